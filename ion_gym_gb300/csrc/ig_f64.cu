@@ -126,42 +126,52 @@ __device__ __forceinline__ Nb neighbours(uint32_t i, uint32_t j, uint32_t k, uin
   return n;
 }
 
-// num and den of the theta-weighted stencil exactly as the reference forms
-// them (solver3d.py:169-191, multigrid3d.py:329-353).
+// The stencil weights of one node exactly as the reference forms them
+// (solver3d.py:169-191, multigrid3d.py:329-353): ghost_linear w[d] =
+// 1/theta_d and their sum; sw the products a neighbour's value is divided
+// by (float32, as the compiled reference types them) and den.
+template <int KIND>
+__device__ __forceinline__ double theta_weights(const float t[6], double w[6]) {
+  if (KIND == kThetaGhost) {
+#pragma unroll
+    for (int d = 0; d < 6; d++) w[d] = __drcp_rn((double)t[d]);
+    return __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(w[0], w[1]), w[2]), w[3]), w[4]),
+                     w[5]);
+  }
+  const float sx = __fadd_rn(t[0], t[1]), sy = __fadd_rn(t[2], t[3]), sz = __fadd_rn(t[4], t[5]);
+  w[0] = (double)__fmul_rn(t[0], sx);
+  w[1] = (double)__fmul_rn(t[1], sx);
+  w[2] = (double)__fmul_rn(t[2], sy);
+  w[3] = (double)__fmul_rn(t[3], sy);
+  w[4] = (double)__fmul_rn(t[4], sz);
+  w[5] = (double)__fmul_rn(t[5], sz);
+  const double px = __drcp_rn((double)__fmul_rn(t[0], t[1]));
+  const double py = __drcp_rn((double)__fmul_rn(t[2], t[3]));
+  const double pz = __drcp_rn((double)__fmul_rn(t[4], t[5]));
+  return __dadd_rn(__dadd_rn(px, py), pz);
+}
+
+// num of the theta-weighted stencil from those weights.
+template <int KIND>
+__device__ __forceinline__ double theta_num(const double v[6], const double w[6]) {
+  double num = KIND == kThetaGhost ? __dmul_rn(v[0], w[0]) : __ddiv_rn(v[0], w[0]);
+#pragma unroll
+  for (int d = 1; d < 6; d++)
+    num = __dadd_rn(num, KIND == kThetaGhost ? __dmul_rn(v[d], w[d]) : __ddiv_rn(v[d], w[d]));
+  return num;
+}
+
 template <int KIND>
 __device__ __forceinline__ void theta_num_den(const double v[6],
                                               const float* __restrict__ th,
                                               size_t N, size_t p, double& num,
                                               double& den) {
-  const float t0 = th[p], t1 = th[N + p], t2 = th[2 * N + p];
-  const float t3 = th[3 * N + p], t4 = th[4 * N + p], t5 = th[5 * N + p];
-  if (KIND == kThetaGhost) {
-    const double w0 = __drcp_rn((double)t0), w1 = __drcp_rn((double)t1);
-    const double w2 = __drcp_rn((double)t2), w3 = __drcp_rn((double)t3);
-    const double w4 = __drcp_rn((double)t4), w5 = __drcp_rn((double)t5);
-    num = __dmul_rn(v[0], w0);
-    num = __dadd_rn(num, __dmul_rn(v[1], w1));
-    num = __dadd_rn(num, __dmul_rn(v[2], w2));
-    num = __dadd_rn(num, __dmul_rn(v[3], w3));
-    num = __dadd_rn(num, __dmul_rn(v[4], w4));
-    num = __dadd_rn(num, __dmul_rn(v[5], w5));
-    den = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(w0, w1), w2), w3), w4), w5);
-  } else {
-    const float sx = __fadd_rn(t0, t1), sy = __fadd_rn(t2, t3), sz = __fadd_rn(t4, t5);
-    const float a0 = __fmul_rn(t0, sx), a1 = __fmul_rn(t1, sx);
-    const float a2 = __fmul_rn(t2, sy), a3 = __fmul_rn(t3, sy);
-    const float a4 = __fmul_rn(t4, sz), a5 = __fmul_rn(t5, sz);
-    num = __ddiv_rn(v[0], (double)a0);
-    num = __dadd_rn(num, __ddiv_rn(v[1], (double)a1));
-    num = __dadd_rn(num, __ddiv_rn(v[2], (double)a2));
-    num = __dadd_rn(num, __ddiv_rn(v[3], (double)a3));
-    num = __dadd_rn(num, __ddiv_rn(v[4], (double)a4));
-    num = __dadd_rn(num, __ddiv_rn(v[5], (double)a5));
-    const double px = __drcp_rn((double)__fmul_rn(t0, t1));
-    const double py = __drcp_rn((double)__fmul_rn(t2, t3));
-    const double pz = __drcp_rn((double)__fmul_rn(t4, t5));
-    den = __dadd_rn(__dadd_rn(px, py), pz);
-  }
+  float t[6];
+  double w[6];
+#pragma unroll
+  for (int d = 0; d < 6; d++) t[d] = th[d * N + p];
+  den = theta_weights<KIND>(t, w);
+  num = theta_num<KIND>(v, w);
 }
 
 __device__ __forceinline__ double sum6(const double v[6]) {
@@ -255,6 +265,202 @@ k_residual(const double* __restrict__ phi, const uint8_t* __restrict__ fixed,
     mb = absbits(r);
   }
   if (absmax) block_max_to(mb, absmax);
+}
+
+// ---- theta solves by a plan -----------------------------------------------
+//
+// The general theta kernels spend 6 reciprocals (ghost_linear) or 6
+// divisions and 3 reciprocals (sw) on every node, although only nodes beside
+// a surface have a leg shorter than 1 (0.4 % of a 57 x 71 x 90 deck).  The
+// FP64 pipe bounds them (2 lanes per clock and SM): 43 us a half-sweep on
+// that deck, either stencil.  A solve therefore sorts its nodes once:
+// nodes with six unit legs take the plain update, whose result is the
+// general one's -- ghost_linear: every weight is 1 and den 6; sw: every
+// product is 2 and den 3, and halving commutes with rounding unless
+// something is subnormal or overflows, where plain_sw_num takes the
+// divisions as written -- and the cut nodes are listed by colour with their
+// weights.  One launch does both: the first blocks the list, the rest the
+// grid; nodes of one colour do not read each other.
+
+// num / den of a node with six unit legs under sw, as the general kernel
+// evaluates it.
+__device__ __noinline__ double plain_sw_num(const double v[6]) {
+  double num = __ddiv_rn(v[0], 2.0);
+  for (int d = 1; d < 6; d++) num = __dadd_rn(num, __ddiv_rn(v[d], 2.0));
+  return num;
+}
+
+// Whether sum6's S of the values v may be halved after the fact: |S| >=
+// 2^-900 and finite (values small enough for v / 2 to round are below
+// 2^-1021 and vanish in such a sum, halved or not), or every value is zero.
+__device__ __forceinline__ bool sw_halves(double S, const double v[6]) {
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(S));
+  const unsigned eb = static_cast<unsigned>(b >> 52) & 0x7ffu;
+  if (eb - 123u <= 2040u - 123u) return true;
+  unsigned long long any = 0;
+#pragma unroll
+  for (int d = 0; d < 6; d++) any |= static_cast<unsigned long long>(__double_as_longlong(v[d]));
+  return (any << 1) == 0ULL;
+}
+
+__global__ void __launch_bounds__(kThreads)
+k_theta_class(const uint8_t* __restrict__ fixed, const float* __restrict__ th, FlatGeom g,
+              uint8_t* __restrict__ cls, uint32_t* counts) {
+  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  int cut = -1;  // the colour of a cut node
+  if (t < g.total) {
+    uint8_t c = 1;
+    if (!fixed[t]) {
+      bool unit = true;
+#pragma unroll
+      for (int d = 0; d < 6; d++) unit = unit && th[(size_t)d * g.total + t] == 1.0f;
+      c = unit ? 0 : 2;
+    }
+    cls[t] = c;
+    if (c == 2) {
+      const uint32_t ij = fdiv(t, g.div_nz);
+      const uint32_t i = fdiv(ij, g.div_ny);
+      cut = (int)((i + (ij - i * g.div_ny.d) + (t - ij * g.div_nz.d)) & 1u);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const int n = __syncthreads_count(cut == c);
+    if (threadIdx.x == 0 && n) atomicAdd(counts + c, (uint32_t)n);
+  }
+}
+
+// The list position of a cut node comes from an atomic counter: the order of
+// a colour's nodes in the list changes no result.
+template <int KIND>
+__global__ void __launch_bounds__(kThreads)
+k_theta_fill(const uint8_t* __restrict__ cls, const float* __restrict__ th, FlatGeom g,
+             uint32_t n0, uint32_t total, uint32_t* cursor, uint32_t* __restrict__ idx,
+             double* __restrict__ w) {
+  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  if (t >= g.total || cls[t] != 2) return;
+  const uint32_t ij = fdiv(t, g.div_nz);
+  const uint32_t i = fdiv(ij, g.div_ny);
+  const uint32_t c = (i + (ij - i * g.div_ny.d) + (t - ij * g.div_nz.d)) & 1u;
+  const uint32_t e = (c ? n0 : 0u) + atomicAdd(cursor + c, 1u);
+  float tv[6];
+  double wv[6];
+#pragma unroll
+  for (int d = 0; d < 6; d++) tv[d] = th[(size_t)d * g.total + t];
+  const double den = theta_weights<KIND>(tv, wv);
+  idx[e] = t;
+#pragma unroll
+  for (int d = 0; d < 6; d++) w[(size_t)d * total + e] = wv[d];
+  w[(size_t)6 * total + e] = den;
+}
+
+// Node e of the cut list: its index, neighbour values and weights.
+template <int KIND>
+__device__ __forceinline__ uint32_t cut_node(const double* __restrict__ phi,
+                                             const ThetaPlan& P, uint32_t e, const FastDiv& dnz,
+                                             const FastDiv& dny, uint32_t nx, double& num,
+                                             double& den) {
+  const uint32_t p = P.idx[e], total = P.total();
+  const uint32_t ij = fdiv(p, dnz);
+  const uint32_t i = fdiv(ij, dny);
+  const Nb n = neighbours(i, ij - i * dny.d, p - ij * dnz.d, nx, dny.d, dnz.d);
+  double v[6], w[6];
+  load6(phi, n, v);
+#pragma unroll
+  for (int d = 0; d < 6; d++) w[d] = P.w[(size_t)d * total + e];
+  den = P.w[(size_t)6 * total + e];
+  num = theta_num<KIND>(v, w);
+  return p;
+}
+
+// One colour of the theta sweep (k_sweep<KIND>'s bits).  Whole solves, the
+// general kernels against the plan (GB300): solve3d, sw, 57 x 71 x 90 with
+// 0.4 % cut nodes 22.6 -> 7.6 ms; the basis door, ghost_linear, four bases of
+// a 65 x 65 x 129 ring deck 71.5 -> 49.3 ms.
+template <int KIND, bool CTL, bool DELTA>
+__global__ void __launch_bounds__(kThreads)
+k_sweep_plan(double* __restrict__ phi, const ThetaPlan P, SweepGeom g, FastDiv dnz,
+             uint32_t list_blocks, double omega, int colour, unsigned long long* dslot,
+             PairCtl* ctl, int lp) {
+  if (CTL) {
+    if (pair_skip(ctl, colour, lp)) return;
+    dslot = &ctl->slot[2 * lp + colour];
+  }
+  unsigned long long mb = 0;
+  uint32_t p = 0xffffffffu;
+  double q = 0.0;
+  if (blockIdx.x < list_blocks) {
+    const uint32_t e = blockIdx.x * kThreads + threadIdx.x;
+    if (e < P.count[colour]) {
+      double num, den;
+      p = cut_node<KIND>(phi, P, (colour ? P.count[0] : 0u) + e, dnz, g.div_ny,
+                         (uint32_t)g.nx, num, den);
+      q = __ddiv_rn(num, den);
+    }
+  } else {
+    const uint32_t t = (blockIdx.x - list_blocks) * kThreads + threadIdx.x;
+    if (t < g.total) {
+      const uint32_t ij = fdiv(t, g.div_kk);
+      const uint32_t kk = t - ij * g.div_kk.d;
+      const uint32_t i = fdiv(ij, g.div_ny);
+      const uint32_t j = ij - i * g.div_ny.d;
+      const uint32_t k = 2 * kk + ((i + j + colour) & 1);
+      const uint32_t o = (i * (uint32_t)g.ny + j) * (uint32_t)g.nz + k;
+      if (k < (uint32_t)g.nz && P.cls[o] == 0) {
+        const Nb n = neighbours(i, j, k, g.nx, g.ny, g.nz);
+        double v[6];
+        load6(phi, n, v);
+        const double S = sum6(v);
+        p = o;
+        if (KIND == kThetaSW && !sw_halves(S, v))
+          q = __ddiv_rn(plain_sw_num(v), 3.0);
+        else
+          q = div6(S);
+      }
+    }
+  }
+  if (p != 0xffffffffu) {
+    const double old = phi[p];
+    const double nw = __dadd_rn(old, omega_step(old, q, omega));
+    if (DELTA) mb = absbits(__dsub_rn(nw, old));
+    phi[p] = nw;
+  }
+  if (DELTA) block_max_to(mb, dslot);
+}
+
+// The fine residual num - den phi (k_residual<KIND>'s bits).
+template <int KIND>
+__global__ void __launch_bounds__(kThreads)
+k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
+                uint32_t list_blocks, double* __restrict__ out) {
+  if (blockIdx.x < list_blocks) {
+    const uint32_t e = blockIdx.x * kThreads + threadIdx.x;
+    if (e >= P.total()) return;
+    double num, den;
+    const uint32_t p = cut_node<KIND>(phi, P, e, g.div_nz, g.div_ny, (uint32_t)g.nx, num, den);
+    out[p] = __dsub_rn(num, __dmul_rn(den, phi[p]));
+    return;
+  }
+  const uint32_t t = (blockIdx.x - list_blocks) * kThreads + threadIdx.x;
+  if (t >= g.total) return;
+  const uint8_t c = P.cls[t];
+  if (c == 2) return;  // the list's
+  double r = 0.0;
+  if (c == 0) {
+    const uint32_t ij = fdiv(t, g.div_nz);
+    const uint32_t i = fdiv(ij, g.div_ny);
+    const Nb n = neighbours(i, ij - i * g.div_ny.d, t - ij * g.div_nz.d, g.nx, g.ny, g.nz);
+    double v[6];
+    load6(phi, n, v);
+    const double S = sum6(v);
+    if (KIND == kThetaGhost)
+      r = __dsub_rn(S, __dmul_rn(6.0, phi[t]));
+    else if (sw_halves(S, v))
+      r = __dsub_rn(__dmul_rn(S, 0.5), __dmul_rn(3.0, phi[t]));
+    else
+      r = __dsub_rn(plain_sw_num(v), __dmul_rn(3.0, phi[t]));
+  }
+  out[t] = r;
 }
 
 // multigrid3d._sweep_rhs (multigrid3d.py:357-391).
@@ -746,6 +952,60 @@ void launch_residual(cudaStream_t s, const double* phi, const uint8_t* fixed,
     k_residual<kThetaGhost><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
   else
     k_residual<kThetaSW><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
+}
+
+void launch_theta_class(cudaStream_t s, const uint8_t* fixed, const float* th, Dims d,
+                        uint8_t* cls, uint32_t* counts) {
+  const FlatGeom g = flat_geom(d);
+  cudaMemsetAsync(counts, 0, 2 * sizeof(uint32_t), s);
+  k_theta_class<<<blocks_for(g.total), kThreads, 0, s>>>(fixed, th, g, cls, counts);
+  counted();
+}
+
+void launch_theta_fill(cudaStream_t s, const uint8_t* cls, const float* th, int kind, Dims d,
+                       const uint32_t count[2], uint32_t* cursor, uint32_t* idx, double* w) {
+  const FlatGeom g = flat_geom(d);
+  const unsigned nb = blocks_for(g.total);
+  const uint32_t total = count[0] + count[1];
+  cudaMemsetAsync(cursor, 0, 2 * sizeof(uint32_t), s);
+  if (total == 0) return;
+  if (kind == kThetaGhost)
+    k_theta_fill<kThetaGhost><<<nb, kThreads, 0, s>>>(cls, th, g, count[0], total, cursor, idx, w);
+  else
+    k_theta_fill<kThetaSW><<<nb, kThreads, 0, s>>>(cls, th, g, count[0], total, cursor, idx, w);
+  counted();
+}
+
+void launch_sweep_plan(cudaStream_t s, double* phi, const ThetaPlan& plan, int kind, Dims d,
+                       double omega, int colour, unsigned long long* dslot, PairCtl* ctl,
+                       int lp) {
+  const SweepGeom g = sweep_geom(d);
+  const FastDiv dnz((uint32_t)d.nz);
+  const uint32_t lb = blocks_for(plan.count[colour]);
+  const unsigned nb = lb + blocks_for(g.total);
+  counted();
+#define IG_SWEEP(K)                                                                          \
+  if (ctl) k_sweep_plan<K, true, true><<<nb, kThreads, 0, s>>>(phi, plan, g, dnz, lb, omega, \
+                                                               colour, dslot, ctl, lp);      \
+  else if (dslot) k_sweep_plan<K, false, true><<<nb, kThreads, 0, s>>>(                      \
+      phi, plan, g, dnz, lb, omega, colour, dslot, ctl, lp);                                 \
+  else k_sweep_plan<K, false, false><<<nb, kThreads, 0, s>>>(phi, plan, g, dnz, lb, omega,   \
+                                                             colour, dslot, ctl, lp);
+  if (kind == kThetaGhost) { IG_SWEEP(kThetaGhost) }
+  else { IG_SWEEP(kThetaSW) }
+#undef IG_SWEEP
+}
+
+void launch_residual_plan(cudaStream_t s, const double* phi, const ThetaPlan& plan, int kind,
+                          Dims d, double* out) {
+  const FlatGeom g = flat_geom(d);
+  const uint32_t lb = blocks_for(plan.total());
+  const unsigned nb = lb + blocks_for(g.total);
+  counted();
+  if (kind == kThetaGhost)
+    k_residual_plan<kThetaGhost><<<nb, kThreads, 0, s>>>(phi, plan, g, lb, out);
+  else
+    k_residual_plan<kThetaSW><<<nb, kThreads, 0, s>>>(phi, plan, g, lb, out);
 }
 
 void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,

@@ -59,7 +59,35 @@ enum StencilKind : int {
                      // its sweeps equal kPlain's
 };
 
+// The theta of a solve sorted by what its nodes need (ig_f64.cu,
+// k_theta_class / k_theta_fill): cls per node (0 free with six unit legs,
+// 1 fixed, 2 free with a cut leg) and the cut nodes of each colour with
+// their stencil weights -- ghost_linear: the six 1/theta and their sum; sw:
+// the six leg products v is divided by, and den -- as `total`-long arrays,
+// w[q * total + e].  Device memory, built once per solve.
+struct ThetaPlan {
+  const uint8_t* cls = nullptr;
+  const uint32_t* idx = nullptr;  // colour 0's cut nodes, then colour 1's
+  const double* w = nullptr;      // 7 * total
+  uint32_t count[2] = {0, 0};
+  __host__ __device__ uint32_t total() const { return count[0] + count[1]; }
+};
+constexpr int kThetaWeights = 7;
+
 // ---- exact FP64 kernels (ig_f64.cu) ----
+// cls, and the cut nodes of each colour counted into counts[2] (zeroed here)
+void launch_theta_class(cudaStream_t s, const uint8_t* fixed, const float* th, Dims d,
+                        uint8_t* cls, uint32_t* counts);
+// idx and w of the plan; cursor[2] is scratch (zeroed here)
+void launch_theta_fill(cudaStream_t s, const uint8_t* cls, const float* th, int kind, Dims d,
+                       const uint32_t count[2], uint32_t* cursor, uint32_t* idx, double* w);
+// launch_sweep / launch_residual of a solve whose theta is in a plan (kind
+// kThetaGhost or kThetaSW): the same bits.
+void launch_sweep_plan(cudaStream_t s, double* phi, const ThetaPlan& plan, int kind, Dims d,
+                       double omega, int colour, unsigned long long* dslot, PairCtl* ctl,
+                       int lp);
+void launch_residual_plan(cudaStream_t s, const double* phi, const ThetaPlan& plan, int kind,
+                          Dims d, double* out);
 // One colour of the reference SOR sweep.  dslot: where the max |update| goes
 // when ctl == nullptr; with ctl the slot is ctl->slot[2*lp + colour].
 void launch_sweep(cudaStream_t s, double* phi, const uint8_t* fixed,

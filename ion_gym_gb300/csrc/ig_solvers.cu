@@ -130,8 +130,8 @@ int stencil_check(int stencil) {
 
 // Sweep kernel kind for a fine grid: theta None reduces both stencils to
 // sum/6 (Shortley-Weller with unit legs halves num and den alike).
-int sweep_kind(const float* th, int stencil) {
-  if (!th) return kPlain;
+int sweep_kind(bool theta, int stencil) {
+  if (!theta) return kPlain;
   return stencil == 0 ? kThetaGhost : kThetaSW;
 }
 
@@ -243,14 +243,59 @@ double device_absmax(ThreadCtx& c, const double* a, const double* b, size_t n,
 }
 
 // ---------------------------------------------------------------- SOR
+// A solve's theta in plan form (empty: no theta, or the general kernels).
+struct Theta {
+  DBuf<uint8_t> cls;
+  DBuf<uint32_t> idx;
+  DBuf<double> w;
+  ThetaPlan plan;
+  bool on() const { return plan.cls != nullptr; }
+};
+
 struct FineGrid {
   Dims d;
   DBuf<uint8_t> fixed;
   DBuf<double> phi;
-  DBuf<float> th;  // empty when theta is None
+  DBuf<float> th;  // empty when theta is None, or once the plan holds it
   int stencil = 0;
-  const float* thp() const { return th.p; }
+  bool theta = false;
+  Theta plan;
 };
+
+// The theta of one solve as a plan, where that pays: few cut nodes (at most
+// a tenth of the grid; every geometry's surface nodes are far fewer), so
+// that the lists (60 bytes a cut node) and cls stay below the theta array
+// they replace and no solve needs more memory than with that array.
+// theta arrays with more cut nodes keep the general kernels.  `th` is freed
+// when the plan took it over.
+void plan_theta(ThreadCtx& c, Theta& t, DBuf<float>& th, const uint8_t* fixed, Dims d,
+                int stencil) {
+  if (!th.p) return;
+  const size_t n = d.n();
+  t.cls.alloc(n, c.s);
+  DBuf<uint32_t> cnt(2, c.s);
+  launch_theta_class(c.s, fixed, th.p, d, t.cls.p, cnt.p);
+  CK(cudaGetLastError());
+  uint32_t count[2] = {0, 0};
+  CK(cudaMemcpyAsync(count, cnt.p, sizeof(count), cudaMemcpyDeviceToHost, c.s));
+  CK(cudaStreamSynchronize(c.s));
+  const size_t total = (size_t)count[0] + count[1];
+  if (total > n / 10) {
+    t.cls.release();
+    return;
+  }
+  t.idx.alloc(total, c.s);
+  t.w.alloc(kThetaWeights * total, c.s);
+  launch_theta_fill(c.s, t.cls.p, th.p, stencil == 0 ? kThetaGhost : kThetaSW, d, count, cnt.p,
+                    t.idx.p, t.w.p);
+  CK(cudaGetLastError());
+  t.plan.cls = t.cls.p;
+  t.plan.idx = t.idx.p;
+  t.plan.w = t.w.p;
+  t.plan.count[0] = count[0];
+  t.plan.count[1] = count[1];
+  th.release();
+}
 
 // phi = phi0 (or 0); phi[fixed] = val[fixed]  (solver3d.py:263-265)
 void init_phi(ThreadCtx& c, FineGrid& g, const double* val_h,
@@ -265,14 +310,23 @@ void init_phi(ThreadCtx& c, FineGrid& g, const double* val_h,
   launch_set_fixed(c.s, g.phi.p, g.fixed.p, val_d.p, n);
 }
 
+// One colour of a fine grid's sweep by the plan or the general kernels.
+void fine_sweep(cudaStream_t s, double* phi, const uint8_t* fx, const float* th, const Theta& t,
+                int kind, Dims d, double omega, int colour, PairCtl* ctl, int lp) {
+  if (t.on())
+    launch_sweep_plan(s, phi, t.plan, kind, d, omega, colour, nullptr, ctl, lp);
+  else
+    launch_sweep(s, phi, fx, th, kind, d, omega, colour, nullptr, ctl, lp);
+}
+
 PairsResult sor_loop(ThreadCtx& c, double* phi, const uint8_t* fx,
-                     const float* th, int stencil, Dims d, double omega,
+                     const float* th, const Theta& t, int stencil, Dims d, double omega,
                      double tol, long max_pairs, PairCtl* ctl_d) {
-  const int kind = sweep_kind(th, stencil);
+  const int kind = sweep_kind(th || t.on(), stencil);
   cudaStream_t s = c.s;
   return run_pairs(c, ctl_d, tol, max_pairs, d.n(), [&](int lp, PairCtl* ctl) {
-    launch_sweep(s, phi, fx, th, kind, d, omega, 0, nullptr, ctl, lp);
-    launch_sweep(s, phi, fx, th, kind, d, omega, 1, nullptr, ctl, lp);
+    for (int colour = 0; colour < 2; colour++)
+      fine_sweep(s, phi, fx, th, t, kind, d, omega, colour, ctl, lp);
   });
 }
 
@@ -418,8 +472,8 @@ VmgOut vmg_loop(ThreadCtx& c, FineGrid& g, VCycle& v, double tol,
                 int max_cycles, int accept_stagnation,
                 const std::vector<int>& sym) {
   const size_t n = g.d.n();
-  const int kind = sweep_kind(g.thp(), g.stencil);
-  const int rkind = g.thp() ? kind : (g.stencil == 0 ? kPlain : kPlainSWResid);
+  const int kind = sweep_kind(g.theta, g.stencil);
+  const int rkind = g.theta ? kind : (g.stencil == 0 ? kPlain : kPlainSWResid);
   DBuf<double> r(n, c.s), phi_c0(n, c.s);
   ErrLevel& e0 = v.lv[0];
   long sweeps = 0;
@@ -429,8 +483,8 @@ VmgOut vmg_loop(ThreadCtx& c, FineGrid& g, VCycle& v, double tol,
     if (g_stop.load()) return {IG_INTERRUPTED, sweeps, prev, cyc, prev};
     CK(cudaMemcpyAsync(phi_c0.p, g.phi.p, n * 8, cudaMemcpyDeviceToDevice, c.s));
     for (int q = 0; q < v.nu1; q++) {
-      launch_sweep(c.s, g.phi.p, g.fixed.p, g.thp(), kind, g.d, 1.0, 0, nullptr, nullptr, 0);
-      launch_sweep(c.s, g.phi.p, g.fixed.p, g.thp(), kind, g.d, 1.0, 1, nullptr, nullptr, 0);
+      for (int colour = 0; colour < 2; colour++)
+        fine_sweep(c.s, g.phi.p, g.fixed.p, g.th.p, g.plan, kind, g.d, 1.0, colour, nullptr, 0);
       sweeps++;
     }
     CK(cudaGetLastError());
@@ -438,14 +492,17 @@ VmgOut vmg_loop(ThreadCtx& c, FineGrid& g, VCycle& v, double tol,
       CK(cudaStreamSynchronize(c.s));
       return {IG_INTERRUPTED, sweeps, prev, cyc, prev};
     }
-    launch_residual(c.s, g.phi.p, g.fixed.p, g.thp(), rkind, g.d, r.p, nullptr);
+    if (g.plan.on())
+      launch_residual_plan(c.s, g.phi.p, g.plan.plan, rkind, g.d, r.p);
+    else
+      launch_residual(c.s, g.phi.p, g.fixed.p, g.th.p, rkind, g.d, r.p, nullptr);
     launch_restrict(c.s, r.p, g.d, e0.f.p, e0.d, 1);
     CK(cudaGetLastError());
     solve_err(c, v, 0);
     launch_prolong_add(c.s, e0.e.p, e0.d, g.phi.p, g.fixed.p, g.d);
     for (int q = 0; q < v.nu2; q++) {
-      launch_sweep(c.s, g.phi.p, g.fixed.p, g.thp(), kind, g.d, 1.0, 0, nullptr, nullptr, 0);
-      launch_sweep(c.s, g.phi.p, g.fixed.p, g.thp(), kind, g.d, 1.0, 1, nullptr, nullptr, 0);
+      for (int colour = 0; colour < 2; colour++)
+        fine_sweep(c.s, g.phi.p, g.fixed.p, g.th.p, g.plan, kind, g.d, 1.0, colour, nullptr, 0);
       sweeps++;
     }
     for (int a : sym) launch_sym_project(c.s, g.phi.p, g.d, a);
@@ -483,8 +540,10 @@ void load_fine(ThreadCtx& c, FineGrid& g, const uint8_t* fixed,
   CK(cudaMemcpyAsync(g.fixed.p, fixed, n, cudaMemcpyDefault, c.s));
   g.phi.alloc(n, c.s);
   if (theta) {
+    g.theta = true;
     g.th.alloc(6 * n, c.s);
     CK(cudaMemcpyAsync(g.th.p, theta, 6 * n * 4, cudaMemcpyDefault, c.s));
+    plan_theta(c, g.plan, g.th, g.fixed.p, g.d, g.stencil);
   }
 }
 
@@ -592,7 +651,7 @@ int ig_solve3d(const uint8_t* fixed, const double* val, const float* theta,
     DBuf<double> val_d;
     init_phi(c, g, val, phi0, val_d);
     DBuf<PairCtl> ctl(1, c.s);
-    const PairsResult r = sor_loop(c, g.phi.p, g.fixed.p, g.thp(), g.stencil, g.d,
+    const PairsResult r = sor_loop(c, g.phi.p, g.fixed.p, g.th.p, g.plan, g.stencil, g.d,
                                     omega, tol, max_sweeps, ctl.p);
     copy_out(c, g.phi.p, phi_out, g.d.n());
     if (sweeps_out) *sweeps_out = r.pairs;
@@ -641,9 +700,12 @@ int ig_solve3d_mg(const uint8_t* fixed, const double* val, const float* theta,
     };
     DBuf<PairCtl> ctl(1, c.s);
     DBuf<float> th_d;
+    Theta plan;
+    const Theta none;
     if (theta) {
       th_d.alloc(6 * d0.n(), c.s);
       CK(cudaMemcpyAsync(th_d.p, theta, 6 * d0.n() * 4, cudaMemcpyDefault, c.s));
+      plan_theta(c, plan, th_d, lv[0].fixed.p, d0, stencil);
     }
     // coarsest level: cold solve with theta None (multigrid3d.py:200-204);
     // then each finer level from the prolongated guess (multigrid3d.py:206-226)
@@ -661,14 +723,15 @@ int ig_solve3d_mg(const uint8_t* fixed, const double* val, const float* theta,
       // the coarsest solve always uses the plain stencil; with a one-level
       // hierarchy the reference then solves the fine grid again from zero
       // with theta (multigrid3d.py:201-203, 220-226)
-      const float* th = (L == 0 && nl > 1) ? th_d.p : nullptr;
+      const bool with_theta = L == 0 && nl > 1;
       const double ltol = (L == 0 || L == nl - 1) ? tol : tol * level_tol_factor;
-      PairsResult r = sor_loop(c, phi.p, M.fixed.p, th, stencil, M.d,
-                               omega_of(L), ltol, max_sweeps, ctl.p);
-      if (nl == 1 && r.converged && th_d.p) {
+      PairsResult r = sor_loop(c, phi.p, M.fixed.p, with_theta ? th_d.p : nullptr,
+                               with_theta ? plan : none, stencil, M.d, omega_of(L), ltol,
+                               max_sweeps, ctl.p);
+      if (nl == 1 && r.converged && theta) {
         CK(cudaMemsetAsync(phi.p, 0, n * 8, c.s));
         launch_set_fixed(c.s, phi.p, M.fixed.p, M.val.p, n);
-        r = sor_loop(c, phi.p, M.fixed.p, th_d.p, stencil, M.d, omega_of(0),
+        r = sor_loop(c, phi.p, M.fixed.p, th_d.p, plan, stencil, M.d, omega_of(0),
                      tol, max_sweeps, ctl.p);
       }
       if (!r.converged || L == 0) {
@@ -857,7 +920,7 @@ int ig_sweep_dev(double* phi, const uint8_t* fixed, const float* theta,
     cudaStream_t s = as_stream(stream);
     unsigned long long* slot = kscratch();
     CK(cudaMemsetAsync(slot, 0, 8, s));
-    launch_sweep(s, phi, fixed, theta, sweep_kind(theta, stencil), Dims{nx, ny, nz},
+    launch_sweep(s, phi, fixed, theta, sweep_kind(theta != nullptr, stencil), Dims{nx, ny, nz},
                  omega, colour & 1, slot, nullptr, 0);
     const double d = finish_max(s, slot);
     if (dmax_out) *dmax_out = d;
@@ -871,7 +934,7 @@ int ig_residual_dev(const double* phi, const uint8_t* fixed, const float* theta,
   return guard([&] {
     check_dims(nx, ny, nz);
     stencil_check(stencil);
-    const int kind = theta ? sweep_kind(theta, stencil) : (stencil == 0 ? kPlain : kPlainSWResid);
+    const int kind = theta ? sweep_kind(theta != nullptr, stencil) : (stencil == 0 ? kPlain : kPlainSWResid);
     launch_residual(as_stream(stream), phi, fixed, theta, kind, Dims{nx, ny, nz}, out, nullptr);
     CK(cudaGetLastError());
     return (int)IG_OK;
