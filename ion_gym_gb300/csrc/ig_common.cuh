@@ -53,65 +53,6 @@ __device__ __forceinline__ double div6(double x) {
   return __longlong_as_double(static_cast<long long>((b & 0x8000000000000000ULL) | mag));
 }
 
-// RN(omega * RN(q - old)), the SOR step of every sweep, on the integer pipe
-// where that is exact.  With q = Mq*2^(eq-1075) and old = Mo*2^(eo-1075)
-// (53-bit integer significands, biased exponents no more than one apart) the
-// difference is the exact integer D = +-Mq*2^(eq-e) -+ Mo*2^(eo-e), e the
-// smaller exponent; when |D| < 2^53 it is RN(q - old) itself.  The product
-// W*|D| (W omega's significand) is exact in 128 bits and is rounded once to
-// 53 bits, to nearest, ties to even -- RN(omega * d).  Lanes outside that
-// window (zeros, subnormals, exponents more than one apart, a difference
-// that would round, a subnormal or overflowing product, omega not a
-// positive normal number) take the two FP64 operations.  q == old gives +0,
-// as q - old does.  Checked bit-for-bit against the FP64 expression by the
-// test-suite.
-__device__ __forceinline__ double omega_step(double old, double q, double omega) {
-  constexpr unsigned long long kFrac = 0x000fffffffffffffULL, kHid = 0x0010000000000000ULL;
-  const unsigned long long bq = static_cast<unsigned long long>(__double_as_longlong(q));
-  const unsigned long long bo = static_cast<unsigned long long>(__double_as_longlong(old));
-  const unsigned long long bw = static_cast<unsigned long long>(__double_as_longlong(omega));
-  const unsigned eq = static_cast<unsigned>(bq >> 52) & 0x7ffu;
-  const unsigned eo = static_cast<unsigned>(bo >> 52) & 0x7ffu;
-  const unsigned ew = static_cast<unsigned>(bw >> 52);  // sign bit included
-  const unsigned emin = min(eq, eo);
-  bool ok = eq - 1u < 2046u && eo - 1u < 2046u && max(eq, eo) - emin <= 1u &&
-            ew - 1u < 2046u;
-  unsigned long long out = 0;
-  if (ok) {
-    long long a = static_cast<long long>(((bq & kFrac) | kHid) << (eq - emin));
-    long long b = static_cast<long long>(((bo & kFrac) | kHid) << (eo - emin));
-    if (static_cast<long long>(bq) < 0) a = -a;
-    if (static_cast<long long>(bo) < 0) b = -b;
-    const long long dd = a - b;
-    if (dd == 0) return 0.0;
-    const unsigned long long ad = static_cast<unsigned long long>(dd < 0 ? -dd : dd);
-    ok = (ad >> 53) == 0ULL;
-    if (ok) {
-      const unsigned long long w = (bw & kFrac) | kHid;
-      const unsigned long long lo = w * ad, hi = __umul64hi(w, ad);
-      int sh = (hi ? 128 - __clzll(static_cast<long long>(hi))
-                   : 64 - __clzll(static_cast<long long>(lo))) - 53;  // 0..53
-      unsigned long long m = lo;
-      if (sh > 0) {
-        m = (lo >> sh) | (hi << (64 - sh));
-        const unsigned long long rem = lo & ((1ULL << sh) - 1ULL), half = 1ULL << (sh - 1);
-        m += (rem > half || (rem == half && (m & 1ULL))) ? 1ULL : 0ULL;
-        if (m >> 53) {
-          m >>= 1;
-          sh++;
-        }
-      }
-      const int eu = sh + static_cast<int>(ew) + static_cast<int>(emin) - 1075;
-      ok = eu >= 1 && eu <= 2046;
-      // m carries the implicit bit: (eu - 1) << 52 plus m has exponent eu
-      out = (dd < 0 ? 0x8000000000000000ULL : 0ULL) |
-            ((static_cast<unsigned long long>(eu - 1) << 52) + m);
-    }
-  }
-  if (!ok) return __dmul_rn(omega, __dsub_rn(q, old));
-  return __longlong_as_double(static_cast<long long>(out));
-}
-
 // |d| as an order-preserving 64-bit key (d >= 0, so the IEEE bit pattern
 // orders like the value).  NaN maps to 0: the reference's "if d > dmax"
 // never takes a NaN.
@@ -119,6 +60,157 @@ __device__ __forceinline__ unsigned long long absbits(double d) {
   unsigned long long b =
       static_cast<unsigned long long>(__double_as_longlong(d)) & 0x7fffffffffffffffULL;
   return b > 0x7ff0000000000000ULL ? 0ULL : b;
+}
+
+// The FP64 operations behind the integer forms below, as calls: written in
+// line, a fallback this short is predicated instead of branched around, and
+// instructions that every lane has switched off still take their turn in
+// the FP64 pipe -- 3 on top of the sum's 5.
+static __device__ __noinline__ double sor_slow(double old, double q, double omega) {
+  return __dadd_rn(old, __dmul_rn(omega, __dsub_rn(q, old)));
+}
+static __device__ __noinline__ double sub_slow(double a, double b) { return __dsub_rn(a, b); }
+static __device__ __noinline__ double resid_slow(double S, double phi) {
+  return __dsub_rn(S, __dmul_rn(6.0, phi));
+}
+
+// One node of a sweep from its quotient q: nw = RN(old + RN(omega * RN(q -
+// old))), the key of |RN(nw - old)| to *key when DELTA, on the integer pipe
+// where that is exact, so that a node costs the FP64 pipe its neighbour sum
+// alone (the pipe does 2 lanes per clock and SM, the integer pipe 64; the
+// sweep is bound by the former).
+//
+//  * difference: q = Mq*2^(eq-1075) and old = Mo*2^(eo-1075) (53-bit integer
+//    significands, biased exponents no more than one apart) differ by the
+//    exact integer D = +-Mq*2^(eq-e) -+ Mo*2^(eo-e), e the smaller exponent;
+//    when |D| < 2^53 it is RN(q - old) itself.
+//  * omega 1 (ONE): then old + D is q, exactly.
+//  * step: omega's significand W times |D| is formed with both normalised,
+//    so its top bit is one of two places, and rounded once to the 53 bits m
+//    (to nearest, ties to even; a set low bit stands for every bit below).
+//  * sum: in units of old's ulp / 512, old is Mo*2^9 and the step m*2^9
+//    shifted right by the exponents' distance, again with a low bit for
+//    what is shifted out (an even half-way point is never mistaken for
+//    it); while the sum keeps old's exponent its rounding to a multiple of
+//    2^9 is RN(old + step), and the integer |rr - Mo| is |nw - old|.
+//    (Leaving the half-way cases to the FP64 operations saves ten integer
+//    instructions and loses: omega 1.85 is 37/20, whose products are halves
+//    once in twenty lanes, so most warps would run both paths: 68 against 52
+//    us a half-sweep of a 257^3 quadrupole.)
+//
+// Zero on zero stays +0 (cold starts are mostly zeros).  Everything else
+// (other zeros, subnormals, exponents further apart, a rounded difference, a
+// subnormal step, a sum that leaves old's binade, omega not a positive
+// normal number) takes the FP64 operations as the reference writes them.
+// Checked bit-for-bit against those by the test-suite.
+//
+// The 257^3 quadrupole's cascadic solve (omega 1.85): 278 ms with the
+// difference and the product alone on the integer pipe (6 FP64 instructions
+// a node), 250 ms now (5, the neighbour sum); both pipes are then about
+// equally busy (320 FP64 and some 340 integer issue cycles a node and
+// scheduler), so moving more of the sum over would not help.
+__device__ __forceinline__ unsigned long long sor_key(unsigned long long ad, int e) {
+  // the IEEE bits of ad * 2^(e - 1075), 0 < ad < 2^54, where that is normal;
+  // ~0 where it is not
+  const int lz = __clzll(static_cast<long long>(ad)) - 11;
+  const unsigned long long m = lz >= 0 ? ad << lz : ad >> 1;  // lz = -1: ad is even
+  return e - lz >= 1 ? (static_cast<unsigned long long>(e - lz - 1) << 52) + m : ~0ULL;
+}
+
+template <bool DELTA, bool ONE>
+__device__ __forceinline__ double sor_apply(double old, double q, double omega,
+                                            unsigned long long* key) {
+  constexpr unsigned long long kFrac = 0x000fffffffffffffULL, kHid = 0x0010000000000000ULL;
+  const unsigned long long bq = static_cast<unsigned long long>(__double_as_longlong(q));
+  const unsigned long long bo = static_cast<unsigned long long>(__double_as_longlong(old));
+  const unsigned long long bw = static_cast<unsigned long long>(__double_as_longlong(omega));
+  const int eq = static_cast<int>(bq >> 52) & 0x7ff, eo = static_cast<int>(bo >> 52) & 0x7ff;
+  const int ew = static_cast<int>(bw >> 52);  // sign bit included
+  const int emin = min(eq, eo), de = eq - eo;
+  const bool wok = ONE || static_cast<unsigned>(ew - 1) < 2046u;
+  const unsigned long long mo = (bo & kFrac) | kHid, mq = (bq & kFrac) | kHid;
+  const unsigned long long a = de > 0 ? mq << 1 : mq, b = de < 0 ? mo << 1 : mo;
+  const bool opp = static_cast<long long>(bq ^ bo) < 0;
+  const long long dd = static_cast<long long>(opp ? a + b : a - b);
+  const unsigned long long ad = static_cast<unsigned long long>(dd < 0 ? -dd : dd);
+  bool ok = wok && static_cast<unsigned>(eq - 1) < 2046u && static_cast<unsigned>(eo - 1) < 2046u &&
+            static_cast<unsigned>(de + 1) <= 2u && (ad >> 53) == 0ULL;
+  unsigned long long k = 0;
+  double nw;
+  if (ONE) {
+    nw = q;
+    if (DELTA && ad) {
+      k = sor_key(ad, emin);
+      ok = ok && k != ~0ULL;
+    }
+  } else {
+    const int lz = __clzll(static_cast<long long>(ad | 1ULL));
+    const unsigned long long an = ad << lz, wn = ((bw & kFrac) | kHid) << 10;
+    const unsigned long long hi = __umul64hi(wn, an), lo = wn * an;
+    const int s = 9 + static_cast<int>(hi >> 62);
+    const unsigned long long h = hi | (lo ? 1ULL : 0ULL);
+    const unsigned long long m = (h + ((1ULL << (s - 1)) - 1ULL) + ((h >> s) & 1ULL)) >> s;
+    const int eu = emin + ew + s - lz - 1021;  // the step is m * 2^(eu - 1075)
+    const int sh = min(eo - eu, 63);
+    const unsigned long long m9 = m << 9, t0 = m9 >> (sh & 63);
+    const unsigned long long t = t0 | ((t0 << (sh & 63)) != m9 ? 1ULL : 0ULL);
+    const unsigned long long A = mo << 9;
+    // the step has q's sign if |q|'s side of the difference won, and old's
+    // side if not: it adds to |old| when q and old agree and |q| is larger
+    const unsigned long long R = (!opp && dd > 0) ? A + t : A - t;
+    const unsigned long long rr = (R + 255ULL + ((R >> 9) & 1ULL)) >> 9;
+    const unsigned long long out = (bo & 0x8000000000000000ULL) |
+                                   ((static_cast<unsigned long long>(eo - 1) << 52) + rr);
+    nw = ad ? __longlong_as_double(static_cast<long long>(out)) : old;
+    ok = ok && (!ad || (eu >= 1 && sh >= 0 && (R >> 61) == 1ULL));
+    if (DELTA && ad && rr != mo) {
+      k = sor_key(rr > mo ? rr - mo : mo - rr, eo);
+      ok = ok && k != ~0ULL;
+    }
+  }
+  if (!ok) {
+    if (wok && ((bq | bo) << 1) == 0ULL) {
+      nw = 0.0;
+      k = 0;
+    } else {
+      nw = sor_slow(old, q, ONE ? 1.0 : omega);
+      if (DELTA) k = absbits(sub_slow(nw, old));
+    }
+  }
+  if (DELTA) *key = k;
+  return nw;
+}
+
+// RN(S - RN(6 phi)), the residual of a node whose legs are all 1, on the
+// integer pipe where that is exact: 6 phi's significand is 3 Mo rounded by
+// one or two bits, and the difference of two numbers at most one binade
+// apart is an exact integer (see sor_apply).  Zero minus zero, and every
+// case that is not exact, take the FP64 operations.  Checked against them
+// by the test-suite.
+__device__ __forceinline__ double resid6(double S, double phi) {
+  constexpr unsigned long long kFrac = 0x000fffffffffffffULL, kHid = 0x0010000000000000ULL;
+  const unsigned long long bs = static_cast<unsigned long long>(__double_as_longlong(S));
+  const unsigned long long bo = static_cast<unsigned long long>(__double_as_longlong(phi));
+  const int es = static_cast<int>(bs >> 52) & 0x7ff, eo = static_cast<int>(bo >> 52) & 0x7ff;
+  const unsigned long long m3 = 3ULL * ((bo & kFrac) | kHid);  // [3, 6) * 2^52
+  const int sh = 1 + static_cast<int>(m3 >> 54);
+  const unsigned long long mp =
+      (m3 + ((1ULL << (sh - 1)) - 1ULL) + ((m3 >> sh) & 1ULL)) >> sh;  // up to 2^53
+  const int ep = eo + 1 + sh;  // 6 phi = mp * 2^(ep - 1075)
+  const unsigned long long ms = (bs & kFrac) | kHid;
+  const int emin = min(es, ep), de = es - ep;
+  const unsigned long long a = de > 0 ? ms << 1 : ms, b = de < 0 ? mp << 1 : mp;
+  const bool opp = static_cast<long long>(bs ^ bo) < 0;
+  const long long dd = static_cast<long long>(opp ? a + b : a - b);
+  const unsigned long long ad = static_cast<unsigned long long>(dd < 0 ? -dd : dd);
+  const bool ok = static_cast<unsigned>(es - 1) < 2046u && static_cast<unsigned>(eo - 1) < 2040u &&
+                  static_cast<unsigned>(de + 1) <= 2u && (ad >> 53) == 0ULL;
+  const unsigned long long k = ad ? sor_key(ad, emin) : 0ULL;
+  if (ok && k != ~0ULL)  // an exact zero difference is +0
+    return __longlong_as_double(static_cast<long long>(
+        k | (ad ? (bs ^ (dd < 0 ? 0x8000000000000000ULL : 0ULL)) & 0x8000000000000000ULL
+                : 0ULL)));
+  return resid_slow(S, phi);
 }
 
 // Warp max of a 64-bit key with two 32-bit warp reductions (REDUX): the

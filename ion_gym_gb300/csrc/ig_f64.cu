@@ -6,7 +6,8 @@
 // GB300 (about 1/64 of the FP32 rate), so the kernels spend it only where the
 // reference does: masks, indices, maxima and absolute values run on the
 // integer pipe, and the theta == 1 stencil divides by 6 on the integer pipe
-// (ig::div6) instead of a full division.
+// (ig::div6) instead of a full division and the relaxation step runs there
+// too (ig::sor_apply).
 //
 // Layout: C-order (nx, ny, nz), z contiguous; theta (6, nx, ny, nz) float32.
 // Sweeps map one thread to one (i, j, k-pair) cell so a warp reads 64
@@ -37,10 +38,11 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
 struct SweepGeom {
   long nx, ny, nz;
   FastDiv div_kk, div_ny;
-  uint32_t total;  // nx*ny*nkk
+  uint32_t total;  // ceil(nx/U)*ny*nkk threads
 };
 
-inline SweepGeom sweep_geom(Dims d) {
+// U: consecutive x-planes per thread.
+inline SweepGeom sweep_geom(Dims d, int U = 1) {
   SweepGeom g;
   g.nx = d.nx;
   g.ny = d.ny;
@@ -48,8 +50,25 @@ inline SweepGeom sweep_geom(Dims d) {
   const long nkk = (d.nz + 1) / 2;
   g.div_kk = FastDiv((uint32_t)nkk);
   g.div_ny = FastDiv((uint32_t)d.ny);
-  g.total = (uint32_t)(d.nx * d.ny * nkk);
+  g.total = (uint32_t)((d.nx + U - 1) / U * d.ny * nkk);
   return g;
+}
+
+// Planes per sweep thread: 2 where the colour still fills the GPU's threads
+// (152 SMs x 2048) with half as many, else 1 (a small level waits for its
+// loads, and more threads have more of them in flight).  The 257^3
+// quadrupole's cascadic solve with 1 / 2 / 4 planes on its large levels: 249
+// / 243 / 303 ms (four planes leave too few warps).
+inline int sweep_planes(Dims d) {
+  return d.nx * d.ny * ((d.nz + 1) / 2) >= 2L * 152 * 2048 ? 2 : 1;
+}
+
+// Threads per block of the sweeps: the pipe-bound blocks of 256 run in step
+// (all in their loads, then all in their sums); the same solve with 64 / 128
+// / 256 threads: 244 / 243 / 254 ms.
+constexpr int kSweepThreads = 128;
+inline unsigned sweep_blocks(const SweepGeom& g) {
+  return (g.total + kSweepThreads - 1) / kSweepThreads;
 }
 
 struct FlatGeom {
@@ -188,9 +207,51 @@ __device__ __forceinline__ void load6(const double* __restrict__ a, const Nb& n,
   v[5] = a[n.zp];
 }
 
-// solver3d._sweep (solver3d.py:131-198).
-template <int KIND, bool CTL, bool DELTA = true>
-__global__ void __launch_bounds__(kThreads)
+// The nodes of one colour a sweep thread owns: the same y, z slot kk and U
+// consecutive x-planes (the colour's node alternates between k = 2 kk and
+// 2 kk + 1), so that one index split and one pair of y-neighbour offsets
+// serve U nodes.
+template <int U>
+struct SweepNodes {
+  uint32_t i0, j, kk, par, sx;
+  int ym, yp;  // y-neighbours, relative
+  uint32_t nx, nz;
+  __device__ __forceinline__ SweepNodes(const SweepGeom& g, uint32_t t, int colour) {
+    const uint32_t ij = fdiv(t, g.div_kk), ny = (uint32_t)g.ny;
+    nx = (uint32_t)g.nx;
+    nz = (uint32_t)g.nz;
+    kk = t - ij * g.div_kk.d;
+    const uint32_t ib = fdiv(ij, g.div_ny);
+    j = ij - ib * g.div_ny.d;
+    i0 = ib * U;
+    par = (i0 + j + (uint32_t)colour) & 1u;
+    sx = ny * nz;
+    const int ry = ny > 1 ? (int)nz : 0;
+    ym = j > 0 ? -(int)nz : ry;
+    yp = j + 1 < ny ? (int)nz : -ry;
+  }
+  __device__ __forceinline__ uint32_t k(int u) const { return 2 * kk + (par ^ (u & 1)); }
+  __device__ __forceinline__ bool valid(int u) const { return i0 + u < nx && k(u) < nz; }
+  __device__ __forceinline__ uint32_t at(int u) const {
+    return (i0 + u) * sx + j * nz + k(u);
+  }
+  __device__ __forceinline__ Nb nb(int u, uint32_t p) const {
+    const uint32_t i = i0 + u, kz = k(u);
+    const uint32_t rx = nx > 1 ? sx : 0u, rz = nz > 1 ? 1u : 0u;
+    Nb n;
+    n.xm = i > 0 ? p - sx : p + rx;
+    n.xp = i + 1 < nx ? p + sx : p - rx;
+    n.ym = p + ym;
+    n.yp = p + yp;
+    n.zm = kz > 0 ? p - 1 : p + rz;
+    n.zp = kz + 1 < nz ? p + 1 : p - rz;
+    return n;
+  }
+};
+
+// solver3d._sweep (solver3d.py:131-198).  ONE: omega is 1.
+template <int KIND, bool CTL, bool DELTA, bool ONE, int U>
+__global__ void __launch_bounds__(kSweepThreads)
 k_sweep(double* __restrict__ phi, const uint8_t* __restrict__ fixed,
         const float* __restrict__ th, SweepGeom g, double omega, int colour,
         unsigned long long* dslot, PairCtl* ctl, int lp) {
@@ -198,71 +259,94 @@ k_sweep(double* __restrict__ phi, const uint8_t* __restrict__ fixed,
     if (pair_skip(ctl, colour, lp)) return;
     dslot = &ctl->slot[2 * lp + colour];
   }
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
   unsigned long long mb = 0;
   if (t < g.total) {
-    const uint32_t ij = fdiv(t, g.div_kk);
-    const uint32_t kk = t - ij * g.div_kk.d;
-    const uint32_t i = fdiv(ij, g.div_ny);
-    const uint32_t j = ij - i * g.div_ny.d;
-    const uint32_t k = 2 * kk + ((i + j + colour) & 1);
-    if (k < (uint32_t)g.nz) {
-      const uint32_t p = (i * (uint32_t)g.ny + j) * (uint32_t)g.nz + k;
-      if (!fixed[p]) {
-        const Nb n = neighbours(i, j, k, g.nx, g.ny, g.nz);
-        double v[6];
-        load6(phi, n, v);
-        const double old = phi[p];
-        double q;
-        if (KIND == kPlain) {
-          q = div6(sum6(v));
-        } else {
-          double num, den;
-          theta_num_den<KIND>(v, th, (size_t)g.nx * g.ny * g.nz, p, num, den);
-          q = __ddiv_rn(num, den);
-        }
-        const double nw = __dadd_rn(old, omega_step(old, q, omega));
-        if (DELTA) mb = absbits(__dsub_rn(nw, old));
-        phi[p] = nw;
+    const SweepNodes<U> sn(g, t, colour);
+    bool go[U];
+    double q[U], old[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) go[u] = sn.valid(u) && !fixed[sn.at(u)];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!go[u]) continue;
+      const uint32_t p = sn.at(u);
+      double v[6];
+      load6(phi, sn.nb(u, p), v);
+      old[u] = phi[p];
+      if (KIND == kPlain) {
+        q[u] = sum6(v);
+      } else {
+        double num, den;
+        theta_num_den<KIND>(v, th, (size_t)g.nx * g.ny * g.nz, p, num, den);
+        q[u] = __ddiv_rn(num, den);
       }
     }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!go[u]) continue;
+      unsigned long long key = 0;
+      phi[sn.at(u)] = sor_apply<DELTA, ONE>(old[u], KIND == kPlain ? div6(q[u]) : q[u], omega,
+                                            &key);
+      if (DELTA && key > mb) mb = key;
+    }
   }
-  // without a slot (DELTA false) nobody reads the max |update|: skip the
-  // subtraction and the block reduction
+  // without a slot (DELTA false) nobody reads the max |update|: skip it and
+  // the block reduction
   if (DELTA) block_max_to(mb, dslot);
 }
 
 // multigrid3d._residual (multigrid3d.py:305-354): num - den*phi, 0 at fixed.
+// A thread owns the nodes (i0 .. i0 + U - 1, j, k): its x-neighbours are its
+// own column, so U nodes take 5 U + 2 loads and one index split.
+constexpr int kResidPlanes = 4;
 template <int KIND>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSweepThreads)
 k_residual(const double* __restrict__ phi, const uint8_t* __restrict__ fixed,
            const float* __restrict__ th, FlatGeom g, double* __restrict__ out,
            unsigned long long* absmax) {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  constexpr int U = kResidPlanes;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
+  const uint32_t nx = (uint32_t)g.nx, ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
   unsigned long long mb = 0;
-  if (t < g.total) {
-    const uint32_t ij = fdiv(t, g.div_nz);
-    const uint32_t k = t - ij * g.div_nz.d;
-    const uint32_t i = fdiv(ij, g.div_ny);
-    const uint32_t j = ij - i * g.div_ny.d;
-    double r = 0.0;
-    if (!fixed[t]) {
-      const Nb n = neighbours(i, j, k, g.nx, g.ny, g.nz);
-      double v[6];
-      load6(phi, n, v);
-      if (KIND == kPlain) {
-        r = __dsub_rn(sum6(v), __dmul_rn(6.0, phi[t]));
-      } else if (KIND == kPlainSW) {
-        // unit legs: num = sum of v/2 (== sum/2 exactly), den = 3
-        r = __dsub_rn(__dmul_rn(sum6(v), 0.5), __dmul_rn(3.0, phi[t]));
-      } else {
-        double num, den;
-        theta_num_den<KIND>(v, th, g.total, t, num, den);
-        r = __dsub_rn(num, __dmul_rn(den, phi[t]));
-      }
+  const uint32_t ij = fdiv(t, g.div_nz);
+  const uint32_t k = t - ij * g.div_nz.d;
+  const uint32_t ib = fdiv(ij, g.div_ny);
+  const uint32_t j = ij - ib * g.div_ny.d;
+  const uint32_t i0 = ib * U;
+  if (i0 < nx) {
+    const Nb n = neighbours(i0, j, k, nx, ny, nz);
+    const uint32_t sx = ny * nz, p0 = i0 * sx + j * nz + k;
+    double c[U + 2];
+    c[0] = phi[n.xm];
+#pragma unroll
+    for (int u = 0; u <= U; u++) {
+      const uint32_t i = i0 + u;  // past the last plane: the reflected one
+      c[u + 1] = i < nx ? phi[p0 + u * sx] : (i == nx ? phi[nx > 1 ? p0 + (u - 2) * sx : p0] : 0.0);
     }
-    if (out) out[t] = r;
-    mb = absbits(r);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (i0 + u >= nx) break;
+      const uint32_t o = u * sx, p = p0 + o;
+      double r = 0.0;
+      if (!fixed[p]) {
+        const double v[6] = {c[u], c[u + 2], phi[n.ym + o], phi[n.yp + o], phi[n.zm + o],
+                             phi[n.zp + o]};
+        if (KIND == kPlain) {
+          r = resid6(sum6(v), c[u + 1]);
+        } else if (KIND == kPlainSW) {
+          // unit legs: num = sum of v/2 (== sum/2 exactly), den = 3
+          r = __dsub_rn(__dmul_rn(sum6(v), 0.5), __dmul_rn(3.0, c[u + 1]));
+        } else {
+          double num, den;
+          theta_num_den<KIND>(v, th, (size_t)nx * ny * nz, p, num, den);
+          r = __dsub_rn(num, __dmul_rn(den, c[u + 1]));
+        }
+      }
+      if (out) out[p] = r;
+      const unsigned long long key = absbits(r);
+      if (key > mb) mb = key;
+    }
   }
   if (absmax) block_max_to(mb, absmax);
 }
@@ -377,7 +461,7 @@ __device__ __forceinline__ uint32_t cut_node(const double* __restrict__ phi,
 // general kernels against the plan (GB300): solve3d, sw, 57 x 71 x 90 with
 // 0.4 % cut nodes 22.6 -> 7.6 ms; the basis door, ghost_linear, four bases of
 // a 65 x 65 x 129 ring deck 71.5 -> 49.3 ms.
-template <int KIND, bool CTL, bool DELTA>
+template <int KIND, bool CTL, bool DELTA, bool ONE>
 __global__ void __launch_bounds__(kThreads)
 k_sweep_plan(double* __restrict__ phi, const ThetaPlan P, SweepGeom g, FastDiv dnz,
              uint32_t list_blocks, double omega, int colour, unsigned long long* dslot,
@@ -421,9 +505,7 @@ k_sweep_plan(double* __restrict__ phi, const ThetaPlan P, SweepGeom g, FastDiv d
   }
   if (p != 0xffffffffu) {
     const double old = phi[p];
-    const double nw = __dadd_rn(old, omega_step(old, q, omega));
-    if (DELTA) mb = absbits(__dsub_rn(nw, old));
-    phi[p] = nw;
+    phi[p] = sor_apply<DELTA, ONE>(old, q, omega, &mb);
   }
   if (DELTA) block_max_to(mb, dslot);
 }
@@ -454,7 +536,7 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
     load6(phi, n, v);
     const double S = sum6(v);
     if (KIND == kThetaGhost)
-      r = __dsub_rn(S, __dmul_rn(6.0, phi[t]));
+      r = resid6(S, phi[t]);
     else if (sw_halves(S, v))
       r = __dsub_rn(__dmul_rn(S, 0.5), __dmul_rn(3.0, phi[t]));
     else
@@ -463,9 +545,9 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
   out[t] = r;
 }
 
-// multigrid3d._sweep_rhs (multigrid3d.py:357-391).
-template <bool CTL>
-__global__ void __launch_bounds__(kThreads)
+// multigrid3d._sweep_rhs (multigrid3d.py:357-391).  ONE: omega is 1.
+template <bool CTL, bool DELTA, bool ONE, int U>
+__global__ void __launch_bounds__(kSweepThreads)
 k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
             const double* __restrict__ f, SweepGeom g, double omega,
             int colour, unsigned long long* dslot, PairCtl* ctl, int lp) {
@@ -473,31 +555,33 @@ k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
     if (pair_skip(ctl, colour, lp)) return;
     dslot = &ctl->slot[2 * lp + colour];
   }
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
   unsigned long long mb = 0;
   if (t < g.total) {
-    const uint32_t ij = fdiv(t, g.div_kk);
-    const uint32_t kk = t - ij * g.div_kk.d;
-    const uint32_t i = fdiv(ij, g.div_ny);
-    const uint32_t j = ij - i * g.div_ny.d;
-    const uint32_t k = 2 * kk + ((i + j + colour) & 1);
-    if (k < (uint32_t)g.nz) {
-      const uint32_t p = (i * (uint32_t)g.ny + j) * (uint32_t)g.nz + k;
-      if (!fixed[p]) {
-        const Nb n = neighbours(i, j, k, g.nx, g.ny, g.nz);
-        double v[6];
-        load6(e, n, v);
-        const double old = e[p];
-        const double nv = div6(__dsub_rn(sum6(v), f[p]));
-        const double nw = __dadd_rn(old, omega_step(old, nv, omega));
-        mb = absbits(__dsub_rn(nw, old));
-        e[p] = nw;
-      }
+    const SweepNodes<U> sn(g, t, colour);
+    bool go[U];
+    double q[U], old[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) go[u] = sn.valid(u) && !fixed[sn.at(u)];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!go[u]) continue;
+      const uint32_t p = sn.at(u);
+      double v[6];
+      load6(e, sn.nb(u, p), v);
+      old[u] = e[p];
+      q[u] = __dsub_rn(sum6(v), f[p]);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (!go[u]) continue;
+      unsigned long long key = 0;
+      e[sn.at(u)] = sor_apply<DELTA, ONE>(old[u], div6(q[u]), omega, &key);
+      if (DELTA && key > mb) mb = key;
     }
   }
-  block_max_to(mb, dslot);
+  if (DELTA) block_max_to(mb, dslot);
 }
-
 
 // multigrid3d._restrict_fw_njit (multigrid3d.py:420-455) at coarse node
 // (ic, jc, kc): 27-point full weighting with clamped edges, /8, and
@@ -644,10 +728,9 @@ __device__ unsigned long long cta_sweep(double* e, const uint8_t* fx, const doub
     load6(e, nb, v);
     const double old = e[p];
     const double nv = div6(__dsub_rn(sum6(v), f[p]));
-    const double nw = __dadd_rn(old, omega_step(old, nv, omega));
-    const unsigned long long x = absbits(__dsub_rn(nw, old));
+    unsigned long long x = 0;
+    e[p] = sor_apply<true, false>(old, nv, omega, &x);
     if (x > mb) mb = x;
-    e[p] = nw;
   }
   __syncthreads();
   return cta_max(mb, red);
@@ -704,7 +787,7 @@ k_residual_rhs(const double* __restrict__ e, const uint8_t* __restrict__ fixed,
     const Nb n = neighbours(i, j, k, g.nx, g.ny, g.nz);
     double v[6];
     load6(e, n, v);
-    r = __dsub_rn(__dsub_rn(sum6(v), __dmul_rn(6.0, e[t])), f[t]);
+    r = __dsub_rn(resid6(sum6(v), e[t]), f[t]);
   }
   out[t] = r;
 }
@@ -920,20 +1003,26 @@ __global__ void k_fill_ones_f32(float* a, size_t n) {
 void launch_sweep(cudaStream_t s, double* phi, const uint8_t* fixed,
                   const float* th, int kind, Dims d, double omega, int colour,
                   unsigned long long* dslot, PairCtl* ctl, int lp) {
-  const SweepGeom g = sweep_geom(d);
-  const unsigned nb = blocks_for(g.total);
+  const int U = kind == kPlain ? sweep_planes(d) : 1;
+  const SweepGeom g = sweep_geom(d, U);
+  const unsigned nb = sweep_blocks(g);
   if (nb == 0) return;
   counted();
-#define IG_SWEEP(K)                                                              \
-  if (ctl) k_sweep<K, true><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, omega,    \
-                                                    colour, dslot, ctl, lp);     \
-  else if (dslot) k_sweep<K, false><<<nb, kThreads, 0, s>>>(phi, fixed, th, g,   \
-                                                 omega, colour, dslot, ctl, lp); \
-  else k_sweep<K, false, false><<<nb, kThreads, 0, s>>>(phi, fixed, th, g,       \
-                                                 omega, colour, dslot, ctl, lp);
-  if (kind == kPlain) { IG_SWEEP(kPlain) }
-  else if (kind == kThetaGhost) { IG_SWEEP(kThetaGhost) }
-  else { IG_SWEEP(kThetaSW) }
+  const bool one = omega == 1.0 && !ctl;
+#define IG_SWEEP_T(K, C, D, O, P)                                                            \
+  k_sweep<K, C, D, O, P><<<nb, kSweepThreads, 0, s>>>(phi, fixed, th, g, omega, colour, dslot,    \
+                                                 ctl, lp)
+#define IG_SWEEP(K, P)                                                                       \
+  if (ctl) IG_SWEEP_T(K, true, true, false, P);                                              \
+  else if (dslot && one) IG_SWEEP_T(K, false, true, true, P);                                \
+  else if (dslot) IG_SWEEP_T(K, false, true, false, P);                                      \
+  else if (one) IG_SWEEP_T(K, false, false, true, P);                                        \
+  else IG_SWEEP_T(K, false, false, false, P);
+  if (kind == kPlain && U == 2) { IG_SWEEP(kPlain, 2) }
+  else if (kind == kPlain) { IG_SWEEP(kPlain, 1) }
+  else if (kind == kThetaGhost) { IG_SWEEP(kThetaGhost, 1) }
+  else { IG_SWEEP(kThetaSW, 1) }
+#undef IG_SWEEP_T
 #undef IG_SWEEP
 }
 
@@ -941,17 +1030,18 @@ void launch_residual(cudaStream_t s, const double* phi, const uint8_t* fixed,
                      const float* th, int kind, Dims d, double* out,
                      unsigned long long* absmax) {
   const FlatGeom g = flat_geom(d);
-  const unsigned nb = blocks_for(g.total);
+  const unsigned nb = (unsigned)((((size_t)(d.nx + kResidPlanes - 1) / kResidPlanes) * d.ny * d.nz +
+                                  kSweepThreads - 1) / kSweepThreads);
   if (nb == 0) return;
   counted();
   if (kind == kPlain)
-    k_residual<kPlain><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
+    k_residual<kPlain><<<nb, kSweepThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
   else if (kind == kPlainSW)
-    k_residual<kPlainSW><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
+    k_residual<kPlainSW><<<nb, kSweepThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
   else if (kind == kThetaGhost)
-    k_residual<kThetaGhost><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
+    k_residual<kThetaGhost><<<nb, kSweepThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
   else
-    k_residual<kThetaSW><<<nb, kThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
+    k_residual<kThetaSW><<<nb, kSweepThreads, 0, s>>>(phi, fixed, th, g, out, absmax);
 }
 
 void launch_theta_class(cudaStream_t s, const uint8_t* fixed, const float* th, Dims d,
@@ -977,22 +1067,24 @@ void launch_theta_fill(cudaStream_t s, const uint8_t* cls, const float* th, int 
 }
 
 void launch_sweep_plan(cudaStream_t s, double* phi, const ThetaPlan& plan, int kind, Dims d,
-                       double omega, int colour, unsigned long long* dslot, PairCtl* ctl,
-                       int lp) {
+                       double omega, int colour, PairCtl* ctl, int lp) {
+  unsigned long long* const dslot = nullptr;  // with ctl the kernel takes its slot from it
   const SweepGeom g = sweep_geom(d);
   const FastDiv dnz((uint32_t)d.nz);
   const uint32_t lb = blocks_for(plan.count[colour]);
   const unsigned nb = lb + blocks_for(g.total);
   counted();
+  const bool one = omega == 1.0 && !ctl;
+#define IG_SWEEP_T(K, C, D, O)                                                               \
+  k_sweep_plan<K, C, D, O><<<nb, kThreads, 0, s>>>(phi, plan, g, dnz, lb, omega, colour,     \
+                                                   dslot, ctl, lp)
 #define IG_SWEEP(K)                                                                          \
-  if (ctl) k_sweep_plan<K, true, true><<<nb, kThreads, 0, s>>>(phi, plan, g, dnz, lb, omega, \
-                                                               colour, dslot, ctl, lp);      \
-  else if (dslot) k_sweep_plan<K, false, true><<<nb, kThreads, 0, s>>>(                      \
-      phi, plan, g, dnz, lb, omega, colour, dslot, ctl, lp);                                 \
-  else k_sweep_plan<K, false, false><<<nb, kThreads, 0, s>>>(phi, plan, g, dnz, lb, omega,   \
-                                                             colour, dslot, ctl, lp);
+  if (ctl) IG_SWEEP_T(K, true, true, false);                                                 \
+  else if (one) IG_SWEEP_T(K, false, false, true);                                           \
+  else IG_SWEEP_T(K, false, false, false);
   if (kind == kThetaGhost) { IG_SWEEP(kThetaGhost) }
   else { IG_SWEEP(kThetaSW) }
+#undef IG_SWEEP_T
 #undef IG_SWEEP
 }
 
@@ -1011,14 +1103,25 @@ void launch_residual_plan(cudaStream_t s, const double* phi, const ThetaPlan& pl
 void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,
                       const double* f, Dims d, double omega, int colour,
                       unsigned long long* dslot, PairCtl* ctl, int lp) {
-  const SweepGeom g = sweep_geom(d);
-  const unsigned nb = blocks_for(g.total);
+  const int U = sweep_planes(d);
+  const SweepGeom g = sweep_geom(d, U);
+  const unsigned nb = sweep_blocks(g);
   if (nb == 0) return;
   counted();
-  if (ctl)
-    k_sweep_rhs<true><<<nb, kThreads, 0, s>>>(e, fixed, f, g, omega, colour, dslot, ctl, lp);
-  else
-    k_sweep_rhs<false><<<nb, kThreads, 0, s>>>(e, fixed, f, g, omega, colour, dslot, ctl, lp);
+  const bool one = omega == 1.0 && !ctl;
+#define IG_SWEEP_T(C, D, O, P)                                                               \
+  k_sweep_rhs<C, D, O, P><<<nb, kSweepThreads, 0, s>>>(e, fixed, f, g, omega, colour, dslot, ctl, \
+                                                  lp)
+#define IG_SWEEP(P)                                                                          \
+  if (ctl) IG_SWEEP_T(true, true, false, P);                                                 \
+  else if (dslot && one) IG_SWEEP_T(false, true, true, P);                                   \
+  else if (dslot) IG_SWEEP_T(false, true, false, P);                                         \
+  else if (one) IG_SWEEP_T(false, false, true, P);                                           \
+  else IG_SWEEP_T(false, false, false, P);
+  if (U == 2) { IG_SWEEP(2) }
+  else { IG_SWEEP(1) }
+#undef IG_SWEEP_T
+#undef IG_SWEEP
 }
 
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,

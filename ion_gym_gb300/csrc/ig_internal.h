@@ -84,12 +84,12 @@ void launch_theta_fill(cudaStream_t s, const uint8_t* cls, const float* th, int 
 // launch_sweep / launch_residual of a solve whose theta is in a plan (kind
 // kThetaGhost or kThetaSW): the same bits.
 void launch_sweep_plan(cudaStream_t s, double* phi, const ThetaPlan& plan, int kind, Dims d,
-                       double omega, int colour, unsigned long long* dslot, PairCtl* ctl,
-                       int lp);
+                       double omega, int colour, PairCtl* ctl, int lp);
 void launch_residual_plan(cudaStream_t s, const double* phi, const ThetaPlan& plan, int kind,
                           Dims d, double* out);
 // One colour of the reference SOR sweep.  dslot: where the max |update| goes
-// when ctl == nullptr; with ctl the slot is ctl->slot[2*lp + colour].
+// when ctl == nullptr (nullptr: not formed); with ctl the slot is
+// ctl->slot[2*lp + colour].
 void launch_sweep(cudaStream_t s, double* phi, const uint8_t* fixed,
                   const float* th, int kind, Dims d, double omega, int colour,
                   unsigned long long* dslot, PairCtl* ctl, int lp);

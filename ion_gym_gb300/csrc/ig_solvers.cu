@@ -314,7 +314,7 @@ void init_phi(ThreadCtx& c, FineGrid& g, const double* val_h,
 void fine_sweep(cudaStream_t s, double* phi, const uint8_t* fx, const float* th, const Theta& t,
                 int kind, Dims d, double omega, int colour, PairCtl* ctl, int lp) {
   if (t.on())
-    launch_sweep_plan(s, phi, t.plan, kind, d, omega, colour, nullptr, ctl, lp);
+    launch_sweep_plan(s, phi, t.plan, kind, d, omega, colour, ctl, lp);
   else
     launch_sweep(s, phi, fx, th, kind, d, omega, colour, nullptr, ctl, lp);
 }
@@ -340,7 +340,7 @@ struct ErrLevel {
 
 struct VCycle {
   std::vector<ErrLevel> lv;  // lv[0]: the first coarse (error) level
-  DBuf<unsigned long long> slots;  // per-pair max keys of fixed-count sweeps
+  DBuf<unsigned long long> slots;  // the max keys of a cycle's last sweep pair
   DBuf<unsigned long long> red;    // absmax scratch
   DBuf<PairCtl> ctl;
   double bottom_omega = 1.0;
@@ -406,22 +406,23 @@ void solve_err(ThreadCtx& c, VCycle& v, size_t L) {
   unsigned long long* sl = v.slots.p;
   for (int cyc = 0; cyc < v.max_cycles_err; cyc++) {
     for (int q = 0; q < v.nu1; q++) {
-      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 0, sl, nullptr, 0);
-      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 1, sl, nullptr, 0);
+      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 0, nullptr, nullptr, 0);
+      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 1, nullptr, nullptr, 0);
     }
     launch_residual_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, a.r.p);
     launch_restrict(c.s, a.r.p, a.d, b.f.p, b.d, 1);
     solve_err(c, v, L + 1);
     launch_prolong_add(c.s, b.e.p, b.d, a.e.p, a.fixed.p, a.d);
     if (v.nu2 > 0) {
-      CK(cudaMemsetAsync(sl, 0, 2 * v.nu2 * 8, c.s));
-      for (int q = 0; q < v.nu2; q++) {
-        launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 0, sl + 2 * q, nullptr, 0);
-        launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 1, sl + 2 * q + 1, nullptr, 0);
-      }
+      // the last pair's max |update| decides; the others' are not formed
+      CK(cudaMemsetAsync(sl, 0, 16, c.s));
+      for (int q = 0; q < v.nu2; q++)
+        for (int colour = 0; colour < 2; colour++)
+          launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, colour,
+                           q + 1 == v.nu2 ? sl + colour : nullptr, nullptr, 0);
       CK(cudaGetLastError());
       unsigned long long last[2];
-      CK(cudaMemcpyAsync(last, sl + 2 * (v.nu2 - 1), 16, cudaMemcpyDeviceToHost, c.s));
+      CK(cudaMemcpyAsync(last, sl, 16, cudaMemcpyDeviceToHost, c.s));
       CK(cudaStreamSynchronize(c.s));
       if (umax(last[0], last[1]) < tol) break;
     } else {
@@ -524,8 +525,7 @@ void prepare_vcycle(ThreadCtx& c, VCycle& v, FineGrid& g, int nu1, int nu2,
   v.nu2 = nu2;
   build_err_levels(c, v, g.fixed.p, g.d);
   v.bottom_omega = bottom_omega > 0 ? bottom_omega : optimal_omega_libm(v.lv.back().d);
-  v.slots.alloc(2 * std::max(1, std::max(nu1, nu2)) + 2, c.s);
-  CK(cudaMemsetAsync(v.slots.p, 0, v.slots.n * 8, c.s));
+  v.slots.alloc(2, c.s);
   v.red.alloc(2, c.s);
   v.ctl.alloc(1, c.s);
 }
