@@ -13,6 +13,7 @@
 // Sweeps map one thread to one (i, j, k-pair) cell so a warp reads 64
 // consecutive doubles of a row and every lane does useful FP64 work; the
 // flattened index is split with 32-bit multiplicative division.
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -586,64 +587,88 @@ k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
 // multigrid3d._restrict_fw_njit (multigrid3d.py:420-455) at coarse node
 // (ic, jc, kc): 27-point full weighting with clamped edges, /8, and
 // -4x when neg4 (the caller's scaling).
-__device__ __forceinline__ double restrict_node(const double* __restrict__ fine, long nx,
-                                                long ny, long nz, long ic, long jc, long kc,
-                                                int neg4) {
-  const long i = 2 * ic, j = 2 * jc, k = 2 * kc;
+//
+// The weights are powers of two, so RN(acc + RN(w x)) is one fused
+// multiply-add as long as w x is exact: always, unless x is subnormal or
+// within a factor of 8 of it (restrict_slow).  27 FP64 instructions a node
+// instead of 54 on a pipe of 2 lanes per clock and SM: 8.9 -> 4.9 us a
+// launch, averaged over a 97 x 97 x 193 deck's levels.
+static __device__ __noinline__ double restrict_slow(const double* __restrict__ fine, int nx,
+                                                    int ny, int nz, int i, int j, int k) {
   double acc = 0.0;
+  for (int di = -1; di <= 1; di++)
+    for (int dj = -1; dj <= 1; dj++)
+      for (int dk = -1; dk <= 1; dk++) {
+        const int ii = min(max(i + di, 0), nx - 1), jj = min(max(j + dj, 0), ny - 1);
+        const int kk = min(max(k + dk, 0), nz - 1);
+        const double w = (di ? 0.5 : 1.0) * (dj ? 0.5 : 1.0) * (dk ? 0.5 : 1.0);
+        acc = __dadd_rn(acc, __dmul_rn(w, fine[((size_t)ii * ny + jj) * nz + kk]));
+      }
+  return acc;
+}
+
+__device__ __forceinline__ double restrict_node(const double* __restrict__ fine, int nx,
+                                                int ny, int nz, int ic, int jc, int kc,
+                                                int neg4) {
+  const int i = 2 * ic, j = 2 * jc, k = 2 * kc;
+  const int km = max(k - 1, 0), kp = min(k + 1, nz - 1);
+  double acc = 0.0;
+  unsigned tiny = 0xffffffffu;  // smallest |x| key but for zeros
 #pragma unroll
   for (int di = -1; di <= 1; di++) {
-    long ii = i + di;
-    ii = ii < 0 ? 0 : (ii > nx - 1 ? nx - 1 : ii);
+    const int ii = min(max(i + di, 0), nx - 1);
     const double wi = di == 0 ? 1.0 : 0.5;
 #pragma unroll
     for (int dj = -1; dj <= 1; dj++) {
-      long jj = j + dj;
-      jj = jj < 0 ? 0 : (jj > ny - 1 ? ny - 1 : jj);
+      const int jj = min(max(j + dj, 0), ny - 1);
       const double wj = dj == 0 ? 1.0 : 0.5;
       const double* row = fine + ((size_t)ii * ny + jj) * nz;
+      const double x[3] = {row[km], row[k], row[kp]};
 #pragma unroll
-      for (int dk = -1; dk <= 1; dk++) {
-        long kk = k + dk;
-        kk = kk < 0 ? 0 : (kk > nz - 1 ? nz - 1 : kk);
-        const double wk = dk == 0 ? 1.0 : 0.5;
-        // wi*wj*wk is a power of two, folded at compile time
-        acc = __dadd_rn(acc, __dmul_rn(wi * wj * wk, row[kk]));
+      for (int q = 0; q < 3; q++) {
+        // (high word << 1 | low word != 0) - 1: zeros wrap to the top
+        const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x[q]));
+        const unsigned key = (static_cast<unsigned>(b >> 32) << 1) |
+                             (static_cast<unsigned>(b) ? 1u : 0u);
+        tiny = min(tiny, key - 1u);
+        acc = __fma_rn(wi * wj * (q == 1 ? 1.0 : 0.5), x[q], acc);
       }
     }
   }
+  if (tiny < 0x00800000u) acc = restrict_slow(fine, nx, ny, nz, i, j, k);  // 2^-1019
   double r = __dmul_rn(acc, 0.125);  // == acc / 8.0 (power-of-two scale)
   if (neg4) r = -__dmul_rn(r, 4.0);
   return r;
 }
 
+// A prolongation axis: fine node i sits at i / 2 in coarse units, so its
+// weight on a1 is 0, 1/2 or 1 (half = 0, 1, 2) and on a0 the rest.
 struct Lerp {
-  long a0, a1;
-  double t;
+  int a0, a1, half;
+  __device__ __forceinline__ double t() const { return 0.5 * half; }
 };
 
-// multigrid3d.py:465-481 (prolong-add coordinates)
-__device__ __forceinline__ Lerp pa_axis(long i, long c) {
-  double xf = __dmul_rn((double)i, 0.5);
-  if (xf > (double)(c - 1)) xf = (double)c - 1.0;
-  long x0 = (long)xf;
-  if (x0 > c - 2) x0 = c > 1 ? c - 2 : 0;
+// multigrid3d.py:465-481 (prolong-add coordinates: a0 kept below the top)
+__device__ __forceinline__ Lerp pa_axis(int i, int c) {
   Lerp l;
-  l.a0 = x0;
-  l.a1 = c > 1 ? x0 + 1 : x0;
-  l.t = __dsub_rn(xf, (double)x0);
+  const bool over = i > 2 * (c - 1);
+  l.a0 = over ? c - 1 : i >> 1;
+  l.half = over ? 0 : i & 1;
+  if (l.a0 > c - 2) {
+    l.half = c > 1 ? l.half + 2 * (l.a0 - (c - 2)) : l.half + 2 * l.a0;
+    l.a0 = c > 1 ? c - 2 : 0;
+  }
+  l.a1 = c > 1 ? l.a0 + 1 : l.a0;
   return l;
 }
 
 // multigrid3d.py:144-156 (cascadic prolongation coordinates)
-__device__ __forceinline__ Lerp pl_axis(long i, long c) {
-  double xf = __ddiv_rn((double)i, 2.0);
-  if (xf > (double)(c - 1)) xf = (double)(c - 1);
-  const long x0 = (long)floor(xf);
+__device__ __forceinline__ Lerp pl_axis(int i, int c) {
   Lerp l;
-  l.a0 = x0;
-  l.a1 = x0 + 1 < c - 1 ? x0 + 1 : c - 1;
-  l.t = __dsub_rn(xf, (double)x0);
+  const bool over = i > 2 * (c - 1);
+  l.a0 = over ? c - 1 : i >> 1;
+  l.half = over ? 0 : i & 1;
+  l.a1 = min(l.a0 + 1, c - 1);
   return l;
 }
 
@@ -652,18 +677,59 @@ __device__ __forceinline__ double lerp_ref(double a, double b, double t) {
   return __dadd_rn(__dmul_rn(a, __dsub_rn(1.0, t)), __dmul_rn(b, t));
 }
 
-__device__ __forceinline__ double trilinear(const double* __restrict__ c,
-                                            long cy, long cz, const Lerp& x,
-                                            const Lerp& y, const Lerp& z) {
+static __device__ __noinline__ double trilinear_slow(const double* __restrict__ c, int cy,
+                                                     int cz, Lerp x, Lerp y, Lerp z) {
 #define C(a, b, d) c[((size_t)(a) * cy + (b)) * cz + (d)]
-  const double c00 = lerp_ref(C(x.a0, y.a0, z.a0), C(x.a1, y.a0, z.a0), x.t);
-  const double c10 = lerp_ref(C(x.a0, y.a1, z.a0), C(x.a1, y.a1, z.a0), x.t);
-  const double c01 = lerp_ref(C(x.a0, y.a0, z.a1), C(x.a1, y.a0, z.a1), x.t);
-  const double c11 = lerp_ref(C(x.a0, y.a1, z.a1), C(x.a1, y.a1, z.a1), x.t);
+  const double c00 = lerp_ref(C(x.a0, y.a0, z.a0), C(x.a1, y.a0, z.a0), x.t());
+  const double c10 = lerp_ref(C(x.a0, y.a1, z.a0), C(x.a1, y.a1, z.a0), x.t());
+  const double c01 = lerp_ref(C(x.a0, y.a0, z.a1), C(x.a1, y.a0, z.a1), x.t());
+  const double c11 = lerp_ref(C(x.a0, y.a1, z.a1), C(x.a1, y.a1, z.a1), x.t());
 #undef C
-  const double c0 = lerp_ref(c00, c10, y.t);
-  const double c1 = lerp_ref(c01, c11, y.t);
-  return lerp_ref(c0, c1, z.t);
+  return lerp_ref(lerp_ref(c00, c10, y.t()), lerp_ref(c01, c11, y.t()), z.t());
+}
+
+// The trilinear value of the reference's nested lerps (28 FP64 instructions
+// and more for the coordinates) with at most 7 additions: a weight 0 or 1
+// picks one value, and the halvings of a mean commute with its rounding, so
+// sums are formed and scaled once at the end.  Holds while every value is
+// +0 or has an exponent that leaves room for three halvings and two
+// doublings (no subnormal, overflow, infinity or NaN, skipped weight-0
+// values included, since 0 x inf is NaN); -0 also takes the nested form.
+// The prolongation's launch, averaged over the same levels: 16.5 -> 4.2 us.
+__device__ __forceinline__ double trilinear(const double* __restrict__ c, int cy, int cz,
+                                            const Lerp& x, const Lerp& y, const Lerp& z) {
+  double v[8];
+  bool ok = x.half <= 2 && y.half <= 2 && z.half <= 2;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    v[q] = c[((size_t)(q & 4 ? x.a1 : x.a0) * cy + (q & 2 ? y.a1 : y.a0)) * cz +
+             (q & 1 ? z.a1 : z.a0)];
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v[q]));
+    ok = ok && ((static_cast<unsigned>(b >> 52) & 0x7ffu) - 64u <= 1976u || b == 0ULL);
+  }
+  if (!ok) return trilinear_slow(c, cy, cz, x, y, z);
+  double p[4];
+  if (x.half == 1) {
+#pragma unroll
+    for (int q = 0; q < 4; q++) p[q] = __dadd_rn(v[q], v[4 + q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; q++) p[q] = x.half ? v[4 + q] : v[q];
+  }
+  if (y.half == 1) {
+    p[0] = __dadd_rn(p[0], p[2]);
+    p[1] = __dadd_rn(p[1], p[3]);
+  } else if (y.half) {
+    p[0] = p[2];
+    p[1] = p[3];
+  }
+  // a single z value is doubled, so that every lane of a row takes one
+  // addition and one halving more
+  const double r = __dadd_rn(z.half == 2 ? p[1] : p[0], z.half ? p[1] : p[0]);
+  const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(r));
+  const unsigned long long halvings =
+      1u + (x.half == 1 ? 1u : 0u) + (y.half == 1 ? 1u : 0u);
+  return (b << 1) ? __longlong_as_double(static_cast<long long>(b - (halvings << 52))) : r;
 }
 
 // One CTA solving the bottom of multigrid3d._solve_err
@@ -671,104 +737,126 @@ __device__ __forceinline__ double trilinear(const double* __restrict__ c,
 // launched kernel's arithmetic and the maxima are order-free, so the result
 // and the pair count equal the launched loop's, without a launch per pair or
 // a host synchronisation per batch.
+//
+// What bounds it is one SM's FP64 pipe (2 lanes per clock, 6 instructions a
+// node) and the latency of a half-sweep's chain, so everything else is taken
+// out of the pairs: the free nodes of each colour are listed once (their
+// order changes no result), a thread keeps its first node of each colour
+// with its neighbours' slots in registers (bottoms up to 2048 nodes need no
+// other), and a pair has two barriers, its maximum going through the second.
+// 637 nodes (7 x 7 x 13): 50 -> 31.5 us a solve, most of it pairs.
 constexpr int kBottomCta = 1024;
 
+// A node of the shared-memory level: its slot and its neighbours'.
+struct BottomNode {
+  int p = -1;
+  Nb n;
+};
+
+struct BottomGeom {
+  int nx, ny, nz;
+  FastDiv dny, dnz;
+};
+
+__device__ __forceinline__ BottomNode bottom_node(int p, const BottomGeom& g) {
+  BottomNode b;
+  b.p = p;
+  const uint32_t ij = fdiv((uint32_t)p, g.dnz);
+  const uint32_t i = fdiv(ij, g.dny);
+  b.n = neighbours(i, ij - i * g.dny.d, (uint32_t)p - ij * g.dnz.d, (uint32_t)g.nx,
+                   (uint32_t)g.ny, (uint32_t)g.nz);
+  return b;
+}
+
+__device__ __forceinline__ unsigned long long bottom_update(double* e, const double* f,
+                                                            const BottomNode& b, double omega) {
+  double v[6];
+  load6(e, b.n, v);
+  unsigned long long key = 0;
+  e[b.p] = sor_apply<true, false>(e[b.p], div6(__dsub_rn(sum6(v), f[b.p])), omega, &key);
+  return key;
+}
+
+// Block-wide maximum of a key; red: two rows of 32, alternated by the caller
+// (row), so that one barrier orders the write and the next call's.
 __device__ __forceinline__ unsigned long long cta_max(unsigned long long v,
-                                                      unsigned long long* red) {
+                                                      unsigned long long* red, int row) {
   v = warp_max_u64(v);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) red[wid] = v;
+  const int lane = threadIdx.x & 31;
+  if (lane == 0) red[32 * row + (threadIdx.x >> 5)] = v;
   __syncthreads();
-  if (wid == 0) {
-    v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0ull;
-    v = warp_max_u64(v);
-    if (lane == 0) red[32] = v;
-  }
-  __syncthreads();
-  const unsigned long long r = red[32];
-  __syncthreads();
-  return r;
-}
-
-// tol = rel_tol * max(max|f|, 1e-300) / 6 of a level in shared memory (NaN
-// in f makes it NaN, as numpy's max does).
-__device__ double cta_level_tol(const double* f, long n, double rel_tol,
-                                unsigned long long* red) {
-  unsigned long long fk = 0;
-  bool nan = false;
-  for (long t = threadIdx.x; t < n; t += blockDim.x) {
-    const unsigned long long x =
-        static_cast<unsigned long long>(__double_as_longlong(f[t])) & 0x7fffffffffffffffULL;
-    if (x > 0x7ff0000000000000ULL) nan = true;
-    else if (x > fk) fk = x;
-  }
-  nan = __syncthreads_or(nan);
-  fk = cta_max(fk, red);
-  double scale = nan ? __longlong_as_double(0x7ff8000000000000LL) : bits_to_double(fk);
-  scale = (1e-300 > scale) ? 1e-300 : scale;  // max(|f|.max(), 1e-300)
-  return __ddiv_rn(__dmul_rn(rel_tol, scale), 6.0);
-}
-
-// One colour of _sweep_rhs over a level in shared memory; returns the
-// largest |update| key (all threads).
-__device__ unsigned long long cta_sweep(double* e, const uint8_t* fx, const double* f,
-                                        long nx, long ny, long nz, double omega, int colour,
-                                        unsigned long long* red) {
-  const long half = nz / 2 + 1;  // slots of one colour in a row
-  unsigned long long mb = 0;
-  for (long t = threadIdx.x; t < nx * ny * half; t += blockDim.x) {
-    const long ij = t / half, kk = t - ij * half;
-    const long i = ij / ny, j = ij - i * ny;
-    const long k = 2 * kk + ((i + j + colour) & 1);
-    if (k >= nz) continue;
-    const long p = (i * ny + j) * nz + k;
-    if (fx[p]) continue;
-    const Nb nb = neighbours(i, j, k, nx, ny, nz);
-    double v[6];
-    load6(e, nb, v);
-    const double old = e[p];
-    const double nv = div6(__dsub_rn(sum6(v), f[p]));
-    unsigned long long x = 0;
-    e[p] = sor_apply<true, false>(old, nv, omega, &x);
-    if (x > mb) mb = x;
-  }
-  __syncthreads();
-  return cta_max(mb, red);
-}
-
-// The bottom: e = 0; SOR pairs at omega until the larger of a pair's two
-// max |update| is below 0.02 * tol, at most max_pairs pairs.
-__device__ void cta_bottom(double* e, const uint8_t* fx, const double* f, long nx, long ny,
-                           long nz, double rel_tol, double omega, long max_pairs,
-                           unsigned long long* red) {
-  const long n = nx * ny * nz;
-  for (long t = threadIdx.x; t < n; t += blockDim.x) e[t] = 0.0;
-  const double tol = __dmul_rn(0.02, cta_level_tol(f, n, rel_tol, red));
-  for (long pr = 0; pr < max_pairs; pr++) {
-    const unsigned long long k0 = cta_sweep(e, fx, f, nx, ny, nz, omega, 0, red);
-    const unsigned long long k1 = cta_sweep(e, fx, f, nx, ny, nz, omega, 1, red);
-    if (bits_to_double(k0 > k1 ? k0 : k1) < tol) break;
-  }
+  return warp_max_u64(lane < (int)(blockDim.x >> 5) ? red[32 * row + lane] : 0ULL);
 }
 
 __global__ void __launch_bounds__(kBottomCta)
 k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
-             const double* __restrict__ f_g, long nx, long ny, long nz, double rel_tol,
+             const double* __restrict__ f_g, BottomGeom g, double rel_tol,
              double omega, long max_pairs) {
   extern __shared__ double sm[];
-  __shared__ unsigned long long red[33];
-  const long n = nx * ny * nz;
+  __shared__ unsigned long long red[64];
+  __shared__ int count[2];
+  const int n = g.nx * g.ny * g.nz, lane = threadIdx.x & 31;
   double* e = sm;
   double* f = sm + n;
-  uint8_t* fx = reinterpret_cast<uint8_t*>(sm + 2 * n);
-  for (long t = threadIdx.x; t < n; t += blockDim.x) {
-    f[t] = f_g[t];
-    fx[t] = fixed_g[t];
+  uint16_t* list = reinterpret_cast<uint16_t*>(sm + 2 * n);  // colour 0 up, colour 1 down
+  if (threadIdx.x < 2) count[threadIdx.x] = 0;
+  __syncthreads();
+  // e = 0, f, the free nodes by colour, and max|f| (NaN in f makes it NaN,
+  // as numpy's max does)
+  unsigned long long fk = 0;
+  bool nan = false;
+  for (int t0 = 0; t0 < n; t0 += blockDim.x) {
+    const int t = t0 + threadIdx.x;
+    int c = -1;
+    if (t < n) {
+      const double x = f_g[t];
+      f[t] = x;
+      e[t] = 0.0;
+      const unsigned long long b =
+          static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7fffffffffffffffULL;
+      if (b > 0x7ff0000000000000ULL) nan = true;
+      else if (b > fk) fk = b;
+      if (!fixed_g[t]) {
+        const uint32_t ij = fdiv((uint32_t)t, g.dnz);
+        const uint32_t i = fdiv(ij, g.dny);
+        c = (int)((i + (ij - i * g.dny.d) + ((uint32_t)t - ij * g.dnz.d)) & 1u);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const unsigned m = __ballot_sync(0xffffffffu, c == q);
+      int base = 0;
+      if (lane == 0 && m) base = atomicAdd(&count[q], __popc(m));
+      base = __shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+      if (c == q) list[q ? n - 1 - base : base] = (uint16_t)t;
+    }
   }
-  __syncthreads();
-  cta_bottom(e, fx, f, nx, ny, nz, rel_tol, omega, max_pairs, red);
-  __syncthreads();
-  for (long t = threadIdx.x; t < n; t += blockDim.x) e_out[t] = e[t];
+  nan = __syncthreads_or(nan);
+  fk = cta_max(fk, red, 0);
+  double scale = nan ? __longlong_as_double(0x7ff8000000000000LL) : bits_to_double(fk);
+  scale = (1e-300 > scale) ? 1e-300 : scale;  // max(|f|.max(), 1e-300)
+  // SOR pairs at omega until the larger of a pair's two max |update| is
+  // below 0.02 * (rel_tol * scale / 6), at most max_pairs pairs
+  const double tol = __dmul_rn(0.02, __ddiv_rn(__dmul_rn(rel_tol, scale), 6.0));
+  const int n0 = count[0], n1 = count[1], tid = (int)threadIdx.x, nt = (int)blockDim.x;
+  BottomNode own[2];
+  if (tid < n0) own[0] = bottom_node(list[tid], g);
+  if (tid < n1) own[1] = bottom_node(list[n - 1 - tid], g);
+  for (long pr = 0; pr < max_pairs; pr++) {
+    unsigned long long mb = 0;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      if (own[c].p >= 0) mb = max(mb, bottom_update(e, f, own[c], omega));
+      for (int q = tid + nt; q < (c ? n1 : n0); q += nt)
+        mb = max(mb, bottom_update(e, f, bottom_node(list[c ? n - 1 - q : q], g), omega));
+      if (c == 0) __syncthreads();
+    }
+    mb = cta_max(mb, red, (int)(pr & 1) ^ 1);
+    if (bits_to_double(mb) < tol) break;
+  }
+  // the last pair's barrier (cta_max) came after its last update
+  if (max_pairs <= 0) __syncthreads();
+  for (int t = tid; t < n; t += nt) e_out[t] = e[t];
 }
 
 // multigrid3d._residual_rhs (multigrid3d.py:394-417).
@@ -792,45 +880,42 @@ k_residual_rhs(const double* __restrict__ e, const uint8_t* __restrict__ fixed,
   out[t] = r;
 }
 
-__global__ void __launch_bounds__(kThreads)
-k_restrict(const double* __restrict__ fine, long nx, long ny, long nz,
+__global__ void __launch_bounds__(kSweepThreads)
+k_restrict(const double* __restrict__ fine, int nx, int ny, int nz,
            double* __restrict__ out, FlatGeom c, int neg4) {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
   if (t >= c.total) return;
   const uint32_t ij = fdiv(t, c.div_nz);
-  const long kc = t - ij * c.div_nz.d;
-  const long ic = fdiv(ij, c.div_ny);
-  const long jc = ij - ic * c.div_ny.d;
-  out[t] = restrict_node(fine, nx, ny, nz, ic, jc, kc, neg4);
+  const uint32_t ic = fdiv(ij, c.div_ny);
+  out[t] = restrict_node(fine, nx, ny, nz, (int)ic, (int)(ij - ic * c.div_ny.d),
+                         (int)(t - ij * c.div_nz.d), neg4);
 }
 
 // multigrid3d._prolong_add_njit (multigrid3d.py:458-499).
-__global__ void __launch_bounds__(kThreads)
-k_prolong_add(const double* __restrict__ coarse, long cx, long cy, long cz,
+__global__ void __launch_bounds__(kSweepThreads)
+k_prolong_add(const double* __restrict__ coarse, int cx, int cy, int cz,
               double* __restrict__ out, const uint8_t* __restrict__ fixed,
               FlatGeom g) {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
   if (t >= g.total) return;
   if (fixed[t]) return;
   const uint32_t ij = fdiv(t, g.div_nz);
-  const long k = t - ij * g.div_nz.d;
-  const long i = fdiv(ij, g.div_ny);
-  const long j = ij - i * g.div_ny.d;
-  const Lerp x = pa_axis(i, cx), y = pa_axis(j, cy), z = pa_axis(k, cz);
+  const uint32_t i = fdiv(ij, g.div_ny);
+  const Lerp x = pa_axis((int)i, cx), y = pa_axis((int)(ij - i * g.div_ny.d), cy);
+  const Lerp z = pa_axis((int)(t - ij * g.div_nz.d), cz);
   out[t] = __dadd_rn(out[t], trilinear(coarse, cy, cz, x, y, z));
 }
 
 // multigrid3d._prolongate (multigrid3d.py:138-171).
-__global__ void __launch_bounds__(kThreads)
-k_prolongate(const double* __restrict__ coarse, long cx, long cy, long cz,
+__global__ void __launch_bounds__(kSweepThreads)
+k_prolongate(const double* __restrict__ coarse, int cx, int cy, int cz,
              double* __restrict__ out, FlatGeom g) {
-  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  const uint32_t t = blockIdx.x * kSweepThreads + threadIdx.x;
   if (t >= g.total) return;
   const uint32_t ij = fdiv(t, g.div_nz);
-  const long k = t - ij * g.div_nz.d;
-  const long i = fdiv(ij, g.div_ny);
-  const long j = ij - i * g.div_ny.d;
-  const Lerp x = pl_axis(i, cx), y = pl_axis(j, cy), z = pl_axis(k, cz);
+  const uint32_t i = fdiv(ij, g.div_ny);
+  const Lerp x = pl_axis((int)i, cx), y = pl_axis((int)(ij - i * g.div_ny.d), cy);
+  const Lerp z = pl_axis((int)(t - ij * g.div_nz.d), cz);
   out[t] = trilinear(coarse, cy, cz, x, y, z);
 }
 
@@ -1127,15 +1212,23 @@ void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
                        Dims d, double rel_tol, double omega, long max_pairs) {
   const size_t n = d.n();
-  const size_t bytes = 17 * n;
-  if (n == 0 || bytes > kBottomSmemMax) return false;
+  if (n == 0 || 17 * n > kBottomSmemMax) return false;
+  const size_t bytes = 18 * n;
   static std::once_flag once;
   std::call_once(once, [] {
     cudaFuncSetAttribute(k_bottom_err, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)kBottomSmemMax);
+                         (int)(18 * (kBottomSmemMax / 17)));
   });
-  k_bottom_err<<<1, kBottomCta, (bytes + 7) / 8 * 8, s>>>(e, fixed, f, d.nx, d.ny, d.nz,
-                                                         rel_tol, omega, max_pairs);
+  BottomGeom g;
+  g.nx = (int)d.nx;
+  g.ny = (int)d.ny;
+  g.nz = (int)d.nz;
+  g.dny = FastDiv((uint32_t)d.ny);
+  g.dnz = FastDiv((uint32_t)d.nz);
+  // a thread per node of one colour, in whole warps: fewer warps, cheaper
+  // barriers
+  const int nt = std::min<long>(kBottomCta, std::max<long>(64, ((long)(n + 1) / 2 + 31) / 32 * 32));
+  k_bottom_err<<<1, nt, (bytes + 7) / 8 * 8, s>>>(e, fixed, f, g, rel_tol, omega, max_pairs);
   counted();
   return true;
 }
@@ -1153,9 +1246,9 @@ void launch_residual_rhs(cudaStream_t s, const double* e, const uint8_t* fixed,
 void launch_restrict(cudaStream_t s, const double* fine, Dims d, double* out,
                      Dims c, int neg4) {
   const FlatGeom g = flat_geom(c);
-  const unsigned nb = blocks_for(g.total);
+  const unsigned nb = (g.total + kSweepThreads - 1) / kSweepThreads;
   if (nb) {
-    k_restrict<<<nb, kThreads, 0, s>>>(fine, d.nx, d.ny, d.nz, out, g, neg4);
+    k_restrict<<<nb, kSweepThreads, 0, s>>>(fine, (int)d.nx, (int)d.ny, (int)d.nz, out, g, neg4);
     counted();
   }
 }
@@ -1163,9 +1256,9 @@ void launch_restrict(cudaStream_t s, const double* fine, Dims d, double* out,
 void launch_prolong_add(cudaStream_t s, const double* coarse, Dims c,
                         double* out, const uint8_t* fixed, Dims d) {
   const FlatGeom g = flat_geom(d);
-  const unsigned nb = blocks_for(g.total);
+  const unsigned nb = (g.total + kSweepThreads - 1) / kSweepThreads;
   if (nb) {
-    k_prolong_add<<<nb, kThreads, 0, s>>>(coarse, c.nx, c.ny, c.nz, out, fixed, g);
+    k_prolong_add<<<nb, kSweepThreads, 0, s>>>(coarse, (int)c.nx, (int)c.ny, (int)c.nz, out, fixed, g);
     counted();
   }
 }
@@ -1173,9 +1266,9 @@ void launch_prolong_add(cudaStream_t s, const double* coarse, Dims c,
 void launch_prolongate(cudaStream_t s, const double* coarse, Dims c,
                        double* out, Dims d) {
   const FlatGeom g = flat_geom(d);
-  const unsigned nb = blocks_for(g.total);
+  const unsigned nb = (g.total + kSweepThreads - 1) / kSweepThreads;
   if (nb) {
-    k_prolongate<<<nb, kThreads, 0, s>>>(coarse, c.nx, c.ny, c.nz, out, g);
+    k_prolongate<<<nb, kSweepThreads, 0, s>>>(coarse, (int)c.nx, (int)c.ny, (int)c.nz, out, g);
     counted();
   }
 }

@@ -98,8 +98,8 @@ void launch_residual(cudaStream_t s, const double* phi, const uint8_t* fixed,
                      unsigned long long* absmax /* nullable */);
 // The whole bottom solve of multigrid3d._solve_err (e = 0, tol from
 // max|f|, SOR pairs to 0.02 tol, at most max_pairs) in one CTA with the
-// level in shared memory; false (nothing launched) when the level does not
-// fit in kBottomSmemMax bytes (17 per node).
+// level in shared memory (18 bytes a node); false (nothing launched) when
+// the level has more than kBottomSmemMax / 17 nodes.
 constexpr size_t kBottomSmemMax = 200 * 1024;
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
                        Dims d, double rel_tol, double omega, long max_pairs);
