@@ -17,6 +17,8 @@
 #include <atomic>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "ig_common.cuh"
 #include "ig_internal.h"
 
@@ -198,14 +200,22 @@ __device__ __forceinline__ double sum6(const double v[6]) {
   return __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(v[0], v[1]), v[2]), v[3]), v[4]), v[5]);
 }
 
+// CG: the value comes from L2, for data that other SMs write within the
+// same kernel.
+template <bool CG>
+__device__ __forceinline__ double ldv(const double* a, size_t o) {
+  return CG ? __ldcg(a + o) : a[o];
+}
+
+template <bool CG = false>
 __device__ __forceinline__ void load6(const double* __restrict__ a, const Nb& n,
                                       double v[6]) {
-  v[0] = a[n.xm];
-  v[1] = a[n.xp];
-  v[2] = a[n.ym];
-  v[3] = a[n.yp];
-  v[4] = a[n.zm];
-  v[5] = a[n.zp];
+  v[0] = ldv<CG>(a, n.xm);
+  v[1] = ldv<CG>(a, n.xp);
+  v[2] = ldv<CG>(a, n.ym);
+  v[3] = ldv<CG>(a, n.yp);
+  v[4] = ldv<CG>(a, n.zm);
+  v[5] = ldv<CG>(a, n.zp);
 }
 
 // The nodes of one colour a sweep thread owns: the same y, z slot kk and U
@@ -593,6 +603,7 @@ k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
 // within a factor of 8 of it (restrict_slow).  27 FP64 instructions a node
 // instead of 54 on a pipe of 2 lanes per clock and SM: 8.9 -> 4.9 us a
 // launch, averaged over a 97 x 97 x 193 deck's levels.
+template <bool CG>
 static __device__ __noinline__ double restrict_slow(const double* __restrict__ fine, int nx,
                                                     int ny, int nz, int i, int j, int k) {
   double acc = 0.0;
@@ -602,11 +613,12 @@ static __device__ __noinline__ double restrict_slow(const double* __restrict__ f
         const int ii = min(max(i + di, 0), nx - 1), jj = min(max(j + dj, 0), ny - 1);
         const int kk = min(max(k + dk, 0), nz - 1);
         const double w = (di ? 0.5 : 1.0) * (dj ? 0.5 : 1.0) * (dk ? 0.5 : 1.0);
-        acc = __dadd_rn(acc, __dmul_rn(w, fine[((size_t)ii * ny + jj) * nz + kk]));
+        acc = __dadd_rn(acc, __dmul_rn(w, ldv<CG>(fine, ((size_t)ii * ny + jj) * nz + kk)));
       }
   return acc;
 }
 
+template <bool CG>
 __device__ __forceinline__ double restrict_node(const double* __restrict__ fine, int nx,
                                                 int ny, int nz, int ic, int jc, int kc,
                                                 int neg4) {
@@ -623,7 +635,7 @@ __device__ __forceinline__ double restrict_node(const double* __restrict__ fine,
       const int jj = min(max(j + dj, 0), ny - 1);
       const double wj = dj == 0 ? 1.0 : 0.5;
       const double* row = fine + ((size_t)ii * ny + jj) * nz;
-      const double x[3] = {row[km], row[k], row[kp]};
+      const double x[3] = {ldv<CG>(row, km), ldv<CG>(row, k), ldv<CG>(row, kp)};
 #pragma unroll
       for (int q = 0; q < 3; q++) {
         // (high word << 1 | low word != 0) - 1: zeros wrap to the top
@@ -635,7 +647,7 @@ __device__ __forceinline__ double restrict_node(const double* __restrict__ fine,
       }
     }
   }
-  if (tiny < 0x00800000u) acc = restrict_slow(fine, nx, ny, nz, i, j, k);  // 2^-1019
+  if (tiny < 0x00800000u) acc = restrict_slow<CG>(fine, nx, ny, nz, i, j, k);  // 2^-1019
   double r = __dmul_rn(acc, 0.125);  // == acc / 8.0 (power-of-two scale)
   if (neg4) r = -__dmul_rn(r, 4.0);
   return r;
@@ -677,9 +689,10 @@ __device__ __forceinline__ double lerp_ref(double a, double b, double t) {
   return __dadd_rn(__dmul_rn(a, __dsub_rn(1.0, t)), __dmul_rn(b, t));
 }
 
+template <bool CG>
 static __device__ __noinline__ double trilinear_slow(const double* __restrict__ c, int cy,
                                                      int cz, Lerp x, Lerp y, Lerp z) {
-#define C(a, b, d) c[((size_t)(a) * cy + (b)) * cz + (d)]
+#define C(a, b, d) ldv<CG>(c, ((size_t)(a) * cy + (b)) * cz + (d))
   const double c00 = lerp_ref(C(x.a0, y.a0, z.a0), C(x.a1, y.a0, z.a0), x.t());
   const double c10 = lerp_ref(C(x.a0, y.a1, z.a0), C(x.a1, y.a1, z.a0), x.t());
   const double c01 = lerp_ref(C(x.a0, y.a0, z.a1), C(x.a1, y.a0, z.a1), x.t());
@@ -696,18 +709,19 @@ static __device__ __noinline__ double trilinear_slow(const double* __restrict__ 
 // doublings (no subnormal, overflow, infinity or NaN, skipped weight-0
 // values included, since 0 x inf is NaN); -0 also takes the nested form.
 // The prolongation's launch, averaged over the same levels: 16.5 -> 4.2 us.
+template <bool CG>
 __device__ __forceinline__ double trilinear(const double* __restrict__ c, int cy, int cz,
                                             const Lerp& x, const Lerp& y, const Lerp& z) {
   double v[8];
   bool ok = x.half <= 2 && y.half <= 2 && z.half <= 2;
 #pragma unroll
   for (int q = 0; q < 8; q++) {
-    v[q] = c[((size_t)(q & 4 ? x.a1 : x.a0) * cy + (q & 2 ? y.a1 : y.a0)) * cz +
-             (q & 1 ? z.a1 : z.a0)];
+    v[q] = ldv<CG>(c, ((size_t)(q & 4 ? x.a1 : x.a0) * cy + (q & 2 ? y.a1 : y.a0)) * cz +
+                          (q & 1 ? z.a1 : z.a0));
     const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v[q]));
     ok = ok && ((static_cast<unsigned>(b >> 52) & 0x7ffu) - 64u <= 1976u || b == 0ULL);
   }
-  if (!ok) return trilinear_slow(c, cy, cz, x, y, z);
+  if (!ok) return trilinear_slow<CG>(c, cy, cz, x, y, z);
   double p[4];
   if (x.half == 1) {
 #pragma unroll
@@ -788,13 +802,14 @@ __device__ __forceinline__ unsigned long long cta_max(unsigned long long v,
   return warp_max_u64(lane < (int)(blockDim.x >> 5) ? red[32 * row + lane] : 0ULL);
 }
 
-__global__ void __launch_bounds__(kBottomCta)
-k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
-             const double* __restrict__ f_g, BottomGeom g, double rel_tol,
-             double omega, long max_pairs) {
-  extern __shared__ double sm[];
-  __shared__ unsigned long long red[64];
-  __shared__ int count[2];
+// The whole bottom solve by the calling CTA: sm holds 18 bytes a node, red
+// and count are its scratch.  Every thread must call it.
+__device__ __forceinline__ void bottom_solve(double* __restrict__ e_out,
+                                             const uint8_t* __restrict__ fixed_g,
+                                             const double* __restrict__ f_g,
+                                             const BottomGeom& g, double rel_tol, double omega,
+                                             long max_pairs, double* sm,
+                                             unsigned long long* red, int* count) {
   const int n = g.nx * g.ny * g.nz, lane = threadIdx.x & 31;
   double* e = sm;
   double* f = sm + n;
@@ -809,7 +824,7 @@ k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
     const int t = t0 + threadIdx.x;
     int c = -1;
     if (t < n) {
-      const double x = f_g[t];
+      const double x = __ldcg(f_g + t);
       f[t] = x;
       e[t] = 0.0;
       const unsigned long long b =
@@ -856,7 +871,208 @@ k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
   }
   // the last pair's barrier (cta_max) came after its last update
   if (max_pairs <= 0) __syncthreads();
-  for (int t = tid; t < n; t += nt) e_out[t] = e[t];
+  for (int t = tid; t < n; t += nt) __stcg(e_out + t, e[t]);
+}
+
+__global__ void __launch_bounds__(kBottomCta)
+k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
+             const double* __restrict__ f_g, BottomGeom g, double rel_tol,
+             double omega, long max_pairs) {
+  extern __shared__ double sm[];
+  __shared__ unsigned long long red[64];
+  __shared__ int count[2];
+  bottom_solve(e_out, fixed_g, f_g, g, rel_tol, omega, max_pairs, sm, red, count);
+}
+
+// ---- the small error levels in one launch ----------------------------------
+//
+// multigrid3d._solve_err (multigrid3d.py:553-599) from one level down to the
+// bottom, by one cluster of CTAs.  On the launched path a level of some
+// 10^4 nodes costs about 20 launches, two memsets and two host decisions a
+// cycle, each a few microseconds for well under one of work, and the eight
+// bases of a door call queue for the driver as well (75,000 launches in 165
+// ms).  Here the host decisions are the cluster's: every CTA forms the same
+// maxima (exchanged through distributed shared memory) and takes the same
+// branches.
+//
+// The levels' arrays stay in global memory; nodes are dealt to the
+// cluster's threads in flat order, values that other CTAs write are read
+// and written through L2 (ldv<true>, __stcg) and a cluster barrier
+// (release / acquire) separates the phases.  Every node's arithmetic is the
+// launched kernels', so the bits are theirs.  The bottom is CTA 0's
+// (bottom_solve).  16 CTAs of 512 threads: a half-sweep of 25 x 25 x 49
+// nodes is then some two nodes a thread and bound by its chain of load, sum
+// and barrier (a microsecond or two) rather than by the 16 SMs' FP64 pipes.
+// The door: 8 bases of a 97 x 97 x 193 ring deck 165 -> 109 ms, 4 with theta
+// at 65 x 65 x 129 46 -> 30.6 ms.
+struct TailGeom {
+  int nx, ny, nz, n, slots;
+  FastDiv dkk, dny, dnz;
+};
+
+// One half-sweep at omega 1; the largest |update| key with DELTA.
+template <bool DELTA>
+__device__ __forceinline__ unsigned long long tail_sweep(const TailLevel& L, const TailGeom& g,
+                                                         int colour, int gt, int gn) {
+  unsigned long long mb = 0;
+  for (int t = gt; t < g.slots; t += gn) {
+    const uint32_t ij = fdiv((uint32_t)t, g.dkk);
+    const uint32_t i = fdiv(ij, g.dny);
+    const uint32_t j = ij - i * g.dny.d;
+    const uint32_t k = 2 * ((uint32_t)t - ij * g.dkk.d) + ((i + j + (uint32_t)colour) & 1u);
+    if (k >= (uint32_t)g.nz) continue;
+    const uint32_t p = ij * (uint32_t)g.nz + k;
+    if (L.fixed[p]) continue;
+    const Nb n = neighbours(i, j, k, (uint32_t)g.nx, (uint32_t)g.ny, (uint32_t)g.nz);
+    double v[6];
+    load6<true>(L.e, n, v);
+    const double f = __ldcg(L.f + p), old = __ldcg(L.e + p);
+    unsigned long long key = 0;
+    __stcg(L.e + p, sor_apply<DELTA, true>(old, div6(__dsub_rn(sum6(v), f)), 1.0, &key));
+    if (DELTA && key > mb) mb = key;
+  }
+  return mb;
+}
+
+__global__ void __launch_bounds__(kTailThreads)
+k_err_tail(TailArgs A) {
+  namespace cg = cooperative_groups;
+  extern __shared__ double sm[];
+  __shared__ unsigned long long red[64], wred[32], slot[2][kTailCtas];
+  __shared__ int count[2];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const int gn = ctas * kTailThreads, gt = rank * kTailThreads + (int)threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int par = 0;
+  // the cluster's maximum of a key, ending in a cluster barrier
+  auto cluster_max = [&](unsigned long long v) {
+    v = warp_max_u64(v);
+    if (lane == 0) wred[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+      v = warp_max_u64(lane < kTailThreads / 32 ? wred[lane] : 0ULL);
+      if (lane < ctas) *cl.map_shared_rank(&slot[par][rank], lane) = v;
+    }
+    cl.sync();
+    v = warp_max_u64(lane < ctas ? slot[par][lane] : 0ULL);
+    par ^= 1;
+    return v;
+  };
+  // max|f| as a key, ~0 standing for NaN
+  auto fkey = [](double f) {
+    const unsigned long long b =
+        static_cast<unsigned long long>(__double_as_longlong(f)) & 0x7fffffffffffffffULL;
+    return b > 0x7ff0000000000000ULL ? ~0ULL : b;
+  };
+  auto geom = [](const TailLevel& L) {
+    TailGeom g;
+    g.nx = L.nx;
+    g.ny = L.ny;
+    g.nz = L.nz;
+    g.n = L.nx * L.ny * L.nz;
+    g.dkk = L.dkk;
+    g.dny = L.dny;
+    g.dnz = L.dnz;
+    g.slots = L.nx * L.ny * (int)L.dkk.d;
+    return g;
+  };
+  double tol[kTailLevels];
+  int cyc[kTailLevels];
+  auto enter = [&](int l, unsigned long long fk) {
+    double scale = fk == ~0ULL ? __longlong_as_double(0x7ff8000000000000LL) : bits_to_double(fk);
+    scale = (1e-300 > scale) ? 1e-300 : scale;  // max(|f|.max(), 1e-300)
+    tol[l] = __ddiv_rn(__dmul_rn(A.rel_tol, scale), 6.0);
+    cyc[l] = 0;
+  };
+  int l = 0;
+  {
+    const TailLevel& L = A.lv[0];
+    const TailGeom g = geom(L);
+    unsigned long long fk = 0;
+    for (int t = gt; t < g.n; t += gn) {
+      fk = max(fk, fkey(__ldcg(L.f + t)));
+      __stcg(L.e + t, 0.0);
+    }
+    enter(0, cluster_max(fk));
+  }
+  while (true) {
+    // level l: pre-smoothing, and its residual restricted to level l + 1
+    const TailLevel& L = A.lv[l];
+    const TailLevel& C = A.lv[l + 1];
+    const TailGeom g = geom(L), c = geom(C);
+    for (int q = 0; q < 2 * A.nu1; q++) {
+      tail_sweep<false>(L, g, q & 1, gt, gn);
+      cl.sync();
+    }
+    for (int t = gt; t < g.n; t += gn) {
+      double r = 0.0;
+      if (!L.fixed[t]) {
+        const uint32_t ij = fdiv((uint32_t)t, g.dnz);
+        const uint32_t i = fdiv(ij, g.dny);
+        const Nb n = neighbours(i, ij - i * g.dny.d, (uint32_t)t - ij * g.dnz.d, (uint32_t)g.nx,
+                                (uint32_t)g.ny, (uint32_t)g.nz);
+        double v[6];
+        load6<true>(L.e, n, v);
+        r = __dsub_rn(resid6(sum6(v), __ldcg(L.e + t)), __ldcg(L.f + t));
+      }
+      __stcg(L.r + t, r);
+    }
+    cl.sync();
+    unsigned long long fk = 0;
+    for (int t = gt; t < c.n; t += gn) {
+      const uint32_t ij = fdiv((uint32_t)t, c.dnz);
+      const uint32_t ic = fdiv(ij, c.dny);
+      const double f = restrict_node<true>(L.r, g.nx, g.ny, g.nz, (int)ic,
+                                           (int)(ij - ic * c.dny.d),
+                                           (int)((uint32_t)t - ij * c.dnz.d), 1);
+      __stcg(C.f + t, f);
+      __stcg(C.e + t, 0.0);
+      fk = max(fk, fkey(f));
+    }
+    enter(l + 1, cluster_max(fk));
+    l++;
+    if (l + 1 < A.nlev) continue;
+    if (rank == 0) {
+      BottomGeom b;
+      b.nx = C.nx;
+      b.ny = C.ny;
+      b.nz = C.nz;
+      b.dny = C.dny;
+      b.dnz = C.dnz;
+      bottom_solve(C.e, C.fixed, C.f, b, A.rel_tol, A.bottom_omega, A.bottom_pairs, sm, red,
+                   count);
+    }
+    cl.sync();
+    // back up: correction, post-smoothing, and the cycle's decision
+    bool done = true;
+    while (done && l > 0) {
+      const TailLevel& F = A.lv[l - 1];
+      const TailLevel& K = A.lv[l];
+      const TailGeom h = geom(F);
+      l--;
+      for (int t = gt; t < h.n; t += gn) {
+        if (F.fixed[t]) continue;
+        const uint32_t ij = fdiv((uint32_t)t, h.dnz);
+        const uint32_t i = fdiv(ij, h.dny);
+        const Lerp x = pa_axis((int)i, K.nx), y = pa_axis((int)(ij - i * h.dny.d), K.ny);
+        const Lerp z = pa_axis((int)((uint32_t)t - ij * h.dnz.d), K.nz);
+        __stcg(F.e + t, __dadd_rn(__ldcg(F.e + t), trilinear<true>(K.e, K.ny, K.nz, x, y, z)));
+      }
+      cl.sync();
+      for (int q = 0; q < 2 * A.nu2 - 2; q++) {
+        tail_sweep<false>(F, h, q & 1, gt, gn);
+        cl.sync();
+      }
+      unsigned long long mb = tail_sweep<true>(F, h, 0, gt, gn);
+      cl.sync();
+      mb = cluster_max(max(mb, tail_sweep<true>(F, h, 1, gt, gn)));
+      cyc[l]++;
+      done = bits_to_double(mb) < tol[l] || cyc[l] >= A.max_cycles;
+    }
+    if (done) break;
+  }
+  cl.sync();  // no CTA leaves while another may still write to its shared memory
 }
 
 // multigrid3d._residual_rhs (multigrid3d.py:394-417).
@@ -887,7 +1103,7 @@ k_restrict(const double* __restrict__ fine, int nx, int ny, int nz,
   if (t >= c.total) return;
   const uint32_t ij = fdiv(t, c.div_nz);
   const uint32_t ic = fdiv(ij, c.div_ny);
-  out[t] = restrict_node(fine, nx, ny, nz, (int)ic, (int)(ij - ic * c.div_ny.d),
+  out[t] = restrict_node<false>(fine, nx, ny, nz, (int)ic, (int)(ij - ic * c.div_ny.d),
                          (int)(t - ij * c.div_nz.d), neg4);
 }
 
@@ -903,7 +1119,7 @@ k_prolong_add(const double* __restrict__ coarse, int cx, int cy, int cz,
   const uint32_t i = fdiv(ij, g.div_ny);
   const Lerp x = pa_axis((int)i, cx), y = pa_axis((int)(ij - i * g.div_ny.d), cy);
   const Lerp z = pa_axis((int)(t - ij * g.div_nz.d), cz);
-  out[t] = __dadd_rn(out[t], trilinear(coarse, cy, cz, x, y, z));
+  out[t] = __dadd_rn(out[t], trilinear<false>(coarse, cy, cz, x, y, z));
 }
 
 // multigrid3d._prolongate (multigrid3d.py:138-171).
@@ -916,7 +1132,7 @@ k_prolongate(const double* __restrict__ coarse, int cx, int cy, int cz,
   const uint32_t i = fdiv(ij, g.div_ny);
   const Lerp x = pl_axis((int)i, cx), y = pl_axis((int)(ij - i * g.div_ny.d), cy);
   const Lerp z = pl_axis((int)(t - ij * g.div_nz.d), cz);
-  out[t] = trilinear(coarse, cy, cz, x, y, z);
+  out[t] = trilinear<false>(coarse, cy, cz, x, y, z);
 }
 
 // multigrid3d._coarsen_fixed_any (multigrid3d.py:507-526).
@@ -1229,6 +1445,67 @@ bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const do
   // barriers
   const int nt = std::min<long>(kBottomCta, std::max<long>(64, ((long)(n + 1) / 2 + 31) / 32 * 32));
   k_bottom_err<<<1, nt, (bytes + 7) / 8 * 8, s>>>(e, fixed, f, g, rel_tol, omega, max_pairs);
+  counted();
+  return true;
+}
+
+TailLevel tail_level(Dims d, double* e, double* f, double* r, const uint8_t* fixed) {
+  TailLevel L;
+  L.e = e;
+  L.f = f;
+  L.r = r;
+  L.fixed = fixed;
+  L.nx = (int)d.nx;
+  L.ny = (int)d.ny;
+  L.nz = (int)d.nz;
+  L.dkk = FastDiv((uint32_t)((d.nz + 1) / 2));
+  L.dny = FastDiv((uint32_t)d.ny);
+  L.dnz = FastDiv((uint32_t)d.nz);
+  return L;
+}
+
+bool launch_err_tail(cudaStream_t s, const TailArgs& a) {
+  const TailLevel& b = a.lv[a.nlev - 1];
+  const size_t nb = (size_t)b.nx * b.ny * b.nz;
+  // the cluster size this device takes (16 CTAs, else the portable 8; 0:
+  // neither), found once
+  static std::once_flag once;
+  static int ctas = 0;
+  auto config = [](cudaLaunchConfig_t* c, cudaLaunchAttribute* at, int n, size_t smem,
+                   cudaStream_t st) {
+    *c = cudaLaunchConfig_t{};
+    c->gridDim = dim3(n);
+    c->blockDim = dim3(kTailThreads);
+    c->dynamicSmemBytes = smem;
+    c->stream = st;
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = n;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    c->attrs = at;
+    c->numAttrs = 1;
+  };
+  std::call_once(once, [&] {
+    const size_t most = 18 * (kBottomSmemMax / 17);
+    cudaFuncSetAttribute(k_err_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    cudaFuncSetAttribute(k_err_tail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (int n : {kTailCtas, 8}) {
+      cudaLaunchConfig_t c;
+      cudaLaunchAttribute at[1];
+      config(&c, at, n, most, nullptr);
+      int active = 0;
+      if (cudaOccupancyMaxActiveClusters(&active, k_err_tail, &c) == cudaSuccess && active > 0) {
+        ctas = n;
+        break;
+      }
+      cudaGetLastError();
+    }
+  });
+  if (!ctas || nb == 0 || 17 * nb > kBottomSmemMax) return false;
+  cudaLaunchConfig_t c;
+  cudaLaunchAttribute at[1];
+  config(&c, at, ctas, (18 * nb + 7) / 8 * 8, s);
+  if (cudaLaunchKernelEx(&c, k_err_tail, a) != cudaSuccess) return true;  // the caller reads the error
   counted();
   return true;
 }

@@ -24,7 +24,7 @@ inline Dims coarse_of(const Dims& d) {
 // m = floor(2^32 (2^s - d) / d) + 1, exact for every n < 2^31.
 struct FastDiv {
   uint32_t d, m, s;
-  FastDiv() : d(1), m(1), s(0) {}
+  __host__ __device__ FastDiv() : d(1), m(1), s(0) {}
   explicit FastDiv(uint32_t div) : d(div) {
     s = 0;
     while ((1ull << s) < div) ++s;
@@ -103,6 +103,25 @@ void launch_residual(cudaStream_t s, const double* phi, const uint8_t* fixed,
 constexpr size_t kBottomSmemMax = 200 * 1024;
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
                        Dims d, double rel_tol, double omega, long max_pairs);
+// multigrid3d._solve_err from level lv[0] (its right-hand side in f) down to
+// the bottom lv[nlev - 1] (nlev >= 2) in one launch (k_err_tail); false
+// (nothing launched) when the bottom does not fit in shared memory or the
+// device takes no such cluster.
+constexpr int kTailLevels = 12, kTailCtas = 16, kTailThreads = 512;
+struct TailLevel {
+  double *e, *f, *r;
+  const uint8_t* fixed;
+  int nx, ny, nz;
+  FastDiv dkk, dny, dnz;
+};
+struct TailArgs {
+  TailLevel lv[kTailLevels];
+  int nlev, nu1, nu2, max_cycles;
+  double rel_tol, bottom_omega;
+  long bottom_pairs;
+};
+TailLevel tail_level(Dims d, double* e, double* f, double* r, const uint8_t* fixed);
+bool launch_err_tail(cudaStream_t s, const TailArgs& a);
 void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,
                       const double* f, Dims d, double omega, int colour,
                       unsigned long long* dslot, PairCtl* ctl, int lp);

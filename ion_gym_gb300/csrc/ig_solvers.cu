@@ -375,11 +375,42 @@ void build_err_levels(ThreadCtx& c, VCycle& v, const uint8_t* fine_fixed,
   CK(cudaGetLastError());
 }
 
+// Nodes up to which a level and everything below it run in one launch
+// (k_err_tail, 16 SMs): above, the launched kernels' 152 SMs win.
+constexpr size_t kTailNodes = 65536;
+// max|f| up to which a level's error solve cannot overflow.  Beyond it (NaN
+// and infinities included) the cycles may run to their caps, which the host
+// should be driving.
+constexpr double kTailMaxF = 1e200;
+
+// Level L's error solve as one launch; false: not done.
+bool solve_err_tail(ThreadCtx& c, VCycle& v, size_t L, double fmax) {
+  if (v.lv[L].bottom || v.lv[L].d.n() > kTailNodes || v.lv.size() - L > (size_t)kTailLevels ||
+      v.nu2 < 1 || !(fmax < kTailMaxF))
+    return false;
+  TailArgs t;
+  t.nlev = (int)(v.lv.size() - L);
+  for (size_t q = L; q < v.lv.size(); q++)
+    t.lv[q - L] = tail_level(v.lv[q].d, v.lv[q].e.p, v.lv[q].f.p, v.lv[q].r.p, v.lv[q].fixed.p);
+  t.nu1 = v.nu1;
+  t.nu2 = v.nu2;
+  t.max_cycles = v.max_cycles_err;
+  t.rel_tol = v.rel_tol;
+  t.bottom_omega = v.bottom_omega;
+  t.bottom_pairs = 20000;
+  if (!launch_err_tail(c.s, t)) return false;
+  CK(cudaGetLastError());
+  return true;
+}
+
 // multigrid3d._solve_err (multigrid3d.py:553-599) on level L; the level's
 // right-hand side is already in lv[L].f, the solution lands in lv[L].e.
-void solve_err(ThreadCtx& c, VCycle& v, size_t L) {
+// above: max|f| of the level above (its corrections' right-hand sides stay
+// within a few powers of ten of it).
+void solve_err(ThreadCtx& c, VCycle& v, size_t L, double above) {
   ErrLevel& a = v.lv[L];
   const size_t n = a.d.n();
+  if (solve_err_tail(c, v, L, above)) return;
   if (a.bottom && launch_bottom_err(c.s, a.e.p, a.fixed.p, a.f.p, a.d, v.rel_tol,
                                     v.bottom_omega, 20000)) {
     CK(cudaGetLastError());
@@ -411,7 +442,7 @@ void solve_err(ThreadCtx& c, VCycle& v, size_t L) {
     }
     launch_residual_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, a.r.p);
     launch_restrict(c.s, a.r.p, a.d, b.f.p, b.d, 1);
-    solve_err(c, v, L + 1);
+    solve_err(c, v, L + 1, fmax);
     launch_prolong_add(c.s, b.e.p, b.d, a.e.p, a.fixed.p, a.d);
     if (v.nu2 > 0) {
       // the last pair's max |update| decides; the others' are not formed
@@ -499,7 +530,12 @@ VmgOut vmg_loop(ThreadCtx& c, FineGrid& g, VCycle& v, double tol,
       launch_residual(c.s, g.phi.p, g.fixed.p, g.th.p, rkind, g.d, r.p, nullptr);
     launch_restrict(c.s, r.p, g.d, e0.f.p, e0.d, 1);
     CK(cudaGetLastError());
-    solve_err(c, v, 0);
+    // a first level small enough for one launch is checked here; a larger
+    // one reads its own max|f|
+    const double f0 = !e0.bottom && e0.d.n() <= kTailNodes
+                          ? device_absmax(c, e0.f.p, nullptr, e0.d.n(), v.red)
+                          : std::numeric_limits<double>::infinity();
+    solve_err(c, v, 0, f0);
     launch_prolong_add(c.s, e0.e.p, e0.d, g.phi.p, g.fixed.p, g.d);
     for (int q = 0; q < v.nu2; q++) {
       for (int colour = 0; colour < 2; colour++)
