@@ -556,6 +556,167 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
   out[t] = r;
 }
 
+// ---- SOR to its tolerance in one launch ------------------------------------
+//
+// A grid of some 10^5 nodes is 1.4 us of FP64 work a half-sweep, and a
+// launch 7 us of latency around it (control block, mask, values, sum, block
+// maximum, each waiting for the one before; 43 us with theta's divisions on
+// the last block's chain).  Here one CTA per SM stays for the whole loop (a
+// cooperative launch, so that all of them are resident): a half-sweep ends
+// in a grid barrier, values pass through L2 (__ldcg / __stcg), and after a
+// pair every CTA reads all CTAs' maxima and takes the same decision, the
+// reference's per-pair test.  The node arithmetic is the launched sweeps'.
+//
+// A cut node of a theta plan goes to six lanes, one per leg (its division
+// or product), and the lanes add the six in the reference's order: the FP64
+// pipe takes a warp's instruction as long for two lanes as for 32, so six
+// legs side by side are a sixth of the divisions in line.
+//
+// What is left at 65^3 (one node a thread) is the chain: barrier 2.2 us
+// (arrival counter in L2, 152 pollers), load 0.5, sums and integer step 2.5
+// with 32 warps an SM, the pair's decision 0.6 every second half-sweep.
+// solve3d at 65^3 4.64 -> 2.80 ms, with theta (sw, 57 x 71 x 90) 7.6 -> 4.9.
+//
+// The barrier's wait is bounded (kCoopWait clocks, seconds): a CTA that
+// gives up raises *status and leaves, the others follow, and the call
+// reports an error.
+constexpr long long kCoopWait = 8000000000LL;
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+  unsigned v;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Every CTA of the grid; false when the wait was given up.
+__device__ __forceinline__ bool coop_barrier(CoopCtl* c, unsigned target, int* ok) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(&c->arrived, 1u);
+    const long long t0 = clock64();
+    int good = 1;
+    for (unsigned polls = 1; ld_acquire(&c->arrived) < target; polls++) {
+      if ((polls & 255u) == 0 &&
+          (clock64() - t0 > kCoopWait || *reinterpret_cast<volatile int*>(&c->status))) {
+        c->status = 1;
+        good = 0;
+        break;
+      }
+    }
+    *ok = good;
+  }
+  __syncthreads();
+  return *ok != 0;
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(kCoopThreads, 1)
+k_sor_coop(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, SweepGeom g,
+           FastDiv dnz, double omega, double tol, int pairs, CoopCtl* ctl) {
+  __shared__ unsigned long long red[33];
+  __shared__ int ok;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kCoopThreads / 32;
+  const uint32_t gn = gridDim.x * kCoopThreads, gt = blockIdx.x * kCoopThreads + threadIdx.x;
+  // cut nodes start at the last warp of every CTA, the plain ones' shortest
+  const uint32_t cw = (uint32_t)(nw - 1 - wid) * gridDim.x + blockIdx.x;
+  unsigned target = 0;
+  unsigned long long key = 0;
+  int pr = 0;
+  bool hit = false;
+  for (; pr < pairs && !hit; pr++) {
+    unsigned long long mb = 0;
+    for (int colour = 0; colour < 2; colour++) {
+      if (KIND != kPlain) {
+        const uint32_t first = colour ? P.count[0] : 0u, total = P.total();
+        for (uint32_t q = cw * 5u; q < P.count[colour]; q += gridDim.x * (uint32_t)nw * 5u) {
+          const int who = lane / 6, leg = lane - 6 * who;
+          const bool act = who < 5 && q + who < P.count[colour];
+          const uint32_t e = first + q + (act ? who : 0);
+          const uint32_t p = P.idx[e];
+          const uint32_t ij = fdiv(p, dnz);
+          const uint32_t i = fdiv(ij, g.div_ny);
+          const Nb n = neighbours(i, ij - i * g.div_ny.d, p - ij * dnz.d, (uint32_t)g.nx,
+                                  g.div_ny.d, dnz.d);
+          const uint32_t o = leg == 0 ? n.xm : leg == 1 ? n.xp : leg == 2 ? n.ym
+                             : leg == 3 ? n.yp : leg == 4 ? n.zm : n.zp;
+          const double v = __ldcg(phi + o), w = P.w[(size_t)leg * total + e];
+          const double old = __ldcg(phi + p), den = P.w[(size_t)6 * total + e];
+          const double term = KIND == kThetaGhost ? __dmul_rn(v, w) : __ddiv_rn(v, w);
+          const int l0 = lane < 30 ? 6 * who : 24;
+          double num = __shfl_sync(0xffffffffu, term, l0);
+#pragma unroll
+          for (int d = 1; d < 6; d++)
+            num = __dadd_rn(num, __shfl_sync(0xffffffffu, term, l0 + d));
+          unsigned long long k = 0;
+          const double nv = sor_apply<true, false>(old, __ddiv_rn(num, den), omega, &k);
+          if (act && leg == 0) {
+            __stcg(phi + p, nv);
+            if (k > mb) mb = k;
+          }
+        }
+      }
+      // two nodes at a time, so that their loads are in flight together
+      for (uint32_t t = gt; t < g.total; t += 2 * gn) {
+        uint32_t p[2];
+        bool go[2];
+        double S[2], old[2], v[2][6];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const SweepNodes<1> sn(g, t + u * gn, colour);
+          go[u] = t + u * gn < g.total && sn.valid(0) && cls[sn.at(0)] == 0;
+          if (!go[u]) continue;
+          p[u] = sn.at(0);
+          load6<true>(phi, sn.nb(0, p[u]), v[u]);
+          old[u] = __ldcg(phi + p[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          if (!go[u]) continue;
+          S[u] = sum6(v[u]);
+          double q;
+          if (KIND == kThetaSW && !sw_halves(S[u], v[u]))
+            q = __ddiv_rn(plain_sw_num(v[u]), 3.0);
+          else
+            q = div6(S[u]);
+          unsigned long long k = 0;
+          __stcg(phi + p[u], sor_apply<true, false>(old[u], q, omega, &k));
+          if (k > mb) mb = k;
+        }
+      }
+      if (colour == 0) {
+        target += gridDim.x;
+        if (!coop_barrier(ctl, target, &ok)) return;
+      }
+    }
+    // the pair's maximum: this CTA's into its slot, then everyone's
+    mb = warp_max_u64(mb);
+    if (lane == 0) red[wid] = mb;
+    __syncthreads();
+    if (wid == 0) {
+      mb = warp_max_u64(red[lane]);
+      if (lane == 0) __stcg(&ctl->slot[pr & 1][blockIdx.x], mb);
+    }
+    target += gridDim.x;
+    if (!coop_barrier(ctl, target, &ok)) return;
+    if (wid == 0) {
+      key = 0;
+      for (uint32_t b = lane; b < gridDim.x; b += 32)
+        key = max(key, __ldcg(&ctl->slot[pr & 1][b]));
+      key = warp_max_u64(key);
+      if (lane == 0) red[32] = key;
+    }
+    __syncthreads();
+    key = red[32];
+    hit = bits_to_double(key) < tol;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->pairs = pr;
+    ctl->hit = hit ? 1 : 0;
+    ctl->key = key;
+  }
+}
+
 // multigrid3d._sweep_rhs (multigrid3d.py:357-391).  ONE: omega is 1.
 template <bool CTL, bool DELTA, bool ONE, int U>
 __global__ void __launch_bounds__(kSweepThreads)
@@ -1446,6 +1607,39 @@ bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const do
   const int nt = std::min<long>(kBottomCta, std::max<long>(64, ((long)(n + 1) / 2 + 31) / 32 * 32));
   k_bottom_err<<<1, nt, (bytes + 7) / 8 * 8, s>>>(e, fixed, f, g, rel_tol, omega, max_pairs);
   counted();
+  return true;
+}
+
+bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const ThetaPlan* plan,
+                     int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl) {
+  // a whole grid of one CTA per SM, found once per device
+  static std::mutex mu;
+  static int sms[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  int n = 0;
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!sms[dev]) {
+      int coop = 0, count = 0;
+      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+      cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+      sms[dev] = coop && count > 0 ? std::min(count, kCoopCtas) : -1;
+    }
+    n = sms[dev];
+  }
+  if (n < 1) return false;
+  SweepGeom g = sweep_geom(d);
+  FastDiv dnz((uint32_t)d.nz);
+  ThetaPlan P = plan ? *plan : ThetaPlan();
+  if (cudaMemsetAsync(ctl, 0, sizeof(CoopCtl), s) != cudaSuccess) return true;
+  void* args[] = {&phi, &cls, &P, &g, &dnz, &omega, &tol, &pairs, &ctl};
+  const void* fn = kind == kThetaGhost ? (const void*)k_sor_coop<kThetaGhost>
+                   : kind == kThetaSW  ? (const void*)k_sor_coop<kThetaSW>
+                                       : (const void*)k_sor_coop<kPlain>;
+  // a failed launch leaves its error for the caller's check
+  if (cudaLaunchCooperativeKernel(fn, dim3(n), dim3(kCoopThreads), args, 0, s) == cudaSuccess)
+    counted();
   return true;
 }
 
