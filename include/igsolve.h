@@ -409,6 +409,14 @@ int ig_field_aware_dev(const void *phi, int dtype, long long phi_stride,
                        int n_channels, const uint8_t *metal, long nx, long ny,
                        long nz, double h, int h_is_f64, void *ex, void *ey,
                        void *ez, long long out_stride, void *stream);
+/* ig_field_aware_dev for float32 potentials with the float32 fields written
+ * widened to float64 (the composer's default channel type): the same values
+ * without a conversion pass.  Grids with nx ny nz + 2 ny nz below 2^31. */
+int ig_field_aware_wide_dev(const float *phi, long long phi_stride,
+                            int n_channels, const uint8_t *metal, long nx,
+                            long ny, long nz, double h, int h_is_f64,
+                            double *ex, double *ey, double *ez,
+                            long long out_stride, void *stream);
 int ig_field_aware_3d(const void *phi, int dtype, const uint8_t *metal,
                       long nx, long ny, long nz, double h, int h_is_f64,
                       void *ex, void *ey, void *ez);

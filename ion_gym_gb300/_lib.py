@@ -87,6 +87,8 @@ SIGNATURES = {
     "ig_superpose_dev": (_i, [_p, _i, _i, _p, _p, _ll, _p, _ll, _p]),
     "ig_field_aware_dev": (_i, [_p, _i, _ll, _i, _p, _l, _l, _l, _d, _i, _p,
                                 _p, _p, _ll, _p]),
+    "ig_field_aware_wide_dev": (_i, [_p, _ll, _i, _p, _l, _l, _l, _d, _i, _p,
+                                     _p, _p, _ll, _p]),
     "ig_field_aware_3d": (_i, [_p, _i, _p, _l, _l, _l, _d, _i, _p, _p, _p]),
     "ig_field_check_division": (_i, [_d, ctypes.c_ulonglong, ctypes.c_uint,
                                      _p]),

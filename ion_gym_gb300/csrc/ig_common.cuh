@@ -243,6 +243,23 @@ __device__ __forceinline__ void block_max_to(unsigned long long v,
   }
 }
 
+// float -> double by its bits for zeros and normal floats (exponent rebias,
+// significand moved up 29 bits); subnormals, infinities and NaN convert on
+// the FP64 pipe (a call, so that they alone pay for it).
+static __device__ __noinline__ double widen_slow(float d) { return (double)d; }
+__device__ __forceinline__ double widen(float d) {
+  const unsigned fb = __float_as_uint(d);
+  const unsigned ef = (fb >> 23) & 0xffu;
+  if (ef - 1u < 254u)
+    return __longlong_as_double(static_cast<long long>(
+        (static_cast<unsigned long long>(fb & 0x80000000u) << 32) |
+        (static_cast<unsigned long long>(ef + 896u) << 52) |
+        (static_cast<unsigned long long>(fb & 0x7fffffu) << 29)));
+  if ((fb & 0x7fffffffu) == 0u)
+    return __longlong_as_double(static_cast<long long>(static_cast<unsigned long long>(fb) << 32));
+  return widen_slow(d);
+}
+
 __host__ __device__ __forceinline__ double bits_to_double(unsigned long long b) {
 #ifdef __CUDA_ARCH__
   return __longlong_as_double(static_cast<long long>(b));

@@ -48,9 +48,9 @@ static_assert(sizeof(SupPlan) < 4000, "superposition plan must fit the kernel pa
 // Superposition.  Each thread keeps NCH float32 accumulators and reads
 // the bases B steps at a time (B = 8, fewer for wide float4 accumulators so
 // the registers suffice; the B loads are issued before any is used, so a
-// warp has B independent DRAM reads in flight).  k_superpose4 works on
-// float4 groups [0, n4) when every basis and output row is 16-byte aligned;
-// k_superpose1 on single nodes [first, n).
+// warp has B independent DRAM reads in flight).  VEC: n float4 groups, when
+// every basis and output row is 16-byte aligned, and the `tail` nodes after
+// them; else n single nodes.
 template <int NCH, typename V>
 __device__ __forceinline__ void sup_steps(V* acc, const SupPlan& plan, long long t);
 
@@ -70,10 +70,10 @@ __device__ __forceinline__ float4 sup_load4(const float* p, long long t) {
 
 template <int NCH, bool VEC>
 __global__ void __launch_bounds__(256)
-k_superpose(long long first, long long n, const SupPlan plan, float* __restrict__ out,
+k_superpose(long long n, int tail, const SupPlan plan, float* __restrict__ out,
             long long ostride) {
   using V = typename std::conditional<VEC, float4, float>::type;
-  for (long long t = first + (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
        t += (long long)gridDim.x * blockDim.x) {
     V acc[NCH];
 #pragma unroll
@@ -109,6 +109,16 @@ k_superpose(long long first, long long n, const SupPlan plan, float* __restrict_
     }
 #pragma unroll
     for (int c = 0; c < NCH; c++) reinterpret_cast<V*>(out + c * ostride)[t] = acc[c];
+  }
+  // the up to three nodes past the last float4 group
+  if (VEC && blockIdx.x == 0 && (int)threadIdx.x < tail) {
+    const long long t = 4 * n + threadIdx.x;
+    for (int c = 0; c < NCH; c++) {
+      float a = plan.accumulate ? out[c * ostride + t] : 0.f;
+      for (int s = 0; s < plan.nsteps; s++)
+        for (int m = 0; m < plan.mult[c][s]; m++) sup_add(a, plan.w[c][s], plan.src[s][t]);
+      out[c * ostride + t] = a;
+    }
   }
 }
 
@@ -248,20 +258,29 @@ __global__ void k_check_div64(Dh H, unsigned long long samples, unsigned seed,
 
 constexpr int kBX = 32, kBY = 8, kPlanes = 8;
 
+// A float32 field value as the output holds it: itself, or widened to
+// float64 (on the integer pipe but for subnormals and the like).
+template <typename O>
+__device__ __forceinline__ O field_out(float v);
+template <>
+__device__ __forceinline__ float field_out<float>(float v) { return v; }
+template <>
+__device__ __forceinline__ double field_out<double>(float v) { return widen(v); }
+
 // tracer3d._fa3d_correct at one metal node (o = (i, j, k)) for NC
 // channels, after the plain gradient was stored there: along each axis with
 // vacuum on exactly one side, the field becomes minus the one-sided
 // difference into the vacuum divided (float64) by h.
-template <int NC>
+template <int NC, typename O>
 __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long long pstride,
                                           const uint8_t* __restrict__ metal, int o, int i, int j,
                                           int k, int nx, int ny, int nz, const Dh& e1,
-                                          float* ex, float* ey, float* ez, long long ostride) {
+                                          O* ex, O* ey, O* ez, long long ostride) {
   const int sx = ny * nz, sy = nz;
   const int step[3] = {sx, sy, 1};
   const bool lo[3] = {i > 0, j > 0, k > 0};
   const bool hi[3] = {i + 1 < nx, j + 1 < ny, k + 1 < nz};
-  float* out[3] = {ex, ey, ez};
+  O* out[3] = {ex, ey, ez};
 #pragma unroll
   for (int a = 0; a < 3; a++) {
     const bool vp = hi[a] && !metal[o + step[a]];
@@ -276,7 +295,8 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
       v[c] = phi[c * pstride + dn];
     }
 #pragma unroll
-    for (int c = 0; c < NC; c++) out[a][c * ostride + o] = -div64(__fsub_rn(u[c], v[c]), e1);
+    for (int c = 0; c < NC; c++)
+      out[a][c * ostride + o] = field_out<O>(-div64(__fsub_rn(u[c], v[c]), e1));
   }
 }
 
@@ -290,11 +310,14 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
 // metal_fix to the queue, so a lone metal lane (a box face across the
 // contiguous axis) does not hold its warp.  In-channel offsets are 32-bit
 // (the host checks nx*ny*nz + 2*ny*nz < 2^31).
-template <int NC, bool F64DIV>
+// O = double writes the float32 fields widened, for callers that want
+// float64 channels: a conversion of its own reads and writes the fields once
+// more (@@F64@@).
+template <int NC, bool F64DIV, typename O>
 __global__ void __launch_bounds__(kBX * kBY)
 k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __restrict__ metal,
-          int nx, int ny, int nz, Spacing sp, int nchunks, float* __restrict__ ex,
-          float* __restrict__ ey, float* __restrict__ ez, long long ostride) {
+          int nx, int ny, int nz, Spacing sp, int nchunks, O* __restrict__ ex,
+          O* __restrict__ ey, O* __restrict__ ez, long long ostride) {
   __shared__ unsigned short queue[kBX * kBY * kPlanes];
   __shared__ int queued;
   const int k = blockIdx.x * kBX + threadIdx.x;
@@ -346,9 +369,9 @@ k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __res
         const float dy = grad_div_t<F64DIV>(__fsub_rn(yb[c], ya[c]), ycen, sp);
         const float dz = grad_div_t<F64DIV>(__fsub_rn(zb[c], za[c]), zcen, sp);
         const long long w = ob + c * ostride + o;
-        __stcs(ex + w, -dx);
-        __stcs(ey + w, -dy);
-        __stcs(ez + w, -dz);
+        __stcs(ex + w, field_out<O>(-dx));
+        __stcs(ey + w, field_out<O>(-dy));
+        __stcs(ez + w, field_out<O>(-dz));
         vm[c] = vc[c];
         vc[c] = vp[c];
       }
@@ -474,11 +497,9 @@ void launch_sup(bool vec, long long n, const SupPlan& p, float* out, long long o
                 cudaStream_t st) {
   const unsigned grid = 152u * 32u;   // 32 resident-capable blocks per SM, grid-stride
   if (vec) {
-    const long long n4 = n / 4;
-    if (n4 > 0) k_superpose<NCH, true><<<grid, 256, 0, st>>>(0, n4, p, out, ostride);
-    if (n4 * 4 < n) k_superpose<NCH, false><<<1, 256, 0, st>>>(n4 * 4, n, p, out, ostride);
+    k_superpose<NCH, true><<<grid, 256, 0, st>>>(n / 4, (int)(n % 4), p, out, ostride);
   } else {
-    k_superpose<NCH, false><<<grid, 256, 0, st>>>(0, n, p, out, ostride);
+    k_superpose<NCH, false><<<grid, 256, 0, st>>>(n, 0, p, out, ostride);
   }
 }
 
@@ -518,7 +539,7 @@ int superpose(const float* const* src, int n_steps, int n_channels, const float*
         case 7: launch_sup<7>(vec, n, p, o, ostride, st); break;
         default: launch_sup<8>(vec, n, p, o, ostride, st); break;
       }
-      launches += (vec && n % 4 != 0 && n >= 4) ? 2 : 1;
+      launches++;
       if (n_steps <= 0) break;
     }
   }
@@ -585,29 +606,73 @@ Spacing make_spacing(double h, int h_is_f64) {
   return s;
 }
 
-template <bool F64DIV>
+template <bool F64DIV, typename O>
 void launch_field32(int nc, dim3 grid, dim3 block, cudaStream_t st, const float* P,
                     long long pstride, const uint8_t* metal, int nx, int ny, int nz,
-                    const Spacing& sp, int nchunks, float* X, float* Y, float* Z,
-                    long long ostride) {
+                    const Spacing& sp, int nchunks, O* X, O* Y, O* Z, long long ostride) {
+#define IG_FIELD(NC)                                                                          \
+  k_field32<NC, F64DIV, O><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks, \
+                                                   X, Y, Z, ostride)
   switch (nc) {
-    case 4:
-      k_field32<4, F64DIV><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks,
-                                                   X, Y, Z, ostride);
-      break;
-    case 3:
-      k_field32<3, F64DIV><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks,
-                                                   X, Y, Z, ostride);
-      break;
-    case 2:
-      k_field32<2, F64DIV><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks,
-                                                   X, Y, Z, ostride);
-      break;
-    default:
-      k_field32<1, F64DIV><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks,
-                                                   X, Y, Z, ostride);
-      break;
+    case 4: IG_FIELD(4); break;
+    case 3: IG_FIELD(3); break;
+    case 2: IG_FIELD(2); break;
+    default: IG_FIELD(1); break;
   }
+#undef IG_FIELD
+}
+
+// float32 potentials of fewer than 2^31 nodes, fields of type O.
+template <typename O>
+int field32(const float* P, long long pstride, int nch, const uint8_t* metal, long nx, long ny,
+            long nz, const Spacing& sp, O* X, O* Y, O* Z, long long ostride, cudaStream_t st,
+            long* launches) {
+  const int nchunks = (int)((nx + kPlanes - 1) / kPlanes);
+  for (int c0 = 0; c0 < nch;) {
+    const int left = nch - c0;
+    const int nc = left >= 4 ? 4 : left;
+    const int groups = nc == 4 ? left / 4 : 1;
+    const long long gz = (long long)nchunks * groups;
+    if (gz > 65535) {
+      set_last_error("field: channels x ceil(nx/8) exceeds one launch (65535)");
+      return IG_BAD_ARG;
+    }
+    const dim3 grid((unsigned)((nz + kBX - 1) / kBX), (unsigned)((ny + kBY - 1) / kBY),
+                    (unsigned)gz);
+    const float* Pc = P + (long long)c0 * pstride;
+    const long long oc = (long long)c0 * ostride;
+    if (sp.f64div)
+      launch_field32<true, O>(nc, grid, dim3(kBX, kBY), st, Pc, pstride, metal, (int)nx, (int)ny,
+                              (int)nz, sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
+    else
+      launch_field32<false, O>(nc, grid, dim3(kBX, kBY), st, Pc, pstride, metal, (int)nx,
+                               (int)ny, (int)nz, sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
+    (*launches)++;
+    c0 += nc * groups;
+  }
+  return IG_OK;
+}
+
+int field_launched(long launches) {
+  note_launches(launches);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    set_last_error(std::string("field launch: ") + cudaGetErrorString(e));
+    return IG_CUDA_ERROR;
+  }
+  return IG_OK;
+}
+
+bool field32_fits(long nx, long ny, long nz) {
+  return (long long)nx * ny * nz + 2LL * ny * nz < (1LL << 31);
+}
+
+int check_rows(long ny) {
+  if ((ny + kBY - 1) / kBY > 65535) {
+    set_last_error("field: grid too large for one launch (ceil(ny/8) must be <= 65535)");
+    return IG_BAD_ARG;
+  }
+  return IG_OK;
 }
 
 int field(const void* phi, int dtype, long long pstride, int nch, const uint8_t* metal,
@@ -615,40 +680,13 @@ int field(const void* phi, int dtype, long long pstride, int nch, const uint8_t*
           long long ostride, cudaStream_t st) {
   const Spacing sp = make_spacing(h, h_is_f64);
   const dim3 block(kBX, kBY);
-  const long long n = (long long)nx * ny * nz;
   long launches = 0;
-  if ((ny + kBY - 1) / kBY > 65535) {
-    set_last_error("field: grid too large for one launch (ceil(ny/8) must be <= 65535)");
-    return IG_BAD_ARG;
-  }
-  if (dtype == 0 && n + 2LL * ny * nz < (1LL << 31)) {
-    const int nchunks = (int)((nx + kPlanes - 1) / kPlanes);
-    const float* P = static_cast<const float*>(phi);
-    float* X = static_cast<float*>(ex);
-    float* Y = static_cast<float*>(ey);
-    float* Z = static_cast<float*>(ez);
-    for (int c0 = 0; c0 < nch;) {
-      const int left = nch - c0;
-      const int nc = left >= 4 ? 4 : left;
-      const int groups = nc == 4 ? left / 4 : 1;
-      const long long gz = (long long)nchunks * groups;
-      if (gz > 65535) {
-        set_last_error("field: channels x ceil(nx/8) exceeds one launch (65535)");
-        return IG_BAD_ARG;
-      }
-      const dim3 grid((unsigned)((nz + kBX - 1) / kBX), (unsigned)((ny + kBY - 1) / kBY),
-                      (unsigned)gz);
-      const float* Pc = P + (long long)c0 * pstride;
-      const long long oc = (long long)c0 * ostride;
-      if (sp.f64div)
-        launch_field32<true>(nc, grid, block, st, Pc, pstride, metal, (int)nx, (int)ny, (int)nz,
-                             sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
-      else
-        launch_field32<false>(nc, grid, block, st, Pc, pstride, metal, (int)nx, (int)ny,
-                              (int)nz, sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
-      launches++;
-      c0 += nc * groups;
-    }
+  if (int e = check_rows(ny)) return e;
+  if (dtype == 0 && field32_fits(nx, ny, nz)) {
+    if (int e = field32(static_cast<const float*>(phi), pstride, nch, metal, nx, ny, nz, sp,
+                        static_cast<float*>(ex), static_cast<float*>(ey),
+                        static_cast<float*>(ez), ostride, st, &launches))
+      return e;
   } else {
     const int nchunks = (int)((nx + kIChunk - 1) / kIChunk);
     const long long gz = (long long)nchunks * nch;
@@ -668,13 +706,7 @@ int field(const void* phi, int dtype, long long pstride, int nch, const uint8_t*
           static_cast<double*>(ex), static_cast<double*>(ey), static_cast<double*>(ez), ostride);
     launches++;
   }
-  note_launches(launches);
-  const cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_last_error(std::string("field launch: ") + cudaGetErrorString(e));
-    return IG_CUDA_ERROR;
-  }
-  return IG_OK;
+  return field_launched(launches);
 }
 
 int check_field_args(int dtype, int nch, long nx, long ny, long nz, double h) {
@@ -792,6 +824,31 @@ extern "C" int ig_field_aware_dev(const void* phi, int dtype, long long phi_stri
   }
   return field(phi, dtype, phi_stride, n_channels, metal, nx, ny, nz, h, h_is_f64, ex, ey, ez,
                out_stride, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int ig_field_aware_wide_dev(const float* phi, long long phi_stride, int n_channels,
+                                       const uint8_t* metal, long nx, long ny, long nz,
+                                       double h, int h_is_f64, double* ex, double* ey,
+                                       double* ez, long long out_stride, void* stream) {
+  set_last_error("");
+  if (int st = check_field_args(0, n_channels, nx, ny, nz, h)) return st;
+  const long long n = (long long)nx * ny * nz;
+  if (!phi || !ex || !ey || !ez || (n_channels > 1 && (phi_stride < n || out_stride < n))) {
+    set_last_error("field: invalid buffers or strides");
+    return IG_BAD_ARG;
+  }
+  if (!field32_fits(nx, ny, nz)) {
+    set_last_error("field: grid too large for float64 fields of float32 potentials "
+                   "(nx ny nz + 2 ny nz must be below 2^31)");
+    return IG_BAD_ARG;
+  }
+  if (int st = check_rows(ny)) return st;
+  long launches = 0;
+  if (int st = field32(phi, phi_stride, n_channels, metal, nx, ny, nz,
+                       make_spacing(h, h_is_f64), ex, ey, ez, out_stride,
+                       static_cast<cudaStream_t>(stream), &launches))
+    return st;
+  return field_launched(launches);
 }
 
 extern "C" int ig_field_aware_3d(const void* phi, int dtype, const uint8_t* metal, long nx,

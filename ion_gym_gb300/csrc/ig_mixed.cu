@@ -1481,22 +1481,6 @@ inline unsigned flat_blocks(const SGeo& G, uint32_t R) {
   return (unsigned)((warps + kRowWarps - 1) / kRowWarps);
 }
 
-// float -> double by its bits for zeros and normal floats (exponent rebias,
-// significand moved up 29 bits); subnormals, infinities and NaN convert on
-// the FP64 pipe.
-__device__ __forceinline__ double widen(float d) {
-  const unsigned fb = __float_as_uint(d);
-  const unsigned ef = (fb >> 23) & 0xffu;
-  if ((fb & 0x7fffffffu) == 0u)
-    return __longlong_as_double(static_cast<long long>(static_cast<unsigned long long>(fb) << 32));
-  if (ef - 1u < 254u)
-    return __longlong_as_double(static_cast<long long>(
-        (static_cast<unsigned long long>(fb & 0x80000000u) << 32) |
-        (static_cast<unsigned long long>(ef + 896u) << 52) |
-        (static_cast<unsigned long long>(fb & 0x7fffffu) << 29)));
-  return (double)d;
-}
-
 // Phi += e32 / u_b (rounded to the nearest unit) at free nodes; the
 // per-problem maximum of |e32| (the applied change, to within half a unit)
 // goes to dmax[b] as float64 bits (the refinement's convergence norm, the

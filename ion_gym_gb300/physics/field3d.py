@@ -79,7 +79,7 @@ def _metal_u8(ele):
     """uint8 0/1 of the label grid's truth value (``not ele[...]`` is the
     vacuum test of the reference's metal pass)."""
     if _is_tensor(ele):
-        return (ele != 0).to(_torch().uint8).contiguous()
+        return (ele != 0).contiguous().view(_torch().uint8)
     return np.ascontiguousarray(np.asarray(ele) != 0).view(np.uint8)
 
 
@@ -105,6 +105,11 @@ def build_field_aware_3d(phi, ele, h_mm, electrode_aware=True):
     return tuple(out)
 
 
+# Nodes (plus two planes) below which the device fields' offsets fit 32 bits
+# and float32 potentials can have float64 fields written directly.
+_WIDE_LIMIT = 1 << 31
+
+
 def _field_device(phi, ele, h_mm, electrode_aware, out=None):
     torch = _torch()
     if phi.dim() == 3:
@@ -127,10 +132,12 @@ def _field_device(phi, ele, h_mm, electrode_aware, out=None):
     n = nx * ny * nz
     pstride = phi.stride(0) if nch > 1 else n
     ostride = out.stride(1) if nch > 1 else n
-    st = _lib.lib().ig_field_aware_dev(
-        _p(phi), code, pstride, nch, _p(metal), nx, ny, nz, float(h_mm),
-        int(_h_is_f64(h_mm)), _p(out[0]), _p(out[1]), _p(out[2]), ostride,
-        _stream())
+    rest = (nch, _p(metal), nx, ny, nz, float(h_mm), int(_h_is_f64(h_mm)),
+            _p(out[0]), _p(out[1]), _p(out[2]), ostride, _stream())
+    if code == 0 and out.dtype == torch.float64:
+        st = _lib.lib().ig_field_aware_wide_dev(_p(phi), pstride, *rest)
+    else:
+        st = _lib.lib().ig_field_aware_dev(_p(phi), code, pstride, *rest)
     _lib.check(st, "build_field_aware_3d")
     if nch == 1:
         return out[0, 0], out[1, 0], out[2, 0]
@@ -350,13 +357,16 @@ def compose_drive_channels(spec, bases, ele, verbose=False):
     P = superpose_device(src, plan["rows"], plan["weights"], plan["mult"],
                          shape=shape)
     del src
-    E = torch.empty((3, nch) + shape, dtype=torch.float32, device=dev)
+    n = int(np.prod(shape))
+    wide = not f32_out and n + 2 * shape[1] * shape[2] < _WIDE_LIMIT
+    E = torch.empty((3, nch) + shape, dtype=torch.float64 if wide else torch.float32,
+                    device=dev)
     _field_device(P, ele if eaware else None, h, eaware, out=E)
     if verbose:
         print(f"[compose] {nch} channel(s) composed on the GPU", flush=True)
     if not resident:
         torch.cuda.current_stream().synchronize()
-    conv = (lambda t: t) if f32_out else (lambda t: t.to(torch.float64))
+    conv = (lambda t: t) if f32_out or wide else (lambda t: t.to(torch.float64))
     host = (lambda t: t.cpu().numpy()) if not resident else (lambda t: t)
     K = nch - 1
     out = dict(
