@@ -175,4 +175,44 @@ void note_launches(long n);
 // Sets the calling thread's ig_last_error() message.
 void set_last_error(const std::string& m);
 
+// The calling thread's stream on its current device (created on first use);
+// a status, with the message set, when there is none.
+int call_stream(cudaStream_t* s);
+
+// Waits for the stream when a call leaves, early returns included: copies
+// from pageable memory may still be reading the caller's (or the call's own)
+// arrays.  Declared after them and after the call's CallBufs.
+struct CallSync {
+  cudaStream_t s;
+  ~CallSync() { cudaStreamSynchronize(s); }
+};
+
+// A device buffer of one synchronous call on host arrays.  Small ones come
+// from the device's stream-ordered pool, which keeps them for the next call
+// (cudaMalloc and cudaFree cost more than the work of a small grid: three
+// buffers 200 us); above kPoolBytes, where that no longer shows, the memory
+// goes back to the device at once.
+constexpr size_t kPoolBytes = size_t(64) << 20;
+struct CallBuf {
+  void* p = nullptr;
+  cudaStream_t s = nullptr;
+  bool pooled = false;
+  cudaError_t alloc(size_t bytes, cudaStream_t st) {
+    s = st;
+    pooled = bytes <= kPoolBytes;
+    return pooled ? cudaMallocAsync(&p, bytes ? bytes : 16, st) : cudaMalloc(&p, bytes);
+  }
+  CallBuf() = default;
+  CallBuf(const CallBuf&) = delete;
+  CallBuf& operator=(const CallBuf&) = delete;
+  ~CallBuf() {
+    if (!p) return;
+    if (pooled) {
+      cudaFreeAsync(p, s);
+    } else {
+      cudaFree(p);
+    }
+  }
+};
+
 }  // namespace ig

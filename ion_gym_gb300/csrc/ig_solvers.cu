@@ -698,6 +698,13 @@ using namespace ig;
 
 void ig::set_last_error(const std::string& m) { t_err = m; }
 
+int ig::call_stream(cudaStream_t* s) {
+  return guard([&] {
+    *s = ctx().s;
+    return (int)IG_OK;
+  });
+}
+
 extern "C" {
 
 const char* ig_last_error(void) { return t_err.c_str(); }
