@@ -199,11 +199,35 @@ __device__ __forceinline__ float div64(float d, const Dh& H) {
   return div64_slow(d, H.h);
 }
 
+// Dd: RN64(d / c) for a float64 divisor c fixed per launch, as Dv in float64
+// (y = RN64(1/c)): 5 fused multiply-adds in place of a division on a pipe of
+// 2 lanes per clock and SM.  Inputs outside [2^-900, 2^900], divisors outside
+// [2^-100, 2^100], infinities and NaN take the division itself; +-0 / c is
+// +-0 y.
+struct Dd {
+  double c, y;
+  int ok;
+};
+
+__device__ __noinline__ double ddiv_slow(double d, double c) { return __ddiv_rn(d, c); }
+
+__device__ __forceinline__ double ddiv(double d, const Dd& D) {
+  const unsigned eb =
+      static_cast<unsigned>(static_cast<unsigned long long>(__double_as_longlong(d)) >> 52) &
+      0x7ffu;
+  const bool zero = (__double_as_longlong(d) << 1) == 0;
+  if (!D.ok || (eb - 123u > 1800u && !zero)) return ddiv_slow(d, D.c);
+  const double q0 = __dmul_rn(d, D.y);
+  if (zero) return q0;
+  const double q1 = __fma_rn(__fma_rn(-q0, D.c, d), D.y, q0);
+  return __fma_rn(__fma_rn(-q1, D.c, d), D.y, q1);
+}
+
 // Spacing of one launch: the float32 divisors RN32(2h), RN32(h) (a Python
 // float spacing), the float64 divisors 2h, h (a numpy float64 spacing) and
 // the float64 h of the metal rule.
 struct Spacing {
-  double h2, h1;
+  Dd h2, h1;
   Dv d2, d1;
   Dh e2, e1;
   int f64div;
@@ -256,7 +280,18 @@ __global__ void k_check_div64(Dh H, unsigned long long samples, unsigned seed,
   if (local) atomicAdd(bad, local);
 }
 
-constexpr int kBX = 32, kBY = 8, kPlanes = 8;
+// kPlanes, kIChunk: the most x-planes a thread marches.  A march reuses its
+// planes from registers, but its planes come one after the other: grids whose
+// (y, z) tiles are few get shorter ones, down to one plane, until about
+// four blocks an SM are there.  float64 at 33^3, 16 planes
+// and divisions: 96 us; 2 planes 20 us; and the multiply-adds of ddiv 10 us.
+constexpr int kBX = 32, kBY = 8, kPlanes = 8, kIChunk = 16;
+inline int march_planes(long nx, long ny, long nz, long channels, int most) {
+  const long tiles = (ny + kBY - 1) / kBY * ((nz + kBX - 1) / kBX) * channels;
+  const long want = (4 * 152 + tiles - 1) / tiles;  // chunks along x
+  const long p = nx / (want > 0 ? want : 1);
+  return (int)(p < 1 ? 1 : (p > most ? most : p));
+}
 
 // A float32 field value as the output holds it: itself, or widened to
 // float64 (on the integer pipe but for subnormals and the like).
@@ -301,7 +336,7 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
 }
 
 // E = -grad(phi) for float32 potentials, NC channels per thread.  Thread
-// (j, k) marches over kPlanes x-planes of the chunk blockIdx.z % nchunks
+// (j, k) marches over `planes` x-planes of the chunk blockIdx.z % nchunks
 // for channels [NC*g, NC*g + NC), g = blockIdx.z / nchunks, with the
 // x-neighbours in registers; the y/z neighbours come through L1 from the
 // block's own loads.  Every node gets numpy.gradient's value.  Metal nodes
@@ -312,19 +347,19 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
 // (the host checks nx*ny*nz + 2*ny*nz < 2^31).
 // O = double writes the float32 fields widened, for callers that want
 // float64 channels: a conversion of its own reads and writes the fields once
-// more (@@F64@@).
+// more (193 x 193 x 385, 4 channels: 245 + 670 us of conversions -> 355 us).
 template <int NC, bool F64DIV, typename O>
 __global__ void __launch_bounds__(kBX * kBY)
 k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __restrict__ metal,
-          int nx, int ny, int nz, Spacing sp, int nchunks, O* __restrict__ ex,
+          int nx, int ny, int nz, Spacing sp, int nchunks, int planes, O* __restrict__ ex,
           O* __restrict__ ey, O* __restrict__ ez, long long ostride) {
   __shared__ unsigned short queue[kBX * kBY * kPlanes];
   __shared__ int queued;
   const int k = blockIdx.x * kBX + threadIdx.x;
   const int j = blockIdx.y * kBY + threadIdx.y;
   const int g = blockIdx.z / nchunks;
-  const int i0 = (blockIdx.z % nchunks) * kPlanes;
-  const int i1 = min(i0 + kPlanes, nx);
+  const int i0 = (blockIdx.z % nchunks) * planes;
+  const int i1 = min(i0 + planes, nx);
   if (threadIdx.x == 0 && threadIdx.y == 0) queued = 0;
   __syncthreads();
   const int sx = ny * nz, sy = nz;
@@ -392,10 +427,10 @@ k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __res
 // E = -grad(phi) for float64 potentials (and for float32 grids of 2^31
 // nodes or more): one channel per blockIdx.z / nchunks, 64-bit offsets.
 __device__ __forceinline__ double d64_central(double a, double b, const Spacing& s) {
-  return __ddiv_rn(__dsub_rn(a, b), s.h2);
+  return ddiv(__dsub_rn(a, b), s.h2);
 }
 __device__ __forceinline__ double d64_edge(double a, double b, const Spacing& s) {
-  return __ddiv_rn(__dsub_rn(a, b), s.h1);
+  return ddiv(__dsub_rn(a, b), s.h1);
 }
 __device__ __forceinline__ float d32_central(float a, float b, const Spacing& s) {
   return grad_div(__fsub_rn(a, b), true, s);
@@ -404,7 +439,7 @@ __device__ __forceinline__ float d32_edge(float a, float b, const Spacing& s) {
   return grad_div(__fsub_rn(a, b), false, s);
 }
 __device__ __forceinline__ double onesided(double a, double b, const Spacing& s) {
-  return __ddiv_rn(__dsub_rn(a, b), s.h1);
+  return ddiv(__dsub_rn(a, b), s.h1);
 }
 __device__ __forceinline__ float onesided(float a, float b, const Spacing& s) {
   return div64(__fsub_rn(a, b), s.e1);
@@ -441,19 +476,17 @@ __device__ __forceinline__ T axis_deriv(T vm, T vc, T vp, long q, long n, const 
   return d;
 }
 
-constexpr int kIChunk = 16;
-
 template <typename T>
 __global__ void __launch_bounds__(kBX * kBY)
 k_field(const T* __restrict__ phi, long long pstride, const uint8_t* __restrict__ metal,
-        long nx, long ny, long nz, Spacing sp, int nchunks, T* __restrict__ ex,
+        long nx, long ny, long nz, Spacing sp, int nchunks, int planes, T* __restrict__ ex,
         T* __restrict__ ey, T* __restrict__ ez, long long ostride) {
   const long k = (long)blockIdx.x * kBX + threadIdx.x;
   const long j = (long)blockIdx.y * kBY + threadIdx.y;
   const int ch = blockIdx.z / nchunks;
-  const long i0 = (long)(blockIdx.z % nchunks) * kIChunk;
+  const long i0 = (long)(blockIdx.z % nchunks) * planes;
   if (k >= nz || j >= ny || i0 >= nx) return;
-  const long i1 = i0 + kIChunk < nx ? i0 + kIChunk : nx;
+  const long i1 = i0 + planes < nx ? i0 + planes : nx;
   const T* p = phi + ch * pstride;
   T* oxp = ex + ch * ostride;
   T* oyp = ey + ch * ostride;
@@ -596,8 +629,12 @@ Dh make_dh(double h) {
 
 Spacing make_spacing(double h, int h_is_f64) {
   Spacing s;
-  s.h2 = 2.0 * h;
-  s.h1 = h;
+  auto dd = [](double c) {
+    const double a = std::fabs(c);
+    return Dd{c, 1.0 / c, a >= 0x1p-100 && a <= 0x1p100 ? 1 : 0};
+  };
+  s.h2 = dd(2.0 * h);
+  s.h1 = dd(h);
   s.d2 = make_dv((float)(2.0 * h));
   s.d1 = make_dv((float)h);
   s.e2 = make_dh(2.0 * h);
@@ -609,10 +646,10 @@ Spacing make_spacing(double h, int h_is_f64) {
 template <bool F64DIV, typename O>
 void launch_field32(int nc, dim3 grid, dim3 block, cudaStream_t st, const float* P,
                     long long pstride, const uint8_t* metal, int nx, int ny, int nz,
-                    const Spacing& sp, int nchunks, O* X, O* Y, O* Z, long long ostride) {
+                    const Spacing& sp, int nchunks, int planes, O* X, O* Y, O* Z, long long ostride) {
 #define IG_FIELD(NC)                                                                          \
   k_field32<NC, F64DIV, O><<<grid, block, 0, st>>>(P, pstride, metal, nx, ny, nz, sp, nchunks, \
-                                                   X, Y, Z, ostride)
+                                                   planes, X, Y, Z, ostride)
   switch (nc) {
     case 4: IG_FIELD(4); break;
     case 3: IG_FIELD(3); break;
@@ -627,7 +664,8 @@ template <typename O>
 int field32(const float* P, long long pstride, int nch, const uint8_t* metal, long nx, long ny,
             long nz, const Spacing& sp, O* X, O* Y, O* Z, long long ostride, cudaStream_t st,
             long* launches) {
-  const int nchunks = (int)((nx + kPlanes - 1) / kPlanes);
+  const int planes = march_planes(nx, ny, nz, (nch + 3) / 4, kPlanes);
+  const int nchunks = (int)((nx + planes - 1) / planes);
   for (int c0 = 0; c0 < nch;) {
     const int left = nch - c0;
     const int nc = left >= 4 ? 4 : left;
@@ -643,10 +681,10 @@ int field32(const float* P, long long pstride, int nch, const uint8_t* metal, lo
     const long long oc = (long long)c0 * ostride;
     if (sp.f64div)
       launch_field32<true, O>(nc, grid, dim3(kBX, kBY), st, Pc, pstride, metal, (int)nx, (int)ny,
-                              (int)nz, sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
+                              (int)nz, sp, nchunks, planes, X + oc, Y + oc, Z + oc, ostride);
     else
       launch_field32<false, O>(nc, grid, dim3(kBX, kBY), st, Pc, pstride, metal, (int)nx,
-                               (int)ny, (int)nz, sp, nchunks, X + oc, Y + oc, Z + oc, ostride);
+                               (int)ny, (int)nz, sp, nchunks, planes, X + oc, Y + oc, Z + oc, ostride);
     (*launches)++;
     c0 += nc * groups;
   }
@@ -688,7 +726,8 @@ int field(const void* phi, int dtype, long long pstride, int nch, const uint8_t*
                         static_cast<float*>(ez), ostride, st, &launches))
       return e;
   } else {
-    const int nchunks = (int)((nx + kIChunk - 1) / kIChunk);
+    const int planes = march_planes(nx, ny, nz, nch, kIChunk);
+    const int nchunks = (int)((nx + planes - 1) / planes);
     const long long gz = (long long)nchunks * nch;
     if (gz > 65535) {
       set_last_error("field: channels x ceil(nx/16) exceeds one launch (65535)");
@@ -698,11 +737,11 @@ int field(const void* phi, int dtype, long long pstride, int nch, const uint8_t*
                     (unsigned)gz);
     if (dtype == 0)
       k_field<float><<<grid, block, 0, st>>>(
-          static_cast<const float*>(phi), pstride, metal, nx, ny, nz, sp, nchunks,
+          static_cast<const float*>(phi), pstride, metal, nx, ny, nz, sp, nchunks, planes,
           static_cast<float*>(ex), static_cast<float*>(ey), static_cast<float*>(ez), ostride);
     else
       k_field<double><<<grid, block, 0, st>>>(
-          static_cast<const double*>(phi), pstride, metal, nx, ny, nz, sp, nchunks,
+          static_cast<const double*>(phi), pstride, metal, nx, ny, nz, sp, nchunks, planes,
           static_cast<double*>(ex), static_cast<double*>(ey), static_cast<double*>(ez), ostride);
     launches++;
   }
@@ -740,23 +779,6 @@ int check_plan(int n_steps, const int* rows, int n_channels, const uint8_t* mult
       set_last_error("superposition: basis row out of range");
       return IG_BAD_ARG;
     }
-  return IG_OK;
-}
-
-struct Tmp {
-  void* p = nullptr;
-  ~Tmp() {
-    if (p) cudaFree(p);
-  }
-};
-
-int no_device() {
-  int ndev = 0;
-  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
-    cudaGetLastError();
-    set_last_error("no CUDA device is visible");
-    return IG_NO_DEVICE;
-  }
   return IG_OK;
 }
 
@@ -860,23 +882,26 @@ extern "C" int ig_field_aware_3d(const void* phi, int dtype, const uint8_t* meta
     set_last_error("field: null buffer");
     return IG_BAD_ARG;
   }
-  if (int st = no_device()) return st;
+  cudaStream_t s = nullptr;
+  if (int st = call_stream(&s)) return st;
   const size_t n = (size_t)nx * ny * nz, es = dtype ? 8 : 4;
-  Tmp dp, dm, dout;
-  GF(cudaMalloc(&dp.p, n * es));
-  GF(cudaMemcpy(dp.p, phi, n * es, cudaMemcpyHostToDevice));
+  CallBuf dp, dm, dout;
+  const CallSync sync{s};
+  GF(dp.alloc(n * es, s));
+  GF(cudaMemcpyAsync(dp.p, phi, n * es, cudaMemcpyHostToDevice, s));
   if (metal) {
-    GF(cudaMalloc(&dm.p, n));
-    GF(cudaMemcpy(dm.p, metal, n, cudaMemcpyHostToDevice));
+    GF(dm.alloc(n, s));
+    GF(cudaMemcpyAsync(dm.p, metal, n, cudaMemcpyHostToDevice, s));
   }
-  GF(cudaMalloc(&dout.p, 3 * n * es));
+  GF(dout.alloc(3 * n * es, s));
   char* o = static_cast<char*>(dout.p);
   if (int st = field(dp.p, dtype, (long long)n, 1, static_cast<uint8_t*>(dm.p), nx, ny, nz, h,
-                     h_is_f64, o, o + n * es, o + 2 * n * es, (long long)n, nullptr))
+                     h_is_f64, o, o + n * es, o + 2 * n * es, (long long)n, s))
     return st;
-  GF(cudaMemcpy(ex, o, n * es, cudaMemcpyDeviceToHost));
-  GF(cudaMemcpy(ey, o + n * es, n * es, cudaMemcpyDeviceToHost));
-  GF(cudaMemcpy(ez, o + 2 * n * es, n * es, cudaMemcpyDeviceToHost));
+  GF(cudaMemcpyAsync(ex, o, n * es, cudaMemcpyDeviceToHost, s));
+  GF(cudaMemcpyAsync(ey, o + n * es, n * es, cudaMemcpyDeviceToHost, s));
+  GF(cudaMemcpyAsync(ez, o + 2 * n * es, n * es, cudaMemcpyDeviceToHost, s));
+  GF(cudaStreamSynchronize(s));
   return IG_OK;
 }
 
@@ -892,34 +917,37 @@ extern "C" int ig_compose_fields(const float* bases, int n_bases, int n_steps, c
     set_last_error("compose: null buffer");
     return IG_BAD_ARG;
   }
-  if (int st = no_device()) return st;
+  cudaStream_t s = nullptr;
+  if (int st = call_stream(&s)) return st;
   const size_t n = (size_t)nx * ny * nz;
   const size_t nc = (size_t)n_channels;
-  Tmp db, dm, dphi, de;
+  CallBuf db, dm, dphi, de;
+  const CallSync sync{s};
   if (n_bases > 0) {
-    GF(cudaMalloc(&db.p, (size_t)n_bases * n * 4));
-    GF(cudaMemcpy(db.p, bases, (size_t)n_bases * n * 4, cudaMemcpyHostToDevice));
+    GF(db.alloc((size_t)n_bases * n * 4, s));
+    GF(cudaMemcpyAsync(db.p, bases, (size_t)n_bases * n * 4, cudaMemcpyHostToDevice, s));
   }
   if (metal) {
-    GF(cudaMalloc(&dm.p, n));
-    GF(cudaMemcpy(dm.p, metal, n, cudaMemcpyHostToDevice));
+    GF(dm.alloc(n, s));
+    GF(cudaMemcpyAsync(dm.p, metal, n, cudaMemcpyHostToDevice, s));
   }
-  GF(cudaMalloc(&dphi.p, nc * n * 4));
-  GF(cudaMalloc(&de.p, 3 * nc * n * 4));
+  GF(dphi.alloc(nc * n * 4, s));
+  GF(de.alloc(3 * nc * n * 4, s));
   float* P = static_cast<float*>(dphi.p);
   float* E = static_cast<float*>(de.p);
   std::vector<const float*> src((size_t)n_steps);
   for (int s = 0; s < n_steps; s++) src[s] = static_cast<const float*>(db.p) + (size_t)rows[s] * n;
   if (int st = superpose(src.data(), n_steps, n_channels, weights, mult, (long long)n, P,
-                         (long long)n, nullptr))
+                         (long long)n, s))
     return st;
   if (int st = field(P, 0, (long long)n, n_channels, static_cast<uint8_t*>(dm.p), nx, ny, nz, h,
-                     h_is_f64, E, E + nc * n, E + 2 * nc * n, (long long)n, nullptr))
+                     h_is_f64, E, E + nc * n, E + 2 * nc * n, (long long)n, s))
     return st;
-  GF(cudaMemcpy(phi_out, P, nc * n * 4, cudaMemcpyDeviceToHost));
-  GF(cudaMemcpy(ex_out, E, nc * n * 4, cudaMemcpyDeviceToHost));
-  GF(cudaMemcpy(ey_out, E + nc * n, nc * n * 4, cudaMemcpyDeviceToHost));
-  GF(cudaMemcpy(ez_out, E + 2 * nc * n, nc * n * 4, cudaMemcpyDeviceToHost));
+  GF(cudaMemcpyAsync(phi_out, P, nc * n * 4, cudaMemcpyDeviceToHost, s));
+  GF(cudaMemcpyAsync(ex_out, E, nc * n * 4, cudaMemcpyDeviceToHost, s));
+  GF(cudaMemcpyAsync(ey_out, E + nc * n, nc * n * 4, cudaMemcpyDeviceToHost, s));
+  GF(cudaMemcpyAsync(ez_out, E + 2 * nc * n, nc * n * 4, cudaMemcpyDeviceToHost, s));
+  GF(cudaStreamSynchronize(s));
   return IG_OK;
 }
 
@@ -930,20 +958,23 @@ extern "C" int ig_field_check_division(double h, unsigned long long samples, uns
     set_last_error("division check: h must be a positive finite number");
     return IG_BAD_ARG;
   }
-  if (int st = no_device()) return st;
-  Tmp bad;
-  GF(cudaMalloc(&bad.p, 8));
-  GF(cudaMemset(bad.p, 0, 8));
+  cudaStream_t s = nullptr;
+  if (int st = call_stream(&s)) return st;
+  CallBuf bad;
+  const CallSync sync{s};
+  GF(bad.alloc(8, s));
+  GF(cudaMemsetAsync(bad.p, 0, 8, s));
   unsigned long long* b = static_cast<unsigned long long*>(bad.p);
   const Spacing sp = make_spacing(h, 0);
-  k_check_div32<<<152 * 32, 256>>>(sp.d1, b);
-  k_check_div32<<<152 * 32, 256>>>(sp.d2, b);
+  k_check_div32<<<152 * 32, 256, 0, s>>>(sp.d1, b);
+  k_check_div32<<<152 * 32, 256, 0, s>>>(sp.d2, b);
   if (samples) {
-    k_check_div64<<<152 * 32, 256>>>(sp.e1, samples, seed, b);
-    k_check_div64<<<152 * 32, 256>>>(sp.e2, samples, seed ^ 0x9e3779b9u, b);
+    k_check_div64<<<152 * 32, 256, 0, s>>>(sp.e1, samples, seed, b);
+    k_check_div64<<<152 * 32, 256, 0, s>>>(sp.e2, samples, seed ^ 0x9e3779b9u, b);
   }
   note_launches(samples ? 4 : 2);
   GF(cudaGetLastError());
-  GF(cudaMemcpy(mismatches_out, b, 8, cudaMemcpyDeviceToHost));
+  GF(cudaMemcpyAsync(mismatches_out, b, 8, cudaMemcpyDeviceToHost, s));
+  GF(cudaStreamSynchronize(s));
   return IG_OK;
 }

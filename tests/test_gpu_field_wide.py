@@ -50,3 +50,26 @@ def test_superposition_tail(n):
             for _ in range(m[c, s]):
                 acc = acc + w[c, s] * b[rows[s]]
         assert np.array_equal(got[c].view(np.int32), acc.view(np.int32))
+
+
+@pytest.mark.parametrize("h", [0.1, 3.0, 1.0 / 3.0, 2.0 ** -30, 1e-40, np.pi])
+def test_float64_gradients(h):
+    """float64 fields (divided by multiply-adds) are numpy's, over the whole
+    exponent range: quotients near rounding boundaries, zeros of both signs,
+    subnormals, infinities; every march length."""
+    from ion_gym_gb300.physics.field3d import build_field_aware_3d
+    for seed, shape in enumerate([(33, 33, 33), (5, 3, 2), (130, 9, 40), (2, 300, 290)]):
+        rng = np.random.default_rng(seed)
+        phi = rng.uniform(-1, 1, shape) * 2.0 ** rng.choice([0, 0, 0, 900, -900, -1060], shape)
+        phi[rng.random(shape) < 0.1] = 0.0
+        phi[rng.random(shape) < 0.05] = -0.0
+        phi[rng.random(shape) < 0.2] = 0.25
+        phi.flat[1] = np.inf
+        with np.errstate(all="ignore"):
+            want = np.gradient(phi, h)
+        got = build_field_aware_3d(phi, np.zeros(shape, np.int16), h, electrode_aware=False)
+        for g, w in zip(got, want):
+            w = -w
+            nan = np.isnan(w)
+            assert np.array_equal(np.isnan(g), nan)
+            assert np.array_equal(g[~nan].view(np.int64), w[~nan].view(np.int64))
