@@ -1726,20 +1726,22 @@ struct KSum {
   __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
-// The last half-sweep of the finest level's cycle (k_gs4<NG, false>, the
-// same update) with the flexible CG's <z, q_old> formed in the same pass:
-// once the colour-c groups are updated, z is final, so each thread adds
-// both colours of its slots (the other colour from the half-sweep before)
-// against q, and each block writes one partial (part[b * gridDim.x +
-// blockIdx.x]) -- k_cg_dot's read of z folded into the sweep that writes
-// it.  Summation order differs from k_cg_dot (blocks of the sweep's shape),
-// so the partial sums, not the update, may differ in their last bits.
-template <int NG>
-__global__ void k_gs4_dot(float* __restrict__ e, const float* __restrict__ g,
-                          const uint8_t* __restrict__ mask, SGeo G, int c, float omega,
-                          size_t pstride, const float* __restrict__ q,
-                          double* __restrict__ part) {
-  __shared__ double sh[32];
+// The last half-sweep of the finest level's cycle (the same update as k_gs4)
+// with the flexible CG's <z, q_old> formed in the same pass: once the
+// colour-c groups are updated, z is final, so each thread adds both colours
+// of its slots (the other colour from the half-sweep before) against q, and
+// each block writes one partial (part[b * gridDim.x + blockIdx.x]) --
+// k_cg_dot's read of z folded into the sweep that writes it.  Grid-stride
+// with cg_blocks() blocks a problem: a block's float64 sum takes the FP64
+// pipe (2 lanes per clock and SM) about a microsecond, which 192 blocks for
+// each of 24 problems' 98,000 groups made a third of the launch; and the
+// partial sums follow the grid and the problem count alone, not the tuned
+// launch shape, so equal solves have equal bits.
+__global__ void __launch_bounds__(kT)
+k_gs4_dot(float* __restrict__ e, const float* __restrict__ g,
+          const uint8_t* __restrict__ mask, SGeo G, int c, float omega,
+          size_t pstride, const float* __restrict__ q, double* __restrict__ part) {
+  __shared__ double sh[kT / 32];
   mask += (size_t)blockIdx.y * G.msplit;
   const uint32_t nq = G.csz >> 2;
   float* eb = e + blockIdx.y * pstride;
@@ -1749,33 +1751,35 @@ __global__ void k_gs4_dot(float* __restrict__ e, const float* __restrict__ g,
   const uint8_t* mp = mask + (size_t)c * G.csz;
   const float* qo = q + blockIdx.y * pstride + (size_t)c * G.csz;
   const float* qt = q + blockIdx.y * pstride + (size_t)(1 - c) * G.csz;
-  const uint32_t t0 = blockIdx.x * blockDim.x * NG + threadIdx.x;
   KSum acc;
-#pragma unroll
-  for (int u = 0; u < NG; u++) {
-    const uint32_t t = t0 + u * blockDim.x;
-    if (t < nq) {
-      gs4_group<false>(own, oth, gp, mp, G, c, omega, t);
-      const uint32_t ij = fdivu(t, G.dH4);
-      const uint32_t base = ij * (uint32_t)G.H + 4 * (t - ij * G.dH4.d);
-      const float4 za = ld4(own + base), zb = ld4(oth + base);
-      const float4 qa = ld4(qo + base), qb = ld4(qt + base);
-      acc.add(za.x * qa.x); acc.add(za.y * qa.y); acc.add(za.z * qa.z); acc.add(za.w * qa.w);
-      acc.add(zb.x * qb.x); acc.add(zb.y * qb.y); acc.add(zb.z * qb.z); acc.add(zb.w * qb.w);
-    }
+  for (uint32_t t = blockIdx.x * kT + threadIdx.x; t < nq; t += gridDim.x * kT) {
+    const uint32_t ij = fdivu(t, G.dH4);
+    const uint32_t base = ij * (uint32_t)G.H + 4 * (t - ij * G.dH4.d);
+    const float4 qa = ld4(qo + base), qb = ld4(qt + base), zb = ld4(oth + base);
+    gs4_group<false>(own, oth, gp, mp, G, c, omega, t);
+    const float4 za = ld4(own + base);
+    acc.add(za.x * qa.x); acc.add(za.y * qa.y); acc.add(za.z * qa.z); acc.add(za.w * qa.w);
+    acc.add(zb.x * qb.x); acc.add(zb.y * qb.y); acc.add(zb.z * qb.z); acc.add(zb.w * qb.w);
   }
   const double tot = block_sum_d(acc.value(), sh);
   if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
 }
 
+// Blocks of a grid-stride pass with block sums over `groups` float4 groups
+// for each of n problems (or problem colours): together four a SM, the
+// resident ones, so that each sums once over as much as it can.
+inline unsigned cg_blocks(uint32_t groups, unsigned n) {
+  const unsigned most = (groups + kT - 1) / kT;
+  return std::max(1u, std::min(most, 4u * 152u / std::max(1u, n)));
+}
+
 // q = L p (both colours; q = 0 on metal) and block partials of <p, q> and
 // <p, g>; blockIdx.y = colour, blockIdx.z = problem.  Grid-stride over
-// float4 groups (kCgBlocks blocks per colour and problem), so each block
+// float4 groups (cg_blocks() blocks per colour and problem), so each block
 // reduces once.  Blocks start in (x, y, z) order, so the two colours of a
 // problem run side by side over the same rows: the other colour's values
 // one colour reads as neighbours are the ones the other is reading as its
 // own, and come from L2 rather than from a second pass over DRAM.
-constexpr unsigned kCgBlocks = 152 * 2;
 __global__ void __launch_bounds__(kT)
 k_cg_matvec(const float* __restrict__ p, const float* __restrict__ g,
             const uint8_t* __restrict__ mask, SGeo G, float* __restrict__ q,
@@ -1896,7 +1900,7 @@ k_cg_matvec_dir(const float* __restrict__ z, const float* __restrict__ po,
   }
 }
 
-// block partials of <z, q>: grid-stride over float4 groups, kCgBlocks
+// block partials of <z, q>: grid-stride over float4 groups, cg_blocks()
 // blocks per problem
 __global__ void __launch_bounds__(kT)
 k_cg_dot(const float* __restrict__ z, const float* __restrict__ q,
@@ -2273,29 +2277,11 @@ struct Session {
   }
 
   // The finest level's last half-sweep with <z, q> folded in (k_gs4_dot):
-  // its partials go to `part`, their count to dot_nparts.  Returns false
-  // (nothing launched) where the tuned shape has no such form.
-  bool launch_gs_dot(MLevel& a, int c, int nb, float omega) {
-    if (flat(a) || gs_cfg.ng == 8) return false;
-    const uint32_t nq = a.G.csz / 4;
-    const unsigned per = (unsigned)(gs_cfg.threads * gs_cfg.ng);
-    const dim3 grid((nq + per - 1) / per, nb);
-    switch (gs_cfg.ng) {
-      case 4:
-        k_gs4_dot<4><<<grid, gs_cfg.threads, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, c, omega,
-                                                      a.pstride, qb.p, part.p);
-        break;
-      case 2:
-        k_gs4_dot<2><<<grid, gs_cfg.threads, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, c, omega,
-                                                      a.pstride, qb.p, part.p);
-        break;
-      default:
-        k_gs4_dot<1><<<grid, gs_cfg.threads, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, c, omega,
-                                                      a.pstride, qb.p, part.p);
-        break;
-    }
+  // its partials go to `part`, their count to dot_nparts.
+  void launch_gs_dot(MLevel& a, int c, int nb, float omega) {
+    const dim3 grid(cg_blocks(a.G.csz / 4, (unsigned)nb), nb);
+    k_gs4_dot<<<grid, kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, c, omega, a.pstride, qb.p, part.p);
     dot_nparts = (int)grid.x;
-    return true;
   }
 
   // The smoother's launch shape (groups per thread x block size) and its
@@ -2533,8 +2519,8 @@ struct Session {
     }
     for (int q = 0; q < nu2; q++)
       for (int c = 1; c >= 0; c--) {
-        if (l == 0 && dot_next && q + 1 == nu2 && c == 0 &&
-            launch_gs_dot(a, c, B, smooth_omega)) {
+        if (l == 0 && dot_next && q + 1 == nu2 && c == 0 && !flat(a)) {
+          launch_gs_dot(a, c, B, smooth_omega);
           dot_next = false;
           dot_done = true;
           continue;
@@ -2594,8 +2580,8 @@ struct Session {
     MLevel& f = lv[0];
     const uint32_t n = (uint32_t)f.pstride;
     const dim3 gv(nblk(n), B);
-    const unsigned nb4 = std::min(nblk(f.G.csz / 4), kCgBlocks);
-    const unsigned nbd = std::min(nblk(n / 4), kCgBlocks);
+    const unsigned nb4 = cg_blocks(f.G.csz / 4, 2 * (unsigned)B);
+    const unsigned nbd = cg_blocks(n / 4, (unsigned)B);
     float* pcur = from_b2 ? pb2.p : pb.p;
     float* pnext = from_b2 ? pb.p : pb2.p;
     const bool fold = fold_ok();
@@ -2663,7 +2649,7 @@ struct Session {
   // conditions under which vcycle reaches launch_gs_dot)
   bool dot_fused() const {
     return dot_on && method == 1 && lv.size() > 1 && !tail_level(0) && !tb_post(0) &&
-           nu2 >= 1 && !flat(lv[0]) && gs_cfg.ng != 8;
+           nu2 >= 1 && !flat(lv[0]);
   }
 
   bool fold_ok() const {
@@ -3282,7 +3268,7 @@ int ig_mixed_check_fused(void* handle, int n_problems, long long mismatches[8]) 
     if (S->fuse_dir()) {
       MLevel& f = S->lv[0];
       const size_t words = f.pstride * B;
-      const unsigned nb4 = std::min(nblk(f.G.csz / 4), kCgBlocks);
+      const unsigned nb4 = cg_blocks(f.G.csz / 4, 2 * (unsigned)B);
       const size_t nparts = 2 * (size_t)B * 2 * nb4;
       Buf<double> part2;
       part2.alloc(nparts, s);
