@@ -1364,6 +1364,35 @@ __global__ void k_set_fixed(double* __restrict__ phi,
   if (t < n && fixed[t]) phi[t] = val[t];
 }
 
+__global__ void k_set_basis(double* __restrict__ phi, const uint8_t* __restrict__ fixed,
+                            const uint8_t* __restrict__ mask, double v, size_t n) {
+  const size_t t = (size_t)blockIdx.x * kThreads + threadIdx.x;
+  if (t < n && fixed[t]) phi[t] = mask[t] ? v : 0.0;
+}
+
+// The flip test of every axis at once, a node and its three mirror images a
+// thread (the host read every node of a symmetric deck once per axis and
+// basis before the first launch).
+__global__ void __launch_bounds__(kThreads)
+k_sym_check(const uint8_t* __restrict__ fixed, const double* __restrict__ val,
+            const uint8_t* __restrict__ mask, double v, FlatGeom g, int* flags) {
+  const uint32_t t = blockIdx.x * kThreads + threadIdx.x;
+  if (t >= g.total) return;
+  const uint32_t ij = fdiv(t, g.div_nz);
+  const uint32_t k = t - ij * g.div_nz.d;
+  const uint32_t i = fdiv(ij, g.div_ny);
+  const uint32_t j = ij - i * g.div_ny.d;
+  const uint32_t nx = (uint32_t)g.nx, ny = (uint32_t)g.ny, nz = (uint32_t)g.nz;
+  const uint32_t q[3] = {((nx - 1 - i) * ny + j) * nz + k, (i * ny + ny - 1 - j) * nz + k,
+                         ij * nz + nz - 1 - k};
+  auto at = [&](uint32_t p) { return val ? val[p] : (mask[p] ? v : 0.0); };
+  const bool fx = fixed[t] != 0;
+  const double x = at(t);
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    if ((fixed[q[a]] != 0) != fx || !(at(q[a]) == x)) flags[a] = 1;
+}
+
 __global__ void __launch_bounds__(kThreads)
 k_absdiff_max(const double* __restrict__ a, const double* __restrict__ b,
               size_t n, unsigned long long* bits, int* nan_flag) {
@@ -1772,6 +1801,23 @@ void launch_set_fixed(cudaStream_t s, double* phi, const uint8_t* fixed,
     k_set_fixed<<<nb, kThreads, 0, s>>>(phi, fixed, val, n);
     counted();
   }
+}
+
+void launch_set_basis(cudaStream_t s, double* phi, const uint8_t* fixed, const uint8_t* mask,
+                      double v, size_t n) {
+  const unsigned nb = blocks_for(n);
+  if (nb) {
+    k_set_basis<<<nb, kThreads, 0, s>>>(phi, fixed, mask, v, n);
+    counted();
+  }
+}
+
+void launch_sym_check(cudaStream_t s, const uint8_t* fixed, const double* val,
+                      const uint8_t* mask, double v, Dims d, int* flags) {
+  const FlatGeom g = flat_geom(d);
+  cudaMemsetAsync(flags, 0, 3 * sizeof(int), s);
+  k_sym_check<<<blocks_for(g.total), kThreads, 0, s>>>(fixed, val, mask, v, g, flags);
+  counted();
 }
 
 void launch_absdiff_max(cudaStream_t s, const double* a, const double* b,

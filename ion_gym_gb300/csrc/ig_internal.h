@@ -155,6 +155,15 @@ void launch_coarsen_mask(cudaStream_t s, const uint8_t* fixed,
                          Dims c);
 void launch_set_fixed(cudaStream_t s, double* phi, const uint8_t* fixed,
                       const double* val, size_t n);
+// phi[fixed] = v_basis on mask, 0 on the rest of fixed (a basis's Dirichlet
+// values without an array of them)
+void launch_set_basis(cudaStream_t s, double* phi, const uint8_t* fixed, const uint8_t* mask,
+                      double v, size_t n);
+// flags[a] = 1 where fixed or the Dirichlet values -- val, or (val null) v on
+// mask and 0 elsewhere -- are not invariant under the flip of axis a
+// (multigrid3d.py:643-650); flags is zeroed here
+void launch_sym_check(cudaStream_t s, const uint8_t* fixed, const double* val,
+                      const uint8_t* mask, double v, Dims d, int* flags);
 // max |a - b| (b nullable: max |a|) into *bits, NaN noted in *nan_flag
 void launch_absdiff_max(cudaStream_t s, const double* a, const double* b,
                         size_t n, unsigned long long* bits, int* nan_flag);

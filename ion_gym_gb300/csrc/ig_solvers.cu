@@ -16,8 +16,11 @@
 #include <cstdio>
 #include <cstring>
 #include <limits>
+#include <mutex>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "ig_common.cuh"
@@ -51,17 +54,40 @@ struct Status : std::runtime_error {
                                       std::to_string(__LINE__) + ")");         \
   } while (0)
 
-// Per-thread stream and pinned control block, created on first use.
+// A calling thread's stream and pinned control block.  Taken on the thread's
+// first call and handed on when it ends, so a program has as many as it had
+// threads at once: the basis door starts its workers anew on every call, and
+// a stream, two events and a pinned allocation for each (which wait for the
+// device) were made, and lost, every time.
 struct ThreadCtx {
   int dev = -1;
   cudaStream_t s = nullptr;
   PairCtl* ctl_h = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-  ~ThreadCtx() {
-    // process exit: the driver reclaims everything; nothing to do here
-  }
 };
-thread_local ThreadCtx t_ctx;
+
+// The idle ones (never destroyed: the driver reclaims them at process exit).
+struct CtxPool {
+  std::mutex mu;
+  std::vector<ThreadCtx> idle;
+};
+CtxPool& ctx_pool() {
+  static CtxPool* p = new CtxPool;
+  return *p;
+}
+
+struct CtxHolder {
+  ThreadCtx c;
+  void hand_on() {
+    if (c.dev < 0) return;
+    CtxPool& p = ctx_pool();
+    std::lock_guard<std::mutex> lk(p.mu);
+    p.idle.push_back(c);
+    c = ThreadCtx();
+  }
+  ~CtxHolder() { hand_on(); }
+};
+thread_local CtxHolder t_ctx;
 
 ThreadCtx& ctx() {
   int n = 0;
@@ -69,19 +95,32 @@ ThreadCtx& ctx() {
     throw Status(IG_NO_DEVICE, "no CUDA device is visible");
   int dev = 0;
   CK(cudaGetDevice(&dev));
-  if (t_ctx.dev != dev) {
-    t_ctx.dev = dev;
-    CK(cudaStreamCreateWithFlags(&t_ctx.s, cudaStreamNonBlocking));
-    CK(cudaMallocHost(&t_ctx.ctl_h, sizeof(PairCtl)));
-    CK(cudaEventCreate(&t_ctx.ev0));
-    CK(cudaEventCreate(&t_ctx.ev1));
+  if (t_ctx.c.dev != dev) {
+    t_ctx.hand_on();
+    CtxPool& p = ctx_pool();
+    {
+      std::lock_guard<std::mutex> lk(p.mu);
+      for (size_t q = p.idle.size(); q-- > 0;)
+        if (p.idle[q].dev == dev) {
+          t_ctx.c = p.idle[q];
+          p.idle.erase(p.idle.begin() + (long)q);
+          return t_ctx.c;
+        }
+    }
+    ThreadCtx c;
+    CK(cudaStreamCreateWithFlags(&c.s, cudaStreamNonBlocking));
+    CK(cudaMallocHost(&c.ctl_h, sizeof(PairCtl)));
+    CK(cudaEventCreate(&c.ev0));
+    CK(cudaEventCreate(&c.ev1));
     // keep freed stream-ordered allocations cached between solves
     cudaMemPool_t pool;
     CK(cudaDeviceGetDefaultMemPool(&pool, dev));
     uint64_t thr = std::numeric_limits<uint64_t>::max();
     CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
+    c.dev = dev;
+    t_ctx.c = c;
   }
-  return t_ctx;
+  return t_ctx.c;
 }
 
 // Stream-ordered device buffer.
@@ -298,17 +337,42 @@ void plan_theta(ThreadCtx& c, Theta& t, DBuf<float>& th, const uint8_t* fixed, D
   th.release();
 }
 
+// A call's Dirichlet values: val (n), or v on the nodes of mask and 0 on the
+// rest of the metal (a basis).  Caller's memory.
+struct Dirichlet {
+  const double* val = nullptr;
+  const uint8_t* mask = nullptr;
+  double v = 0.0;
+};
+
+// ... and on the device.
+struct DirichletDev {
+  DBuf<double> val;
+  DBuf<uint8_t> mask;
+  void load(ThreadCtx& c, const Dirichlet& b, size_t n) {
+    if (b.val) {
+      val.alloc(n, c.s);
+      CK(cudaMemcpyAsync(val.p, b.val, n * 8, cudaMemcpyDefault, c.s));
+    } else {
+      mask.alloc(n, c.s);
+      CK(cudaMemcpyAsync(mask.p, b.mask, n, cudaMemcpyDefault, c.s));
+    }
+  }
+};
+
 // phi = phi0 (or 0); phi[fixed] = val[fixed]  (solver3d.py:263-265)
-void init_phi(ThreadCtx& c, FineGrid& g, const double* val_h,
-              const double* phi0_h, DBuf<double>& val_d) {
+void init_phi(ThreadCtx& c, FineGrid& g, const Dirichlet& b, const double* phi0_h,
+              DirichletDev& d) {
   const size_t n = g.d.n();
   if (phi0_h)
     CK(cudaMemcpyAsync(g.phi.p, phi0_h, n * 8, cudaMemcpyDefault, c.s));
   else
     CK(cudaMemsetAsync(g.phi.p, 0, n * 8, c.s));
-  val_d.alloc(n, c.s);
-  CK(cudaMemcpyAsync(val_d.p, val_h, n * 8, cudaMemcpyDefault, c.s));
-  launch_set_fixed(c.s, g.phi.p, g.fixed.p, val_d.p, n);
+  d.load(c, b, n);
+  if (b.val)
+    launch_set_fixed(c.s, g.phi.p, g.fixed.p, d.val.p, n);
+  else
+    launch_set_basis(c.s, g.phi.p, g.fixed.p, d.mask.p, b.v, n);
 }
 
 // One colour of a fine grid's sweep by the plan or the general kernels.
@@ -515,32 +579,20 @@ void solve_err(ThreadCtx& c, VCycle& v, size_t L, double above) {
   }
 }
 
-// Axes along which fixed and val are exactly flip-invariant
-// (multigrid3d.py:643-650).  val(p) is read through a callback so a basis
-// solve can test v_basis * mask without materialising val.
-template <class V>
-std::vector<int> sym_axes(const uint8_t* fixed, V&& val, Dims d) {
+// Axes along which fixed and the values are exactly flip-invariant
+// (multigrid3d.py:643-650).
+std::vector<int> sym_axes(ThreadCtx& c, const FineGrid& g, const Dirichlet& b,
+                          const DirichletDev& d) {
+  DBuf<int> flags(3, c.s);
+  launch_sym_check(c.s, g.fixed.p, d.val.p, d.mask.p, b.v, g.d, flags.p);
+  CK(cudaGetLastError());
+  int h[3] = {1, 1, 1};
+  CK(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, c.s));
+  CK(cudaStreamSynchronize(c.s));
+  const long n[3] = {g.d.nx, g.d.ny, g.d.nz};
   std::vector<int> axes;
-  const long n[3] = {d.nx, d.ny, d.nz};
-  for (int a = 0; a < 3; a++) {
-    if (n[a] < 3) continue;
-    bool ok = true;
-    for (long i = 0; i < d.nx && ok; i++)
-      for (long j = 0; j < d.ny && ok; j++)
-        for (long k = 0; k < d.nz; k++) {
-          long mi = i, mj = j, mk = k;
-          if (a == 0) mi = d.nx - 1 - i;
-          else if (a == 1) mj = d.ny - 1 - j;
-          else mk = d.nz - 1 - k;
-          const size_t p = ((size_t)i * d.ny + j) * d.nz + k;
-          const size_t q = ((size_t)mi * d.ny + mj) * d.nz + mk;
-          if ((fixed[p] != 0) != (fixed[q] != 0) || !(val(p) == val(q))) {
-            ok = false;
-            break;
-          }
-        }
-    if (ok) axes.push_back(a);
-  }
+  for (int a = 0; a < 3; a++)
+    if (n[a] >= 3 && !h[a]) axes.push_back(a);
   return axes;
 }
 
@@ -636,6 +688,33 @@ void load_fine(ThreadCtx& c, FineGrid& g, const uint8_t* fixed,
   }
 }
 
+// Brings the pages of a call's pageable output array in while the GPU
+// solves.  A fresh array's pages are otherwise faulted in by the copy at the
+// end, which the bases of a door call do at the same time and on one lock:
+// eight copies of 14.5 MB took 1 to 17 ms, into touched pages 1 to 2.
+struct PageTouch {
+  std::thread t;
+  PageTouch(void* p, size_t bytes) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    if (a.type != cudaMemoryTypeUnregistered || bytes < (size_t(1) << 20)) return;
+    try {
+      t = std::thread([p, bytes] {
+        volatile unsigned char* q = static_cast<unsigned char*>(p);
+        for (size_t o = 0; o < bytes; o += 4096) q[o] = q[o];
+      });
+    } catch (const std::system_error&) {  // no thread: the copy faults them in
+    }
+  }
+  void join() {
+    if (t.joinable()) t.join();
+  }
+  ~PageTouch() { join(); }
+};
+
 void copy_out(ThreadCtx& c, const double* d, double* h, size_t n) {
   CK(cudaMemcpyAsync(h, d, n * 8, cudaMemcpyDefault, c.s));
   CK(cudaStreamSynchronize(c.s));
@@ -691,6 +770,59 @@ int guard(F&& f) {
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
+// ig_solve3d on the values `b`.
+int sor_call(const uint8_t* fixed, const Dirichlet& b, const float* theta, long nx, long ny,
+             long nz, double tol, long max_sweeps, double omega, const double* phi0, int stencil,
+             double* phi_out, long* sweeps_out, double* delta_out) {
+  if (!fixed || !(b.val || b.mask) || !phi_out) throw Status(IG_BAD_ARG, "null array");
+  ThreadCtx& c = ctx();
+  FineGrid g;
+  load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
+  DirichletDev bd;
+  init_phi(c, g, b, phi0, bd);
+  DBuf<PairCtl> ctl(1, c.s);
+  const PairsResult r = sor_loop(c, g.phi.p, g.fixed.p, g.th.p, g.plan, g.stencil, g.d, omega,
+                                 tol, max_sweeps, ctl.p);
+  copy_out(c, g.phi.p, phi_out, g.d.n());
+  if (sweeps_out) *sweeps_out = r.pairs;
+  if (delta_out) *delta_out = r.delta;
+  if (!r.converged) {
+    t_err = "SOR reached its sweep cap";
+    return (int)IG_NOT_CONVERGED;
+  }
+  return (int)IG_OK;
+}
+
+// ig_solve3d_vmg on the values `b`.
+int vmg_call(const uint8_t* fixed, const Dirichlet& b, const float* theta, long nx, long ny,
+             long nz, double tol, int max_cycles, int nu1, int nu2, int stencil,
+             const double* phi0, int accept_stagnation, double bottom_omega, double* phi_out,
+             long* sweeps_out, double* delta_out, int* cycles_out, double* prev_delta_out) {
+  if (!fixed || !(b.val || b.mask) || !phi_out) throw Status(IG_BAD_ARG, "null array");
+  if (nu1 < 0 || nu2 < 0) throw Status(IG_BAD_ARG, "nu1 and nu2 must be >= 0");
+  ThreadCtx& c = ctx();
+  FineGrid g;
+  load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
+  PageTouch touch(phi_out, g.d.n() * 8);
+  std::vector<int> sym;
+  {
+    DirichletDev bd;
+    init_phi(c, g, b, phi0, bd);
+    if (!theta) sym = sym_axes(c, g, b, bd);
+  }
+  VCycle v;
+  prepare_vcycle(c, v, g, nu1, nu2, bottom_omega);
+  const VmgOut o = vmg_loop(c, g, v, tol, max_cycles, accept_stagnation, sym);
+  touch.join();
+  copy_out(c, g.phi.p, phi_out, g.d.n());
+  if (sweeps_out) *sweeps_out = o.sweeps;
+  if (delta_out) *delta_out = o.delta;
+  if (cycles_out) *cycles_out = o.cycles;
+  if (prev_delta_out) *prev_delta_out = o.prev;
+  if (o.status != IG_OK) t_err = "V-cycle did not reach tol";
+  return o.status;
+}
+
 }  // namespace
 }  // namespace ig
 
@@ -739,24 +871,11 @@ int ig_solve3d(const uint8_t* fixed, const double* val, const float* theta,
                long nx, long ny, long nz, double tol, long max_sweeps,
                double omega, const double* phi0, int stencil, double* phi_out,
                long* sweeps_out, double* delta_out) {
+  Dirichlet b;
+  b.val = val;
   return guard([&] {
-    if (!fixed || !val || !phi_out) throw Status(IG_BAD_ARG, "null array");
-    ThreadCtx& c = ctx();
-    FineGrid g;
-    load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
-    DBuf<double> val_d;
-    init_phi(c, g, val, phi0, val_d);
-    DBuf<PairCtl> ctl(1, c.s);
-    const PairsResult r = sor_loop(c, g.phi.p, g.fixed.p, g.th.p, g.plan, g.stencil, g.d,
-                                    omega, tol, max_sweeps, ctl.p);
-    copy_out(c, g.phi.p, phi_out, g.d.n());
-    if (sweeps_out) *sweeps_out = r.pairs;
-    if (delta_out) *delta_out = r.delta;
-    if (!r.converged) {
-      t_err = "SOR reached its sweep cap";
-      return (int)IG_NOT_CONVERGED;
-    }
-    return (int)IG_OK;
+    return sor_call(fixed, b, theta, nx, ny, nz, tol, max_sweeps, omega, phi0, stencil, phi_out,
+                    sweeps_out, delta_out);
   });
 }
 
@@ -765,14 +884,12 @@ int ig_solve_basis_sor(const uint8_t* metal, const uint8_t* mask,
                        long nz, double tol, long max_sweeps, double omega,
                        int stencil, double* phi_out, long* sweeps_out,
                        double* delta_out) {
+  Dirichlet b;
+  b.mask = mask;
+  b.v = v_basis;
   return guard([&] {
-    if (!metal || !mask || !phi_out) throw Status(IG_BAD_ARG, "null array");
-    check_dims(nx, ny, nz);
-    const size_t n = (size_t)nx * ny * nz;
-    std::vector<double> val(n);
-    for (size_t p = 0; p < n; p++) val[p] = mask[p] ? v_basis : 0.0;
-    return ig_solve3d(metal, val.data(), theta, nx, ny, nz, tol, max_sweeps,
-                      omega, nullptr, stencil, phi_out, sweeps_out, delta_out);
+    return sor_call(metal, b, theta, nx, ny, nz, tol, max_sweeps, omega, nullptr, stencil,
+                    phi_out, sweeps_out, delta_out);
   });
 }
 
@@ -856,26 +973,12 @@ int ig_solve3d_vmg(const uint8_t* fixed, const double* val, const float* theta,
                    int accept_stagnation, double bottom_omega, double* phi_out,
                    long* sweeps_out, double* delta_out, int* cycles_out,
                    double* prev_delta_out) {
+  Dirichlet b;
+  b.val = val;
   return guard([&] {
-    if (!fixed || !val || !phi_out) throw Status(IG_BAD_ARG, "null array");
-    if (nu1 < 0 || nu2 < 0) throw Status(IG_BAD_ARG, "nu1 and nu2 must be >= 0");
-    ThreadCtx& c = ctx();
-    FineGrid g;
-    load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
-    DBuf<double> val_d;
-    init_phi(c, g, val, phi0, val_d);
-    std::vector<int> sym;
-    if (!theta) sym = sym_axes(fixed, [&](size_t p) { return val[p]; }, g.d);
-    VCycle v;
-    prepare_vcycle(c, v, g, nu1, nu2, bottom_omega);
-    const VmgOut o = vmg_loop(c, g, v, tol, max_cycles, accept_stagnation, sym);
-    copy_out(c, g.phi.p, phi_out, g.d.n());
-    if (sweeps_out) *sweeps_out = o.sweeps;
-    if (delta_out) *delta_out = o.delta;
-    if (cycles_out) *cycles_out = o.cycles;
-    if (prev_delta_out) *prev_delta_out = o.prev;
-    if (o.status != IG_OK) t_err = "V-cycle did not reach tol";
-    return o.status;
+    return vmg_call(fixed, b, theta, nx, ny, nz, tol, max_cycles, nu1, nu2, stencil, phi0,
+                    accept_stagnation, bottom_omega, phi_out, sweeps_out, delta_out, cycles_out,
+                    prev_delta_out);
   });
 }
 
@@ -885,15 +988,12 @@ int ig_solve_basis_vmg(const uint8_t* metal, const uint8_t* mask,
                        int stencil, double bottom_omega, double* phi_out,
                        long* sweeps_out, double* delta_out, int* cycles_out,
                        double* prev_delta_out) {
+  Dirichlet b;
+  b.mask = mask;
+  b.v = v_basis;
   return guard([&] {
-    if (!metal || !mask || !phi_out) throw Status(IG_BAD_ARG, "null array");
-    check_dims(nx, ny, nz);
-    const size_t n = (size_t)nx * ny * nz;
-    std::vector<double> val(n);
-    for (size_t p = 0; p < n; p++) val[p] = mask[p] ? v_basis : 0.0;
-    return ig_solve3d_vmg(metal, val.data(), theta, nx, ny, nz, tol, max_cycles,
-                          nu1, nu2, stencil, nullptr, 0, bottom_omega, phi_out,
-                          sweeps_out, delta_out, cycles_out, prev_delta_out);
+    return vmg_call(metal, b, theta, nx, ny, nz, tol, max_cycles, nu1, nu2, stencil, nullptr, 0,
+                    bottom_omega, phi_out, sweeps_out, delta_out, cycles_out, prev_delta_out);
   });
 }
 
