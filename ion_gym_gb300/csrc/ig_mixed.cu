@@ -43,6 +43,8 @@
 #include <map>
 #include <mutex>
 
+#include <cooperative_groups.h>
+
 #include "ig_common.cuh"
 #include "ig_internal.h"
 #include "../../include/igsolve.h"
@@ -119,8 +121,18 @@ __device__ __forceinline__ float nbr_sum(const SGeo& g, const float* __restrict_
 
 // ---- FP32 kernels on split arrays (blockIdx.y = problem) ----------------
 
+// CG: from L2, for values that other SMs write within the same kernel.
+template <bool CG = false>
 __device__ __forceinline__ float4 ld4(const float* p) {
-  return *reinterpret_cast<const float4*>(p);
+  return CG ? __ldcg(reinterpret_cast<const float4*>(p)) : *reinterpret_cast<const float4*>(p);
+}
+template <bool CG = false>
+__device__ __forceinline__ float2 ld2(const float* p) {
+  return CG ? __ldcg(reinterpret_cast<const float2*>(p)) : *reinterpret_cast<const float2*>(p);
+}
+template <bool CG = false>
+__device__ __forceinline__ float ld1(const float* p) {
+  return CG ? __ldcg(p) : *p;
 }
 
 // Neighbour sums of the four slots m0..m0+3 (k parity p) of row (i, j),
@@ -132,10 +144,11 @@ __device__ __forceinline__ float4 ld4(const float* p) {
 // group) only feeds unused slots, whose results are never kept.  Sum order:
 // ((xm + xp) + (ym + yp)) + (zm + zp).
 // Values of the other colour's array: plain loads.
+template <bool CG = false>
 struct PlainLd {
   const float* __restrict__ a;
-  __device__ __forceinline__ float4 v4(uint32_t o) const { return ld4(a + o); }
-  __device__ __forceinline__ float v1(uint32_t o) const { return a[o]; }
+  __device__ __forceinline__ float4 v4(uint32_t o) const { return ld4<CG>(a + o); }
+  __device__ __forceinline__ float v1(uint32_t o) const { return ld1<CG>(a + o); }
 };
 // Values of the new CG direction z + beta p, formed where they are read
 // (the expression k_cg_dir stores).
@@ -175,7 +188,7 @@ __device__ __forceinline__ void nbr4(const L& oth, const SGeo& G, int i, int j, 
 
 // One float4 group (slots m0..m0+3 of colour c, row ij) of the update.
 // FLAT: the grid has a size-1 axis (per-slot neighbour sums).
-template <bool FLAT>
+template <bool FLAT, bool CG = false>
 __device__ __forceinline__ void gs4_at(float* __restrict__ own, const float* __restrict__ oth,
                                        const float* __restrict__ gp,
                                        const uint8_t* __restrict__ mp, const SGeo& G, int c,
@@ -189,8 +202,8 @@ __device__ __forceinline__ void gs4_at(float* __restrict__ own, const float* __r
   // its rows.  There the loads (in bounds in every group) are issued with
   // the mask's rather than after it, so a group waits for one memory round
   // trip, not two.
-  const float4 gg = ld4(gp + base);
-  if (!FLAT) nbr4(PlainLd{oth}, G, i, j, m0, p, base, q);
+  const float4 gg = ld4<CG>(gp + base);
+  if (!FLAT) nbr4(PlainLd<CG>{oth}, G, i, j, m0, p, base, q);
   if (mk.x & mk.y & mk.z & mk.w) return;  // all metal or unused slots
   if (FLAT) {
 #pragma unroll
@@ -211,11 +224,16 @@ __device__ __forceinline__ void gs4_at(float* __restrict__ own, const float* __r
   for (int u = 0; u < 4; u++) {
     if (mv[u]) continue;
     const float nv = (q[u] - gv[u]) * (1.0f / 6.0f);
-    own[base + u] = omega == 1.0f ? nv : own[base + u] + omega * (nv - own[base + u]);
+    if (omega == 1.0f) {
+      own[base + u] = nv;
+    } else {
+      const float old = ld1<CG>(own + base + u);
+      own[base + u] = old + omega * (nv - old);
+    }
   }
 }
 
-template <bool FLAT>
+template <bool FLAT, bool CG = false>
 __device__ __forceinline__ void gs4_group(float* __restrict__ own, const float* __restrict__ oth,
                                           const float* __restrict__ gp,
                                           const uint8_t* __restrict__ mp, const SGeo& G,
@@ -224,7 +242,7 @@ __device__ __forceinline__ void gs4_group(float* __restrict__ own, const float* 
   const int m0 = 4 * (int)(t - ij * G.dH4.d);
   const int i = (int)fdivu(ij, G.dny);
   const int j = (int)(ij - (uint32_t)i * G.dny.d);
-  gs4_at<FLAT>(own, oth, gp, mp, G, c, omega, ij, i, j, m0);
+  gs4_at<FLAT, CG>(own, oth, gp, mp, G, c, omega, ij, i, j, m0);
 }
 
 // Red-black Gauss-Seidel half-sweep of colour c on the split layout.  Each
@@ -293,32 +311,26 @@ __global__ void k_gs8(float* __restrict__ e, const float* __restrict__ g,
 __device__ __forceinline__ float zero_start_e0(float g, uint8_t m) {
   return m ? 0.f : (0.f - g) * (1.0f / 6.0f);
 }
-__device__ __forceinline__ float4 zero_start_e0(const float* gp, const uint8_t* mp) {
-  const float4 g = ld4(gp);
-  const uchar4 m = *reinterpret_cast<const uchar4*>(mp);
-  return make_float4(zero_start_e0(g.x, m.x), zero_start_e0(g.y, m.y), zero_start_e0(g.z, m.z),
-                     zero_start_e0(g.w, m.w));
-}
 
 // The right-hand side a cycle reads: g itself, or (FOLD) g + alpha q -- the
 // flexible CG's update of the previous iteration, formed where it is read
 // (k_cg_update's expression, so the same bits).
-template <bool FOLD>
+template <bool FOLD, bool CG = false>
 struct RhsLd {
   const float* __restrict__ g;
   const float* __restrict__ q;
   float al;
   __device__ __forceinline__ float4 v4(uint32_t o) const {
-    float4 v = ld4(g + o);
+    float4 v = ld4<CG>(g + o);
     if (FOLD) {
-      const float4 w = ld4(q + o);
+      const float4 w = ld4<CG>(q + o);
       v.x = __fmaf_rn(al, w.x, v.x); v.y = __fmaf_rn(al, w.y, v.y);
       v.z = __fmaf_rn(al, w.z, v.z); v.w = __fmaf_rn(al, w.w, v.w);
     }
     return v;
   }
   __device__ __forceinline__ float v1(uint32_t o) const {
-    return FOLD ? __fmaf_rn(al, q[o], g[o]) : g[o];
+    return FOLD ? __fmaf_rn(al, ld1<CG>(q + o), ld1<CG>(g + o)) : ld1<CG>(g + o);
   }
 };
 __device__ __forceinline__ float4 zero_start_e0(float4 g, uchar4 m) {
@@ -331,7 +343,7 @@ __device__ __forceinline__ float4 zero_start_e0(float4 g, uchar4 m) {
 // right-hand side is g0 + al q0 (the previous CG iteration's update,
 // formed where it is read), and the thread stores it, both colours of its
 // slots, to gout (a different array: neighbouring threads still read g0).
-template <bool FOLD>
+template <bool FOLD, bool CG = false>
 __device__ __forceinline__ void zero_pair_at(float* e0, const float* g0, const uint8_t* mask,
                                              const SGeo& G, uint32_t t,
                                              const float* q0 = nullptr, float al = 0.f,
@@ -342,8 +354,8 @@ __device__ __forceinline__ void zero_pair_at(float* e0, const float* g0, const u
   const int j = (int)(ij - (uint32_t)i * G.dny.d);
   const uint32_t base = ij * (uint32_t)G.H + m0;
   float* e1 = e0 + G.csz;
-  const RhsLd<FOLD> r0{g0, q0, al};
-  const RhsLd<FOLD> r1{g0 + G.csz, FOLD ? q0 + G.csz : nullptr, al};
+  const RhsLd<FOLD, CG> r0{g0, q0, al};
+  const RhsLd<FOLD, CG> r1{g0 + G.csz, FOLD ? q0 + G.csz : nullptr, al};
   const uint8_t* k0 = mask;
   const uint8_t* k1 = mask + G.csz;
   auto m4 = [&](uint32_t o) { return *reinterpret_cast<const uchar4*>(k0 + o); };
@@ -686,6 +698,7 @@ k_resid0(const float* __restrict__ e, const float* __restrict__ g,
 // float4 store of r.
 // Float4 group t of the colour-0 residual, one problem: eb, gb, mask its
 // split arrays, rb its colour-0 residual (csz floats).
+template <bool CG = false>
 __device__ __forceinline__ void resid0_4_at(const float* eb, const float* gb,
                                             const uint8_t* mask, const SGeo& G, float* rb,
                                             uint32_t t) {
@@ -699,8 +712,8 @@ __device__ __forceinline__ void resid0_4_at(const float* eb, const float* gb,
   // group and go out with the mask's; metal slots select 0 below
   const uchar4 mk = *reinterpret_cast<const uchar4*>(mask + base);
   float q[4];
-  nbr4(PlainLd{eb + G.csz}, G, i, j, m0, (i + j) & 1, base, q);
-  const float4 ev = ld4(eb + base), gg = ld4(gb + base);
+  nbr4(PlainLd<CG>{eb + G.csz}, G, i, j, m0, (i + j) & 1, base, q);
+  const float4 ev = ld4<CG>(eb + base), gg = ld4<CG>(gb + base);
   const float es[4] = {ev.x, ev.y, ev.z, ev.w}, gv[4] = {gg.x, gg.y, gg.z, gg.w};
   const uint8_t mv[4] = {mk.x, mk.y, mk.z, mk.w};
   float o[4];
@@ -759,6 +772,7 @@ k_restrict0(const float* __restrict__ r0, SGeo F, float* __restrict__ gc, SGeo C
 }
 
 // The 13-tap sum of one coarse node (k_restrict0's loop).
+template <bool CG = false>
 __device__ __forceinline__ float restrict0_node(const float* __restrict__ rb, const SGeo& F,
                                                 int ic, int jc, int kc) {
   float acc = 0.f;
@@ -775,11 +789,25 @@ __device__ __forceinline__ float restrict0_node(const float* __restrict__ rb, co
         const int kk = min(max(2 * kc + dk, 0), F.nz - 1);
         if ((ii + jj + kk) & 1) continue;
         const float wk = dk == 0 ? 1.f : 0.5f;
-        acc += wi * wj * wk * rb[sidx(F, ii, jj, kk)];
+        acc += wi * wj * wk * ld1<CG>(rb + sidx(F, ii, jj, kk));
       }
     }
   }
   return acc;
+}
+
+// Coarse node t of that restriction, one thread a node: for grids of fewer
+// groups of four than a cluster has threads (33^3 to 17^3: a group a thread
+// kept three of eight CTAs busy, 14.9e3 -> 5.5e3 clocks).
+template <bool CG = false>
+__device__ __forceinline__ void restrict0_at(const float* rb, const SGeo& F, float* gb,
+                                             const SGeo& C, uint32_t t) {
+  const uint32_t ij = fdivu(t, C.dnz);
+  const int kc = (int)(t - ij * C.dnz.d);
+  const int ic = (int)fdivu(ij, C.dny);
+  const int jc = (int)(ij - (uint32_t)ic * C.dny.d);
+  gb[(size_t)scol(ic, jc, kc) * C.csz + sidx(C, ic, jc, kc)] =
+      0.5f * restrict0_node<CG>(rb, F, ic, jc, kc);
 }
 
 // k_restrict0 for four consecutive coarse z nodes kc = 4g .. 4g+3 of one
@@ -818,7 +846,7 @@ __device__ __forceinline__ void restrict0_4_at(const float* rb, const SGeo& F, f
   float a[4] = {0.f, 0.f, 0.f, 0.f};
   // one tap per node from slot kc of a row, weight w
   auto at = [&](const float* r, float w) {
-    const float4 v = ld4(r);
+    const float4 v = *reinterpret_cast<const float4*>(r);
     a[0] += w * v.x;
     a[1] += w * v.y;
     a[2] += w * v.z;
@@ -826,7 +854,7 @@ __device__ __forceinline__ void restrict0_4_at(const float* rb, const SGeo& F, f
   };
   // two taps per node from slots kc - 1 and kc of a row (dk = -1, +1)
   auto at2 = [&](const float* r, float w) {
-    const float4 v = ld4(r);
+    const float4 v = *reinterpret_cast<const float4*>(r);
     const float m = r[-1];
     a[0] += w * m;
     a[0] += w * v.x;
@@ -1019,6 +1047,7 @@ k_prolong_add4_gather(const float* __restrict__ ec, SGeo C, float* __restrict__ 
 // Fine float4 group t of colour c of the windowed prolongation, one
 // problem: eb its coarse correction, efb its fine correction and maskf its
 // fine split mask.
+template <bool CG = false>
 __device__ __forceinline__ void prolong_add4_at(const float* eb, const SGeo& C, float* efb,
                                                 const uint8_t* maskf, const SGeo& F, int c,
                                                 uint32_t t) {
@@ -1066,14 +1095,14 @@ __device__ __forceinline__ void prolong_add4_at(const float* eb, const SGeo& C, 
       // slots (m0 >> 1) and the next of both colours as 8-byte loads (the
       // row offset is even: H and m0 >> 1 are), in bounds even where they
       // lie past the row's last node (padding), which the guards zero
-      const float2 a01 = *reinterpret_cast<const float2*>(A);
-      const float2 b01 = *reinterpret_cast<const float2*>(Bc);
+      const float2 a01 = ld2<CG>(A);
+      const float2 b01 = ld2<CG>(Bc);
       float cv[5];
       cv[0] = a01.x;
       cv[1] = m0 + 1 < C.nz ? b01.x : 0.f;
       cv[2] = m0 + 2 < C.nz ? a01.y : 0.f;
       cv[3] = m0 + 3 < C.nz ? b01.y : 0.f;
-      cv[4] = m0 + 4 < C.nz ? A[2] : 0.f;
+      cv[4] = m0 + 4 < C.nz ? ld1<CG>(A + 2) : 0.f;
       const float w = xw[a] * yw[b];
 #pragma unroll
       for (int u = 0; u < 4; u++) {
@@ -1085,7 +1114,7 @@ __device__ __forceinline__ void prolong_add4_at(const float* eb, const SGeo& C, 
     }
   if (mk.x & mk.y & mk.z & mk.w) return;  // metal or unused: nothing to add
   float4* out = reinterpret_cast<float4*>(efb + (size_t)c * F.csz + base);
-  float4 v = *out;
+  float4 v = ld4<CG>(reinterpret_cast<const float*>(out));
   v.x += mv[0] ? 0.f : acc[0];
   v.y += mv[1] ? 0.f : acc[1];
   v.z += mv[2] ? 0.f : acc[2];
@@ -1103,64 +1132,115 @@ k_prolong_add4(const float* __restrict__ ec, SGeo C, float* __restrict__ ef,
                   maskf + (size_t)blockIdx.y * F.msplit, F, blockIdx.z, t);
 }
 
-// The coarsest level's SOR pairs for one problem, by the calling CTA
-// (kBottomThreads threads, all of which must call it): eb (out), gb and
-// mask the problem's split arrays, se and sg shared scratch of kBottomMax
-// floats each.
+// The coarsest level's SOR pairs for one problem, by the calling CTA (NT
+// threads, all of which must call it): eb (out), gb and mask the problem's
+// split arrays, se shared scratch of kBottomMax floats.  The free nodes of
+// each colour are listed first, in their order, so that a thread has one node
+// of either colour and a half-sweep no idle lanes among its warps' active
+// ones; a node's neighbour slots, its right-hand side and its own value (no
+// other thread writes it) stay in registers.  In se the nodes of even and of
+// odd index lie apart: a colour's neighbours are then next to each other for
+// the threads of a warp, where the natural order made every load a 2-way bank
+// conflict.  What is left of a half-sweep is the barrier and one round of
+// shared loads and sums: 9^3 nodes, 40 pairs, 22.7e3 -> 17.2e3 clocks.  (A
+// barrier of the occupied warps alone was slower, 18.5e3.)
+__device__ __forceinline__ int bottom_slot(int t) {
+  return (t >> 1) + (t & 1) * (kBottomMax / 2);
+}
+template <int NT, bool CG = false>
 __device__ __forceinline__ void bottom_at(float* eb, const float* gb, const uint8_t* mask,
-                                          const SGeo& G, float omega, int pairs, float* se,
-                                          float* sg) {
-  // A thread's nodes (at most kBottomMax / kBottomThreads): their colour,
-  // whether they are free, and their six neighbours' slots, worked out once
-  // so that the pairs below run on shared memory alone.
-  constexpr int NPT = kBottomMax / kBottomThreads;
-  int nbr[NPT][6];
-  int col[NPT];
+                                          const SGeo& G, float omega, int pairs, float* se) {
+  static_assert(NT % 32 == 0 && 2 * NT >= kBottomMax, "one node of either colour a thread");
+  constexpr int kU = (kBottomMax + NT - 1) / NT, kW = NT / 32;
+  constexpr int kRuns = (kU * kW + 31) / 32;
+  __shared__ uint16_t list[2][kBottomMax / 2];
+  __shared__ uint16_t run[2][kRuns * 32];  // free nodes in each warp's run of 32
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q = threadIdx.x; q < 2 * kRuns * 32; q += NT) (&run[0][0])[q] = 0;
+  __syncthreads();
+  unsigned m[kU][2];
 #pragma unroll
-  for (int u = 0; u < NPT; u++) {
-    const uint32_t t = threadIdx.x + (uint32_t)u * kBottomThreads;
-    col[u] = -1;  // no node, or metal: never updated
+  for (int u = 0; u < kU; u++) {
+    const uint32_t t = threadIdx.x + (uint32_t)u * NT;
+    int col = -1;  // no node, or metal: never updated
     if (t < G.n) {
-      const int k = (int)(t % G.nz);
-      const int j = (int)((t / G.nz) % G.ny);
-      const int i = (int)(t / ((uint32_t)G.nz * G.ny));
+      const uint32_t ij = fdivu(t, G.dnz);
+      const int k = (int)(t - ij * G.dnz.d);
+      const int i = (int)fdivu(ij, G.dny);
+      const int j = (int)(ij - (uint32_t)i * G.dny.d);
       const int c = scol(i, j, k);
-      const uint32_t sl = sidx(G, i, j, k);
-      se[t] = 0.f;
-      sg[t] = gb[(size_t)c * G.csz + sl];
-      if (!mask[(size_t)c * G.csz + sl]) col[u] = c;
-      nbr[u][0] = (lo_i(i, G.nx) * G.ny + j) * G.nz + k;
-      nbr[u][1] = (hi_i(i, G.nx) * G.ny + j) * G.nz + k;
-      nbr[u][2] = (i * G.ny + lo_i(j, G.ny)) * G.nz + k;
-      nbr[u][3] = (i * G.ny + hi_i(j, G.ny)) * G.nz + k;
-      nbr[u][4] = (i * G.ny + j) * G.nz + lo_i(k, G.nz);
-      nbr[u][5] = (i * G.ny + j) * G.nz + hi_i(k, G.nz);
+      se[bottom_slot((int)t)] = 0.f;
+      if (!mask[(size_t)c * G.csz + sidx(G, i, j, k)]) col = c;
+    }
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      m[u][c] = __ballot_sync(0xffffffffu, col == c);
+      if (lane == 0) run[c][u * kW + warp] = (uint16_t)__popc(m[u][c]);
     }
   }
   __syncthreads();
-  for (int it = 0; it < pairs; it++) {
-    for (int c = 0; c < 2; c++) {
+  int count[2] = {0, 0};
 #pragma unroll
-      for (int u = 0; u < NPT; u++) {
-        if (col[u] != c) continue;
-        const uint32_t t = threadIdx.x + (uint32_t)u * kBottomThreads;
-        const float q = ((((se[nbr[u][0]] + se[nbr[u][1]]) + (se[nbr[u][2]] + se[nbr[u][3]])) +
-                          (se[nbr[u][4]] + se[nbr[u][5]])) -
-                         sg[t]) *
+  for (int c = 0; c < 2; c++) {
+    int base[kU];
+#pragma unroll
+    for (int u = 0; u < kU; u++) base[u] = __popc(m[u][c] & ((1u << lane) - 1u));
+#pragma unroll
+    for (int q = 0; q < kRuns; q++) {
+      const int v = run[c][q * 32 + lane];
+      count[c] += (int)__reduce_add_sync(0xffffffffu, (unsigned)v);
+#pragma unroll
+      for (int u = 0; u < kU; u++)
+        base[u] += (int)__reduce_add_sync(0xffffffffu,
+                                          q * 32 + lane < u * kW + warp ? (unsigned)v : 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; u++)
+      if ((m[u][c] >> lane) & 1u) list[c][base[u]] = (uint16_t)(threadIdx.x + u * NT);
+  }
+  __syncthreads();
+  int own[2], nbr[2][6];
+  float ev[2] = {0.f, 0.f}, gv[2];
+#pragma unroll
+  for (int c = 0; c < 2; c++) {
+    const bool has = (int)threadIdx.x < count[c];
+    const uint32_t t = has ? list[c][threadIdx.x] : 0u;
+    const uint32_t ij = fdivu(t, G.dnz);
+    const int k = (int)(t - ij * G.dnz.d);
+    const int i = (int)fdivu(ij, G.dny);
+    const int j = (int)(ij - (uint32_t)i * G.dny.d);
+    own[c] = has ? bottom_slot((int)t) : -1;
+    gv[c] = has ? ld1<CG>(gb + (size_t)c * G.csz + sidx(G, i, j, k)) : 0.f;
+    nbr[c][0] = bottom_slot((lo_i(i, G.nx) * G.ny + j) * G.nz + k);
+    nbr[c][1] = bottom_slot((hi_i(i, G.nx) * G.ny + j) * G.nz + k);
+    nbr[c][2] = bottom_slot((i * G.ny + lo_i(j, G.ny)) * G.nz + k);
+    nbr[c][3] = bottom_slot((i * G.ny + hi_i(j, G.ny)) * G.nz + k);
+    nbr[c][4] = bottom_slot((i * G.ny + j) * G.nz + lo_i(k, G.nz));
+    nbr[c][5] = bottom_slot((i * G.ny + j) * G.nz + hi_i(k, G.nz));
+  }
+  for (int it = 0; it < pairs; it++) {
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      if (own[c] >= 0) {
+        const float q = ((((se[nbr[c][0]] + se[nbr[c][1]]) + (se[nbr[c][2]] + se[nbr[c][3]])) +
+                          (se[nbr[c][4]] + se[nbr[c][5]])) -
+                         gv[c]) *
                         (1.0f / 6.0f);
-        se[t] += omega * (q - se[t]);
+        ev[c] += omega * (q - ev[c]);
+        se[own[c]] = ev[c];
       }
       __syncthreads();
     }
   }
 #pragma unroll
-  for (int u = 0; u < NPT; u++) {
-    const uint32_t t = threadIdx.x + (uint32_t)u * kBottomThreads;
+  for (int u = 0; u < kU; u++) {
+    const uint32_t t = threadIdx.x + (uint32_t)u * NT;
     if (t < G.n) {
-      const int k = (int)(t % G.nz);
-      const int j = (int)((t / G.nz) % G.ny);
-      const int i = (int)(t / ((uint32_t)G.nz * G.ny));
-      eb[(size_t)scol(i, j, k) * G.csz + sidx(G, i, j, k)] = se[t];
+      const uint32_t ij = fdivu(t, G.dnz);
+      const int k = (int)(t - ij * G.dnz.d);
+      const int i = (int)fdivu(ij, G.dny);
+      const int j = (int)(ij - (uint32_t)i * G.dny.d);
+      eb[(size_t)scol(i, j, k) * G.csz + sidx(G, i, j, k)] = se[bottom_slot((int)t)];
     }
   }
 }
@@ -1172,9 +1252,8 @@ k_bottom(float* __restrict__ e, const float* __restrict__ g,
          const uint8_t* __restrict__ mask, SGeo G, float omega, int pairs,
          size_t pstride) {
   __shared__ float se[kBottomMax];
-  __shared__ float sg[kBottomMax];
-  bottom_at(e + blockIdx.x * pstride, g + blockIdx.x * pstride,
-            mask + (size_t)blockIdx.x * G.msplit, G, omega, pairs, se, sg);
+  bottom_at<kBottomThreads>(e + blockIdx.x * pstride, g + blockIdx.x * pstride,
+                            mask + (size_t)blockIdx.x * G.msplit, G, omega, pairs, se);
 }
 
 // The cycle of the level just above the bottom, the bottom solve included,
@@ -1183,21 +1262,19 @@ k_bottom(float* __restrict__ e, const float* __restrict__ g,
 // launches of a few blocks that the separate kernels take on these small
 // grids -- each a few microseconds of latency -- become one.  The phases
 // are the device code of those kernels (zero_pair_at, gs4_group,
-// resid0_4_at, restrict0_4_at, bottom_at, prolong_add4_at) over the CTA's
+// resid0_4_at, restrict0_at, bottom_at, prolong_add4_at) over the CTA's
 // threads, in their order, so the result has their bits.  Shared memory:
-// the bottom's scratch (2 kBottomMax floats), the level's correction and
+// the bottom's scratch (kBottomMax floats), the level's correction and
 // right-hand side (2 csz floats each), its colour-0 residual (csz floats),
 // the bottom's correction and right-hand side (2 csz_b floats each), then
 // both masks (2 csz + 2 csz_b bytes); tail_smem_bytes() gives the total.
-__global__ void __launch_bounds__(kBottomThreads)
-k_tail_cycle(float* __restrict__ e, const float* __restrict__ g,
-             const uint8_t* __restrict__ mask, SGeo A, size_t apstride,
-             const uint8_t* __restrict__ bmask, SGeo Bt, int nu1, int nu2, float omega_b,
-             int pairs) {
-  extern __shared__ float4 tail_smem[];
-  float* se = reinterpret_cast<float*>(tail_smem);
-  float* sg = se + kBottomMax;
-  float* ae = sg + kBottomMax;
+template <int NT, bool CG>
+__device__ __forceinline__ void tail_cycle_at(float* eA, const float* gA, const uint8_t* mA,
+                                              const SGeo& A, const uint8_t* mB, const SGeo& Bt,
+                                              int nu1, int nu2, float omega_b, int pairs,
+                                              float4* smem) {
+  float* se = reinterpret_cast<float*>(smem);
+  float* ae = se + kBottomMax;
   float* ag = ae + 2 * (size_t)A.csz;
   float* ar = ag + 2 * (size_t)A.csz;
   float* be = ar + (size_t)A.csz;
@@ -1205,58 +1282,177 @@ k_tail_cycle(float* __restrict__ e, const float* __restrict__ g,
   uint8_t* am = reinterpret_cast<uint8_t*>(bg + 2 * (size_t)Bt.csz);
   uint8_t* bm = am + 2 * (size_t)A.csz;
   const uint32_t tid = threadIdx.x;
-  const float* gA = g + blockIdx.x * apstride;
-  const uint8_t* mA = mask + (size_t)blockIdx.x * A.msplit;
-  const uint8_t* mB = bmask + (size_t)blockIdx.x * Bt.msplit;
   const uint32_t na4 = (2 * A.csz) >> 2, nb4 = (2 * Bt.csz) >> 2;
-  for (uint32_t q = tid; q < na4; q += kBottomThreads) {
-    reinterpret_cast<float4*>(ag)[q] = ld4(gA + 4 * (size_t)q);
+  for (uint32_t q = tid; q < na4; q += NT) {
+    reinterpret_cast<float4*>(ag)[q] = ld4<CG>(gA + 4 * (size_t)q);
     reinterpret_cast<uchar4*>(am)[q] = reinterpret_cast<const uchar4*>(mA)[q];
   }
-  for (uint32_t q = tid; q < nb4; q += kBottomThreads)
+  for (uint32_t q = tid; q < nb4; q += NT)
     reinterpret_cast<uchar4*>(bm)[q] = reinterpret_cast<const uchar4*>(mB)[q];
   __syncthreads();
   const uint32_t nq = A.csz >> 2;
   // pre-smoothing: the fused first pair from e = 0, then nu1 - 1 pairs
-  for (uint32_t t = tid; t < nq; t += kBottomThreads) zero_pair_at<false>(ae, ag, am, A, t);
+  for (uint32_t t = tid; t < nq; t += NT) zero_pair_at<false>(ae, ag, am, A, t);
   __syncthreads();
   for (int q = 1; q < nu1; q++)
     for (int c = 0; c < 2; c++) {
-      for (uint32_t t = tid; t < nq; t += kBottomThreads)
+      for (uint32_t t = tid; t < nq; t += NT)
         gs4_group<false>(ae + (size_t)c * A.csz, ae + (size_t)(1 - c) * A.csz,
                          ag + (size_t)c * A.csz, am + (size_t)c * A.csz, A, c, 1.f, t);
       __syncthreads();
     }
   // the colour-0 residual, restricted to the bottom's right-hand side
-  for (uint32_t t = tid; t < nq; t += kBottomThreads) resid0_4_at(ae, ag, am, A, ar, t);
+  for (uint32_t t = tid; t < nq; t += NT) resid0_4_at(ae, ag, am, A, ar, t);
   __syncthreads();
-  const uint32_t nr = (uint32_t)Bt.nx * Bt.ny * ((uint32_t)(Bt.nz + 3) >> 2);
-  for (uint32_t t = tid; t < nr; t += kBottomThreads) restrict0_4_at(ar, A, bg, Bt, t);
+  for (uint32_t t = tid; t < Bt.n; t += NT) restrict0_at(ar, A, bg, Bt, t);
   __syncthreads();
-  bottom_at(be, bg, bm, Bt, omega_b, pairs, se, sg);
+  bottom_at<NT>(be, bg, bm, Bt, omega_b, pairs, se);
   __syncthreads();
   // colour 0 takes the prolonged correction (the first post-smoothing
   // half-sweep, colour 1, rewrites every free colour-1 slot)
-  for (uint32_t t = tid; t < nq; t += kBottomThreads) prolong_add4_at(be, Bt, ae, am, A, 0, t);
+  for (uint32_t t = tid; t < nq; t += NT) prolong_add4_at(be, Bt, ae, am, A, 0, t);
   __syncthreads();
   for (int q = 0; q < nu2; q++)
     for (int c = 1; c >= 0; c--) {
-      for (uint32_t t = tid; t < nq; t += kBottomThreads)
+      for (uint32_t t = tid; t < nq; t += NT)
         gs4_group<false>(ae + (size_t)c * A.csz, ae + (size_t)(1 - c) * A.csz,
                          ag + (size_t)c * A.csz, am + (size_t)c * A.csz, A, c, 1.f, t);
       __syncthreads();
     }
-  float* eA = e + blockIdx.x * apstride;
-  for (uint32_t q = tid; q < na4; q += kBottomThreads)
+  for (uint32_t q = tid; q < na4; q += NT)
     reinterpret_cast<float4*>(eA)[q] = reinterpret_cast<const float4*>(ae)[q];
+}
+
+__global__ void __launch_bounds__(kBottomThreads)
+k_tail_cycle(float* __restrict__ e, const float* __restrict__ g,
+             const uint8_t* __restrict__ mask, SGeo A, size_t apstride,
+             const uint8_t* __restrict__ bmask, SGeo Bt, int nu1, int nu2, float omega_b,
+             int pairs) {
+  extern __shared__ float4 tail_smem[];
+  tail_cycle_at<kBottomThreads, false>(
+      e + blockIdx.x * apstride, g + blockIdx.x * apstride,
+      mask + (size_t)blockIdx.x * A.msplit, A, bmask + (size_t)blockIdx.x * Bt.msplit, Bt, nu1,
+      nu2, omega_b, pairs, tail_smem);
 }
 
 // Shared bytes k_tail_cycle needs for level A above the bottom Bt.
 inline size_t tail_smem_bytes(const SGeo& A, const SGeo& Bt) {
-  return 4 * (2 * (size_t)kBottomMax + 5 * (size_t)A.csz + 4 * (size_t)Bt.csz) +
+  return 4 * ((size_t)kBottomMax + 5 * (size_t)A.csz + 4 * (size_t)Bt.csz) +
          2 * (size_t)A.csz + 2 * (size_t)Bt.csz;
 }
 constexpr size_t kTailSmemMax = 200 * 1024;
+
+// ---- the small levels of a cycle in one launch ------------------------------
+//
+// A level of some 10^4 nodes a problem is ten launches of 2 to 6 us each
+// (33^3 in a batch of eight: 60 % of a cycle's time), two to three of which
+// are the launch itself.  Here a cluster of CTAs per problem walks the cycle
+// from such a level down: the phases are the separate kernels' device code
+// over the cluster's threads, with values that other CTAs write read from L2
+// and a cluster barrier (0.25 us, with the L2 round trip about one) between
+// phases, and the last level above the bottom and the bottom are CTA 0's in
+// shared memory (tail_cycle_at).  Every expression and its order are the
+// launches', so the bits are.
+constexpr int kMTailLevels = 6, kMTailCtas = 8, kMTailThreads = 640;
+struct MTailLevel {
+  float *e, *g, *r;
+  const uint8_t* mask;
+  SGeo G;
+  size_t pstride;
+  int visits;  // of the next level, per visit of this one
+};
+struct MTailArgs {
+  MTailLevel lv[kMTailLevels];
+  int n, nu1, nu2, pairs, zero;
+  float omega_b;
+};
+
+__global__ void __launch_bounds__(kMTailThreads)
+k_tail_cluster(const __grid_constant__ MTailArgs A) {
+  namespace cg = cooperative_groups;
+  extern __shared__ float4 tail_smem[];
+  cg::cluster_group cl = cg::this_cluster();
+  const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const uint32_t gn = (uint32_t)(ctas * kMTailThreads);
+  const uint32_t gt = (uint32_t)(rank * kMTailThreads) + threadIdx.x;
+  const size_t b = blockIdx.x / (unsigned)ctas;  // the problem
+  int left[kMTailLevels];
+  int l = 0;
+  bool zero = A.zero != 0, down = true;
+  while (true) {
+    const MTailLevel& L = A.lv[l];
+    const SGeo& G = L.G;
+    float* e = L.e + b * L.pstride;
+    float* g = L.g + b * L.pstride;
+    float* r = L.r + b * (size_t)G.csz;
+    const uint8_t* m = L.mask + b * (size_t)G.msplit;
+    const uint32_t nq = G.csz >> 2;
+    auto sweep = [&](int c) {
+      for (uint32_t t = gt; t < nq; t += gn)
+        gs4_group<false, true>(e + (size_t)c * G.csz, e + (size_t)(1 - c) * G.csz,
+                               g + (size_t)c * G.csz, m + (size_t)c * G.csz, G, c, 1.f, t);
+      cl.sync();
+    };
+    if (down) {
+      if (l + 1 == A.n) {
+        if (rank == 0)
+          bottom_at<kMTailThreads, true>(e, g, m, G, A.omega_b, A.pairs,
+                                         reinterpret_cast<float*>(tail_smem));
+        cl.sync();
+        l--;
+        down = false;
+        continue;
+      }
+      if (l + 2 == A.n && zero) {
+        if (rank == 0) {
+          const MTailLevel& Bt = A.lv[l + 1];
+          tail_cycle_at<kMTailThreads, true>(e, g, m, G, Bt.mask + b * (size_t)Bt.G.msplit, Bt.G,
+                                             A.nu1, A.nu2, A.omega_b, A.pairs, tail_smem);
+        }
+        cl.sync();
+        if (l == 0) break;
+        l--;
+        down = false;
+        continue;
+      }
+      if (zero) {
+        for (uint32_t t = gt; t < nq; t += gn) zero_pair_at<false, true>(e, g, m, G, t);
+        cl.sync();
+      }
+      for (int q = zero ? 1 : 0; q < A.nu1; q++) {
+        sweep(0);
+        sweep(1);
+      }
+      for (uint32_t t = gt; t < nq; t += gn) resid0_4_at<true>(e, g, m, G, r, t);
+      cl.sync();
+      const MTailLevel& C = A.lv[l + 1];
+      for (uint32_t t = gt; t < C.G.n; t += gn)
+        restrict0_at<true>(r, G, C.g + b * C.pstride, C.G, t);
+      cl.sync();
+      left[l] = L.visits;
+      l++;
+      zero = true;
+      continue;
+    }
+    // back from a visit of the next level
+    if (--left[l] > 0) {
+      l++;
+      zero = false;
+      down = true;
+      continue;
+    }
+    const MTailLevel& C = A.lv[l + 1];
+    for (uint32_t t = gt; t < nq; t += gn)
+      prolong_add4_at<true>(C.e + b * C.pstride, C.G, e, m, G, 0, t);
+    cl.sync();
+    for (int q = 0; q < A.nu2; q++) {
+      sweep(1);
+      sweep(0);
+    }
+    if (l == 0) break;
+    l--;
+  }
+}
 
 // Coarse metal of the FP32 correction's hierarchy: injection with a rescue
 // of thin metal.  Coarse node (i, j, k) is metal when fine node
@@ -2263,8 +2459,10 @@ struct Session {
   int tb_levels = 0;
   int tb_max = 6;  // half-sweeps per blocked pass (2, 4 or 6); longer phases split
   bool tb_auto = true;  // the tuner picks tb_levels / tb_max (no environment override)
-  bool tail_on = true;   // k_tail_cycle allowed (IG_MIXED_TAIL=0: the separate launches)
+  bool tail_on = true;   // k_tail_cycle and k_tail_cluster allowed (IG_MIXED_TAIL=0: the separate launches)
   bool tail_ok = false;  // ... and usable on this hierarchy
+  size_t tail_top = 0;   // the finest level that runs as k_tail_cluster (0: none)
+  int tail_ctas = 0;     // its CTAs per problem
   double last_solve_bytes = 0.0;  // algorithmic bytes of the last solve's steps
   int rows_force = -1;  // rows per warp of the residual and update: -1 by rule (flat_rows)
 
@@ -2548,11 +2746,72 @@ struct Session {
         MK(cudaFuncSetAttribute(k_tail_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kTailSmemMax));
     }
+    update_tail_cluster();
   }
 
   // level l's cycle from zero runs as k_tail_cycle (l the last level above
   // the bottom, no temporal blocking there)
   bool tail_level(size_t l) const { return tail_ok && l + 2 == lv.size() && !use_tb(l); }
+
+  // The finest level whose cycle runs as k_tail_cluster: at least two levels
+  // above the bottom (one is k_tail_cycle's), at most kMTailNodes nodes a
+  // problem -- up to there the phases wait for their barriers and loads,
+  // which a launch's few microseconds exceed; past it the launched kernels'
+  // 152 SMs win.  Eight 65^3 decks (levels 33^3 to 9^3): 4.52 -> 4.06 ms a
+  // solve; eight 193 x 193 x 385 bases 37.9 -> 37.5; 24 bases of a
+  // 256 x 64 x 48 board 12.1 -> 11.7.  Threads: 640 and 768 measure alike, 896 is slower (its
+  // barriers are).
+  static constexpr size_t kMTailNodes = 65536;
+  void update_tail_cluster() {
+    tail_top = 0;
+    tail_ctas = 0;
+    if (!tail_ok) return;
+    size_t top = lv.size() - 2;
+    while (top > 1 && lv[top - 1].d.n() <= kMTailNodes && lv.size() - (top - 1) <= kMTailLevels &&
+           !flat(lv[top - 1]))
+      top--;
+    if (top < 1 || top + 2 >= lv.size() || (int)top < tb_levels) return;
+    // CTAs: a group of slots a thread at most, as far as a cluster goes
+    const uint32_t groups = lv[top].G.csz / 4;
+    int n = 1;
+    while (n < kMTailCtas && (uint32_t)(n * kMTailThreads) < groups) n *= 2;
+    if (cudaFuncSetAttribute(k_tail_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kTailSmemMax) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    tail_top = top;
+    tail_ctas = n;
+  }
+  bool tail_cluster(size_t l) const { return tail_top > 0 && l == tail_top && !use_tb(l); }
+
+  void launch_tail_cluster(bool zero) {
+    MTailArgs A;
+    A.n = (int)(lv.size() - tail_top);
+    for (int q = 0; q < A.n; q++) {
+      MLevel& L = lv[tail_top + q];
+      A.lv[q] = MTailLevel{L.e.p, L.g.p, L.r.p, L.mask.p, L.G, L.pstride,
+                           coarse_visits(tail_top + q)};
+    }
+    A.nu1 = nu1;
+    A.nu2 = nu2;
+    A.pairs = bottom_pairs;
+    A.zero = zero ? 1 : 0;
+    A.omega_b = bottom_omega;
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at[1];
+    c.gridDim = dim3((unsigned)(B * tail_ctas));
+    c.blockDim = dim3(kMTailThreads);
+    c.dynamicSmemBytes = tail_smem_bytes(lv[lv.size() - 2].G, lv.back().G);
+    c.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)tail_ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    MK(cudaLaunchKernelEx(&c, k_tail_cluster, A));
+  }
 
   bool fuse_zero_pair(const MLevel& a) const {
     return nu1 >= 1 && smooth_omega == 1.f && !flat(a);
@@ -2572,6 +2831,10 @@ struct Session {
     if (l + 1 == lv.size()) {
       k_bottom<<<B, kBottomThreads, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, bottom_omega,
                                             bottom_pairs, a.pstride);
+      return;
+    }
+    if (tail_cluster(l)) {
+      launch_tail_cluster(zero);
       return;
     }
     if (zero && tail_level(l)) {
@@ -2823,7 +3086,7 @@ struct Session {
 
   long cycle_launches(size_t l, bool zero) const {
     if (l + 1 == lv.size()) return 1;
-    if (zero && tail_level(l)) return 1;
+    if (tail_cluster(l) || (zero && tail_level(l))) return 1;
     const int reps = coarse_visits(l);
     long n = 3;                                         // residual, restriction, prolongation
     if (tb_pre(l, zero)) n += tb_passes(2 * nu1);
@@ -3099,7 +3362,7 @@ int open_session(const uint8_t* metal, int nmetal, long nx, long ny, long nz,
     if (const char* v = std::getenv("IG_MIXED_DOT")) S->dot_on = std::atoi(v) != 0;
     // IG_MIXED_FOLD=0: the flexible CG's updates by separate launches
     if (const char* v = std::getenv("IG_MIXED_FOLD")) S->fold_on = std::atoi(v) != 0;
-    // IG_MIXED_TAIL=0: the last level above the bottom by separate launches
+    // IG_MIXED_TAIL=0: the small levels by separate launches
     if (const char* v = std::getenv("IG_MIXED_TAIL")) S->tail_on = std::atoi(v) != 0;
     // IG_MIXED_TB_LEVELS: how many of the finest levels smooth temporally
     // blocked, fixed instead of left to the smoother tuner
