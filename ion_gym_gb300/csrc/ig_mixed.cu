@@ -696,18 +696,12 @@ k_resid0(const float* __restrict__ e, const float* __restrict__ g,
 // k_resid0 over float4 groups (grids with no size-1 axis): the same
 // expressions per slot, 16-byte loads of the colour-1 neighbour rows, one
 // float4 store of r.
-// Float4 group t of the colour-0 residual, one problem: eb, gb, mask its
-// split arrays, rb its colour-0 residual (csz floats).
+// Float4 group of row (i, j) from slot m0 (base its first slot) of the
+// colour-0 residual, one problem: eb, gb, mask its split arrays.
 template <bool CG = false>
-__device__ __forceinline__ void resid0_4_at(const float* eb, const float* gb,
-                                            const uint8_t* mask, const SGeo& G, float* rb,
-                                            uint32_t t) {
-  const uint32_t ij = fdivu(t, G.dH4);
-  const int m0 = 4 * (int)(t - ij * G.dH4.d);
-  const int i = (int)fdivu(ij, G.dny);
-  const int j = (int)(ij - (uint32_t)i * G.dny.d);
-  const uint32_t base = ij * (uint32_t)G.H + m0;
-  float4* out = reinterpret_cast<float4*>(rb + base);
+__device__ __forceinline__ float4 resid0_group(const float* eb, const float* gb,
+                                               const uint8_t* mask, const SGeo& G, int i, int j,
+                                               int m0, uint32_t base) {
   // no early exit on an all-metal group: the loads are in bounds in every
   // group and go out with the mask's; metal slots select 0 below
   const uchar4 mk = *reinterpret_cast<const uchar4*>(mask + base);
@@ -722,7 +716,20 @@ __device__ __forceinline__ void resid0_4_at(const float* eb, const float* gb,
     const float a = q[u] - 6.0f * es[u];
     o[u] = mv[u] ? 0.f : gv[u] - a;
   }
-  *out = make_float4(o[0], o[1], o[2], o[3]);
+  return make_float4(o[0], o[1], o[2], o[3]);
+}
+
+// Float4 group t of it, to the problem's colour-0 residual rb (csz floats).
+template <bool CG = false>
+__device__ __forceinline__ void resid0_4_at(const float* eb, const float* gb,
+                                            const uint8_t* mask, const SGeo& G, float* rb,
+                                            uint32_t t) {
+  const uint32_t ij = fdivu(t, G.dH4);
+  const int m0 = 4 * (int)(t - ij * G.dH4.d);
+  const int i = (int)fdivu(ij, G.dny);
+  const int j = (int)(ij - (uint32_t)i * G.dny.d);
+  const uint32_t base = ij * (uint32_t)G.H + m0;
+  *reinterpret_cast<float4*>(rb + base) = resid0_group<CG>(eb, gb, mask, G, i, j, m0, base);
 }
 
 __global__ void __launch_bounds__(kT)
@@ -889,6 +896,178 @@ k_restrict0_4(const float* __restrict__ r0, SGeo F, float* __restrict__ gc, SGeo
   const uint32_t t = blockIdx.x * kT + threadIdx.x;
   if (t >= (uint32_t)C.nx * C.ny * ((uint32_t)(C.nz + 3) >> 2)) return;
   restrict0_4_at(r0 + blockIdx.y * (size_t)F.csz, F, gc + blockIdx.y * cstride, C, t);
+}
+
+// k_resid0_4 and k_restrict0_4 in one pass: the residual goes no further than
+// shared memory.  A block has TJ coarse rows of coarse planes [ic0, ic0 + MI)
+// and marches along i: of the fine planes 2ic - 1, 2ic, 2ic + 1 that coarse
+// plane ic needs, the first is the last step's, so a step forms two planes of
+// 2 TJ + 1 rows (one of them shared with the next block), a float4 group a
+// thread, and then sums.  A thread keeps its group's colour-1 values of the
+// planes around in registers: read through L1 as k_resid0_4 does they come
+// from L2 three times beside this much shared memory.  A ring of five planes
+// lets a warp form the next two while others still sum.  The expressions and
+// the taps' order are those of the two kernels, clamped taps included, so the
+// bits are.  The residual's store and second reading (a third of the two
+// kernels' bytes) and a launch are gone: fine level of eight 193 x 193 x 385,
+// 286 -> 214 us; of 24 of 256 x 64 x 48, 58 -> 43; of 257^3, 54 -> 35; of
+// eight 65^3, 11.7 -> 6.8.  (The same without the registers: 229, 47, 42,
+// 8.9.)
+constexpr int kRrThreads = 512;
+__global__ void __launch_bounds__(kRrThreads, 2)
+k_resid_restrict0(const float* __restrict__ e, const float* __restrict__ g,
+                  const uint8_t* __restrict__ mask, SGeo F, float* __restrict__ gc, SGeo C,
+                  size_t fstride, size_t cstride, int TJ, int MI, int jtiles) {
+  extern __shared__ float4 rr_smem[];
+  float* ring = reinterpret_cast<float*>(rr_smem);
+  const int NR = 2 * TJ + 1;
+  const uint32_t plane = (uint32_t)NR * F.H;
+  const int it = (int)(blockIdx.x / (unsigned)jtiles);
+  const int jc0 = (int)(blockIdx.x - (unsigned)it * (unsigned)jtiles) * TJ;
+  const int ic0 = it * MI, ic1 = min(ic0 + MI, C.nx);
+  const int jf0 = 2 * jc0 - 1;  // the fine row of the ring's row 0
+  const float* e0 = e + blockIdx.y * fstride;
+  const float* e1 = e0 + F.csz;
+  const float* gb = g + blockIdx.y * fstride;
+  const uint8_t* mb = mask + (size_t)blockIdx.y * F.msplit;
+  float* cb = gc + blockIdx.y * cstride;
+  const uint32_t C4 = (uint32_t)(C.nz + 3) >> 2, nc = (uint32_t)TJ * C4;
+  // this thread's group
+  const uint32_t row = fdivu(threadIdx.x, F.dH4);
+  const int m0 = 4 * (int)(threadIdx.x - row * F.dH4.d);
+  const int j = jf0 + (int)row;
+  const bool mine = (int)row < NR && j >= 0 && j < F.ny;
+  const int jj0 = mine ? j : 0;
+  const uint32_t ps = (uint32_t)F.ny * F.H;  // a plane's slots
+  const uint32_t o = (uint32_t)jj0 * F.H + m0;
+  const uint32_t olo = (uint32_t)lo_i(jj0, F.ny) * F.H + m0;
+  const uint32_t ohi = (uint32_t)hi_i(jj0, F.ny) * F.H + m0;
+  struct In {
+    float4 ym, yp, ev, gg;
+    uchar4 mk;
+    float z;
+  };
+  auto load = [&](int i) {
+    In v;
+    const uint32_t b = (uint32_t)i * ps;
+    v.ym = ld4(e1 + b + olo);
+    v.yp = ld4(e1 + b + ohi);
+    v.ev = ld4(e0 + b + o);
+    v.gg = ld4(gb + b + o);
+    v.mk = *reinterpret_cast<const uchar4*>(mb + b + o);
+    const int p = (i + j) & 1;
+    v.z = 0.f;
+    if (p == 0 ? m0 > 0 : m0 + 4 < F.H) v.z = e1[b + o + (p == 0 ? -1 : 4)];
+    return v;
+  };
+  auto form = [&](int i, const In& v, const float4& xm, const float4& zc, const float4& xp) {
+    const int p = (i + j) & 1;
+    float z[5];
+    if (p == 0) {
+      z[0] = m0 > 0 ? v.z : zc.x;
+      z[1] = zc.x; z[2] = zc.y; z[3] = zc.z; z[4] = zc.w;
+    } else {
+      z[0] = zc.x; z[1] = zc.y; z[2] = zc.z; z[3] = zc.w; z[4] = v.z;
+    }
+    const int utop = F.nz - 1 - p - 2 * m0;  // 2u == utop: node nz-1
+    const float sx[4] = {(xm.x + xp.x) + (v.ym.x + v.yp.x), (xm.y + xp.y) + (v.ym.y + v.yp.y),
+                         (xm.z + xp.z) + (v.ym.z + v.yp.z), (xm.w + xp.w) + (v.ym.w + v.yp.w)};
+    const float es[4] = {v.ev.x, v.ev.y, v.ev.z, v.ev.w};
+    const float gv[4] = {v.gg.x, v.gg.y, v.gg.z, v.gg.w};
+    const uint8_t mv[4] = {v.mk.x, v.mk.y, v.mk.z, v.mk.w};
+    float r[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const float q = sx[u] + (z[u] + (2 * u == utop ? z[u] : z[u + 1]));
+      const float a = q - 6.0f * es[u];
+      r[u] = mv[u] ? 0.f : gv[u] - a;
+    }
+    *reinterpret_cast<float4*>(ring + (uint32_t)(i % 5) * plane + row * F.H + m0) =
+        make_float4(r[0], r[1], r[2], r[3]);
+  };
+  float4 em = make_float4(0.f, 0.f, 0.f, 0.f), ec = em;  // e1 of planes 2ic - 1, 2ic
+  if (mine) {
+    ec = ld4(e1 + (uint32_t)(2 * ic0) * ps + o);
+    if (ic0 > 0) {
+      const int i = 2 * ic0 - 1;
+      const In v = load(i);
+      const float4 x0 = ld4(e1 + (uint32_t)(i - 1) * ps + o);
+      em = ld4(e1 + (uint32_t)i * ps + o);
+      form(i, v, x0, em, ec);
+    }
+  }
+  for (int ic = ic0; ic < ic1; ic++) {
+    if (mine) {
+      const int i = 2 * ic;
+      const bool two = i + 1 < F.nx;
+      const In v0 = load(i);
+      float4 en = em, e2 = ec;  // past the face: the plane before
+      In v1;
+      if (two) {
+        en = ld4(e1 + (uint32_t)(i + 1) * ps + o);
+        if (i + 2 < F.nx) e2 = ld4(e1 + (uint32_t)(i + 2) * ps + o);
+        v1 = load(i + 1);
+      }
+      form(i, v0, i > 0 ? em : en, ec, en);
+      if (two) form(i + 1, v1, ec, en, e2);
+      em = en;
+      ec = e2;
+    }
+    __syncthreads();
+    for (uint32_t q = threadIdx.x; q < nc; q += blockDim.x) {
+      const uint32_t jr = q / C4;
+      const int kc0 = 4 * (int)(q - jr * C4);
+      const int jc = jc0 + (int)jr;
+      if (jc >= C.ny) break;
+      float a[4] = {0.f, 0.f, 0.f, 0.f};
+      // the coarse node whose tap dk = +1 is clamped onto its centre
+      const int ktop = F.nz - 1 - 2 * kc0;  // u == ktop / 2 if even and in 0..6
+#pragma unroll
+      for (int di = -1; di <= 1; di++) {
+        const int ii = min(max(2 * ic + di, 0), F.nx - 1);
+        const float* pl = ring + (uint32_t)(ii % 5) * plane;
+#pragma unroll
+        for (int dj = -1; dj <= 1; dj++) {
+          const int jj = min(max(2 * jc + dj, 0), F.ny - 1);
+          const float* r = pl + (uint32_t)(jj - jf0) * F.H + kc0;
+          const float w = (di == 0 ? 1.f : 0.5f) * (dj == 0 ? 1.f : 0.5f);
+          const float4 v = *reinterpret_cast<const float4*>(r);
+          const float vv[4] = {v.x, v.y, v.z, v.w};
+          if (((ii + jj) & 1) == 0) {
+            // slot kc alone, and once more for a tap clamped onto it
+            if (kc0 == 0) a[0] += 0.5f * w * v.x;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              a[u] += w * vv[u];
+              if (2 * u == ktop) a[u] += 0.5f * w * vv[u];
+            }
+          } else {
+            // slots kc - 1 and kc (dk = -1, +1); past the top face the slot
+            // is unused and holds 0
+            const float m = kc0 > 0 ? r[-1] : 0.f;
+            a[0] += 0.5f * w * m;
+            a[0] += 0.5f * w * v.x;
+#pragma unroll
+            for (int u = 1; u < 4; u++) {
+              a[u] += 0.5f * w * vv[u - 1];
+              a[u] += 0.5f * w * vv[u];
+            }
+          }
+        }
+      }
+      const int ca = scol(ic, jc, kc0);
+      float* c0 = cb + (size_t)ca * C.csz + ((uint32_t)ic * C.ny + jc) * C.H + (kc0 >> 1);
+      float* c1 = cb + (size_t)(1 - ca) * C.csz + ((uint32_t)ic * C.ny + jc) * C.H + (kc0 >> 1);
+      if (kc0 + 3 < C.nz) {
+        *reinterpret_cast<float2*>(c0) = make_float2(0.5f * a[0], 0.5f * a[2]);
+        *reinterpret_cast<float2*>(c1) = make_float2(0.5f * a[1], 0.5f * a[3]);
+      } else {
+        c0[0] = 0.5f * a[0];
+        if (kc0 + 1 < C.nz) c1[0] = 0.5f * a[1];
+        if (kc0 + 2 < C.nz) c0[1] = 0.5f * a[2];
+      }
+    }
+  }
 }
 
 // r = g - A e on natural layout (0 at metal).
@@ -2823,6 +3002,37 @@ struct Session {
     return (int)l < tb_levels && l + 1 < lv.size() && !flat(lv[l]) && smooth_omega == 1.f;
   }
 
+  // The residual and its restriction in one kernel: grids with no size-1
+  // axis with at least one coarse row's three fine rows a block.
+  static bool resid_restrict(const SGeo& G) {
+    return G.nx > 1 && G.ny > 1 && G.nz > 1 && 3 * (G.H / 4) <= kRrThreads;
+  }
+  // TJ: as many rows as the threads hold (the shared row costs least), evened
+  // over the tiles.  MI: the fewest rounds of resident blocks (two an SM),
+  // each of 2 MI + 1 planes; measured best 8 and 4 (alike) on the fine level
+  // of eight 193 x 193 x 385, 4 on 24 of 256 x 64 x 48, 2 on eight 65^3 and 1
+  // on the smaller levels, where 8 takes 2.5 times as long.
+  void launch_resid_restrict(MLevel& a, MLevel& b) {
+    const int H4 = a.G.H / 4;
+    int TJ = std::min((kRrThreads / H4 - 1) / 2, b.G.ny);
+    const int jt = (b.G.ny + TJ - 1) / TJ;
+    TJ = (b.G.ny + jt - 1) / jt;
+    int MI = 1;
+    long best = 0;
+    for (int m = 1; m <= 8; m *= 2) {
+      const long blocks = (long)jt * ((b.G.nx + m - 1) / m) * B;
+      const long cost = (blocks + 303) / 304 * (2 * m + 1);
+      if (m == 1 || cost <= best) {
+        best = cost;
+        MI = m;
+      }
+    }
+    const unsigned nt = (unsigned)((2 * TJ + 1) * H4 + 31) & ~31u;
+    k_resid_restrict0<<<dim3((unsigned)(jt * ((b.G.nx + MI - 1) / MI)), B), nt,
+                        5 * (size_t)(2 * TJ + 1) * a.G.H * 4, s>>>(
+        a.e.p, a.g.p, a.mask.p, a.G, b.g.p, b.G, a.pstride, b.pstride, TJ, MI, jt);
+  }
+
   // One cycle on level l.  zero: the level's correction starts at 0 (the
   // cycle zeroes it, or its first Gauss-Seidel pair writes every slot).
   void vcycle(size_t l, bool zero) {
@@ -2883,13 +3093,17 @@ struct Session {
     MLevel& b = lv[l + 1];
     if (nu1 > 0 && smooth_omega == 1.f) {
       // Gauss-Seidel ended on colour 1: its residual is zero
-      if (flat(a))
-        k_resid0<<<gs, kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, a.r.p, a.pstride);
-      else
-        k_resid0_4<<<dim3(nblk(a.G.csz / 4), B), kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G,
-                                                            a.r.p, a.pstride);
-      k_restrict0_4<<<dim3(nblk((uint32_t)b.G.nx * b.G.ny * ((b.G.nz + 3) / 4)), B), kT, 0, s>>>(
-          a.r.p, a.G, b.g.p, b.G, b.pstride);
+      if (resid_restrict(a.G)) {
+        launch_resid_restrict(a, b);
+      } else {
+        if (flat(a))
+          k_resid0<<<gs, kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, a.r.p, a.pstride);
+        else
+          k_resid0_4<<<dim3(nblk(a.G.csz / 4), B), kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G,
+                                                              a.r.p, a.pstride);
+        k_restrict0_4<<<dim3(nblk((uint32_t)b.G.nx * b.G.ny * ((b.G.nz + 3) / 4)), B), kT, 0,
+                        s>>>(a.r.p, a.G, b.g.p, b.G, b.pstride);
+      }
     } else {
       k_resid<<<gn, kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, a.r.p, a.pstride, a.rstride);
       k_restrict<<<dim3(nblk(b.G.n), B), kT, 0, s>>>(a.r.p, a.G, b.g.p, b.G, a.rstride, b.pstride);
@@ -3088,7 +3302,8 @@ struct Session {
     if (l + 1 == lv.size()) return 1;
     if (tail_cluster(l) || (zero && tail_level(l))) return 1;
     const int reps = coarse_visits(l);
-    long n = 3;                                         // residual, restriction, prolongation
+    // residual, restriction, prolongation
+    long n = nu1 > 0 && smooth_omega == 1.f && resid_restrict(lv[l].G) ? 2 : 3;
     if (tb_pre(l, zero)) n += tb_passes(2 * nu1);
     else n += 2 * nu1 - ((zero && fuse_zero_pair(lv[l])) ? 1 : 0);
     n += tb_post(l) ? tb_passes(2 * nu2) : 2 * nu2;
@@ -3120,7 +3335,8 @@ struct Session {
     b += 2.0 * (nu1 - q0) * 6.5 * n;                    // half-sweeps
     const double nc = (double)lv[l + 1].G.n;
     if (nu1 > 0 && smooth_omega == 1.f)
-      b += 8.5 * n + 2.0 * n + 4.0 * nc;                // colour-0 residual, restriction
+      // colour-0 residual, restriction
+      b += (resid_restrict(a.G) ? 6.5 : 8.5 + 2.0) * n + 4.0 * nc;
     else
       b += 13.0 * n + 4.0 * n + 4.0 * nc;
     const int reps = coarse_visits(l);
@@ -3627,6 +3843,17 @@ int ig_mixed_check_fused(void* handle, int n_problems, long long mismatches[8]) 
           a.r.p, a.G, b.g.p, b.G, b.pstride);
       diff(b.g.p, scrA, b.pstride * B, 4);
       launches += 2;
+      if (Session::resid_restrict(a.G)) {
+        // in one kernel, each over a stand-in right-hand side
+        MK(cudaMemsetAsync(b.g.p, 0x7f, b.pstride * B * 4, s));
+        k_restrict0<<<dim3(nblk(b.G.n), B), kT, 0, s>>>(a.r.p, a.G, b.g.p, b.G, b.pstride);
+        MK(cudaMemcpyAsync(scrA, b.g.p, b.pstride * B * 4, cudaMemcpyDeviceToDevice, s));
+        MK(cudaMemsetAsync(b.g.p, 0x7f, b.pstride * B * 4, s));
+        S->launch_resid_restrict(a, b);
+        diff(b.g.p, scrA, b.pstride * B, 4);
+        MK(cudaMemsetAsync(b.g.p, 0, b.pstride * B * 4, s));
+        launches += 2;
+      }
       // the fused first pair from a zero correction (a stand-in correction
       // left over from an earlier cycle: both ways must overwrite all of it)
       MK(cudaMemsetAsync(a.e.p, 0x7f, bytes, s));
