@@ -1311,6 +1311,113 @@ k_prolong_add4(const float* __restrict__ ec, SGeo C, float* __restrict__ ef,
                   maskf + (size_t)blockIdx.y * F.msplit, F, blockIdx.z, t);
 }
 
+// k_prolong_add4 for colour 0 with a thread at coarse node (I, J): the fine
+// rows (2I, 2J), (2I + 1, 2J), (2I, 2J + 1) and (2I + 1, 2J + 1) read the same
+// four coarse rows, so four slots of each take one fetch of 4 x 5 coarse
+// values, and the weights are known without forming them: colour 0 has the
+// even k (coarse nodes themselves) on the first and last of these rows and
+// the odd k (means of two) on the others.  Sums in the order of
+// k_prolong_add4, so the same bits; its index and weight arithmetic, some 250
+// instructions for four slots, was what that kernel's time went on, where
+// this one comes near its bytes: fine level of eight 193 x 193 x 385,
+// 157 -> 108 us (84 at copy rate), of 24 of 256 x 64 x 48 26.7 -> 13.9, of
+// 257^3 24.5 -> 14.6.
+__global__ void __launch_bounds__(kT)
+k_prolong_rows0(const float* __restrict__ ec, SGeo C, float* __restrict__ ef,
+                const uint8_t* __restrict__ maskf, SGeo F, size_t cstride, size_t fstride) {
+  const uint32_t t = blockIdx.x * kT + threadIdx.x;
+  const uint32_t IJ = fdivu(t, F.dH4);
+  const int I = (int)fdivu(IJ, C.dny);
+  if (I >= C.nx) return;
+  const int J = (int)(IJ - (uint32_t)I * C.dny.d);
+  const int m0 = 4 * (int)(t - IJ * F.dH4.d);
+  const bool i1 = 2 * I + 1 < F.nx, j1 = 2 * J + 1 < F.ny;  // the odd fine rows exist
+  const bool ih = i1 && I + 1 < C.nx, jh = j1 && J + 1 < C.ny;  // and lie between two coarse ones
+  const float* eb = ec + blockIdx.y * cstride;
+  float* efb = ef + blockIdx.y * fstride;
+  const uint8_t* mf = maskf + (size_t)blockIdx.y * F.msplit;
+  // coarse values kc = m0 .. m0 + 4 of row (I', J'), 0 past its last node
+  auto coarse = [&](int Ic, int Jc, float cv[5]) {
+    const uint32_t row = ((uint32_t)Ic * C.ny + Jc) * C.H + (m0 >> 1);
+    const int ca = (Ic + Jc) & 1;
+    const float* A = eb + (size_t)ca * C.csz + row;
+    const float* Bc = eb + (size_t)(1 - ca) * C.csz + row;
+    const float2 a01 = ld2(A), b01 = ld2(Bc);
+    cv[0] = a01.x;
+    cv[1] = m0 + 1 < C.nz ? b01.x : 0.f;
+    cv[2] = m0 + 2 < C.nz ? a01.y : 0.f;
+    cv[3] = m0 + 3 < C.nz ? b01.y : 0.f;
+    cv[4] = m0 + 4 < C.nz ? A[2] : 0.f;
+  };
+  // the four odd-k values of a row: a mean, or the top coarse node alone
+  auto mean = [&](const float cv[5], float z[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const bool top = m0 + u + 1 >= C.nz;
+      z[u] = top ? cv[u] : __fmaf_rn(0.5f, cv[u + 1], 0.5f * cv[u]);
+    }
+  };
+  auto add = [&](int i, int j, const float v[4]) {
+    const uint32_t base = ((uint32_t)i * F.ny + j) * F.H + m0;
+    const uchar4 mk = *reinterpret_cast<const uchar4*>(mf + base);
+    float4* out = reinterpret_cast<float4*>(efb + base);
+    float4 x = *out;
+    x.x += mk.x ? 0.f : v[0];
+    x.y += mk.y ? 0.f : v[1];
+    x.z += mk.z ? 0.f : v[2];
+    x.w += mk.w ? 0.f : v[3];
+    *out = x;
+  };
+  float c00[5], c10[5], c01[5], c11[5];
+  coarse(I, J, c00);
+  if (ih) coarse(I + 1, J, c10);
+  if (jh) coarse(I, J + 1, c01);
+  if (ih && jh) coarse(I + 1, J + 1, c11);
+  float z00[4], z[4], v[4];
+  mean(c00, z00);
+  add(2 * I, 2 * J, c00);
+  if (i1) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = z00[u];
+    if (ih) {
+      mean(c10, z);
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = __fmaf_rn(0.5f, z[u], 0.5f * z00[u]);
+    }
+    add(2 * I + 1, 2 * J, v);
+  }
+  if (j1) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) v[u] = z00[u];
+    if (jh) {
+      mean(c01, z);
+#pragma unroll
+      for (int u = 0; u < 4; u++) v[u] = __fmaf_rn(0.5f, z[u], 0.5f * z00[u]);
+    }
+    add(2 * I, 2 * J + 1, v);
+  }
+  if (i1 && j1) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      float a;
+      if (ih && jh) {
+        a = 0.25f * c00[u];
+        a = __fmaf_rn(0.25f, c01[u], a);
+        a = __fmaf_rn(0.25f, c10[u], a);
+        a = __fmaf_rn(0.25f, c11[u], a);
+      } else if (ih) {
+        a = __fmaf_rn(0.5f, c10[u], 0.5f * c00[u]);
+      } else if (jh) {
+        a = __fmaf_rn(0.5f, c01[u], 0.5f * c00[u]);
+      } else {
+        a = c00[u];
+      }
+      v[u] = a;
+    }
+    add(2 * I + 1, 2 * J + 1, v);
+  }
+}
+
 // The coarsest level's SOR pairs for one problem, by the calling CTA (NT
 // threads, all of which must call it): eb (out), gb and mask the problem's
 // split arrays, se shared scratch of kBottomMax floats.  The free nodes of
@@ -2899,7 +3006,10 @@ struct Session {
   // fine a.e += trilinear(coarse b.e) for colours 0 .. ncol-1
   void launch_prolong(MLevel& b, MLevel& a, int nb, unsigned ncol) {
     const dim3 grid(nblk(a.G.csz / 4), nb, ncol);
-    if (two_or_more(a) && two_or_more(b))
+    if (ncol == 1 && two_or_more(a) && two_or_more(b))
+      k_prolong_rows0<<<dim3(nblk((uint32_t)b.G.nx * b.G.ny * (a.G.H / 4)), nb), kT, 0, s>>>(
+          b.e.p, b.G, a.e.p, a.mask.p, a.G, b.pstride, a.pstride);
+    else if (two_or_more(a) && two_or_more(b))
       k_prolong_add4<<<grid, kT, 0, s>>>(b.e.p, b.G, a.e.p, a.mask.p, a.G, b.pstride, a.pstride);
     else
       k_prolong_add4_gather<<<grid, kT, 0, s>>>(b.e.p, b.G, a.e.p, a.mask.p, a.G, b.pstride,
@@ -3826,7 +3936,15 @@ int ig_mixed_check_fused(void* handle, int n_problems, long long mismatches[8]) 
       k_prolong_add4_gather<<<dim3(nblk(a.G.csz / 4), B, 2), kT, 0, s>>>(
           b.e.p, b.G, a.e.p, a.mask.p, a.G, b.pstride, a.pstride);
       diff(a.e.p, scrB, words, 2);
-      launches += 2;
+      // colour 0 alone
+      MK(cudaMemcpyAsync(a.e.p, scrA, bytes, cudaMemcpyDeviceToDevice, s));
+      S->launch_prolong(b, a, B, 1);
+      MK(cudaMemcpyAsync(scrB, a.e.p, bytes, cudaMemcpyDeviceToDevice, s));
+      MK(cudaMemcpyAsync(a.e.p, scrA, bytes, cudaMemcpyDeviceToDevice, s));
+      k_prolong_add4_gather<<<dim3(nblk(a.G.csz / 4), B, 1), kT, 0, s>>>(
+          b.e.p, b.G, a.e.p, a.mask.p, a.G, b.pstride, a.pstride);
+      diff(a.e.p, scrB, words, 2);
+      launches += 4;
       if (Session::flat(a)) continue;
       // the colour-0 residual after a Gauss-Seidel pair
       k_resid0<<<dim3(nblk(a.G.csz), B), kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, a.r.p,
