@@ -755,6 +755,16 @@ k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
   if (DELTA) block_max_to(mb, dslot);
 }
 
+// A level's values by (row, k), row the grid row's index ij = i ny + j: a
+// flat array.
+struct FlatRows {
+  const double* __restrict__ a;
+  uint32_t nz;
+  typedef const double* Row;
+  __device__ __forceinline__ Row row(uint32_t ij) const { return a + (size_t)ij * nz; }
+  __device__ __forceinline__ double at(Row r, int k) const { return r[k]; }
+};
+
 // multigrid3d._restrict_fw_njit (multigrid3d.py:420-455) at coarse node
 // (ic, jc, kc): 27-point full weighting with clamped edges, /8, and
 // -4x when neg4 (the caller's scaling).
@@ -764,9 +774,9 @@ k_sweep_rhs(double* __restrict__ e, const uint8_t* __restrict__ fixed,
 // within a factor of 8 of it (restrict_slow).  27 FP64 instructions a node
 // instead of 54 on a pipe of 2 lanes per clock and SM: 8.9 -> 4.9 us a
 // launch, averaged over a 97 x 97 x 193 deck's levels.
-template <bool CG>
-static __device__ __noinline__ double restrict_slow(const double* __restrict__ fine, int nx,
-                                                    int ny, int nz, int i, int j, int k) {
+template <class A>
+static __device__ __noinline__ double restrict_slow(const A fine, int nx, int ny, int nz, int i,
+                                                    int j, int k) {
   double acc = 0.0;
   for (int di = -1; di <= 1; di++)
     for (int dj = -1; dj <= 1; dj++)
@@ -774,15 +784,14 @@ static __device__ __noinline__ double restrict_slow(const double* __restrict__ f
         const int ii = min(max(i + di, 0), nx - 1), jj = min(max(j + dj, 0), ny - 1);
         const int kk = min(max(k + dk, 0), nz - 1);
         const double w = (di ? 0.5 : 1.0) * (dj ? 0.5 : 1.0) * (dk ? 0.5 : 1.0);
-        acc = __dadd_rn(acc, __dmul_rn(w, ldv<CG>(fine, ((size_t)ii * ny + jj) * nz + kk)));
+        acc = __dadd_rn(acc, __dmul_rn(w, fine.at(fine.row((uint32_t)(ii * ny + jj)), kk)));
       }
   return acc;
 }
 
-template <bool CG>
-__device__ __forceinline__ double restrict_node(const double* __restrict__ fine, int nx,
-                                                int ny, int nz, int ic, int jc, int kc,
-                                                int neg4) {
+template <class A>
+__device__ __forceinline__ double restrict_node(const A& fine, int nx, int ny, int nz, int ic,
+                                                int jc, int kc, int neg4) {
   const int i = 2 * ic, j = 2 * jc, k = 2 * kc;
   const int km = max(k - 1, 0), kp = min(k + 1, nz - 1);
   double acc = 0.0;
@@ -795,8 +804,8 @@ __device__ __forceinline__ double restrict_node(const double* __restrict__ fine,
     for (int dj = -1; dj <= 1; dj++) {
       const int jj = min(max(j + dj, 0), ny - 1);
       const double wj = dj == 0 ? 1.0 : 0.5;
-      const double* row = fine + ((size_t)ii * ny + jj) * nz;
-      const double x[3] = {ldv<CG>(row, km), ldv<CG>(row, k), ldv<CG>(row, kp)};
+      const typename A::Row row = fine.row((uint32_t)(ii * ny + jj));
+      const double x[3] = {fine.at(row, km), fine.at(row, k), fine.at(row, kp)};
 #pragma unroll
       for (int q = 0; q < 3; q++) {
         // (high word << 1 | low word != 0) - 1: zeros wrap to the top
@@ -808,7 +817,7 @@ __device__ __forceinline__ double restrict_node(const double* __restrict__ fine,
       }
     }
   }
-  if (tiny < 0x00800000u) acc = restrict_slow<CG>(fine, nx, ny, nz, i, j, k);  // 2^-1019
+  if (tiny < 0x00800000u) acc = restrict_slow<A>(fine, nx, ny, nz, i, j, k);  // 2^-1019
   double r = __dmul_rn(acc, 0.125);  // == acc / 8.0 (power-of-two scale)
   if (neg4) r = -__dmul_rn(r, 4.0);
   return r;
@@ -850,10 +859,9 @@ __device__ __forceinline__ double lerp_ref(double a, double b, double t) {
   return __dadd_rn(__dmul_rn(a, __dsub_rn(1.0, t)), __dmul_rn(b, t));
 }
 
-template <bool CG>
-static __device__ __noinline__ double trilinear_slow(const double* __restrict__ c, int cy,
-                                                     int cz, Lerp x, Lerp y, Lerp z) {
-#define C(a, b, d) ldv<CG>(c, ((size_t)(a) * cy + (b)) * cz + (d))
+template <class A>
+static __device__ __noinline__ double trilinear_slow(const A c, int cy, Lerp x, Lerp y, Lerp z) {
+#define C(a, b, d) c.at(c.row((uint32_t)((a) * cy + (b))), d)
   const double c00 = lerp_ref(C(x.a0, y.a0, z.a0), C(x.a1, y.a0, z.a0), x.t());
   const double c10 = lerp_ref(C(x.a0, y.a1, z.a0), C(x.a1, y.a1, z.a0), x.t());
   const double c01 = lerp_ref(C(x.a0, y.a0, z.a1), C(x.a1, y.a0, z.a1), x.t());
@@ -870,19 +878,19 @@ static __device__ __noinline__ double trilinear_slow(const double* __restrict__ 
 // doublings (no subnormal, overflow, infinity or NaN, skipped weight-0
 // values included, since 0 x inf is NaN); -0 also takes the nested form.
 // The prolongation's launch, averaged over the same levels: 16.5 -> 4.2 us.
-template <bool CG>
-__device__ __forceinline__ double trilinear(const double* __restrict__ c, int cy, int cz,
-                                            const Lerp& x, const Lerp& y, const Lerp& z) {
+template <class A>
+__device__ __forceinline__ double trilinear(const A& c, int cy, const Lerp& x, const Lerp& y,
+                                            const Lerp& z) {
   double v[8];
   bool ok = x.half <= 2 && y.half <= 2 && z.half <= 2;
 #pragma unroll
   for (int q = 0; q < 8; q++) {
-    v[q] = ldv<CG>(c, ((size_t)(q & 4 ? x.a1 : x.a0) * cy + (q & 2 ? y.a1 : y.a0)) * cz +
-                          (q & 1 ? z.a1 : z.a0));
+    v[q] = c.at(c.row((uint32_t)((q & 4 ? x.a1 : x.a0) * cy + (q & 2 ? y.a1 : y.a0))),
+                q & 1 ? z.a1 : z.a0);
     const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(v[q]));
     ok = ok && ((static_cast<unsigned>(b >> 52) & 0x7ffu) - 64u <= 1976u || b == 0ULL);
   }
-  if (!ok) return trilinear_slow<CG>(c, cy, cz, x, y, z);
+  if (!ok) return trilinear_slow<A>(c, cy, x, y, z);
   double p[4];
   if (x.half == 1) {
 #pragma unroll
@@ -964,10 +972,11 @@ __device__ __forceinline__ unsigned long long cta_max(unsigned long long v,
 }
 
 // The whole bottom solve by the calling CTA: sm holds 18 bytes a node, red
-// and count are its scratch.  Every thread must call it.
-__device__ __forceinline__ void bottom_solve(double* __restrict__ e_out,
+// and count are its scratch; f(t, ij, k) reads and put(t, ij, k, e) takes the
+// value of node t = ij nz + k.  Every thread must call it.
+template <class F, class P>
+__device__ __forceinline__ void bottom_solve(const F& f_of, const P& put,
                                              const uint8_t* __restrict__ fixed_g,
-                                             const double* __restrict__ f_g,
                                              const BottomGeom& g, double rel_tol, double omega,
                                              long max_pairs, double* sm,
                                              unsigned long long* red, int* count) {
@@ -985,7 +994,8 @@ __device__ __forceinline__ void bottom_solve(double* __restrict__ e_out,
     const int t = t0 + threadIdx.x;
     int c = -1;
     if (t < n) {
-      const double x = __ldcg(f_g + t);
+      const uint32_t ij = fdiv((uint32_t)t, g.dnz), k = (uint32_t)t - ij * g.dnz.d;
+      const double x = f_of((uint32_t)t, ij, k);
       f[t] = x;
       e[t] = 0.0;
       const unsigned long long b =
@@ -993,9 +1003,8 @@ __device__ __forceinline__ void bottom_solve(double* __restrict__ e_out,
       if (b > 0x7ff0000000000000ULL) nan = true;
       else if (b > fk) fk = b;
       if (!fixed_g[t]) {
-        const uint32_t ij = fdiv((uint32_t)t, g.dnz);
         const uint32_t i = fdiv(ij, g.dny);
-        c = (int)((i + (ij - i * g.dny.d) + ((uint32_t)t - ij * g.dnz.d)) & 1u);
+        c = (int)((i + (ij - i * g.dny.d) + k) & 1u);
       }
     }
 #pragma unroll
@@ -1032,7 +1041,10 @@ __device__ __forceinline__ void bottom_solve(double* __restrict__ e_out,
   }
   // the last pair's barrier (cta_max) came after its last update
   if (max_pairs <= 0) __syncthreads();
-  for (int t = tid; t < n; t += nt) __stcg(e_out + t, e[t]);
+  for (int t = tid; t < n; t += nt) {
+    const uint32_t ij = fdiv((uint32_t)t, g.dnz);
+    put((uint32_t)t, ij, (uint32_t)t - ij * g.dnz.d, e[t]);
+  }
 }
 
 __global__ void __launch_bounds__(kBottomCta)
@@ -1042,7 +1054,9 @@ k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
   extern __shared__ double sm[];
   __shared__ unsigned long long red[64];
   __shared__ int count[2];
-  bottom_solve(e_out, fixed_g, f_g, g, rel_tol, omega, max_pairs, sm, red, count);
+  bottom_solve([=](uint32_t t, uint32_t, uint32_t) { return f_g[t]; },
+               [=](uint32_t t, uint32_t, uint32_t, double e) { e_out[t] = e; }, fixed_g, g,
+               rel_tol, omega, max_pairs, sm, red, count);
 }
 
 // ---- the small error levels in one launch ----------------------------------
@@ -1056,54 +1070,155 @@ k_bottom_err(double* __restrict__ e_out, const uint8_t* __restrict__ fixed_g,
 // maxima (exchanged through distributed shared memory) and takes the same
 // branches.
 //
-// The levels' arrays stay in global memory; nodes are dealt to the
-// cluster's threads in flat order, values that other CTAs write are read
-// and written through L2 (ldv<true>, __stcg) and a cluster barrier
-// (release / acquire) separates the phases.  Every node's arithmetic is the
-// launched kernels', so the bits are theirs.  The bottom is CTA 0's
+// A CTA owns some rows (of k) of each level and their work.  DS: it also
+// holds them, values, right-hand sides, masks and the residual, in its shared
+// memory for the whole solve, and the others read them there: a phase then
+// waits for a remote shared load (some 200 clocks) and a barrier with nothing
+// of global memory behind it, where the levels in global memory cost two L2
+// round trips and a fence, 5200 clocks a half-sweep even on 13 x 13 x 25
+// nodes.  Levels too large for that (long rows in few of them) stay in
+// global memory, read and written through L2.  Every node's arithmetic is
+// the launched kernels', so the bits are theirs.  The bottom is CTA 0's
 // (bottom_solve).  16 CTAs of 512 threads: a half-sweep of 25 x 25 x 49
 // nodes is then some two nodes a thread and bound by its chain of load, sum
-// and barrier (a microsecond or two) rather than by the 16 SMs' FP64 pipes.
-// The door: 8 bases of a 97 x 97 x 193 ring deck 165 -> 109 ms, 4 with theta
-// at 65 x 65 x 129 46 -> 30.6 ms.
-struct TailGeom {
-  int nx, ny, nz, n, slots;
-  FastDiv dkk, dny, dnz;
+// and barrier rather than by the 16 SMs' FP64 pipes.
+// A launch's time, values in global memory and here: 8 bases of a 97 x 97 x
+// 193 ring deck 723 -> 576 us beside one another (a third of it the bottom),
+// the door 96 -> 82 ms; 4 with theta at 65 x 65 x 129 282 -> 246 us (two
+// thirds the bottom), 28.8 -> 27.5 ms.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return (uint32_t)__cvta_generic_to_shared(p);
+}
+// Shared address a of CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ double ld_cluster(uint32_t a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+  return v;
+}
+__device__ __forceinline__ void st_cluster(uint32_t a, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// A level's values by row and k wherever they live (FlatRows' interface):
+// s the owner's shared address of them (the same in every CTA), or g.
+template <bool DS>
+struct TailRows;
+template <>
+struct TailRows<true> {
+  uint32_t s, nz;
+  FastDiv drow;  // rows a CTA
+  typedef uint32_t Row;
+  __device__ __forceinline__ Row row(uint32_t ij) const {
+    const uint32_t o = fdiv(ij, drow);
+    return cluster_addr(s + (ij - o * drow.d) * nz * 8u, o);
+  }
+  __device__ __forceinline__ double at(Row r, int k) const { return ld_cluster(r + 8u * k); }
+  __device__ __forceinline__ void put(Row r, int k, double v) const { st_cluster(r + 8u * k, v); }
+};
+template <>
+struct TailRows<false> {
+  double* g;
+  uint32_t nz;
+  typedef double* Row;
+  __device__ __forceinline__ Row row(uint32_t ij) const { return g + (size_t)ij * nz; }
+  __device__ __forceinline__ double at(Row r, int k) const { return __ldcg(r + k); }
+  __device__ __forceinline__ void put(Row r, int k, double v) const { __stcg(r + k, v); }
 };
 
-// One half-sweep at omega 1; the largest |update| key with DELTA.
-template <bool DELTA>
-__device__ __forceinline__ unsigned long long tail_sweep(const TailLevel& L, const TailGeom& g,
-                                                         int colour, int gt, int gn) {
+// What a CTA has of a level: rows [row0, row0 + rows), their arrays.
+template <bool DS>
+struct TailPart {
+  uint32_t row0;
+  int rows;
+  double *e, *f, *r;
+  const uint8_t* fixed;
+  // own values: DS in this CTA's shared memory, else through L2
+  static __device__ __forceinline__ double ld(const double* p) { return DS ? *p : __ldcg(p); }
+  static __device__ __forceinline__ void st(double* p, double v) {
+    if (DS) *p = v;
+    else __stcg(p, v);
+  }
+};
+
+template <bool DS>
+__device__ __forceinline__ TailPart<DS> tail_part(const TailArgs& A, const TailLevel& L, int rank,
+                                                  unsigned char* sm) {
+  TailPart<DS> t;
+  t.row0 = (uint32_t)rank * L.drow.d;
+  t.rows = min((int)L.drow.d, L.nx * L.ny - (int)t.row0);
+  const size_t o = (size_t)t.row0 * L.nz;
+  t.e = DS ? reinterpret_cast<double*>(sm + L.oe) : L.e + o;
+  t.f = DS ? reinterpret_cast<double*>(sm + L.of) : L.f + o;
+  t.r = DS ? reinterpret_cast<double*>(sm + A.orr) : L.r + o;
+  t.fixed = DS ? sm + L.om : L.fixed + o;
+  return t;
+}
+
+template <bool DS>
+__device__ __forceinline__ TailRows<DS> tail_rows(const TailLevel& L, double* g, uint32_t s) {
+  if constexpr (DS) return TailRows<true>{s, (uint32_t)L.nz, L.drow};
+  else return TailRows<false>{g, (uint32_t)L.nz};
+}
+
+// The six neighbours of node (row ij = (i, j), k) of a level: x and y ones by
+// row, z ones in the node's own row (own), as neighbours() has them.
+template <bool DS>
+__device__ __forceinline__ void tail_load6(const TailRows<DS>& e, const double* own,
+                                           const TailLevel& L, uint32_t ij, uint32_t i,
+                                           uint32_t j, uint32_t k, double v[6]) {
+  const uint32_t ny = (uint32_t)L.ny, nx = (uint32_t)L.nx, nz = (uint32_t)L.nz;
+  const uint32_t rx = nx > 1 ? ny : 0u, ry = ny > 1 ? 1u : 0u, rz = nz > 1 ? 1u : 0u;
+  v[0] = e.at(e.row(i > 0 ? ij - ny : ij + rx), (int)k);
+  v[1] = e.at(e.row(i + 1 < nx ? ij + ny : ij - rx), (int)k);
+  v[2] = e.at(e.row(j > 0 ? ij - 1 : ij + ry), (int)k);
+  v[3] = e.at(e.row(j + 1 < ny ? ij + 1 : ij - ry), (int)k);
+  v[4] = TailPart<DS>::ld(own + (k > 0 ? k - 1 : k + rz));
+  v[5] = TailPart<DS>::ld(own + (k + 1 < nz ? k + 1 : k - rz));
+}
+
+// One half-sweep at omega 1 of a CTA's rows; the largest |update| key with
+// DELTA.
+template <bool DS, bool DELTA>
+__device__ __forceinline__ unsigned long long tail_sweep(const TailLevel& L,
+                                                         const TailPart<DS>& own,
+                                                         const TailRows<DS>& e, int colour) {
   unsigned long long mb = 0;
-  for (int t = gt; t < g.slots; t += gn) {
-    const uint32_t ij = fdiv((uint32_t)t, g.dkk);
-    const uint32_t i = fdiv(ij, g.dny);
-    const uint32_t j = ij - i * g.dny.d;
-    const uint32_t k = 2 * ((uint32_t)t - ij * g.dkk.d) + ((i + j + (uint32_t)colour) & 1u);
-    if (k >= (uint32_t)g.nz) continue;
-    const uint32_t p = ij * (uint32_t)g.nz + k;
-    if (L.fixed[p]) continue;
-    const Nb n = neighbours(i, j, k, (uint32_t)g.nx, (uint32_t)g.ny, (uint32_t)g.nz);
+  const int slots = own.rows * (int)L.dkk.d;
+  for (int t = (int)threadIdx.x; t < slots; t += kTailThreads) {
+    const uint32_t lr = fdiv((uint32_t)t, L.dkk), ij = own.row0 + lr;
+    const uint32_t i = fdiv(ij, L.dny);
+    const uint32_t j = ij - i * L.dny.d;
+    const uint32_t k = 2 * ((uint32_t)t - lr * L.dkk.d) + ((i + j + (uint32_t)colour) & 1u);
+    if (k >= (uint32_t)L.nz) continue;
+    const uint32_t row = lr * (uint32_t)L.nz;
+    if (own.fixed[row + k]) continue;
     double v[6];
-    load6<true>(L.e, n, v);
-    const double f = __ldcg(L.f + p), old = __ldcg(L.e + p);
+    tail_load6<DS>(e, own.e + row, L, ij, i, j, k, v);
+    const double f = own.ld(own.f + row + k), old = own.ld(own.e + row + k);
     unsigned long long key = 0;
-    __stcg(L.e + p, sor_apply<DELTA, true>(old, div6(__dsub_rn(sum6(v), f)), 1.0, &key));
+    own.st(own.e + row + k,
+           sor_apply<DELTA, true>(old, div6(__dsub_rn(sum6(v), f)), 1.0, &key));
     if (DELTA && key > mb) mb = key;
   }
   return mb;
 }
 
+template <bool DS>
 __global__ void __launch_bounds__(kTailThreads)
-k_err_tail(TailArgs A) {
+k_err_tail(const __grid_constant__ TailArgs A) {
   namespace cg = cooperative_groups;
-  extern __shared__ double sm[];
+  extern __shared__ double dyn[];
   __shared__ unsigned long long red[64], wred[32], slot[2][kTailCtas];
   __shared__ int count[2];
+  unsigned char* sm = reinterpret_cast<unsigned char*>(dyn);
+  const uint32_t sb = smem_u32(sm);
   cg::cluster_group cl = cg::this_cluster();
   const int ctas = (int)cl.num_blocks(), rank = (int)cl.block_rank();
-  const int gn = ctas * kTailThreads, gt = rank * kTailThreads + (int)threadIdx.x;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   int par = 0;
   // the cluster's maximum of a key, ending in a cluster barrier
@@ -1126,18 +1241,8 @@ k_err_tail(TailArgs A) {
         static_cast<unsigned long long>(__double_as_longlong(f)) & 0x7fffffffffffffffULL;
     return b > 0x7ff0000000000000ULL ? ~0ULL : b;
   };
-  auto geom = [](const TailLevel& L) {
-    TailGeom g;
-    g.nx = L.nx;
-    g.ny = L.ny;
-    g.nz = L.nz;
-    g.n = L.nx * L.ny * L.nz;
-    g.dkk = L.dkk;
-    g.dny = L.dny;
-    g.dnz = L.dnz;
-    g.slots = L.nx * L.ny * (int)L.dkk.d;
-    return g;
-  };
+  auto part = [&](const TailLevel& L) { return tail_part<DS>(A, L, rank, sm); };
+  auto e_rows = [&](const TailLevel& L) { return tail_rows<DS>(L, L.e, sb + L.oe); };
   double tol[kTailLevels];
   int cyc[kTailLevels];
   auto enter = [&](int l, unsigned long long fk) {
@@ -1147,13 +1252,25 @@ k_err_tail(TailArgs A) {
     cyc[l] = 0;
   };
   int l = 0;
+  cl.sync();  // every CTA of the cluster runs
   {
+    if (DS) {
+      // the masks, and the first level's right-hand side
+      for (int q = 0; q + 1 < A.nlev; q++) {
+        const TailLevel& L = A.lv[q];
+        const TailPart<DS> own = part(L);
+        for (int t = threadIdx.x; t < own.rows * L.nz; t += kTailThreads)
+          sm[L.om + t] = L.fixed[(size_t)own.row0 * L.nz + t];
+      }
+    }
     const TailLevel& L = A.lv[0];
-    const TailGeom g = geom(L);
+    const TailPart<DS> own = part(L);
     unsigned long long fk = 0;
-    for (int t = gt; t < g.n; t += gn) {
-      fk = max(fk, fkey(__ldcg(L.f + t)));
-      __stcg(L.e + t, 0.0);
+    for (int t = threadIdx.x; t < own.rows * L.nz; t += kTailThreads) {
+      const double f = __ldcg(L.f + (size_t)own.row0 * L.nz + t);
+      fk = max(fk, fkey(f));
+      if (DS) own.st(own.f + t, f);
+      own.st(own.e + t, 0.0);
     }
     enter(0, cluster_max(fk));
   }
@@ -1161,37 +1278,42 @@ k_err_tail(TailArgs A) {
     // level l: pre-smoothing, and its residual restricted to level l + 1
     const TailLevel& L = A.lv[l];
     const TailLevel& C = A.lv[l + 1];
-    const TailGeom g = geom(L), c = geom(C);
-    for (int q = 0; q < 2 * A.nu1; q++) {
-      tail_sweep<false>(L, g, q & 1, gt, gn);
+    {
+      const TailPart<DS> own = part(L);
+      const TailRows<DS> e = e_rows(L);
+      for (int q = 0; q < 2 * A.nu1; q++) {
+        tail_sweep<DS, false>(L, own, e, q & 1);
+        cl.sync();
+      }
+      for (int t = threadIdx.x; t < own.rows * L.nz; t += kTailThreads) {
+        double r = 0.0;
+        if (!own.fixed[t]) {
+          const uint32_t lr = fdiv((uint32_t)t, L.dnz), ij = own.row0 + lr;
+          const uint32_t i = fdiv(ij, L.dny);
+          const uint32_t row = lr * (uint32_t)L.nz;
+          double v[6];
+          tail_load6<DS>(e, own.e + row, L, ij, i, ij - i * L.dny.d, (uint32_t)t - row, v);
+          r = __dsub_rn(resid6(sum6(v), own.ld(own.e + t)), own.ld(own.f + t));
+        }
+        own.st(own.r + t, r);
+      }
       cl.sync();
     }
-    for (int t = gt; t < g.n; t += gn) {
-      double r = 0.0;
-      if (!L.fixed[t]) {
-        const uint32_t ij = fdiv((uint32_t)t, g.dnz);
-        const uint32_t i = fdiv(ij, g.dny);
-        const Nb n = neighbours(i, ij - i * g.dny.d, (uint32_t)t - ij * g.dnz.d, (uint32_t)g.nx,
-                                (uint32_t)g.ny, (uint32_t)g.nz);
-        double v[6];
-        load6<true>(L.e, n, v);
-        r = __dsub_rn(resid6(sum6(v), __ldcg(L.e + t)), __ldcg(L.f + t));
+    {
+      const TailPart<DS> own = part(C);
+      const TailRows<DS> r = tail_rows<DS>(L, L.r, sb + A.orr);
+      unsigned long long fk = 0;
+      for (int t = threadIdx.x; t < own.rows * C.nz; t += kTailThreads) {
+        const uint32_t lr = fdiv((uint32_t)t, C.dnz), ij = own.row0 + lr;
+        const uint32_t ic = fdiv(ij, C.dny);
+        const double f = restrict_node(r, L.nx, L.ny, L.nz, (int)ic, (int)(ij - ic * C.dny.d),
+                                       (int)((uint32_t)t - lr * C.dnz.d), 1);
+        own.st(own.f + t, f);
+        own.st(own.e + t, 0.0);
+        fk = max(fk, fkey(f));
       }
-      __stcg(L.r + t, r);
+      enter(l + 1, cluster_max(fk));
     }
-    cl.sync();
-    unsigned long long fk = 0;
-    for (int t = gt; t < c.n; t += gn) {
-      const uint32_t ij = fdiv((uint32_t)t, c.dnz);
-      const uint32_t ic = fdiv(ij, c.dny);
-      const double f = restrict_node<true>(L.r, g.nx, g.ny, g.nz, (int)ic,
-                                           (int)(ij - ic * c.dny.d),
-                                           (int)((uint32_t)t - ij * c.dnz.d), 1);
-      __stcg(C.f + t, f);
-      __stcg(C.e + t, 0.0);
-      fk = max(fk, fkey(f));
-    }
-    enter(l + 1, cluster_max(fk));
     l++;
     if (l + 1 < A.nlev) continue;
     if (rank == 0) {
@@ -1201,8 +1323,12 @@ k_err_tail(TailArgs A) {
       b.nz = C.nz;
       b.dny = C.dny;
       b.dnz = C.dnz;
-      bottom_solve(C.e, C.fixed, C.f, b, A.rel_tol, A.bottom_omega, A.bottom_pairs, sm, red,
-                   count);
+      const TailRows<DS> e = e_rows(C), f = tail_rows<DS>(C, C.f, sb + C.of);
+      bottom_solve(
+          [&](uint32_t, uint32_t ij, uint32_t k) { return f.at(f.row(ij), (int)k); },
+          [&](uint32_t, uint32_t ij, uint32_t k, double v) { e.put(e.row(ij), (int)k, v); },
+          C.fixed, b, A.rel_tol, A.bottom_omega, A.bottom_pairs,
+          reinterpret_cast<double*>(sm + A.ob), red, count);
     }
     cl.sync();
     // back up: correction, post-smoothing, and the cycle's decision
@@ -1210,30 +1336,37 @@ k_err_tail(TailArgs A) {
     while (done && l > 0) {
       const TailLevel& F = A.lv[l - 1];
       const TailLevel& K = A.lv[l];
-      const TailGeom h = geom(F);
+      const TailPart<DS> own = part(F);
+      const TailRows<DS> e = e_rows(F), ec = e_rows(K);
       l--;
-      for (int t = gt; t < h.n; t += gn) {
-        if (F.fixed[t]) continue;
-        const uint32_t ij = fdiv((uint32_t)t, h.dnz);
-        const uint32_t i = fdiv(ij, h.dny);
-        const Lerp x = pa_axis((int)i, K.nx), y = pa_axis((int)(ij - i * h.dny.d), K.ny);
-        const Lerp z = pa_axis((int)((uint32_t)t - ij * h.dnz.d), K.nz);
-        __stcg(F.e + t, __dadd_rn(__ldcg(F.e + t), trilinear<true>(K.e, K.ny, K.nz, x, y, z)));
+      for (int t = threadIdx.x; t < own.rows * F.nz; t += kTailThreads) {
+        if (own.fixed[t]) continue;
+        const uint32_t lr = fdiv((uint32_t)t, F.dnz), ij = own.row0 + lr;
+        const uint32_t i = fdiv(ij, F.dny);
+        const Lerp x = pa_axis((int)i, K.nx), y = pa_axis((int)(ij - i * F.dny.d), K.ny);
+        const Lerp z = pa_axis((int)((uint32_t)t - lr * F.dnz.d), K.nz);
+        own.st(own.e + t, __dadd_rn(own.ld(own.e + t), trilinear(ec, K.ny, x, y, z)));
       }
       cl.sync();
       for (int q = 0; q < 2 * A.nu2 - 2; q++) {
-        tail_sweep<false>(F, h, q & 1, gt, gn);
+        tail_sweep<DS, false>(F, own, e, q & 1);
         cl.sync();
       }
-      unsigned long long mb = tail_sweep<true>(F, h, 0, gt, gn);
+      unsigned long long mb = tail_sweep<DS, true>(F, own, e, 0);
       cl.sync();
-      mb = cluster_max(max(mb, tail_sweep<true>(F, h, 1, gt, gn)));
+      mb = cluster_max(max(mb, tail_sweep<DS, true>(F, own, e, 1)));
       cyc[l]++;
       done = bits_to_double(mb) < tol[l] || cyc[l] >= A.max_cycles;
     }
     if (done) break;
   }
-  cl.sync();  // no CTA leaves while another may still write to its shared memory
+  if (DS) {
+    const TailLevel& L = A.lv[0];
+    const TailPart<DS> own = part(L);
+    for (int t = threadIdx.x; t < own.rows * L.nz; t += kTailThreads)
+      L.e[(size_t)own.row0 * L.nz + t] = own.e[t];
+  }
+  cl.sync();  // no CTA leaves while another may still reach its shared memory
 }
 
 // multigrid3d._residual_rhs (multigrid3d.py:394-417).
@@ -1264,7 +1397,7 @@ k_restrict(const double* __restrict__ fine, int nx, int ny, int nz,
   if (t >= c.total) return;
   const uint32_t ij = fdiv(t, c.div_nz);
   const uint32_t ic = fdiv(ij, c.div_ny);
-  out[t] = restrict_node<false>(fine, nx, ny, nz, (int)ic, (int)(ij - ic * c.div_ny.d),
+  out[t] = restrict_node(FlatRows{fine, (uint32_t)nz}, nx, ny, nz, (int)ic, (int)(ij - ic * c.div_ny.d),
                          (int)(t - ij * c.div_nz.d), neg4);
 }
 
@@ -1280,7 +1413,7 @@ k_prolong_add(const double* __restrict__ coarse, int cx, int cy, int cz,
   const uint32_t i = fdiv(ij, g.div_ny);
   const Lerp x = pa_axis((int)i, cx), y = pa_axis((int)(ij - i * g.div_ny.d), cy);
   const Lerp z = pa_axis((int)(t - ij * g.div_nz.d), cz);
-  out[t] = __dadd_rn(out[t], trilinear<false>(coarse, cy, cz, x, y, z));
+  out[t] = __dadd_rn(out[t], trilinear(FlatRows{coarse, (uint32_t)cz}, cy, x, y, z));
 }
 
 // multigrid3d._prolongate (multigrid3d.py:138-171).
@@ -1293,7 +1426,7 @@ k_prolongate(const double* __restrict__ coarse, int cx, int cy, int cz,
   const uint32_t i = fdiv(ij, g.div_ny);
   const Lerp x = pl_axis((int)i, cx), y = pl_axis((int)(ij - i * g.div_ny.d), cy);
   const Lerp z = pl_axis((int)(t - ij * g.div_nz.d), cz);
-  out[t] = trilinear<false>(coarse, cy, cz, x, y, z);
+  out[t] = trilinear(FlatRows{coarse, (uint32_t)cz}, cy, x, y, z);
 }
 
 // multigrid3d._coarsen_fixed_any (multigrid3d.py:507-526).
@@ -1687,11 +1820,38 @@ TailLevel tail_level(Dims d, double* e, double* f, double* r, const uint8_t* fix
   return L;
 }
 
-bool launch_err_tail(cudaStream_t s, const TailArgs& a) {
+// Gives each CTA its rows and, in shared memory, its part of every level;
+// the bytes that takes.
+static size_t tail_layout(TailArgs& a, int ctas) {
+  size_t o = 0, rmax = 0, m = 0;
+  for (int q = 0; q < a.nlev; q++) {
+    TailLevel& L = a.lv[q];
+    const uint32_t rows = ((uint32_t)(L.nx * L.ny) + ctas - 1) / ctas;
+    L.drow = FastDiv(rows);
+    const size_t n = (size_t)rows * L.nz;
+    L.oe = (uint32_t)o;
+    L.of = (uint32_t)(o + 8 * n);
+    o += 16 * n;
+    if (q + 1 < a.nlev) rmax = std::max(rmax, n);
+  }
+  a.orr = (uint32_t)o;
+  o += 8 * rmax;
+  a.ob = (uint32_t)o;  // the bottom's 18 bytes a node, CTA 0's
+  const TailLevel& b = a.lv[a.nlev - 1];
+  o += ((size_t)b.nx * b.ny * b.nz * 18 + 7) / 8 * 8;
+  for (int q = 0; q + 1 < a.nlev; q++) {
+    TailLevel& L = a.lv[q];
+    L.om = (uint32_t)(o + m);
+    m += (size_t)L.drow.d * L.nz;
+  }
+  return (o + m + 7) / 8 * 8;
+}
+
+bool launch_err_tail(cudaStream_t s, TailArgs a) {
   const TailLevel& b = a.lv[a.nlev - 1];
   const size_t nb = (size_t)b.nx * b.ny * b.nz;
-  // the cluster size this device takes (16 CTAs, else the portable 8; 0:
-  // neither), found once
+  // the cluster size this device takes with all of an SM's shared memory (16
+  // CTAs, else the portable 8; 0: neither), found once
   static std::once_flag once;
   static int ctas = 0;
   auto config = [](cudaLaunchConfig_t* c, cudaLaunchAttribute* at, int n, size_t smem,
@@ -1708,16 +1868,20 @@ bool launch_err_tail(cudaStream_t s, const TailArgs& a) {
     c->attrs = at;
     c->numAttrs = 1;
   };
+  constexpr size_t most = 18 * (kBottomSmemMax / 17);
   std::call_once(once, [&] {
-    const size_t most = 18 * (kBottomSmemMax / 17);
-    cudaFuncSetAttribute(k_err_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
-    cudaFuncSetAttribute(k_err_tail, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    for (const void* fn : {(const void*)k_err_tail<false>, (const void*)k_err_tail<true>}) {
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    }
     for (int n : {kTailCtas, 8}) {
       cudaLaunchConfig_t c;
       cudaLaunchAttribute at[1];
       config(&c, at, n, most, nullptr);
-      int active = 0;
-      if (cudaOccupancyMaxActiveClusters(&active, k_err_tail, &c) == cudaSuccess && active > 0) {
+      int active = 0, other = 0;
+      if (cudaOccupancyMaxActiveClusters(&active, k_err_tail<true>, &c) == cudaSuccess &&
+          cudaOccupancyMaxActiveClusters(&other, k_err_tail<false>, &c) == cudaSuccess &&
+          active > 0 && other > 0) {
         ctas = n;
         break;
       }
@@ -1725,10 +1889,15 @@ bool launch_err_tail(cudaStream_t s, const TailArgs& a) {
     }
   });
   if (!ctas || nb == 0 || 17 * nb > kBottomSmemMax) return false;
+  const size_t bytes = tail_layout(a, ctas);
+  const bool ds = bytes <= most;
+  if (!ds) a.ob = 0;  // the bottom's scratch alone
   cudaLaunchConfig_t c;
   cudaLaunchAttribute at[1];
-  config(&c, at, ctas, (18 * nb + 7) / 8 * 8, s);
-  if (cudaLaunchKernelEx(&c, k_err_tail, a) != cudaSuccess) return true;  // the caller reads the error
+  config(&c, at, ctas, ds ? bytes : (18 * nb + 7) / 8 * 8, s);
+  // an error is the caller's to read
+  if (cudaLaunchKernelEx(&c, ds ? k_err_tail<true> : k_err_tail<false>, a) != cudaSuccess)
+    return true;
   counted();
   return true;
 }

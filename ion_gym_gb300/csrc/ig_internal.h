@@ -127,15 +127,20 @@ struct TailLevel {
   const uint8_t* fixed;
   int nx, ny, nz;
   FastDiv dkk, dny, dnz;
+  // set by the launch: rows a CTA, and the byte offsets of its part in
+  // shared memory (values, right-hand side, mask)
+  FastDiv drow;
+  uint32_t oe, of, om;
 };
 struct TailArgs {
   TailLevel lv[kTailLevels];
   int nlev, nu1, nu2, max_cycles;
   double rel_tol, bottom_omega;
   long bottom_pairs;
+  uint32_t orr, ob;  // the residual's and the bottom's scratch
 };
 TailLevel tail_level(Dims d, double* e, double* f, double* r, const uint8_t* fixed);
-bool launch_err_tail(cudaStream_t s, const TailArgs& a);
+bool launch_err_tail(cudaStream_t s, TailArgs a);
 void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,
                       const double* f, Dims d, double omega, int colour,
                       unsigned long long* dslot, PairCtl* ctl, int lp);
