@@ -172,6 +172,8 @@ void launch_sym_check(cudaStream_t s, const uint8_t* fixed, const double* val,
 // max |a - b| (b nullable: max |a|) into *bits, NaN noted in *nan_flag
 void launch_absdiff_max(cudaStream_t s, const double* a, const double* b,
                         size_t n, unsigned long long* bits, int* nan_flag);
+// Two words of the device to mapped host memory.
+void launch_report(cudaStream_t s, const unsigned long long* d, unsigned long long* host);
 void launch_sym_project(cudaStream_t s, double* phi, Dims d, int axis);
 void launch_residual_audit(cudaStream_t s, const double* u,
                            const uint8_t* fixed, const float* th, Dims d,

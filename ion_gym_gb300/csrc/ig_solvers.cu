@@ -262,15 +262,23 @@ PairsResult run_pairs(ThreadCtx& c, PairCtl* ctl_d, double tol, long max_pairs,
   return {max_pairs, last, false};
 }
 
-// Reads back one 64-bit max key (sync) as a double, NaN when flagged.
-double read_absmax(ThreadCtx& c, unsigned long long* bits_d, int* nan_d) {
-  unsigned long long b = 0;
-  int nanf = 0;
-  CK(cudaMemcpyAsync(&b, bits_d, 8, cudaMemcpyDeviceToHost, c.s));
-  if (nan_d) CK(cudaMemcpyAsync(&nanf, nan_d, 4, cudaMemcpyDeviceToHost, c.s));
+// Two 64-bit words of the device (sync), written by a kernel to the context's
+// pinned memory: the copy engine takes the copies of all streams in turn, so
+// a few bytes behind a copy that waits for another solve's kernels wait for
+// them too (eight bases at once: one read in ten 400 to 880 us).
+const unsigned long long* read_words(ThreadCtx& c, const unsigned long long* d) {
+  launch_report(c.s, d, c.ctl_h->slot);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c.s));
-  if (nanf) return std::numeric_limits<double>::quiet_NaN();
-  return bits_to_double(b);
+  return c.ctl_h->slot;
+}
+
+// Reads back one 64-bit max key (sync) as a double; words[1], an int in its
+// low half, flags NaN when `nan`.
+double read_absmax(ThreadCtx& c, const unsigned long long* words_d, bool nan) {
+  const unsigned long long* w = read_words(c, words_d);
+  if (nan && (int)w[1]) return std::numeric_limits<double>::quiet_NaN();
+  return bits_to_double(w[0]);
 }
 
 double device_absmax(ThreadCtx& c, const double* a, const double* b, size_t n,
@@ -279,7 +287,7 @@ double device_absmax(ThreadCtx& c, const double* a, const double* b, size_t n,
   CK(cudaMemsetAsync(scratch.p, 0, 16, c.s));
   launch_absdiff_max(c.s, a, b, n, scratch.p, (int*)(scratch.p + 1));
   CK(cudaGetLastError());
-  return read_absmax(c, scratch.p, (int*)(scratch.p + 1));
+  return read_absmax(c, scratch.p, true);
 }
 
 // ---------------------------------------------------------------- SOR
@@ -568,10 +576,7 @@ void solve_err(ThreadCtx& c, VCycle& v, size_t L, double above) {
         for (int colour = 0; colour < 2; colour++)
           launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, colour,
                            q + 1 == v.nu2 ? sl + colour : nullptr, nullptr, 0);
-      CK(cudaGetLastError());
-      unsigned long long last[2];
-      CK(cudaMemcpyAsync(last, sl, 16, cudaMemcpyDeviceToHost, c.s));
-      CK(cudaStreamSynchronize(c.s));
+      const unsigned long long* last = read_words(c, sl);
       if (umax(last[0], last[1]) < tol) break;
     } else {
       if (0.0 < tol) break;
@@ -1027,7 +1032,7 @@ int ig_cascadic_relres(const uint8_t* fixed, const double* val, long nx,
       launch_set_fixed(c.s, nxt.p, M.fixed.p, M.val.p, n);
       CK(cudaMemsetAsync(red.p, 0, 16, c.s));
       launch_residual(c.s, nxt.p, M.fixed.p, nullptr, kPlain, M.d, nullptr, red.p);
-      const double bnorm = read_absmax(c, red.p, nullptr);
+      const double bnorm = read_absmax(c, red.p, false);
       if (L < nl - 1) {
         launch_prolongate(c.s, cur.p, cd, nxt.p, M.d);
         launch_set_fixed(c.s, nxt.p, M.fixed.p, M.val.p, n);
@@ -1039,7 +1044,7 @@ int ig_cascadic_relres(const uint8_t* fixed, const double* val, long nx,
       while (true) {
         CK(cudaMemsetAsync(red.p, 0, 16, c.s));
         launch_residual(c.s, nxt.p, M.fixed.p, nullptr, kPlain, M.d, nullptr, red.p);
-        const double rmax = read_absmax(c, red.p, nullptr);
+        const double rmax = read_absmax(c, red.p, false);
         rr = bnorm > 0 ? rmax / bnorm : rmax;
         if (rr < ltol || pairs >= max_sweeps) break;
         const int chunk = (int)std::min<long>(check_every, max_sweeps - pairs);
