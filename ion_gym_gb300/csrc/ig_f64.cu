@@ -26,13 +26,18 @@ namespace ig {
 
 std::atomic<long> g_launches{0};
 long launch_total() { return g_launches.load(); }
+static thread_local long t_launches = 0;
+long launch_total_thread() { return t_launches; }
 void note_launches(long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
 namespace {
 
 constexpr int kThreads = 256;
 
-inline void counted() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+inline void counted() {
+  t_launches++;
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+}
 
 __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv& f) {
   return (__umulhi(n, f.m) + n) >> f.s;

@@ -187,6 +187,8 @@ void launch_fill_ones_f32(cudaStream_t s, float* a, size_t n);
 long launch_total();
 // Adds n launches issued by another translation unit to that count.
 void note_launches(long n);
+// Launches this thread counted, recordings included.
+long launch_total_thread();
 
 // Sets the calling thread's ig_last_error() message.
 void set_last_error(const std::string& m);

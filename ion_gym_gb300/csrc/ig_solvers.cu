@@ -262,21 +262,17 @@ PairsResult run_pairs(ThreadCtx& c, PairCtl* ctl_d, double tol, long max_pairs,
   return {max_pairs, last, false};
 }
 
-// Two 64-bit words of the device (sync), written by a kernel to the context's
+// Two 64-bit words of the device, written by a kernel to the context's
 // pinned memory: the copy engine takes the copies of all streams in turn, so
 // a few bytes behind a copy that waits for another solve's kernels wait for
 // them too (eight bases at once: one read in ten 400 to 880 us).
-const unsigned long long* read_words(ThreadCtx& c, const unsigned long long* d) {
-  launch_report(c.s, d, c.ctl_h->slot);
+// As a 64-bit max key (sync) and, with `nan`, an int in the second word's low
+// half that flags NaN.
+double read_absmax(ThreadCtx& c, const unsigned long long* words_d, bool nan) {
+  launch_report(c.s, words_d, c.ctl_h->slot);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(c.s));
-  return c.ctl_h->slot;
-}
-
-// Reads back one 64-bit max key (sync) as a double; words[1], an int in its
-// low half, flags NaN when `nan`.
-double read_absmax(ThreadCtx& c, const unsigned long long* words_d, bool nan) {
-  const unsigned long long* w = read_words(c, words_d);
+  const unsigned long long* w = c.ctl_h->slot;
   if (nan && (int)w[1]) return std::numeric_limits<double>::quiet_NaN();
   return bits_to_double(w[0]);
 }
@@ -286,7 +282,6 @@ double device_absmax(ThreadCtx& c, const double* a, const double* b, size_t n,
   // scratch: [0] = max bits, [1] = NaN flag (as int in the low word)
   CK(cudaMemsetAsync(scratch.p, 0, 16, c.s));
   launch_absdiff_max(c.s, a, b, n, scratch.p, (int*)(scratch.p + 1));
-  CK(cudaGetLastError());
   return read_absmax(c, scratch.p, true);
 }
 
@@ -456,11 +451,66 @@ PairsResult sor_loop(ThreadCtx& c, double* phi, const uint8_t* fx,
 }
 
 // ---------------------------------------------------------------- V-cycle
+//
+// The launches between two decisions of a cycle, the same ones each time (the
+// solve's buffers, grid and options): enqueued one by one the first kDirect
+// times and run as a graph from then on.  With eight bases at once each
+// launch waits its turn in the driver and a graph of twenty is one turn (2 us
+// of the host against 30): 4.1 -> 0.7 us between two sweeps of a stream
+// (median), 8 bases of a 97 x 97 x 193 ring deck 78 -> 75 ms, 4 with theta at
+// 65 x 65 x 129 24.8 -> 23.1 ms.  Making one takes 30 to 60 us, two runs'
+// launches.  Where nothing can be captured it keeps enqueuing.
+struct Replay {
+  static constexpr int kDirect = 3;
+  cudaGraphExec_t x = nullptr;
+  int runs = 0;
+  long kernels = 0;
+  Replay() = default;
+  Replay(Replay&& o) noexcept : x(o.x), runs(o.runs), kernels(o.kernels) { o.x = nullptr; }
+  Replay& operator=(Replay&&) = delete;
+  ~Replay() {
+    if (x) cudaGraphExecDestroy(x);
+  }
+  // Runs what `enqueue` enqueues.  false: nothing was run (not yet a graph, or
+  // none to be had).
+  template <class F>
+  bool operator()(ThreadCtx& c, F&& enqueue) {
+    if (!x && runs++ == kDirect) capture(c, enqueue);
+    if (!x) return false;
+    CK(cudaGraphLaunch(x, c.s));
+    note_launches(kernels);
+    return true;
+  }
+
+ private:
+  template <class F>
+  void capture(ThreadCtx& c, F&& enqueue) {
+    if (cudaStreamBeginCapture(c.s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    cudaGraph_t g = nullptr;
+    bool ok = false;
+    const long before = launch_total_thread();
+    try {
+      ok = enqueue();
+    } catch (...) {
+    }
+    kernels = launch_total_thread() - before;
+    note_launches(-kernels);  // recorded, not run
+    ok = cudaStreamEndCapture(c.s, &g) == cudaSuccess && ok;
+    if (!ok || cudaGraphInstantiate(&x, g, 0) != cudaSuccess) x = nullptr;
+    if (g) cudaGraphDestroy(g);
+    cudaGetLastError();
+  }
+};
+
 struct ErrLevel {
   Dims d;
   DBuf<uint8_t> fixed;
   DBuf<double> e, f, r;
   bool bottom = false;
+  Replay cycle;  // of a level above one that runs in one launch
 };
 
 struct VCycle {
@@ -508,22 +558,27 @@ constexpr size_t kTailNodes = 65536;
 // should be driving.
 constexpr double kTailMaxF = 1e200;
 
-// Level L's error solve as one launch; false: not done.
-bool solve_err_tail(ThreadCtx& c, VCycle& v, size_t L, double fmax) {
+// Level L's error solve as one launch: its arguments; false: not possible.
+bool err_tail_args(VCycle& v, size_t L, double fmax, TailArgs* t) {
   if (v.lv[L].bottom || v.lv[L].d.n() > kTailNodes || v.lv.size() - L > (size_t)kTailLevels ||
       v.nu2 < 1 || !(fmax < kTailMaxF))
     return false;
-  TailArgs t;
-  t.nlev = (int)(v.lv.size() - L);
+  t->nlev = (int)(v.lv.size() - L);
   for (size_t q = L; q < v.lv.size(); q++)
-    t.lv[q - L] = tail_level(v.lv[q].d, v.lv[q].e.p, v.lv[q].f.p, v.lv[q].r.p, v.lv[q].fixed.p);
-  t.nu1 = v.nu1;
-  t.nu2 = v.nu2;
-  t.max_cycles = v.max_cycles_err;
-  t.rel_tol = v.rel_tol;
-  t.bottom_omega = v.bottom_omega;
-  t.bottom_pairs = 20000;
-  if (!launch_err_tail(c.s, t)) return false;
+    t->lv[q - L] = tail_level(v.lv[q].d, v.lv[q].e.p, v.lv[q].f.p, v.lv[q].r.p, v.lv[q].fixed.p);
+  t->nu1 = v.nu1;
+  t->nu2 = v.nu2;
+  t->max_cycles = v.max_cycles_err;
+  t->rel_tol = v.rel_tol;
+  t->bottom_omega = v.bottom_omega;
+  t->bottom_pairs = 20000;
+  return true;
+}
+
+// Runs it; false: not done.
+bool solve_err_tail(ThreadCtx& c, VCycle& v, size_t L, double fmax) {
+  TailArgs t;
+  if (!err_tail_args(v, L, fmax, &t) || !launch_err_tail(c.s, t)) return false;
   CK(cudaGetLastError());
   return true;
 }
@@ -560,24 +615,40 @@ void solve_err(ThreadCtx& c, VCycle& v, size_t L, double above) {
   }
   ErrLevel& b = v.lv[L + 1];
   unsigned long long* sl = v.slots.p;
-  for (int cyc = 0; cyc < v.max_cycles_err; cyc++) {
-    for (int q = 0; q < v.nu1; q++) {
-      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 0, nullptr, nullptr, 0);
-      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, 1, nullptr, nullptr, 0);
-    }
+  const auto down = [&] {
+    for (int q = 0; q < 2 * v.nu1; q++)
+      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, q & 1, nullptr, nullptr, 0);
     launch_residual_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, a.r.p);
     launch_restrict(c.s, a.r.p, a.d, b.f.p, b.d, 1);
-    solve_err(c, v, L + 1, fmax);
+  };
+  const auto up = [&] {
     launch_prolong_add(c.s, b.e.p, b.d, a.e.p, a.fixed.p, a.d);
+    if (v.nu2 <= 0) return;
+    // the last pair's max |update| decides; the others' are not formed
+    CK(cudaMemsetAsync(sl, 0, 16, c.s));
+    for (int q = 0; q < 2 * v.nu2; q++)
+      launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, q & 1,
+                       q / 2 + 1 == v.nu2 ? sl + (q & 1) : nullptr, nullptr, 0);
+    launch_report(c.s, sl, c.ctl_h->slot);
+  };
+  TailArgs tail;
+  const bool one = err_tail_args(v, L + 1, fmax, &tail);
+  for (int cyc = 0; cyc < v.max_cycles_err; cyc++) {
+    const bool replayed = one && a.cycle(c, [&] {
+      down();
+      if (!launch_err_tail(c.s, tail)) return false;
+      up();
+      return true;
+    });
+    if (!replayed) {
+      down();
+      solve_err(c, v, L + 1, fmax);
+      up();
+    }
+    CK(cudaGetLastError());
     if (v.nu2 > 0) {
-      // the last pair's max |update| decides; the others' are not formed
-      CK(cudaMemsetAsync(sl, 0, 16, c.s));
-      for (int q = 0; q < v.nu2; q++)
-        for (int colour = 0; colour < 2; colour++)
-          launch_sweep_rhs(c.s, a.e.p, a.fixed.p, a.f.p, a.d, 1.0, colour,
-                           q + 1 == v.nu2 ? sl + colour : nullptr, nullptr, 0);
-      const unsigned long long* last = read_words(c, sl);
-      if (umax(last[0], last[1]) < tol) break;
+      CK(cudaStreamSynchronize(c.s));
+      if (umax(c.ctl_h->slot[0], c.ctl_h->slot[1]) < tol) break;
     } else {
       if (0.0 < tol) break;
     }
