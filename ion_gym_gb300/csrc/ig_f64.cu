@@ -567,24 +567,42 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
 // launch 7 us of latency around it (control block, mask, values, sum, block
 // maximum, each waiting for the one before; 43 us with theta's divisions on
 // the last block's chain).  Here one CTA per SM stays for the whole loop (a
-// cooperative launch, so that all of them are resident): a half-sweep ends
-// in a grid barrier, values pass through L2 (__ldcg / __stcg), and after a
-// pair every CTA reads all CTAs' maxima and takes the same decision, the
-// reference's per-pair test.  The node arithmetic is the launched sweeps'.
+// cooperative launch, so that all of them are resident).  The node arithmetic
+// is the launched sweeps'.
 //
-// A cut node of a theta plan goes to six lanes, one per leg (its division
-// or product), and the lanes add the six in the reference's order: the FP64
-// pipe takes a warp's instruction as long for two lanes as for 32, so six
-// legs side by side are a sixth of the divisions in line.
+// A grid barrier after each half-sweep would be four trips to L2 one after
+// the other (the values' stores, the arrival, the poll, the next loads), 4000
+// clocks at 65^3 beside 7500 of work that all warps do in step, the FP64 pipe
+// idle while they are in the integer part.  So there is none: a node's value
+// travels with its version, the number of updates it has had, in one 16-byte
+// word (a 128-bit access is single).  Colour 0 of pair n takes colour-1
+// neighbours of version n, colour 1 colour-0 ones of version n + 1, each lane
+// waiting for its own six.  No node can get further ahead: its next update
+// waits for neighbours that have read it.  So every CTA runs on as its own
+// neighbours allow.
 //
-// What is left at 65^3 (one node a thread) is the chain: barrier 2.2 us
-// (arrival counter in L2, 152 pollers), load 0.5, sums and integer step 2.5
-// with 32 warps an SM, the pair's decision 0.6 every second half-sweep.
-// solve3d at 65^3 4.64 -> 2.80 ms, with theta (sw, 57 x 71 x 90) 7.6 -> 4.9.
+// The reference's test after each pair is made a pair late: a CTA publishes
+// its maximum of pair n and goes on, and at the end of pair n + 1 reads all
+// of pair n; when that met tol, pair n + 1 is undone (prev holds each node's
+// value before its last update).  All CTAs see the same maxima and stop
+// alike.
 //
-// The barrier's wait is bounded (kCoopWait clocks, seconds): a CTA that
-// gives up raises *status and leaves, the others follow, and the call
-// reports an error.
+// A CTA has an even share of the slots in a row; where a thread's neighbours
+// lie is worked out once, into shared memory (1500 clocks a half-sweep of
+// divisions and masks otherwise).  Words lie by colour and slot, so a warp's
+// loads are contiguous.  A cut node of a theta plan goes to six lanes, one
+// per leg (its division or product), and the lanes add the six in the
+// reference's order: the FP64 pipe takes a warp's instruction as long for two
+// lanes as for 32, so six legs side by side are a sixth of the divisions in
+// line.
+//
+// What is left at 65^3 is a half-sweep's chain: the neighbours' words 0.8 us,
+// sums and integer step 2.2 (28 warps an SM, FP64 alone 1.4).  solve3d at 65^3
+// 4.73 ms launched, 2.75 with barriers, 1.78 so; with theta (sw, 57 x 71 x 90)
+// 22.5, 6.0 and 3.3.
+//
+// Waits are bounded (kCoopWait clocks, seconds): a warp that gives up raises
+// *status and leaves, the others follow, and the call reports an error.
 constexpr long long kCoopWait = 8000000000LL;
 
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
@@ -615,38 +633,164 @@ __device__ __forceinline__ bool coop_barrier(CoopCtl* c, unsigned target, int* o
   return *ok != 0;
 }
 
+constexpr size_t kFlowBytes = 20;  // of shared memory a slot
+struct FlowGeom {
+  SweepGeom g;
+  FastDiv dnz;
+  uint32_t share;    // slots a CTA
+  int rounds;        // and a thread
+  ulonglong2* word;  // 2 * g.total
+  double* prev;      // 2 * g.total
+};
+
+__device__ __forceinline__ void ld_word(const ulonglong2* p, unsigned long long& v,
+                                        unsigned long long& n) {
+  asm volatile("{ .reg .b128 w; ld.relaxed.gpu.global.b128 w, [%2]; mov.b128 {%0, %1}, w; }"
+               : "=l"(v), "=l"(n) : "l"(p));
+}
+__device__ __forceinline__ void st_word(ulonglong2* p, unsigned long long v,
+                                        unsigned long long n) {
+  asm volatile("{ .reg .b128 w; mov.b128 w, {%1, %2}; st.relaxed.gpu.global.b128 [%0], w; }"
+               ::"l"(p), "l"(v), "l"(n) : "memory");
+}
+
+// Polls until done() (every lane of the warp calls it); false: given up.
+template <class F>
+__device__ __forceinline__ bool flow_wait(CoopCtl* c, F&& done) {
+  if (__all_sync(0xffffffffu, done())) return true;
+  const long long t0 = clock64();
+  for (unsigned polls = 1; !__all_sync(0xffffffffu, done()); polls++)
+    if ((polls & 255u) == 0 &&
+        __any_sync(0xffffffffu, clock64() - t0 > kCoopWait ||
+                                    *reinterpret_cast<volatile int*>(&c->status))) {
+      c->status = 1;
+      return false;
+    }
+  return true;
+}
+
+// A node of colour c at slot t = (row ij, kk): its k and its neighbours' slots
+// of the other colour (t itself along a size-1 axis).
+struct FlowNode {
+  uint32_t k, o, t[6];
+};
+__device__ __forceinline__ FlowNode flow_node(const FlowGeom& G, uint32_t t, int c) {
+  const uint32_t nkk = G.g.div_kk.d, ny = G.g.div_ny.d;
+  const uint32_t nx = (uint32_t)G.g.nx, nz = (uint32_t)G.g.nz;
+  const uint32_t ij = fdiv(t, G.g.div_kk), kk = t - ij * nkk;
+  const uint32_t i = fdiv(ij, G.g.div_ny), j = ij - i * ny;
+  FlowNode f;
+  f.k = 2 * kk + ((i + j + (uint32_t)c) & 1u);
+  f.o = ij * nz + f.k;
+  const uint32_t sx = ny * nkk, r = ij * nkk;
+  const uint32_t rx = nx > 1 ? sx : 0u, ry = ny > 1 ? nkk : 0u;
+  f.t[0] = i > 0 ? t - sx : t + rx;
+  f.t[1] = i + 1 < nx ? t + sx : t - rx;
+  f.t[2] = j > 0 ? t - nkk : t + ry;
+  f.t[3] = j + 1 < ny ? t + nkk : t - ry;
+  f.t[4] = r + ((f.k > 0 ? f.k - 1 : 1u) >> 1);
+  f.t[5] = r + (nz == 1 ? 0u : (f.k + 1 < nz ? f.k + 1 : f.k - 1) >> 1);
+  return f;
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(kCoopThreads, 1)
-k_sor_coop(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, SweepGeom g,
-           FastDiv dnz, double omega, double tol, int pairs, CoopCtl* ctl) {
-  __shared__ unsigned long long red[33];
+k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, FlowGeom G,
+           double omega, double tol, int pairs, CoopCtl* ctl) {
+  // this thread's slots: the x and y neighbours', and bits: plain of either
+  // colour (0, 1), z neighbours' distances + 1 (two bits each from 2)
+  extern __shared__ uint4 near_xy[];
+  uint32_t* near_z = reinterpret_cast<uint32_t*>(near_xy + (size_t)G.rounds * kCoopThreads);
+  __shared__ unsigned long long red[2][32], all[2];
   __shared__ int ok;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kCoopThreads / 32;
-  const uint32_t gn = gridDim.x * kCoopThreads, gt = blockIdx.x * kCoopThreads + threadIdx.x;
-  // cut nodes start at the last warp of every CTA, the plain ones' shortest
+  const uint32_t S = G.g.total, nz = (uint32_t)G.g.nz;
+  const unsigned same = (G.g.nx > 1 ? 0u : 3u) | (G.g.ny > 1 ? 0u : 12u) | (nz > 1 ? 0u : 48u);
+  // slot r of this thread: t0 + r kCoopThreads, below t1
+  const uint32_t t0 = blockIdx.x * G.share + threadIdx.x;
+  const uint32_t t1 = min(S, (blockIdx.x + 1) * G.share);
   const uint32_t cw = (uint32_t)(nw - 1 - wid) * gridDim.x + blockIdx.x;
-  unsigned target = 0;
-  unsigned long long key = 0;
+  for (int r = 0; r < G.rounds; r++) {
+    const uint32_t t = t0 + (uint32_t)r * kCoopThreads;
+    uint32_t bits = 0;
+    for (int c = 0; c < 2 && t < t1; c++) {
+      const FlowNode f = flow_node(G, t, c);
+      unsigned long long v = 0, n = ~0ULL;
+      if (f.k < nz) {
+        v = static_cast<unsigned long long>(__double_as_longlong(phi[f.o]));
+        const uint8_t k = cls[f.o];
+        n = k == 0 || (KIND != kPlain && k == 2) ? 0ULL : ~0ULL;  // metal: any version
+        bits |= (k == 0 ? 1u << c : 0u) | (f.t[4] - t + 1u) << (2 + 4 * c) |
+                (f.t[5] - t + 1u) << (4 + 4 * c);
+      }
+      st_word(G.word + (size_t)c * S + t, v, n);
+      near_xy[r * kCoopThreads + threadIdx.x] = make_uint4(f.t[0], f.t[1], f.t[2], f.t[3]);
+    }
+    near_z[r * kCoopThreads + threadIdx.x] = bits;
+  }
+  if (!coop_barrier(ctl, gridDim.x, &ok)) return;
+
   int pr = 0;
-  bool hit = false;
+  bool hit = false, undo = false;
+  unsigned long long key = 0;
+  // all CTAs' maxima of pair q (warp 0); false: given up
+  auto maxima = [&](int q, unsigned long long* out) {
+    unsigned long long m = 0;
+    const bool good = flow_wait(ctl, [&] {
+      m = 0;
+      bool all = true;
+      const ulonglong2* w = reinterpret_cast<const ulonglong2*>(ctl->word[q & 3]);
+      for (uint32_t b0 = lane; b0 < gridDim.x; b0 += 160) {
+        unsigned long long v[5], n[5];
+#pragma unroll
+        for (int d = 0; d < 5; d++) ld_word(w + min(b0 + 32 * d, gridDim.x - 1), v[d], n[d]);
+#pragma unroll
+        for (int d = 0; d < 5; d++) {
+          m = max(m, v[d]);
+          all = all && n[d] == (unsigned long long)(q + 1);
+        }
+      }
+      return all;
+    });
+    *out = warp_max_u64(m);
+    return good;
+  };
   for (; pr < pairs && !hit; pr++) {
     unsigned long long mb = 0;
-    for (int colour = 0; colour < 2; colour++) {
+    for (int c = 0; c < 2; c++) {
+      const unsigned long long want = (unsigned long long)(pr + c);
+      ulonglong2* own = G.word + (size_t)c * S;
+      const ulonglong2* oth = G.word + (size_t)(1 - c) * S;
+      double* prev = G.prev + (size_t)c * S;
       if (KIND != kPlain) {
-        const uint32_t first = colour ? P.count[0] : 0u, total = P.total();
-        for (uint32_t q = cw * 5u; q < P.count[colour]; q += gridDim.x * (uint32_t)nw * 5u) {
+        // the cut nodes from the CTA's last warps on, which have fewer of the rest
+        const uint32_t first = c ? P.count[0] : 0u, total = P.total();
+        for (uint32_t q = cw * 5u; q < P.count[c]; q += gridDim.x * (uint32_t)nw * 5u) {
           const int who = lane / 6, leg = lane - 6 * who;
-          const bool act = who < 5 && q + who < P.count[colour];
+          const bool act = who < 5 && q + who < P.count[c];
           const uint32_t e = first + q + (act ? who : 0);
-          const uint32_t p = P.idx[e];
-          const uint32_t ij = fdiv(p, dnz);
-          const uint32_t i = fdiv(ij, g.div_ny);
-          const Nb n = neighbours(i, ij - i * g.div_ny.d, p - ij * dnz.d, (uint32_t)g.nx,
-                                  g.div_ny.d, dnz.d);
-          const uint32_t o = leg == 0 ? n.xm : leg == 1 ? n.xp : leg == 2 ? n.ym
-                             : leg == 3 ? n.yp : leg == 4 ? n.zm : n.zp;
-          const double v = __ldcg(phi + o), w = P.w[(size_t)leg * total + e];
-          const double old = __ldcg(phi + p), den = P.w[(size_t)6 * total + e];
+          const uint32_t p = P.idx[e], ij = fdiv(p, G.dnz);
+          const uint32_t t = ij * G.g.div_kk.d + ((p - ij * nz) >> 1);
+          const FlowNode f = flow_node(G, t, c);
+          const bool self = (same >> leg) & 1u;
+          uint32_t u = f.t[0];
+#pragma unroll
+          for (int d = 1; d < 6; d++) u = leg == d ? f.t[d] : u;
+          const ulonglong2* src = self ? own + t : oth + u;
+          unsigned long long vb, n, ob, on;
+          ld_word(own + t, ob, on);
+          const double w = P.w[(size_t)leg * total + e], den = P.w[(size_t)6 * total + e];
+          bool have = false;
+          if (!flow_wait(ctl, [&] {
+                if (!have) {
+                  ld_word(src, vb, n);
+                  have = self || !act || n >= want;
+                }
+                return have;
+              }))
+            return;
+          const double v = __longlong_as_double((long long)vb);
+          const double old = __longlong_as_double((long long)ob);
           const double term = KIND == kThetaGhost ? __dmul_rn(v, w) : __ddiv_rn(v, w);
           const int l0 = lane < 30 ? 6 * who : 24;
           double num = __shfl_sync(0xffffffffu, term, l0);
@@ -656,67 +800,112 @@ k_sor_coop(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Swee
           unsigned long long k = 0;
           const double nv = sor_apply<true, false>(old, __ddiv_rn(num, den), omega, &k);
           if (act && leg == 0) {
-            __stcg(phi + p, nv);
+            st_word(own + t, (unsigned long long)__double_as_longlong(nv), pr + 1ULL);
+            prev[t] = old;
             if (k > mb) mb = k;
           }
         }
       }
-      // two nodes at a time, so that their loads are in flight together
-      for (uint32_t t = gt; t < g.total; t += 2 * gn) {
-        uint32_t p[2];
-        bool go[2];
-        double S[2], old[2], v[2][6];
+      for (int r = 0; r < G.rounds; r++) {
+        const uint32_t t = t0 + (uint32_t)r * kCoopThreads;
+        const uint4 xy = near_xy[r * kCoopThreads + threadIdx.x];
+        const uint32_t bits = near_z[r * kCoopThreads + threadIdx.x] >> c;
+        const bool go = bits & 1u;
+        const uint32_t z = bits >> (2 + 3 * c);
+        const uint32_t nt[6] = {xy.x, xy.y, xy.z, xy.w, t + (z & 3u) - 1u,
+                                t + ((z >> 2) & 3u) - 1u};
+        unsigned long long b[6], ob = 0, on;
+        bool have = !go;
+        if (go) ld_word(own + t, ob, on);
+        if (!flow_wait(ctl, [&] {
+              if (!have) {
+                unsigned long long n[6];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          const SweepNodes<1> sn(g, t + u * gn, colour);
-          go[u] = t + u * gn < g.total && sn.valid(0) && cls[sn.at(0)] == 0;
-          if (!go[u]) continue;
-          p[u] = sn.at(0);
-          load6<true>(phi, sn.nb(0, p[u]), v[u]);
-          old[u] = __ldcg(phi + p[u]);
-        }
+                for (int d = 0; d < 6; d++) ld_word(oth + nt[d], b[d], n[d]);
+                have = true;
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          if (!go[u]) continue;
-          S[u] = sum6(v[u]);
-          double q;
-          if (KIND == kThetaSW && !sw_halves(S[u], v[u]))
-            q = __ddiv_rn(plain_sw_num(v[u]), 3.0);
-          else
-            q = div6(S[u]);
-          unsigned long long k = 0;
-          __stcg(phi + p[u], sor_apply<true, false>(old[u], q, omega, &k));
-          if (k > mb) mb = k;
-        }
-      }
-      if (colour == 0) {
-        target += gridDim.x;
-        if (!coop_barrier(ctl, target, &ok)) return;
+                for (int d = 0; d < 6; d++) have = have && (n[d] >= want || ((same >> d) & 1u));
+              }
+              return have;
+            }))
+          return;
+        if (!go) continue;
+        double v[6];
+#pragma unroll
+        for (int d = 0; d < 6; d++)
+          v[d] = __longlong_as_double((long long)((same >> d) & 1u ? ob : b[d]));
+        const double old = __longlong_as_double((long long)ob), sum = sum6(v);
+        double q;
+        if (KIND == kThetaSW && !sw_halves(sum, v))
+          q = __ddiv_rn(plain_sw_num(v), 3.0);
+        else
+          q = div6(sum);
+        unsigned long long k = 0;
+        const double nv = sor_apply<true, false>(old, q, omega, &k);
+        st_word(own + t, (unsigned long long)__double_as_longlong(nv), pr + 1ULL);
+        prev[t] = old;
+        if (k > mb) mb = k;
       }
     }
-    // the pair's maximum: this CTA's into its slot, then everyone's
+    // the last pair's maximum of all CTAs in (by the warp with the fewest
+    // nodes, while the others finish), this pair's of this one out
     mb = warp_max_u64(mb);
-    if (lane == 0) red[wid] = mb;
-    __syncthreads();
-    if (wid == 0) {
-      mb = warp_max_u64(red[lane]);
-      if (lane == 0) __stcg(&ctl->slot[pr & 1][blockIdx.x], mb);
-    }
-    target += gridDim.x;
-    if (!coop_barrier(ctl, target, &ok)) return;
-    if (wid == 0) {
-      key = 0;
-      for (uint32_t b = lane; b < gridDim.x; b += 32)
-        key = max(key, __ldcg(&ctl->slot[pr & 1][b]));
-      key = warp_max_u64(key);
-      if (lane == 0) red[32] = key;
+    if (lane == 0) red[pr & 1][wid] = mb;
+    if (wid == nw - 1 && pr > 0) {
+      const bool good = maxima(pr - 1, &key);
+      if (lane == 0) {
+        all[pr & 1] = key;
+        if (!good) ok = 0;
+      }
     }
     __syncthreads();
-    key = red[32];
+    if (!ok) return;
+    if (wid == 0) {
+      mb = warp_max_u64(red[pr & 1][lane]);
+      if (lane == 0)
+        st_word(reinterpret_cast<ulonglong2*>(ctl->word[pr & 3]) + blockIdx.x, mb, pr + 1ULL);
+    }
+    if (pr > 0) {
+      key = all[pr & 1];
+      hit = undo = bits_to_double(key) < tol;
+    }
+  }
+  if (!hit) {
+    // the last pair's own test
+    if (wid == nw - 1) {
+      const bool good = maxima(pairs - 1, &key);
+      if (lane == 0) {
+        all[pairs & 1] = key;
+        if (!good) ok = 0;
+      }
+    }
+    __syncthreads();
+    if (!ok) return;
+    key = all[pairs & 1];
     hit = bits_to_double(key) < tol;
   }
+  auto put = [&](uint32_t o, uint32_t t, int c) {
+    unsigned long long v, n;
+    ld_word(G.word + (size_t)c * S + t, v, n);
+    phi[o] = undo ? G.prev[(size_t)c * S + t] : __longlong_as_double((long long)v);
+  };
+  for (int c = 0; c < 2; c++) {
+    if (KIND != kPlain) {
+      for (uint32_t q = cw * 5u; q < P.count[c]; q += gridDim.x * (uint32_t)nw * 5u) {
+        const int who = lane / 6;
+        if (who < 5 && lane == 6 * who && q + who < P.count[c]) {
+          const uint32_t p = P.idx[(c ? P.count[0] : 0u) + q + who], ij = fdiv(p, G.dnz);
+          put(p, ij * G.g.div_kk.d + ((p - ij * nz) >> 1), c);
+        }
+      }
+    }
+    for (uint32_t t = t0; t < t1; t += kCoopThreads) {
+      const FlowNode f = flow_node(G, t, c);
+      if (f.k < nz && cls[f.o] == 0) put(f.o, t, c);
+    }
+  }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    ctl->pairs = pr;
+    ctl->pairs = undo ? pr - 1 : pr;
     ctl->hit = hit ? 1 : 0;
     ctl->key = key;
   }
@@ -1782,7 +1971,8 @@ bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const do
 }
 
 bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const ThetaPlan* plan,
-                     int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl) {
+                     int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl,
+                     void* word, double* prev) {
   // a whole grid of one CTA per SM, found once per device
   static std::mutex mu;
   static int sms[64] = {0};
@@ -1799,17 +1989,27 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
     }
     n = sms[dev];
   }
-  if (n < 1) return false;
+  if (n < 1 || !word) return false;
   SweepGeom g = sweep_geom(d);
   FastDiv dnz((uint32_t)d.nz);
   ThetaPlan P = plan ? *plan : ThetaPlan();
   if (cudaMemsetAsync(ctl, 0, sizeof(CoopCtl), s) != cudaSuccess) return true;
-  void* args[] = {&phi, &cls, &P, &g, &dnz, &omega, &tol, &pairs, &ctl};
-  const void* fn = kind == kThetaGhost ? (const void*)k_sor_coop<kThetaGhost>
-                   : kind == kThetaSW  ? (const void*)k_sor_coop<kThetaSW>
-                                       : (const void*)k_sor_coop<kPlain>;
+  FlowGeom G;
+  G.g = g;
+  G.dnz = dnz;
+  G.share = (g.total + (uint32_t)n - 1) / (uint32_t)n;
+  G.rounds = (int)((G.share + kCoopThreads - 1) / kCoopThreads);
+  G.word = static_cast<ulonglong2*>(word);
+  G.prev = prev;
+  const size_t smem = (size_t)G.rounds * kCoopThreads * kFlowBytes;
+  void* args[] = {&phi, &cls, &P, &G, &omega, &tol, &pairs, &ctl};
+  const void* fn = kind == kThetaGhost ? (const void*)k_sor_flow<kThetaGhost>
+                   : kind == kThetaSW  ? (const void*)k_sor_flow<kThetaSW>
+                                       : (const void*)k_sor_flow<kPlain>;
   // a failed launch leaves its error for the caller's check
-  if (cudaLaunchCooperativeKernel(fn, dim3(n), dim3(kCoopThreads), args, 0, s) == cudaSuccess)
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
+          cudaSuccess &&
+      cudaLaunchCooperativeKernel(fn, dim3(n), dim3(kCoopThreads), args, smem, s) == cudaSuccess)
     counted();
   return true;
 }

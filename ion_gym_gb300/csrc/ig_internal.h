@@ -104,19 +104,21 @@ constexpr size_t kBottomSmemMax = 200 * 1024;
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
                        Dims d, double rel_tol, double omega, long max_pairs);
 // SOR pairs until one meets tol, at most `pairs`, in one cooperative launch
-// (k_sor_coop): cls holds 0 at the nodes the plain update owns, plan the cut
+// (k_sor_flow): cls holds 0 at the nodes the plain update owns, plan the cut
 // nodes of a theta solve (kind kThetaGhost / kThetaSW) or null.  ctl gets
 // the pairs run, whether the last met tol and its max |update| key; status 1
-// means a barrier gave up.  false: the device takes no such launch.
+// means a wait gave up.  word (32 bytes a slot of one colour) and prev (16)
+// are scratch.  false: the device takes no such launch.
 constexpr int kCoopThreads = 1024, kCoopCtas = 512;
 struct CoopCtl {
   unsigned arrived;
   int status, pairs, hit;
   unsigned long long key;
-  unsigned long long slot[2][kCoopCtas];
+  alignas(16) unsigned long long word[4][2 * kCoopCtas];  // a CTA's maximum, pair + 1
 };
 bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const ThetaPlan* plan,
-                     int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl);
+                     int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl,
+                     void* word, double* prev);
 // multigrid3d._solve_err from level lv[0] (its right-hand side in f) down to
 // the bottom lv[nlev - 1] (nlev >= 2) in one launch (k_err_tail); false
 // (nothing launched) when the bottom does not fit in shared memory or the

@@ -387,23 +387,27 @@ void fine_sweep(cudaStream_t s, double* phi, const uint8_t* fx, const float* th,
     launch_sweep(s, phi, fx, th, kind, d, omega, colour, nullptr, ctl, lp);
 }
 
-// Slots of one colour up to which the SOR loop is one launch (k_sor_coop):
+// Slots of one colour up to which the SOR loop is one launch (k_sor_flow):
 // eight nodes a thread.  A half-sweep of solve3d, launched against resident
-// (us, host copies of the call included): 33^3 7.1 / 6.5, 65^3 11.1 / 6.7,
-// 97^3 22.9 / 12.8, 129^3 31.3 / 23.8; with theta (sw) 33^3 9.6 / 8.5, 65^3
-// 14.6 / 8.8, 129^3 44.6 / 27.7.  Past that the margin is gone (the sweep
-// itself fills the GPU) and one call would hold every SM for long.
+// (us, host copies of the call included): 33^3 7.1 / 2.4, 65^3 11.1 / 4.1,
+// 97^3 22.9 / 9.3, 129^3 31.3 / 20.7; with theta (sw) 33^3 9.6 / 3.1, 65^3
+// 14.6 / 4.2, 129^3 44.6 / 20.6.  Past that the sweep itself fills the GPU,
+// one call would hold every SM for long, and a thread's neighbour slots fill
+// its SM's shared memory.
 constexpr long kCoopSlots = 8L * 152 * kCoopThreads;
 // Pairs per launch: the host looks in between.
 constexpr int kCoopPairs = 4096;
 
-// The SOR loop by k_sor_coop; false: not done.
+// The SOR loop by k_sor_flow; false: not done.
 bool sor_loop_coop(ThreadCtx& c, double* phi, const uint8_t* fx, const float* th, const Theta& t,
                    int kind, Dims d, double omega, double tol, long max_pairs,
                    PairsResult* out) {
   if ((th && !t.on()) || d.nx * d.ny * ((d.nz + 1) / 2) > kCoopSlots || max_pairs < 1)
     return false;
   DBuf<CoopCtl> ctl(1, c.s);
+  const size_t slots = (size_t)(d.nx * d.ny * ((d.nz + 1) / 2));
+  DBuf<ulonglong2> word(2 * slots, c.s);
+  DBuf<double> before(2 * slots, c.s);
   const bool prof = g_prof.on.load() != 0;
   long base = 0;
   double last = std::numeric_limits<double>::quiet_NaN();
@@ -411,14 +415,14 @@ bool sor_loop_coop(ThreadCtx& c, double* phi, const uint8_t* fx, const float* th
     const int lim = (int)std::min<long>(kCoopPairs, max_pairs - base);
     if (prof) CK(cudaEventRecord(c.ev0, c.s));
     if (!launch_sor_coop(c.s, phi, t.on() ? t.plan.cls : fx, t.on() ? &t.plan : nullptr, kind, d,
-                         omega, tol, lim, ctl.p))
+                         omega, tol, lim, ctl.p, word.p, before.p))
       return false;
     CK(cudaGetLastError());
     if (prof) CK(cudaEventRecord(c.ev1, c.s));
     CoopCtl h;
-    CK(cudaMemcpyAsync(&h, ctl.p, offsetof(CoopCtl, slot), cudaMemcpyDeviceToHost, c.s));
+    CK(cudaMemcpyAsync(&h, ctl.p, offsetof(CoopCtl, word), cudaMemcpyDeviceToHost, c.s));
     CK(cudaStreamSynchronize(c.s));
-    if (h.status) throw Status(IG_CUDA_ERROR, "SOR loop: a grid barrier ran out of time");
+    if (h.status) throw Status(IG_CUDA_ERROR, "SOR loop: a wait ran out of time");
     if (prof) {
       float ms = 0.f;
       CK(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
