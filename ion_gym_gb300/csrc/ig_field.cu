@@ -335,6 +335,47 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
   }
 }
 
+// The quotient of div32 without its cases: exact for d of +0 or within
+// [2^-100, 2^100] and a divisor the launch found in range; *bad is raised
+// otherwise.
+__device__ __forceinline__ float div32_fast(float d, float c, float y, bool* bad) {
+  const unsigned b = __float_as_uint(d);
+  constexpr unsigned lo = 0x0d800000u, hi = 0x71800000u;  // 2^-100, 2^100
+  *bad = *bad || ((b & 0x7fffffffu) - lo > hi - lo && b != 0u);
+  const float q0 = __fmul_rn(d, y);
+  const float q1 = __fmaf_rn(__fmaf_rn(-q0, c, d), y, q0);
+  return __fmaf_rn(__fmaf_rn(-q1, c, d), y, q1);
+}
+
+// -v as the output holds it, v +-0 or normal.
+template <typename O>
+__device__ __forceinline__ O field_neg(float v);
+template <>
+__device__ __forceinline__ float field_neg<float>(float v) { return -v; }
+template <>
+__device__ __forceinline__ double field_neg<double>(float v) {
+  const unsigned b = __float_as_uint(v), m = b & 0x7fffffffu;
+  const unsigned hi = (m ? (m >> 3) + 0x38000000u : 0u) | (~b & 0x80000000u);
+  return __hiloint2double((int)hi, (int)(b << 29));
+}
+
+// A node of NC channels with every case (differences outside div32_fast's
+// range, divisors that are): what the march stored there is replaced.
+template <int NC, bool F64DIV, typename O>
+__device__ __noinline__ void field_node(const float* p, long long pstride, int o, int i, int j,
+                                        int k, int nx, int ny, int nz, const Spacing& sp, O* ex,
+                                        O* ey, O* ez, long long ostride) {
+  const int st[3] = {ny * nz, nz, 1}, q[3] = {i, j, k}, n[3] = {nx, ny, nz};
+  O* out[3] = {ex, ey, ez};
+  for (int c = 0; c < NC; c++)
+    for (int a = 0; a < 3; a++) {
+      const float* v = p + c * pstride + o;
+      const bool lo = q[a] > 0, hi = q[a] + 1 < n[a];
+      const float d = __fsub_rn(hi ? v[st[a]] : v[0], lo ? v[-st[a]] : v[0]);
+      __stcs(out[a] + c * ostride + o, field_out<O>(-grad_div_t<F64DIV>(d, lo && hi, sp)));
+    }
+}
+
 // E = -grad(phi) for float32 potentials, NC channels per thread.  Thread
 // (j, k) marches over `planes` x-planes of the chunk blockIdx.z % nchunks
 // for channels [NC*g, NC*g + NC), g = blockIdx.z / nchunks, with the
@@ -347,7 +388,8 @@ __device__ __forceinline__ void metal_fix(const float* __restrict__ phi, long lo
 // (the host checks nx*ny*nz + 2*ny*nz < 2^31).
 // O = double writes the float32 fields widened, for callers that want
 // float64 channels: a conversion of its own reads and writes the fields once
-// more (193 x 193 x 385, 4 channels: 245 + 670 us of conversions -> 355 us).
+// more (193 x 193 x 385, 4 channels: 245 + 670 us of conversions -> 330 us; 366 with
+// each value's cases in line).
 template <int NC, bool F64DIV, typename O>
 __global__ void __launch_bounds__(kBX * kBY)
 k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __restrict__ metal,
@@ -368,6 +410,9 @@ k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __res
   if (k < nz && j < ny && i0 < nx) {
     const bool jlo = j > 0, jhi = j + 1 < ny, klo = k > 0, khi = k + 1 < nz;
     const bool ycen = jlo && jhi, zcen = klo && khi;
+    const float yc = ycen ? sp.d2.c : sp.d1.c, yy = ycen ? sp.d2.y : sp.d1.y;
+    const float zc = zcen ? sp.d2.c : sp.d1.c, zy = zcen ? sp.d2.y : sp.d1.y;
+    const bool fast = sp.d1.ok && sp.d2.ok;
     int o = i0 * sx + j * sy + k;
     float vm[NC], vc[NC];
 #pragma unroll
@@ -390,25 +435,48 @@ k_field32(const float* __restrict__ phi, long long pstride, const uint8_t* __res
         queue[atomicAdd(&queued, 1)] =
             (unsigned short)(((i - i0) << 8) | (threadIdx.y << 5) | threadIdx.x);
       const bool xcen = i > 0 && i + 1 < nx;
+      if constexpr (!F64DIV) {
+        // one test a node for the cases (field_node): with them in line, some
+        // 52 instructions a value, the issue slots were 60 % taken
+        const float xc = xcen ? sp.d2.c : sp.d1.c, xy = xcen ? sp.d2.y : sp.d1.y;
+        bool bad = !fast;
 #pragma unroll
-      for (int c = 0; c < NC; c++) {
-        // numpy.gradient: (up - down) / 2h inside, one-sided / h at the
-        // faces (the missing y/z neighbour was replaced by the node itself
-        // above; x takes a branch that is uniform over the block).
-        float dx;
-        if (xcen)
-          dx = grad_div_t<F64DIV>(__fsub_rn(vp[c], vm[c]), true, sp);
-        else
-          dx = grad_div_t<F64DIV>(i == 0 ? __fsub_rn(vp[c], vc[c]) : __fsub_rn(vc[c], vm[c]),
-                                  false, sp);
-        const float dy = grad_div_t<F64DIV>(__fsub_rn(yb[c], ya[c]), ycen, sp);
-        const float dz = grad_div_t<F64DIV>(__fsub_rn(zb[c], za[c]), zcen, sp);
-        const long long w = ob + c * ostride + o;
-        __stcs(ex + w, field_out<O>(-dx));
-        __stcs(ey + w, field_out<O>(-dy));
-        __stcs(ez + w, field_out<O>(-dz));
-        vm[c] = vc[c];
-        vc[c] = vp[c];
+        for (int c = 0; c < NC; c++) {
+          const float xa = i > 0 ? vm[c] : vc[c], xb = i + 1 < nx ? vp[c] : vc[c];
+          const float dx = div32_fast(__fsub_rn(xb, xa), xc, xy, &bad);
+          const float dy = div32_fast(__fsub_rn(yb[c], ya[c]), yc, yy, &bad);
+          const float dz = div32_fast(__fsub_rn(zb[c], za[c]), zc, zy, &bad);
+          const long long w = ob + c * ostride + o;
+          __stcs(ex + w, field_neg<O>(dx));
+          __stcs(ey + w, field_neg<O>(dy));
+          __stcs(ez + w, field_neg<O>(dz));
+          vm[c] = vc[c];
+          vc[c] = vp[c];
+        }
+        if (bad)
+          field_node<NC, F64DIV, O>(p, pstride, o, i, j, k, nx, ny, nz, sp, ex + ob, ey + ob,
+                                    ez + ob, ostride);
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+          // numpy.gradient: (up - down) / 2h inside, one-sided / h at the
+          // faces (the missing y/z neighbour was replaced by the node itself
+          // above; x takes a branch that is uniform over the block).
+          float dx;
+          if (xcen)
+            dx = grad_div_t<F64DIV>(__fsub_rn(vp[c], vm[c]), true, sp);
+          else
+            dx = grad_div_t<F64DIV>(i == 0 ? __fsub_rn(vp[c], vc[c]) : __fsub_rn(vc[c], vm[c]),
+                                    false, sp);
+          const float dy = grad_div_t<F64DIV>(__fsub_rn(yb[c], ya[c]), ycen, sp);
+          const float dz = grad_div_t<F64DIV>(__fsub_rn(zb[c], za[c]), zcen, sp);
+          const long long w = ob + c * ostride + o;
+          __stcs(ex + w, field_out<O>(-dx));
+          __stcs(ey + w, field_out<O>(-dy));
+          __stcs(ez + w, field_out<O>(-dz));
+          vm[c] = vc[c];
+          vc[c] = vp[c];
+        }
       }
     }
   }
