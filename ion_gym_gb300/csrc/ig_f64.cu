@@ -700,18 +700,25 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
   // this thread's slots: the x and y neighbours', and bits: plain of either
   // colour (0, 1), z neighbours' distances + 1 (two bits each from 2)
   extern __shared__ uint4 near_xy[];
-  uint32_t* near_z = reinterpret_cast<uint32_t*>(near_xy + (size_t)G.rounds * kCoopThreads);
-  __shared__ unsigned long long red[2][32], all[2];
+  uint32_t* near_z = reinterpret_cast<uint32_t*>(near_xy + (size_t)G.rounds * blockDim.x);
+  // pair n in slot n & 3: the warps' maxima and how many are in, whether a
+  // warp reads the other CTAs', and the maximum of all once it is known
+  __shared__ volatile unsigned long long red[4][32], all[4];
+  __shared__ unsigned in[4], asked[4];
+  __shared__ volatile unsigned known[4];
   __shared__ int ok;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = kCoopThreads / 32;
+  if (threadIdx.x < 4)
+    in[threadIdx.x] = asked[threadIdx.x] = known[threadIdx.x] = 0;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
+  const uint32_t nt = blockDim.x;
   const uint32_t S = G.g.total, nz = (uint32_t)G.g.nz;
   const unsigned same = (G.g.nx > 1 ? 0u : 3u) | (G.g.ny > 1 ? 0u : 12u) | (nz > 1 ? 0u : 48u);
-  // slot r of this thread: t0 + r kCoopThreads, below t1
+  // slot r of this thread: t0 + r nt, below t1
   const uint32_t t0 = blockIdx.x * G.share + threadIdx.x;
   const uint32_t t1 = min(S, (blockIdx.x + 1) * G.share);
   const uint32_t cw = (uint32_t)(nw - 1 - wid) * gridDim.x + blockIdx.x;
   for (int r = 0; r < G.rounds; r++) {
-    const uint32_t t = t0 + (uint32_t)r * kCoopThreads;
+    const uint32_t t = t0 + (uint32_t)r * nt;
     uint32_t bits = 0;
     for (int c = 0; c < 2 && t < t1; c++) {
       const FlowNode f = flow_node(G, t, c);
@@ -724,16 +731,16 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
                 (f.t[5] - t + 1u) << (4 + 4 * c);
       }
       st_word(G.word + (size_t)c * S + t, v, n);
-      near_xy[r * kCoopThreads + threadIdx.x] = make_uint4(f.t[0], f.t[1], f.t[2], f.t[3]);
+      near_xy[r * nt + threadIdx.x] = make_uint4(f.t[0], f.t[1], f.t[2], f.t[3]);
     }
-    near_z[r * kCoopThreads + threadIdx.x] = bits;
+    near_z[r * nt + threadIdx.x] = bits;
   }
   if (!coop_barrier(ctl, gridDim.x, &ok)) return;
 
   int pr = 0;
   bool hit = false, undo = false;
   unsigned long long key = 0;
-  // all CTAs' maxima of pair q (warp 0); false: given up
+  // all CTAs' maximum of pair q; false: given up
   auto maxima = [&](int q, unsigned long long* out) {
     unsigned long long m = 0;
     const bool good = flow_wait(ctl, [&] {
@@ -754,6 +761,31 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
     });
     *out = warp_max_u64(m);
     return good;
+  };
+  // the same, read from the others by the CTA's first warp to ask and from
+  // shared memory by the rest
+  auto maximum = [&](int q, unsigned long long* out) {
+    const unsigned id = (unsigned)(q + 1);
+    unsigned before = 0;
+    if (lane == 0) before = atomicExch(&asked[q & 3], id);
+    if (__shfl_sync(0xffffffffu, before, 0) != id) {
+      if (!maxima(q, out)) return false;
+      if (lane == 0) {
+        all[q & 3] = *out;
+        __threadfence_block();
+        known[q & 3] = id;
+      }
+      return true;
+    }
+    if (!flow_wait(ctl, [&] {
+          if (known[q & 3] == id) return true;
+          __nanosleep(32);
+          return false;
+        }))
+      return false;
+    __threadfence_block();
+    *out = all[q & 3];
+    return true;
   };
   for (; pr < pairs && !hit; pr++) {
     unsigned long long mb = 0;
@@ -807,9 +839,9 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
         }
       }
       for (int r = 0; r < G.rounds; r++) {
-        const uint32_t t = t0 + (uint32_t)r * kCoopThreads;
-        const uint4 xy = near_xy[r * kCoopThreads + threadIdx.x];
-        const uint32_t bits = near_z[r * kCoopThreads + threadIdx.x] >> c;
+        const uint32_t t = t0 + (uint32_t)r * nt;
+        const uint4 xy = near_xy[r * nt + threadIdx.x];
+        const uint32_t bits = near_z[r * nt + threadIdx.x] >> c;
         const bool go = bits & 1u;
         const uint32_t z = bits >> (2 + 3 * c);
         const uint32_t nt[6] = {xy.x, xy.y, xy.z, xy.w, t + (z & 3u) - 1u,
@@ -847,41 +879,30 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
         if (k > mb) mb = k;
       }
     }
-    // the last pair's maximum of all CTAs in (by the warp with the fewest
-    // nodes, while the others finish), this pair's of this one out
+    // this pair's maximum out, by the CTA's last warp, and the last pair's in
     mb = warp_max_u64(mb);
-    if (lane == 0) red[pr & 1][wid] = mb;
-    if (wid == nw - 1 && pr > 0) {
-      const bool good = maxima(pr - 1, &key);
+    unsigned before = 0;
+    if (lane == 0) {
+      red[pr & 3][wid] = mb;
+      __threadfence_block();
+      before = atomicAdd(&in[pr & 3], 1u);
+    }
+    if (__shfl_sync(0xffffffffu, before, 0) == (unsigned)nw - 1) {
+      __threadfence_block();
+      mb = warp_max_u64(lane < nw ? red[pr & 3][lane] : 0ULL);
       if (lane == 0) {
-        all[pr & 1] = key;
-        if (!good) ok = 0;
+        in[pr & 3] = 0;
+        st_word(reinterpret_cast<ulonglong2*>(ctl->word[pr & 3]) + blockIdx.x, mb, pr + 1ULL);
       }
     }
-    __syncthreads();
-    if (!ok) return;
-    if (wid == 0) {
-      mb = warp_max_u64(red[pr & 1][lane]);
-      if (lane == 0)
-        st_word(reinterpret_cast<ulonglong2*>(ctl->word[pr & 3]) + blockIdx.x, mb, pr + 1ULL);
-    }
     if (pr > 0) {
-      key = all[pr & 1];
+      if (!maximum(pr - 1, &key)) return;
       hit = undo = bits_to_double(key) < tol;
     }
   }
   if (!hit) {
     // the last pair's own test
-    if (wid == nw - 1) {
-      const bool good = maxima(pairs - 1, &key);
-      if (lane == 0) {
-        all[pairs & 1] = key;
-        if (!good) ok = 0;
-      }
-    }
-    __syncthreads();
-    if (!ok) return;
-    key = all[pairs & 1];
+    if (!maximum(pairs - 1, &key)) return;
     hit = bits_to_double(key) < tol;
   }
   auto put = [&](uint32_t o, uint32_t t, int c) {
@@ -899,7 +920,7 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
         }
       }
     }
-    for (uint32_t t = t0; t < t1; t += kCoopThreads) {
+    for (uint32_t t = t0; t < t1; t += nt) {
       const FlowNode f = flow_node(G, t, c);
       if (f.k < nz && cls[f.o] == 0) put(f.o, t, c);
     }
@@ -1998,10 +2019,13 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
   G.g = g;
   G.dnz = dnz;
   G.share = (g.total + (uint32_t)n - 1) / (uint32_t)n;
-  G.rounds = (int)((G.share + kCoopThreads - 1) / kCoopThreads);
+  // no more warps than the share has work for: idle ones only ask whether the
+  // others are done
+  const unsigned nt = std::min((unsigned)kCoopThreads, std::max(64u, (G.share + 31) / 32 * 32));
+  G.rounds = (int)((G.share + nt - 1) / nt);
   G.word = static_cast<ulonglong2*>(word);
   G.prev = prev;
-  const size_t smem = (size_t)G.rounds * kCoopThreads * kFlowBytes;
+  const size_t smem = (size_t)G.rounds * nt * kFlowBytes;
   void* args[] = {&phi, &cls, &P, &G, &omega, &tol, &pairs, &ctl};
   const void* fn = kind == kThetaGhost ? (const void*)k_sor_flow<kThetaGhost>
                    : kind == kThetaSW  ? (const void*)k_sor_flow<kThetaSW>
@@ -2009,7 +2033,7 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
   // a failed launch leaves its error for the caller's check
   if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
           cudaSuccess &&
-      cudaLaunchCooperativeKernel(fn, dim3(n), dim3(kCoopThreads), args, smem, s) == cudaSuccess)
+      cudaLaunchCooperativeKernel(fn, dim3(n), dim3(nt), args, smem, s) == cudaSuccess)
     counted();
   return true;
 }
