@@ -597,9 +597,9 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
 // line.
 //
 // What is left at 65^3 is a half-sweep's chain: the neighbours' words 0.8 us,
-// sums and integer step 2.2 (28 warps an SM, FP64 alone 1.4).  solve3d at 65^3
-// 4.73 ms launched, 2.75 with barriers, 1.78 so; with theta (sw, 57 x 71 x 90)
-// 22.5, 6.0 and 3.3.
+// sums and integer step 2.0 (28 warps an SM, FP64 alone 1.4).  solve3d at 65^3
+// 4.73 ms launched, 2.75 with grid barriers, 1.78 with a block barrier a
+// pair, 1.65 so; with theta (sw, 57 x 71 x 90) 22.5, 6.0, 3.3 and 3.3.
 //
 // Waits are bounded (kCoopWait clocks, seconds): a warp that gives up raises
 // *status and leaves, the others follow, and the call reports an error.
