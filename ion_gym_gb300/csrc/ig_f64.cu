@@ -599,7 +599,8 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
 // What is left at 65^3 is a half-sweep's chain: the neighbours' words 0.8 us,
 // sums and integer step 2.0 (28 warps an SM, FP64 alone 1.4).  solve3d at 65^3
 // 4.73 ms launched, 2.75 with grid barriers, 1.78 with a block barrier a
-// pair, 1.65 so; with theta (sw, 57 x 71 x 90) 22.5, 6.0, 3.3 and 3.3.
+// pair, 1.65 so; with theta (sw, 57 x 71 x 90) 22.5, 6.0, 3.3 and 2.95 (the
+// cut nodes in warps of their own).
 //
 // Waits are bounded (kCoopWait clocks, seconds): a warp that gives up raises
 // *status and leaves, the others follow, and the call reports an error.
@@ -638,7 +639,8 @@ struct FlowGeom {
   SweepGeom g;
   FastDiv dnz;
   uint32_t share;    // slots a CTA
-  int rounds;        // and a thread
+  uint32_t workers;  // threads that have them; the warps after have cut nodes alone
+  int rounds;        // slots a worker
   ulonglong2* word;  // 2 * g.total
   double* prev;      // 2 * g.total
 };
@@ -700,7 +702,7 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
   // this thread's slots: the x and y neighbours', and bits: plain of either
   // colour (0, 1), z neighbours' distances + 1 (two bits each from 2)
   extern __shared__ uint4 near_xy[];
-  uint32_t* near_z = reinterpret_cast<uint32_t*>(near_xy + (size_t)G.rounds * blockDim.x);
+  uint32_t* near_z = reinterpret_cast<uint32_t*>(near_xy + (size_t)G.rounds * G.workers);
   // pair n in slot n & 3: the warps' maxima and how many are in, whether a
   // warp reads the other CTAs', and the maximum of all once it is known
   __shared__ volatile unsigned long long red[4][32], all[4];
@@ -710,14 +712,15 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
   if (threadIdx.x < 4)
     in[threadIdx.x] = asked[threadIdx.x] = known[threadIdx.x] = 0;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (int)blockDim.x >> 5;
-  const uint32_t nt = blockDim.x;
+  const uint32_t nt = G.workers;
+  const int rounds = threadIdx.x < nt ? G.rounds : 0;  // uniform over a warp
   const uint32_t S = G.g.total, nz = (uint32_t)G.g.nz;
   const unsigned same = (G.g.nx > 1 ? 0u : 3u) | (G.g.ny > 1 ? 0u : 12u) | (nz > 1 ? 0u : 48u);
   // slot r of this thread: t0 + r nt, below t1
   const uint32_t t0 = blockIdx.x * G.share + threadIdx.x;
   const uint32_t t1 = min(S, (blockIdx.x + 1) * G.share);
   const uint32_t cw = (uint32_t)(nw - 1 - wid) * gridDim.x + blockIdx.x;
-  for (int r = 0; r < G.rounds; r++) {
+  for (int r = 0; r < rounds; r++) {
     const uint32_t t = t0 + (uint32_t)r * nt;
     uint32_t bits = 0;
     for (int c = 0; c < 2 && t < t1; c++) {
@@ -838,7 +841,7 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
           }
         }
       }
-      for (int r = 0; r < G.rounds; r++) {
+      for (int r = 0; r < rounds; r++) {
         const uint32_t t = t0 + (uint32_t)r * nt;
         const uint4 xy = near_xy[r * nt + threadIdx.x];
         const uint32_t bits = near_z[r * nt + threadIdx.x] >> c;
@@ -920,7 +923,7 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
         }
       }
     }
-    for (uint32_t t = t0; t < t1; t += nt) {
+    for (uint32_t t = t0; rounds && t < t1; t += nt) {
       const FlowNode f = flow_node(G, t, c);
       if (f.k < nz && cls[f.o] == 0) put(f.o, t, c);
     }
@@ -2020,12 +2023,22 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
   G.dnz = dnz;
   G.share = (g.total + (uint32_t)n - 1) / (uint32_t)n;
   // no more warps than the share has work for: idle ones only ask whether the
-  // others are done
-  const unsigned nt = std::min((unsigned)kCoopThreads, std::max(64u, (G.share + 31) / 32 * 32));
-  G.rounds = (int)((G.share + nt - 1) / nt);
+  // others are done.  A theta plan's cut nodes (five a warp) get up to four
+  // warps of their own, since the nodes of a warp that has both wait behind the
+  // divisions (57 x 71 x 90, 0.4 % cut nodes: 3.31 -> 2.98 ms), but none that
+  // would cost the others a round (129^3: 20.6 us a half-sweep, 22.0 with
+  // four).
+  const uint32_t cut = plan ? std::max(plan->count[0], plan->count[1]) : 0u;
+  unsigned cutw = std::min(4u, (cut + 5u * (unsigned)n - 1) / (5u * (unsigned)n));
+  auto rounds_of = [&](unsigned w) { return (G.share + w - 1) / w; };
+  while (cutw && rounds_of(kCoopThreads - 32 * cutw) > rounds_of(kCoopThreads)) cutw--;
+  G.workers = std::min((unsigned)kCoopThreads - 32 * cutw,
+                       std::max(64u, (G.share + 31) / 32 * 32));
+  const unsigned nt = G.workers + 32 * cutw;
+  G.rounds = (int)rounds_of(G.workers);
   G.word = static_cast<ulonglong2*>(word);
   G.prev = prev;
-  const size_t smem = (size_t)G.rounds * nt * kFlowBytes;
+  const size_t smem = (size_t)G.rounds * G.workers * kFlowBytes;
   void* args[] = {&phi, &cls, &P, &G, &omega, &tol, &pairs, &ctl};
   const void* fn = kind == kThetaGhost ? (const void*)k_sor_flow<kThetaGhost>
                    : kind == kThetaSW  ? (const void*)k_sor_flow<kThetaSW>

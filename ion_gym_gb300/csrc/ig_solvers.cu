@@ -390,8 +390,8 @@ void fine_sweep(cudaStream_t s, double* phi, const uint8_t* fx, const float* th,
 // Slots of one colour up to which the SOR loop is one launch (k_sor_flow):
 // eight nodes a thread.  A half-sweep of solve3d, launched against resident
 // (us, host copies of the call included): 33^3 7.1 / 2.1, 65^3 11.1 / 3.8,
-// 97^3 22.9 / 8.6, 129^3 31.3 / 19.9; with theta (sw) 33^3 9.6 / 3.1, 65^3
-// 14.6 / 4.2, 129^3 44.6 / 20.6.  Past that the sweep itself fills the GPU,
+// 97^3 22.9 / 8.6, 129^3 31.3 / 19.9; with theta (sw) 33^3 9.6 / 2.7, 65^3
+// 14.6 / 3.9, 129^3 44.6 / 20.6.  Past that the sweep itself fills the GPU,
 // one call would hold every SM for long, and a thread's neighbour slots fill
 // its SM's shared memory.
 constexpr long kCoopSlots = 8L * 152 * kCoopThreads;
