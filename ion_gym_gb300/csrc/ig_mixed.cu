@@ -1962,7 +1962,10 @@ inline unsigned flat_blocks(const SGeo& G, uint32_t R) {
 // analogue of the V-cycle's full-cycle change, multigrid3d.py:702).  With
 // p given, e32 is e + alpha p: the flexible CG's last step x += alpha p
 // folded in (k_cg_update's expression; its g half is dead, the residual is
-// recomputed next).  One warp per natural row, as k_resid64: lane k's
+// recomputed next).  With e2 given, e and e2 are the directions of a step's
+// first two iterations and hist their alphas: x = a1 p1 + a2 p2, as the
+// direction updates would have summed it.  One warp per natural row, as
+// k_resid64: lane k's
 // potential and mask are 8 and 1 contiguous bytes of the row, its
 // correction slot k >> 1 of the colour (i + j + k) & 1, so a warp's loads
 // of the corrections are two runs of 16 consecutive floats.
@@ -1970,7 +1973,8 @@ __global__ void __launch_bounds__(kT)
 k_update64(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
            const float* __restrict__ e, SGeo G, unsigned long long* dmax,
            const int* __restrict__ fexp, size_t nstride, size_t pstride,
-           const float* __restrict__ p = nullptr, const double* __restrict__ scal = nullptr) {
+           const float* __restrict__ p = nullptr, const double* __restrict__ scal = nullptr,
+           const float* __restrict__ e2 = nullptr, const double* __restrict__ hist = nullptr) {
   const uint32_t r = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   unsigned key32 = 0;
   if (r < (uint32_t)G.nx * (uint32_t)G.ny) {
@@ -1985,7 +1989,11 @@ k_update64(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
     const float* eo = e ? e + ro + (size_t)(1 - ((i + j) & 1)) * G.csz : nullptr;
     const float* pe = p ? p + ro + (size_t)((i + j) & 1) * G.csz : nullptr;
     const float* po = p ? p + ro + (size_t)(1 - ((i + j) & 1)) * G.csz : nullptr;
+    const float* qe = e2 ? e2 + ro + (size_t)((i + j) & 1) * G.csz : nullptr;
+    const float* qo = e2 ? e2 + ro + (size_t)(1 - ((i + j) & 1)) * G.csz : nullptr;
     const float al = p ? (float)scal[4 * blockIdx.y + 1] : 0.f;
+    const float a1 = e2 ? (float)hist[2 * blockIdx.y] : 0.f;
+    const float a2 = e2 ? (float)hist[2 * blockIdx.y + 1] : 0.f;
     const float to_units = pow2f(56 - fexp[blockIdx.y]);
     // The loads do not wait for the mask (all in bounds) and no lane
     // branches on it: metal nodes compute a zero change and skip only the
@@ -1999,6 +2007,7 @@ k_update64(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
       const uint8_t metal = fr[k];
       const long long old = pr[k];
       float ev = e ? ((k & 1) ? eo : ee)[m] : 0.f;
+      if (e2) ev = __fmaf_rn(a2, ((k & 1) ? qo : qe)[m], __fmaf_rn(a1, ev, 0.f));
       if (p) ev = __fmaf_rn(al, ((k & 1) ? po : pe)[m], ev);
       ev = metal ? 0.f : ev;
       const long long nv = old + f2ll_rn(ev * to_units);
@@ -2026,7 +2035,9 @@ __global__ void __launch_bounds__(kT)
 k_update64_flat(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
                 const float* __restrict__ e, SGeo G, unsigned long long* dmax,
                 const int* __restrict__ fexp, size_t nstride, size_t pstride,
-                const float* __restrict__ p, const double* __restrict__ scal, uint32_t R) {
+                const float* __restrict__ p, const double* __restrict__ scal, uint32_t R,
+                const float* __restrict__ e2 = nullptr,
+                const double* __restrict__ hist = nullptr) {
   const uint32_t nrows = (uint32_t)G.nx * (uint32_t)G.ny;
   const uint32_t r0 = (blockIdx.x * kRowWarps + (threadIdx.x >> 5)) * R;
   unsigned key32 = 0;
@@ -2038,6 +2049,8 @@ k_update64_flat(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
     const uint8_t* F = fixed + (size_t)blockIdx.y * G.mnat + (size_t)r0 * nz;
     const size_t pb = blockIdx.y * pstride;
     const float al = p ? (float)scal[4 * blockIdx.y + 1] : 0.f;
+    const float a1 = e2 ? (float)hist[2 * blockIdx.y] : 0.f;
+    const float a2 = e2 ? (float)hist[2 * blockIdx.y + 1] : 0.f;
     const float to_units = pow2f(56 - fexp[blockIdx.y]);
 #pragma unroll 2
     for (uint32_t q = lane; q < span; q += 32) {
@@ -2050,6 +2063,7 @@ k_update64_flat(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
       const uint8_t metal = F[q];
       const long long old = P[q];
       float ev = e ? e[so] : 0.f;
+      if (e2) ev = __fmaf_rn(a2, e2[so], __fmaf_rn(a1, ev, 0.f));
       if (p) ev = __fmaf_rn(al, p[so], ev);
       ev = metal ? 0.f : ev;
       const long long nv = old + f2ll_rn(ev * to_units);
@@ -2532,10 +2546,10 @@ k_cg_dot(const float* __restrict__ z, const float* __restrict__ q,
 
 // Per-problem fixed-order sums of the partials.  mode 0: alpha from <p,q>
 // and <p,g> (also keeps <p,q> for beta); mode 1: beta = -<z,q>/<p,q>.
-// scal[4b + 0] = <p,q>, [1] = alpha, [2] = beta.
+// scal[4b + 0] = <p,q>, [1] = alpha (also to keep[2b]), [2] = beta.
 __global__ void __launch_bounds__(kT)
 k_cg_reduce(const double* __restrict__ part, int nparts, int stride,
-            double* __restrict__ scal, int mode) {
+            double* __restrict__ scal, int mode, double* __restrict__ keep = nullptr) {
   __shared__ double sh[kT / 32];
   const int b = blockIdx.x;
   double a = 0.0, c = 0.0;
@@ -2552,6 +2566,7 @@ k_cg_reduce(const double* __restrict__ part, int nparts, int stride,
     if (mode == 0) {
       S[0] = sa;
       S[1] = sa > 0.0 ? -sc / sa : 0.0;
+      if (keep) keep[2 * b] = S[1];
     } else {
       S[2] = S[0] > 0.0 ? -sa / S[0] : 0.0;
     }
@@ -2706,6 +2721,7 @@ struct Session {
   bool dot_done = false;   // ... and did (its partial count in dot_nparts)
   int dot_nparts = 0;
   Buf<double> part, scal;
+  Buf<double> hist;  // alphas of a step's first two iterations, per problem
   int method = 1;            // 0: defect correction with `vcycles` cycles,
                              // 1: flexible CG preconditioned by one cycle
   int cg_iters = 3;          // CG iterations per FP64 refinement
@@ -2762,6 +2778,7 @@ struct Session {
     qb.release();
     part.release();
     scal.release();
+    hist.release();
     if (s) {
       cudaStreamSynchronize(s);
       cudaStreamDestroy(s);
@@ -2840,6 +2857,7 @@ struct Session {
       const size_t nb4 = nblk(lv[0].G.csz / 4), nbn = nblk((uint32_t)lv[0].pstride);
       part.alloc(std::max(4 * nb4, nbn) * bmax, s);
       scal.alloc(4 * bmax, s);
+      hist.alloc(2 * (size_t)bmax, s);
     }
     MK(cudaGetLastError());
   }
@@ -3246,15 +3264,15 @@ struct Session {
           phi.p, fixed.p, f.G, f.g.p, fexp.p, (float)-resid_scale, f.G.n, f.pstride, R);
   }
   void launch_update64(const float* e, unsigned long long* dm, const float* p,
-                       const double* sc) {
+                       const double* sc, const float* e2 = nullptr) {
     MLevel& f = lv[0];
     const uint32_t R = flat_rows(f.G, rows_force);
     if (R == 1)
       k_update64<<<dim3(rows_blocks(f.G), B), kT, 0, s>>>(phi.p, fixed.p, e, f.G, dm, fexp.p,
-                                                          f.G.n, f.pstride, p, sc);
+                                                          f.G.n, f.pstride, p, sc, e2, hist.p);
     else
       k_update64_flat<<<dim3(flat_blocks(f.G, R), B), kT, 0, s>>>(
-          phi.p, fixed.p, e, f.G, dm, fexp.p, f.G.n, f.pstride, p, sc, R);
+          phi.p, fixed.p, e, f.G, dm, fexp.p, f.G.n, f.pstride, p, sc, R, e2, hist.p);
   }
 
   // one refinement step: FP64 residual, V-cycles on the correction, update
@@ -3288,8 +3306,13 @@ struct Session {
     const unsigned nbd = cg_blocks(n / 4, (unsigned)B);
     float* pcur = from_b2 ? pb2.p : pb.p;
     float* pnext = from_b2 ? pb.p : pb2.p;
-    const bool fold = fold_ok();
+    const bool fold = fold_ok(), three = three_ok();
+    float* dir[3] = {pb.p, pb2.p, xb.p};
     for (int it = 0; it < cg_iters; it++) {
+      if (three) {
+        pcur = dir[it];
+        pnext = dir[(it + 1) % 3];
+      }
       // with fold, iteration it > 0 takes the previous iteration's
       // k_cg_update in two halves: g += alpha q in the finest level's
       // zero-start pair, x += alpha p_old in the direction update
@@ -3307,7 +3330,7 @@ struct Session {
       }
       if (fuse_dir()) {
         const dim3 gm(nb4, 2, B);
-        if (!fold || it == 0)
+        if (!fold || it == 0 || three)
           k_cg_matvec_dir<0><<<gm, kT, 0, s>>>(f.e.p, pcur, pnext, scal.p, f.g.p, f.mask.p,
                                                f.G, qb.p, part.p, f.pstride, nullptr);
         else if (it == 1)
@@ -3322,7 +3345,8 @@ struct Session {
         k_cg_matvec<<<dim3(nb4, 2, B), kT, 0, s>>>(pcur, f.g.p, f.mask.p, f.G, qb.p, part.p,
                                                   f.pstride);
       }
-      k_cg_reduce<<<B, kT, 0, s>>>(part.p, 2 * (int)nb4, 2, scal.p, 0);
+      k_cg_reduce<<<B, kT, 0, s>>>(part.p, 2 * (int)nb4, 2, scal.p, 0,
+                                   three && it < 2 ? hist.p + it : nullptr);
       // the last iteration's x += alpha p is folded into the FP64 update
       // below; the first one writes x = alpha p (no zeroing pass)
       if (fold)
@@ -3336,13 +3360,18 @@ struct Session {
     }
     MK(cudaMemsetAsync(dmax.p, 0, 8 * B, s));
     // phi += x + alpha p (x absent when the step has one iteration)
-    launch_update64(cg_iters > 1 ? xb.p : nullptr, dmax.p, pcur, scal.p);
+    if (three)
+      launch_update64(dir[1], dmax.p, dir[0], scal.p, dir[2]);
+    else
+      launch_update64(cg_iters > 1 ? xb.p : nullptr, dmax.p, pcur, scal.p);
     launch_resid64();
   }
 
   // a step ends with the direction in the other buffer when the fused CG
   // runs an odd number of iterations
-  bool step_swaps() const { return method == 1 && fuse_dir() && (cg_iters & 1); }
+  bool step_swaps() const {
+    return method == 1 && fuse_dir() && (cg_iters & 1) && !three_ok();
+  }
 
   // The CG update folded into the next iteration (k_gs_zero_pair_fold,
   // k_cg_matvec_dir<1|2>): the finest level starts its cycle with the fused
@@ -3361,6 +3390,13 @@ struct Session {
            (cg_iters & 1) && fuse_zero_pair(lv[0]) && !tb_pre(0, true) && !tail_level(0) &&
            lv.size() > 1;
   }
+
+  // A step of three folded iterations keeps their three directions, the last
+  // in the buffer of the one before the step, and the update sums them: the
+  // correction x is not kept: eight 193 x 193 x 385 bases, direction updates
+  // 429 + 551 + 690 -> 3 x 429 us and the update 517 -> 630, a solve 38.2 ->
+  // 36.5 ms; 24 bases of 256 x 64 x 48 11.0 -> 10.9.
+  bool three_ok() const { return fold_ok() && cg_iters == 3; }
 
   void step() {
     const bool from_b2 = method == 1 && p_in_b2;
@@ -3452,14 +3488,14 @@ struct Session {
         b += (fuse_dir() ? 21.0 : 33.0) * n;            // direction, L p
         if (fold) {
           // q in, the updated g out (zero-start pair); x out / in and out
-          if (it > 0) b += 8.0 * n + (it == 1 ? 4.0 : 8.0) * n;
+          if (it > 0) b += 8.0 * n + (three_ok() ? 0.0 : it == 1 ? 4.0 : 8.0) * n;
         } else if (it == 0 && cg_iters > 1) {
           b += 20.0 * n;                                // x = a p, g += a q
         } else if (it + 1 < cg_iters) {
           b += 24.0 * n;
         }
       }
-      b += (cg_iters > 1 ? 25.0 : 21.0) * n;            // phi += x + a p
+      b += (three_ok() ? 29.0 : cg_iters > 1 ? 25.0 : 21.0) * n;  // phi += x + a p
     } else {
       for (int v = 0; v < vcycles; v++) b += cycle_bytes(0, v == 0);
       b += 21.0 * n;                                    // phi += e
