@@ -2172,19 +2172,21 @@ __device__ __forceinline__ double units_out(long long q, int fexp) {
       sor_key(u, e) | (q < 0 ? 0x8000000000000000ULL : 0ULL)));
 }
 
-// In place: the float64 potential of problem b from its units (Phi * u_b,
-// one rounding when |Phi| >= 2^53), with the Dirichlet values written
+// The float64 potential of problem b from its units (Phi * u_b, one rounding
+// when |Phi| >= 2^53) to out, phi itself or a result on the device (a copy
+// would move it once more, 290 us), with the Dirichlet values written
 // exactly at the metal: vals (n per problem) when given, else the basis
 // set's v_basis on mask b (masks, n per problem) and 0 on the rest.
 // 193 x 193 x 385, 8 bases: 527 -> 311 us.
 __global__ void __launch_bounds__(kT)
-k_fixed_out(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
+k_fixed_out(const long long* phi, double* out, const uint8_t* __restrict__ fixed,
             const double* __restrict__ vals, const uint8_t* __restrict__ masks,
             double v, uint32_t n, size_t nstride,
             const int* __restrict__ fexp, size_t fstride) {
   const uint32_t t0 = blockIdx.x * kIo * kT + threadIdx.x;
   fixed += blockIdx.y * fstride;
   phi += blockIdx.y * nstride;
+  out += blockIdx.y * nstride;
   if (vals) vals += blockIdx.y * nstride;
   if (masks) masks += (size_t)blockIdx.y * n;
   const int ex = fexp[blockIdx.y];
@@ -2204,7 +2206,7 @@ k_fixed_out(long long* __restrict__ phi, const uint8_t* __restrict__ fixed,
     if (t >= n) continue;
     double r = units_out(q[u], ex);
     if (metal[u]) r = vals ? vals[t] : (masks[t] ? v : 0.0);
-    reinterpret_cast<double*>(phi)[t] = r;
+    out[t] = r;
   }
 }
 
@@ -3596,6 +3598,17 @@ void set_units(Session& S, const std::vector<double>& vmax) {
 
 // The float64 potentials (Dirichlet values exact at the metal: vals, or
 // v_basis on the basis masks) into phi_out.
+// Memory of the current device, which a kernel may write.
+bool on_device(const void* p) {
+  cudaPointerAttributes a;
+  int dev = -1;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
            double* dmax_out, const double* vals, const uint8_t* masks, double v,
            float* unit_out = nullptr) {
@@ -3605,7 +3618,8 @@ int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
     // float32 unit bases, staged in the finest level's correction buffer
     // (scratch once the refinement is done; it holds pstride >= n floats
     // per problem)
-    float* u = S.lv[0].e.p;
+    const bool direct = on_device(unit_out);
+    float* u = direct ? unit_out : S.lv[0].e.p;
     // every basis of the set has v's exponent as its unit's (set_units)
     UnitScale U;
     U.v = v;
@@ -3617,12 +3631,14 @@ int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
     U.other = (float)(0.0 / v);
     k_unit32_out<<<dim3(io_blocks(n), S.B), kT, 0, S.s>>>(S.phi.p, S.fixed.p, masks, U, n, n, u);
     MK(cudaGetLastError());
-    MK(cudaMemcpyAsync(unit_out, u, (size_t)n * S.B * 4, cudaMemcpyDefault, S.s));
+    if (!direct) MK(cudaMemcpyAsync(unit_out, u, (size_t)n * S.B * 4, cudaMemcpyDefault, S.s));
   } else {
-    k_fixed_out<<<dim3(io_blocks(n), S.B), kT, 0, S.s>>>(S.phi.p, S.fixed.p, vals, masks, v, n, n,
-                                                    S.fexp.p, S.lv[0].G.mnat);
+    const bool direct = on_device(phi_out);
+    double* to = direct ? phi_out : reinterpret_cast<double*>(S.phi.p);
+    k_fixed_out<<<dim3(io_blocks(n), S.B), kT, 0, S.s>>>(S.phi.p, to, S.fixed.p, vals, masks, v, n,
+                                                    n, S.fexp.p, S.lv[0].G.mnat);
     MK(cudaGetLastError());
-    MK(cudaMemcpyAsync(phi_out, S.phi.p, S.d.n() * S.B * 8, cudaMemcpyDefault, S.s));
+    if (!direct) MK(cudaMemcpyAsync(phi_out, to, S.d.n() * S.B * 8, cudaMemcpyDefault, S.s));
   }
   MK(cudaStreamSynchronize(S.s));
   if (steps_out) *steps_out = r.steps;
