@@ -3290,10 +3290,10 @@ struct Session {
   void cg_init() {
     MLevel& f = lv[0];
     launch_resid64();
-    MK(cudaMemsetAsync(xb.p, 0, f.pstride * B * 4, s));
+    // x is written before it is read (the first iteration's x = alpha p, or
+    // the third direction), and q counts only once <p, q> > 0 (scal)
     MK(cudaMemsetAsync(pb.p, 0, f.pstride * B * 4, s));
     p_in_b2 = false;
-    MK(cudaMemsetAsync(qb.p, 0, f.pstride * B * 4, s));
     MK(cudaMemsetAsync(scal.p, 0, 4 * B * 8, s));
   }
 
