@@ -824,10 +824,14 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
                 return have;
               }))
             return;
-          const double v = __longlong_as_double((long long)vb);
-          const double old = __longlong_as_double((long long)ob);
-          const double term = KIND == kThetaGhost ? __dmul_rn(v, w) : __ddiv_rn(v, w);
           const int l0 = lane < 30 ? 6 * who : 24;
+          // along an axis of one node a leg is the node itself: its value from
+          // the lane that stored it (l0), since nothing orders this lane's own
+          // read of the word behind that store
+          const unsigned long long mine = __shfl_sync(0xffffffffu, ob, l0);
+          const double v = __longlong_as_double((long long)(self ? mine : vb));
+          const double old = __longlong_as_double((long long)mine);
+          const double term = KIND == kThetaGhost ? __dmul_rn(v, w) : __ddiv_rn(v, w);
           double num = __shfl_sync(0xffffffffu, term, l0);
 #pragma unroll
           for (int d = 1; d < 6; d++)
@@ -889,14 +893,14 @@ k_sor_flow(double* phi, const uint8_t* __restrict__ cls, const ThetaPlan P, Flow
       red[pr & 3][wid] = mb;
       __threadfence_block();
       before = atomicAdd(&in[pr & 3], 1u);
-    }
-    if (__shfl_sync(0xffffffffu, before, 0) == (unsigned)nw - 1) {
       __threadfence_block();
+    }
+    // a slot's count goes up by nw every four pairs and is never reset
+    if (__shfl_sync(0xffffffffu, before, 0) == (unsigned)(nw * (pr >> 2) + nw - 1)) {
+      __syncwarp();
       mb = warp_max_u64(lane < nw ? red[pr & 3][lane] : 0ULL);
-      if (lane == 0) {
-        in[pr & 3] = 0;
+      if (lane == 0)
         st_word(reinterpret_cast<ulonglong2*>(ctl->word[pr & 3]) + blockIdx.x, mb, pr + 1ULL);
-      }
     }
     if (pr > 0) {
       if (!maximum(pr - 1, &key)) return;

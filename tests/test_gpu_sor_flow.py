@@ -51,3 +51,19 @@ def test_theta(shape, stencil):
     a = S.solve3d(fixed, val, theta=theta, tol=1e-5, omega=1.0, stencil=stencil)
     b = port.solve3d(fixed, val, theta=theta, tol=1e-5, omega=1.0, stencil=stencil)
     assert a[1:] == b[1:] and same_bits(a[0], b[0])
+
+
+# a leg along an axis of one node is the node itself: its value of the pair
+# before, also where most warps have cut nodes alone
+@pytest.mark.parametrize("stencil", ["ghost_linear", "sw"])
+@pytest.mark.parametrize("shape", [(1, 90, 91), (67, 1, 80), (75, 74, 1), (1, 1, 400), (1, 1, 1)])
+def test_theta_on_axes_of_one_node(shape, stencil):
+    from ion_gym_gb300.physics import solver3d as S
+    fixed, val = _deck(shape, 25)
+    rng = np.random.default_rng(26)
+    theta = np.ones((6,) + shape, np.float32)
+    cut = (rng.random(shape) < 0.09) & ~fixed
+    theta[:, cut] = rng.uniform(0.3, 1.0, (6, int(cut.sum()))).astype(np.float32)
+    a = S.solve3d(fixed, val, theta=theta, tol=1e-6, omega=1.0, stencil=stencil)
+    b = port.solve3d(fixed, val, theta=theta, tol=1e-6, omega=1.0, stencil=stencil)
+    assert a[1:] == b[1:] and same_bits(a[0], b[0])
