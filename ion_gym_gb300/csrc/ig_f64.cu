@@ -1998,30 +1998,61 @@ bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const do
   return true;
 }
 
+// A number found once for each device: a kernel's attributes and the launches
+// that fit belong to the device, and another thread's call may be between
+// finding them and launching.
+class PerDevice {
+ public:
+  // find(device) on the current device's first use; 0 where there is no device
+  template <class F>
+  int get(F&& find) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMost) {
+      cudaGetLastError();
+      return 0;
+    }
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!found_[dev]) {
+      value_[dev] = find(dev);
+      found_[dev] = true;
+    }
+    return value_[dev];
+  }
+
+ private:
+  static constexpr int kMost = 64;
+  std::mutex mu_;
+  int value_[kMost] = {0};
+  bool found_[kMost] = {false};
+};
+
+// The largest dynamic shared memory a CTA of k_sor_flow is launched with: its
+// share of the slots of the largest grid on this route (152 SMs).  The
+// attribute is set to this once, never to a call's own size: calls of other
+// threads launch the same kernels.
+constexpr size_t kFlowSmemMax = 8 * kCoopThreads * kFlowBytes;
+
 bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const ThetaPlan* plan,
                      int kind, Dims d, double omega, double tol, int pairs, CoopCtl* ctl,
                      void* word, double* prev) {
-  // a whole grid of one CTA per SM, found once per device
-  static std::mutex mu;
-  static int sms[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  int n = 0;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!sms[dev]) {
-      int coop = 0, count = 0;
-      cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-      cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-      sms[dev] = coop && count > 0 ? std::min(count, kCoopCtas) : -1;
-    }
-    n = sms[dev];
-  }
+  // a whole grid of one CTA per SM
+  static PerDevice sms;
+  const int n = sms.get([](int dev) {
+    int coop = 0, count = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    for (const void* fn : {(const void*)k_sor_flow<kThetaGhost>, (const void*)k_sor_flow<kThetaSW>,
+                           (const void*)k_sor_flow<kPlain>})
+      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kFlowSmemMax) != cudaSuccess)
+        coop = 0;
+    cudaGetLastError();
+    return coop ? std::min(count, kCoopCtas) : 0;
+  });
   if (n < 1 || !word) return false;
   SweepGeom g = sweep_geom(d);
   FastDiv dnz((uint32_t)d.nz);
   ThetaPlan P = plan ? *plan : ThetaPlan();
-  if (cudaMemsetAsync(ctl, 0, sizeof(CoopCtl), s) != cudaSuccess) return true;
   FlowGeom G;
   G.g = g;
   G.dnz = dnz;
@@ -2043,15 +2074,19 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
   G.word = static_cast<ulonglong2*>(word);
   G.prev = prev;
   const size_t smem = (size_t)G.rounds * G.workers * kFlowBytes;
+  if (smem > kFlowSmemMax || cudaMemsetAsync(ctl, 0, sizeof(CoopCtl), s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
   void* args[] = {&phi, &cls, &P, &G, &omega, &tol, &pairs, &ctl};
   const void* fn = kind == kThetaGhost ? (const void*)k_sor_flow<kThetaGhost>
                    : kind == kThetaSW  ? (const void*)k_sor_flow<kThetaSW>
                                        : (const void*)k_sor_flow<kPlain>;
-  // a failed launch leaves its error for the caller's check
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-          cudaSuccess &&
-      cudaLaunchCooperativeKernel(fn, dim3(n), dim3(nt), args, smem, s) == cudaSuccess)
-    counted();
+  if (cudaLaunchCooperativeKernel(fn, dim3(n), dim3(nt), args, smem, s) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  counted();
   return true;
 }
 

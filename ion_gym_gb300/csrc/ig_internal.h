@@ -108,7 +108,8 @@ bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const do
 // nodes of a theta solve (kind kThetaGhost / kThetaSW) or null.  ctl gets
 // the pairs run, whether the last met tol and its max |update| key; status 1
 // means a wait gave up.  word (32 bytes a slot of one colour) and prev (16)
-// are scratch.  false: the device takes no such launch.
+// are scratch.  false: nothing was launched, since the device takes no such
+// launch or refused this one (no error is left behind).
 constexpr int kCoopThreads = 1024, kCoopCtas = 512;
 struct CoopCtl {
   unsigned arrived;

@@ -415,9 +415,11 @@ bool sor_loop_coop(ThreadCtx& c, double* phi, const uint8_t* fx, const float* th
     const int lim = (int)std::min<long>(kCoopPairs, max_pairs - base);
     if (prof) CK(cudaEventRecord(c.ev0, c.s));
     if (!launch_sor_coop(c.s, phi, t.on() ? t.plan.cls : fx, t.on() ? &t.plan : nullptr, kind, d,
-                         omega, tol, lim, ctl.p, word.p, before.p))
-      return false;
-    CK(cudaGetLastError());
+                         omega, tol, lim, ctl.p, word.p, before.p)) {
+      // refused: the launched sweeps, which take the pairs from the first
+      if (base == 0) return false;
+      throw Status(IG_CUDA_ERROR, "SOR loop: a further launch was refused");
+    }
     if (prof) CK(cudaEventRecord(c.ev1, c.s));
     CoopCtl h;
     CK(cudaMemcpyAsync(&h, ctl.p, offsetof(CoopCtl, word), cudaMemcpyDeviceToHost, c.s));

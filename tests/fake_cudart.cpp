@@ -1,0 +1,165 @@
+// The library's launchers over a stand-in CUDA runtime of two devices, which
+// keeps kernel attributes by device and refuses a launch beyond them as the
+// real one does; nothing is computed.  Prints one line per check; the first
+// word says what it is, the rest what happened.
+#include <cstdio>
+#include <cstring>
+#include <map>
+#include <string>
+#include <utility>
+
+#include <cuda_runtime.h>
+
+#include "ig_internal.h"
+
+namespace {
+struct Attr {
+  size_t smem = 48 * 1024;
+  int cluster = 8, lowered = 0;
+};
+struct Config {
+  dim3 grid, block;
+  size_t smem = 0;
+  cudaStream_t s = nullptr;
+};
+int device = 0, launched = 0, refuse = 0;
+cudaError_t last = cudaSuccess;
+std::map<std::pair<int, const void*>, Attr> attrs;
+Config config;
+
+cudaError_t note(cudaError_t e) {
+  if (e != cudaSuccess) last = e;
+  return e;
+}
+cudaError_t launch(const void* fn, size_t smem, int cluster) {
+  const Attr& a = attrs[{device, fn}];
+  if (refuse || smem > a.smem || cluster > a.cluster) return note(cudaErrorInvalidValue);
+  launched++;
+  return cudaSuccess;
+}
+int cluster_of(const cudaLaunchConfig_t* c) {
+  int n = 1;
+  for (unsigned q = 0; q < c->numAttrs; q++)
+    if (c->attrs[q].id == cudaLaunchAttributeClusterDimension)
+      n = (int)c->attrs[q].val.clusterDim.x;
+  return n;
+}
+}  // namespace
+
+extern "C" {
+void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
+void __cudaRegisterFatBinaryEnd(void**) {}
+void __cudaUnregisterFatBinary(void**) {}
+void __cudaRegisterFunction(void**, const char*, char*, const char*, int, uint3*, uint3*, dim3*,
+                            dim3*, int*) {}
+unsigned __cudaPushCallConfiguration(dim3 g, dim3 b, size_t smem, cudaStream_t s) {
+  config.grid = g;
+  config.block = b;
+  config.smem = smem;
+  config.s = s;
+  return 0;
+}
+cudaError_t __cudaPopCallConfiguration(dim3* g, dim3* b, size_t* smem, void* s) {
+  *g = config.grid;
+  *b = config.block;
+  *smem = config.smem;
+  *static_cast<cudaStream_t*>(s) = config.s;
+  return cudaSuccess;
+}
+cudaError_t __cudaGetKernel(cudaKernel_t* k, const void* fn) {
+  *k = reinterpret_cast<cudaKernel_t>(const_cast<void*>(fn));
+  return cudaSuccess;
+}
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t smem, cudaStream_t) {
+  return launch(reinterpret_cast<const void*>(k), smem, 1);
+}
+cudaError_t cudaLaunchKernel(const void* fn, dim3, dim3, void**, size_t smem, cudaStream_t) {
+  return launch(fn, smem, 1);
+}
+cudaError_t cudaLaunchCooperativeKernel(const void* fn, dim3, dim3, void**, size_t smem,
+                                        cudaStream_t) {
+  return launch(fn, smem, 1);
+}
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
+  return launch(fn, c->dynamicSmemBytes, cluster_of(c));
+}
+cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void* fn, const cudaLaunchConfig_t* c) {
+  const Attr& a = attrs[{device, fn}];
+  if (c->dynamicSmemBytes > a.smem || cluster_of(c) > a.cluster)
+    return note(cudaErrorInvalidValue);
+  *n = 1;
+  return cudaSuccess;
+}
+cudaError_t cudaFuncSetAttribute(const void* fn, cudaFuncAttribute what, int v) {
+  Attr& a = attrs[{device, fn}];
+  if (what == cudaFuncAttributeMaxDynamicSharedMemorySize) {
+    if ((size_t)v < a.smem) a.lowered++;
+    a.smem = (size_t)v;
+  }
+  if (what == cudaFuncAttributeNonPortableClusterSizeAllowed) a.cluster = v ? 16 : 8;
+  return cudaSuccess;
+}
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr what, int) {
+  *v = what == cudaDevAttrMultiProcessorCount ? 152 : 1;
+  return cudaSuccess;
+}
+cudaError_t cudaGetDevice(int* d) {
+  *d = device;
+  return cudaSuccess;
+}
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = last;
+  last = cudaSuccess;
+  return e;
+}
+cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
+}
+
+using namespace ig;
+
+static bool sor(long side) {
+  char scratch[64];
+  return launch_sor_coop(nullptr, reinterpret_cast<double*>(scratch),
+                         reinterpret_cast<uint8_t*>(scratch), nullptr, kPlain,
+                         Dims{side, side, side}, 1.5, 1e-3, 8, reinterpret_cast<CoopCtl*>(scratch),
+                         scratch, reinterpret_cast<double*>(scratch));
+}
+
+static bool tail() {
+  TailArgs a{};
+  for (long n : {33L, 17L, 9L})
+    a.lv[a.nlev++] = tail_level(Dims{n, n, n}, nullptr, nullptr, nullptr, nullptr);
+  a.nu1 = a.nu2 = 2;
+  return launch_err_tail(nullptr, a);
+}
+
+static bool bottom(long n) {
+  return launch_bottom_err(nullptr, nullptr, nullptr, nullptr, Dims{n, n, n}, 1e-3, 1.5, 10);
+}
+
+static void say(const char* what, bool took) {
+  std::printf("%s took=%d launched=%d error=%d\n", what, took, launched, (int)cudaGetLastError());
+  launched = 0;
+}
+
+int main() {
+  say("sor-large", sor(129));
+  say("sor-small", sor(40));
+  int lowered = 0;
+  for (auto& a : attrs) lowered += a.second.lowered;
+  std::printf("sor-attribute lowered=%d\n", lowered);
+  device = 1;
+  say("sor-second-device", sor(129));
+  refuse = 1;
+  say("sor-refused", sor(65));
+  refuse = 0;
+  for (device = 0; device < 2; device++) {
+    const std::string d = std::to_string(device);
+    say(("tail-device" + d).c_str(), tail());
+    say(("bottom-device" + d).c_str(), bottom(21));  // 167 KB of shared memory
+  }
+  refuse = 1;
+  say("tail-refused", tail());
+  say("bottom-refused", bottom(21));
+  return 0;
+}

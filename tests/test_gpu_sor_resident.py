@@ -57,3 +57,19 @@ def test_solves_from_several_threads():
     for (f, v), a in zip(decks, got):
         b = port.solve3d(f, v, tol=1e-3, omega=1.5)
         assert a[1:] == b[1:] and same_bits(a[0], b[0])
+
+
+# shared memory from a few KB to over 100 a CTA, in calls of threads that
+# start theirs at any time
+def test_threads_with_small_and_large_grids():
+    from ion_gym_gb300.physics import solver3d as S
+    decks = [_deck(shape, 30 + q) for q, shape in enumerate([(40, 40, 40), (129, 129, 129)] * 3)]
+    want = [S.solve3d(*d, tol=0.5, omega=1.5) for d in decks]
+
+    def calls(q):
+        for _ in range(40 if q % 2 == 0 else 15):
+            a = S.solve3d(*decks[q], tol=0.5, omega=1.5)
+            assert a[1:] == want[q][1:] and same_bits(a[0], want[q][0])
+
+    with ThreadPoolExecutor(len(decks)) as ex:
+        list(ex.map(calls, range(len(decks))))

@@ -1,0 +1,37 @@
+"""The launchers that set kernel attributes, over a stand-in CUDA runtime
+(fake_cudart.cpp): a call's own size is never left behind for other threads'
+calls, every device gets its attributes, and a refused launch is reported as
+not launched, with no error left, so that the caller takes the other route."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def said(tmp_path_factory):
+    from ion_gym_gb300 import build as B
+    if not os.path.exists(os.path.join(B.OUT_DIR, "ig_f64.o")):
+        B.build(force=True)
+    exe = str(tmp_path_factory.mktemp("launchers") / "launchers")
+    include = os.path.join(os.path.dirname(os.path.dirname(B.nvcc())), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", B.CSRC, "-I", include,
+                    os.path.join(HERE, "fake_cudart.cpp"),
+                    os.path.join(B.OUT_DIR, "ig_f64.o"), "-o", exe, "-lpthread"], check=True)
+    out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
+    return dict(line.split(" ", 1) for line in out.splitlines())
+
+
+TOOK, REFUSED = "took=1 launched=1 error=0", "took=0 launched=0 error=0"
+
+
+def test_sor_attribute_is_not_a_calls_own(said):
+    assert said["sor-large"] == said["sor-small"] == TOOK
+    assert said["sor-attribute"] == "lowered=0"
+
+
+def test_sor_on_a_second_device_and_refused(said):
+    assert said["sor-second-device"] == TOOK
+    assert said["sor-refused"] == REFUSED
