@@ -1974,30 +1974,6 @@ void launch_sweep_rhs(cudaStream_t s, double* e, const uint8_t* fixed,
 #undef IG_SWEEP
 }
 
-bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
-                       Dims d, double rel_tol, double omega, long max_pairs) {
-  const size_t n = d.n();
-  if (n == 0 || 17 * n > kBottomSmemMax) return false;
-  const size_t bytes = 18 * n;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(k_bottom_err, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(18 * (kBottomSmemMax / 17)));
-  });
-  BottomGeom g;
-  g.nx = (int)d.nx;
-  g.ny = (int)d.ny;
-  g.nz = (int)d.nz;
-  g.dny = FastDiv((uint32_t)d.ny);
-  g.dnz = FastDiv((uint32_t)d.nz);
-  // a thread per node of one colour, in whole warps: fewer warps, cheaper
-  // barriers
-  const int nt = std::min<long>(kBottomCta, std::max<long>(64, ((long)(n + 1) / 2 + 31) / 32 * 32));
-  k_bottom_err<<<1, nt, (bytes + 7) / 8 * 8, s>>>(e, fixed, f, g, rel_tol, omega, max_pairs);
-  counted();
-  return true;
-}
-
 // A number found once for each device: a kernel's attributes and the launches
 // that fit belong to the device, and another thread's call may be between
 // finding them and launching.
@@ -2025,6 +2001,44 @@ class PerDevice {
   int value_[kMost] = {0};
   bool found_[kMost] = {false};
 };
+
+bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
+                       Dims d, double rel_tol, double omega, long max_pairs) {
+  const size_t n = d.n();
+  if (n == 0 || 17 * n > kBottomSmemMax) return false;
+  const size_t bytes = 18 * n;
+  static PerDevice smem;
+  if (!smem.get([](int) {
+        const int most = (int)(18 * (kBottomSmemMax / 17));
+        const bool ok = cudaFuncSetAttribute(k_bottom_err,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             most) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok ? 1 : 0;
+      }))
+    return false;
+  BottomGeom g;
+  g.nx = (int)d.nx;
+  g.ny = (int)d.ny;
+  g.nz = (int)d.nz;
+  g.dny = FastDiv((uint32_t)d.ny);
+  g.dnz = FastDiv((uint32_t)d.nz);
+  // a thread per node of one colour, in whole warps: fewer warps, cheaper
+  // barriers
+  const int nt = std::min<long>(kBottomCta, std::max<long>(64, ((long)(n + 1) / 2 + 31) / 32 * 32));
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(1);
+  c.blockDim = dim3((unsigned)nt);
+  c.dynamicSmemBytes = (bytes + 7) / 8 * 8;
+  c.stream = s;
+  if (cudaLaunchKernelEx(&c, k_bottom_err, e, fixed, f, g, rel_tol, omega, max_pairs) !=
+      cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  counted();
+  return true;
+}
 
 // The largest dynamic shared memory a CTA of k_sor_flow is launched with: its
 // share of the slots of the largest grid on this route (152 SMs).  The
@@ -2135,10 +2149,6 @@ static size_t tail_layout(TailArgs& a, int ctas) {
 bool launch_err_tail(cudaStream_t s, TailArgs a) {
   const TailLevel& b = a.lv[a.nlev - 1];
   const size_t nb = (size_t)b.nx * b.ny * b.nz;
-  // the cluster size this device takes with all of an SM's shared memory (16
-  // CTAs, else the portable 8; 0: neither), found once
-  static std::once_flag once;
-  static int ctas = 0;
   auto config = [](cudaLaunchConfig_t* c, cudaLaunchAttribute* at, int n, size_t smem,
                    cudaStream_t st) {
     *c = cudaLaunchConfig_t{};
@@ -2154,11 +2164,15 @@ bool launch_err_tail(cudaStream_t s, TailArgs a) {
     c->numAttrs = 1;
   };
   constexpr size_t most = 18 * (kBottomSmemMax / 17);
-  std::call_once(once, [&] {
+  // the cluster size this device takes with all of an SM's shared memory (16
+  // CTAs, else the portable 8; 0: neither)
+  static PerDevice size;
+  const int ctas = size.get([&](int) {
     for (const void* fn : {(const void*)k_err_tail<false>, (const void*)k_err_tail<true>}) {
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
       cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     }
+    cudaGetLastError();
     for (int n : {kTailCtas, 8}) {
       cudaLaunchConfig_t c;
       cudaLaunchAttribute at[1];
@@ -2166,12 +2180,11 @@ bool launch_err_tail(cudaStream_t s, TailArgs a) {
       int active = 0, other = 0;
       if (cudaOccupancyMaxActiveClusters(&active, k_err_tail<true>, &c) == cudaSuccess &&
           cudaOccupancyMaxActiveClusters(&other, k_err_tail<false>, &c) == cudaSuccess &&
-          active > 0 && other > 0) {
-        ctas = n;
-        break;
-      }
+          active > 0 && other > 0)
+        return n;
       cudaGetLastError();
     }
+    return 0;
   });
   if (!ctas || nb == 0 || 17 * nb > kBottomSmemMax) return false;
   const size_t bytes = tail_layout(a, ctas);
@@ -2180,9 +2193,10 @@ bool launch_err_tail(cudaStream_t s, TailArgs a) {
   cudaLaunchConfig_t c;
   cudaLaunchAttribute at[1];
   config(&c, at, ctas, ds ? bytes : (18 * nb + 7) / 8 * 8, s);
-  // an error is the caller's to read
-  if (cudaLaunchKernelEx(&c, ds ? k_err_tail<true> : k_err_tail<false>, a) != cudaSuccess)
-    return true;
+  if (cudaLaunchKernelEx(&c, ds ? k_err_tail<true> : k_err_tail<false>, a) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
   counted();
   return true;
 }

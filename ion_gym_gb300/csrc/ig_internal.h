@@ -98,8 +98,9 @@ void launch_residual(cudaStream_t s, const double* phi, const uint8_t* fixed,
                      unsigned long long* absmax /* nullable */);
 // The whole bottom solve of multigrid3d._solve_err (e = 0, tol from
 // max|f|, SOR pairs to 0.02 tol, at most max_pairs) in one CTA with the
-// level in shared memory (18 bytes a node); false (nothing launched) when
-// the level has more than kBottomSmemMax / 17 nodes.
+// level in shared memory (18 bytes a node); false (nothing launched, no error
+// left behind) when the level has more than kBottomSmemMax / 17 nodes or the
+// launch was refused.
 constexpr size_t kBottomSmemMax = 200 * 1024;
 bool launch_bottom_err(cudaStream_t s, double* e, const uint8_t* fixed, const double* f,
                        Dims d, double rel_tol, double omega, long max_pairs);
@@ -122,8 +123,8 @@ bool launch_sor_coop(cudaStream_t s, double* phi, const uint8_t* cls, const Thet
                      void* word, double* prev);
 // multigrid3d._solve_err from level lv[0] (its right-hand side in f) down to
 // the bottom lv[nlev - 1] (nlev >= 2) in one launch (k_err_tail); false
-// (nothing launched) when the bottom does not fit in shared memory or the
-// device takes no such cluster.
+// (nothing launched, no error left behind) when the bottom does not fit in
+// shared memory or the device takes no such cluster or refused this one.
 constexpr int kTailLevels = 12, kTailCtas = 16, kTailThreads = 512;
 struct TailLevel {
   double *e, *f, *r;

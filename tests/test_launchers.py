@@ -35,3 +35,14 @@ def test_sor_attribute_is_not_a_calls_own(said):
 def test_sor_on_a_second_device_and_refused(said):
     assert said["sor-second-device"] == TOOK
     assert said["sor-refused"] == REFUSED
+
+
+@pytest.mark.parametrize("device", [0, 1])
+def test_cluster_and_bottom_on_every_device(said, device):
+    assert said[f"tail-device{device}"] == TOOK
+    assert said[f"bottom-device{device}"] == TOOK
+
+
+def test_cluster_and_bottom_refused(said):
+    assert said["tail-refused"] == REFUSED
+    assert said["bottom-refused"] == REFUSED
