@@ -952,6 +952,7 @@ extern "C" int ig_field_aware_3d(const void* phi, int dtype, const uint8_t* meta
   }
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   const size_t n = (size_t)nx * ny * nz, es = dtype ? 8 : 4;
   CallBuf dp, dm, dout;
   const CallSync sync{s};
@@ -987,6 +988,7 @@ extern "C" int ig_compose_fields(const float* bases, int n_bases, int n_steps, c
   }
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   const size_t n = (size_t)nx * ny * nz;
   const size_t nc = (size_t)n_channels;
   CallBuf db, dm, dphi, de;
@@ -1028,6 +1030,7 @@ extern "C" int ig_field_check_division(double h, unsigned long long samples, uns
   }
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   CallBuf bad;
   const CallSync sync{s};
   GF(bad.alloc(8, s));

@@ -483,6 +483,7 @@ extern "C" int ig_rasterize(const double* table, int n_prims,
   if (int st = check_table(table, n_prims)) return st;
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   const size_t n = (size_t)nx * ny * nz;
   std::vector<Prim> host;
   CallBuf prims, eidx, lab, cnt;
@@ -524,6 +525,7 @@ extern "C" int ig_theta_scene(const double* table, int n_prims, const uint8_t* m
   if (int st = check_table(table, n_prims)) return st;
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   const size_t n = (size_t)nx * ny * nz;
   std::vector<Prim> host;
   CallBuf prims, m, th;
@@ -552,6 +554,7 @@ extern "C" int ig_shape_xsection(int type, const double* params, int n_params,
   }
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   XSec S{};
   S.type = type;
   for (int q = 0; q < n_params; q++) S.p[q] = params[q];
@@ -614,6 +617,7 @@ extern "C" int ig_shapes_label(const long long* table, int n_shapes, const uint8
   }
   cudaStream_t s = nullptr;
   if (int st = call_stream(&s)) return st;
+  const CallInFlight call(kOtherCall);
   const size_t n = (size_t)nx * ny * nz;
   CallBuf drec, dxs, drng, deidx, dlab, dcnt;
   const CallSync sync{s};

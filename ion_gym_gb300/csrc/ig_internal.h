@@ -2,6 +2,7 @@
 // libigsolve.so (kernel launchers, control blocks).  Not part of the C-ABI;
 // the public entry points are in include/igsolve.h.
 #pragma once
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
 #include <string>
@@ -200,6 +201,20 @@ void set_last_error(const std::string& m);
 // The calling thread's stream on its current device (created on first use);
 // a status, with the message set, when there is none.
 int call_stream(cudaStream_t* s);
+
+// A call that keeps the current device busy, for as long as the object lives.
+// The resident SOR loop fills the device, so it asks who else is there.
+enum CallKind { kSorCall, kOtherCall };
+class CallInFlight {
+ public:
+  explicit CallInFlight(CallKind kind);
+  ~CallInFlight();
+  CallInFlight(const CallInFlight&) = delete;
+  CallInFlight& operator=(const CallInFlight&) = delete;
+
+ private:
+  std::atomic<int>* n_;
+};
 
 // Waits for the stream when a call leaves, early returns included: copies
 // from pageable memory may still be reading the caller's (or the call's own)

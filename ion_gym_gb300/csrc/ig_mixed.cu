@@ -3701,6 +3701,7 @@ int open_session(const uint8_t* metal, int nmetal, long nx, long ny, long nz,
   // an error an earlier call on this thread left behind (and reported
   // itself) is not this session's: start from a clean slate
   cudaGetLastError();
+  const CallInFlight call(kOtherCall);
   Session* S = new Session();
   try {
     MK(cudaStreamCreateWithFlags(&S->s, cudaStreamNonBlocking));
@@ -3787,6 +3788,7 @@ int ig_mixed_rebind(void* handle, const uint8_t* metal, long nx, long ny, long n
     set_last_error("ig_mixed_rebind: the new metal's shape differs from the session's");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     S->load_metal(metal);             // nmetal masks for a per-problem session
     MK(cudaStreamSynchronize(S->s));  // the caller may reuse its mask buffer
@@ -3861,6 +3863,7 @@ int ig_mixed_tuning(void* handle, int n_problems, int* out_ng, int* out_threads,
     set_last_error("null argument or problem count outside 1..max_problems");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     if (!S->gs_tuned) S->tune_gs(n_problems);
     *out_ng = S->gs_cfg.ng;
@@ -3905,6 +3908,7 @@ int ig_mixed_time_gs(void* handle, int n_problems, int pairs, double* ms_per_lau
     set_last_error("bad session, problem count or pair count");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     MLevel& f = S->lv[0];
     if (!S->gs_tuned) S->tune_gs(n_problems);
@@ -3941,6 +3945,7 @@ int ig_mixed_check_fused(void* handle, int n_problems, long long mismatches[8]) 
     set_last_error("bad session (flexible-CG sessions only) or problem count");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     if (!S->gs_tuned) S->tune_gs(n_problems);
     const int B = n_problems;
@@ -4135,6 +4140,7 @@ int solve_bases_to(Session* S, const uint8_t* masks, int n_bases, double v_basis
                    "values (ig_mixed_solve_values), not the bases of one metal union");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     const size_t n = S->d.n();
     S->B = n_bases;
@@ -4202,6 +4208,7 @@ int ig_mixed_solve_values_acc(void* handle, const double* vals, int n_problems,
     set_last_error("null argument or problem count outside 1..max_problems");
     return IG_BAD_ARG;
   }
+  const CallInFlight call(kOtherCall);
   try {
     const size_t n = S->d.n();
     S->B = n_problems;

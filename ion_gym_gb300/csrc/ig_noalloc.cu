@@ -121,6 +121,7 @@ extern "C" int ig_cascadic_relres_noalloc(
                     " bytes of scratch; the static scratch holds " +
                     std::to_string((size_t)IG_NOALLOC_SCRATCH_BYTES) +
                     " bytes (use ig_cascadic_relres for larger grids)");
+  const CallInFlight call(kOtherCall);
   // the array's address on the current device (see the file header)
   void* sym = nullptr;
   NA_CK(cudaGetSymbolAddress(&sym, g_noalloc_scratch));

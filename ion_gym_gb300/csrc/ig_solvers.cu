@@ -76,6 +76,18 @@ CtxPool& ctx_pool() {
   return *p;
 }
 
+// The calls in flight on a device, counted by CallInFlight.
+struct DeviceCalls {
+  std::atomic<int> sor{0}, other{0};
+};
+DeviceCalls& device_calls() {
+  constexpr int kMost = 64;
+  static DeviceCalls k[kMost + 1];  // the last: devices past the rest
+  int dev = kMost;
+  if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+  return k[dev < 0 || dev > kMost ? kMost : dev];
+}
+
 struct CtxHolder {
   ThreadCtx c;
   void hand_on() {
@@ -395,51 +407,77 @@ void fine_sweep(cudaStream_t s, double* phi, const uint8_t* fx, const float* th,
 // one call would hold every SM for long, and a thread's neighbour slots fill
 // its SM's shared memory.
 constexpr long kCoopSlots = 8L * 152 * kCoopThreads;
-// Pairs per launch: the host looks in between.
-constexpr int kCoopPairs = 4096;
 
-// The SOR loop by k_sor_flow; false: not done.
-bool sor_loop_coop(ThreadCtx& c, double* phi, const uint8_t* fx, const float* th, const Theta& t,
-                   int kind, Dims d, double omega, double tol, long max_pairs,
-                   PairsResult* out) {
-  if ((th && !t.on()) || d.nx * d.ny * ((d.nz + 1) / 2) > kCoopSlots || max_pairs < 1)
-    return false;
-  DBuf<CoopCtl> ctl(1, c.s);
-  const size_t slots = (size_t)(d.nx * d.ny * ((d.nz + 1) / 2));
-  DBuf<ulonglong2> word(2 * slots, c.s);
-  DBuf<double> before(2 * slots, c.s);
-  const bool prof = g_prof.on.load() != 0;
-  long base = 0;
-  double last = std::numeric_limits<double>::quiet_NaN();
-  while (base < max_pairs) {
-    const int lim = (int)std::min<long>(kCoopPairs, max_pairs - base);
-    if (prof) CK(cudaEventRecord(c.ev0, c.s));
-    if (!launch_sor_coop(c.s, phi, t.on() ? t.plan.cls : fx, t.on() ? &t.plan : nullptr, kind, d,
-                         omega, tol, lim, ctl.p, word.p, before.p)) {
-      // refused: the launched sweeps, which take the pairs from the first
-      if (base == 0) return false;
-      throw Status(IG_CUDA_ERROR, "SOR loop: a further launch was refused");
+// A resident loop has a CTA on every SM until it ends, and other streams'
+// kernels come in where it leaves room, or between two launches.  So it runs
+// in turns, after each of which the host looks who else is there:
+//  * Calls of another kind in this process (sessions, V-cycles, geometry, host
+//    fields) are many short launches, each of which would wait for a turn:
+//    while there is one, the sweeps are launched.  Beside three solves in a
+//    loop a batch of eight 65^3 decks took 160 ms (solves of 65^3) and 1.8 s
+//    (129^3) without this, 6.6 and 36 ms beside launched sweeps.
+//  * Up to kCoopCalls solves keep their loops, which then take turns; with
+//    more, launched sweeps overlap better, unless two loops fit on an SM.
+//    Solves a second, launched / resident: 65^3 two calls 378 / 638, four
+//    594 / 658, six 749 / 660, eight 807 / 663; 49^3 eight 1372 / 2064; 33^3
+//    eight 2875 / 8368.
+// A turn is about 2 ms (kernels of other libraries and processes wait for no
+// more than that), a pair some 3 us and 34 ps a slot; a turn costs some 25 us
+// besides.
+constexpr int kCoopCalls = 4;
+constexpr long kCoopShared = 512L * 152;  // slots: half an SM's registers
+inline int coop_turn(long slots) { return (int)(2e9 / (3e6 + 34.0 * (double)slots)); }
+// Launched pairs before the host looks again.
+constexpr long kLaunchedTurn = 2 * kMaxBatch;
+
+bool may_stay(long slots) {
+  const DeviceCalls& k = device_calls();
+  return k.other.load() == 0 && (slots <= kCoopShared || k.sor.load() <= kCoopCalls);
+}
+
+// What a solve's resident loop needs; `on` while it may still be had.
+struct Resident {
+  bool on = false;
+  DBuf<CoopCtl> ctl;
+  DBuf<ulonglong2> word;
+  DBuf<double> before;
+};
+
+// Up to `pairs` pairs by k_sor_flow; false: nothing was run (no memory for it,
+// or the device refused the launch).
+bool resident_pairs(ThreadCtx& c, Resident& R, double* phi, const uint8_t* fx, const Theta& t,
+                    int kind, Dims d, double omega, double tol, int pairs, PairsResult* out) {
+  if (!R.before.p) {
+    const size_t slots = (size_t)(d.nx * d.ny * ((d.nz + 1) / 2));
+    try {
+      R.ctl.alloc(1, c.s);
+      R.word.alloc(2 * slots, c.s);
+      R.before.alloc(2 * slots, c.s);
+    } catch (const Status&) {
+      cudaGetLastError();
+      R.ctl.release();
+      R.word.release();
+      return false;
     }
-    if (prof) CK(cudaEventRecord(c.ev1, c.s));
-    CoopCtl h;
-    CK(cudaMemcpyAsync(&h, ctl.p, offsetof(CoopCtl, word), cudaMemcpyDeviceToHost, c.s));
-    CK(cudaStreamSynchronize(c.s));
-    if (h.status) throw Status(IG_CUDA_ERROR, "SOR loop: a wait ran out of time");
-    if (prof) {
-      float ms = 0.f;
-      CK(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-      g_prof.ms += ms;
-      g_prof.launches += 1;
-      g_prof.nodes += (long)d.n() * h.pairs;
-    }
-    last = bits_to_double(h.key);
-    if (h.hit) {
-      *out = {base + h.pairs, last, true};
-      return true;
-    }
-    base += lim;
   }
-  *out = {max_pairs, last, false};
+  const bool prof = g_prof.on.load() != 0;
+  if (prof) CK(cudaEventRecord(c.ev0, c.s));
+  if (!launch_sor_coop(c.s, phi, t.on() ? t.plan.cls : fx, t.on() ? &t.plan : nullptr, kind, d,
+                       omega, tol, pairs, R.ctl.p, R.word.p, R.before.p))
+    return false;
+  if (prof) CK(cudaEventRecord(c.ev1, c.s));
+  CoopCtl h;
+  CK(cudaMemcpyAsync(&h, R.ctl.p, offsetof(CoopCtl, word), cudaMemcpyDeviceToHost, c.s));
+  CK(cudaStreamSynchronize(c.s));
+  if (h.status) throw Status(IG_CUDA_ERROR, "SOR loop: a wait ran out of time");
+  if (prof) {
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
+    g_prof.ms += ms;
+    g_prof.launches += 1;
+    g_prof.nodes += (long)d.n() * h.pairs;
+  }
+  *out = {h.pairs, bits_to_double(h.key), h.hit != 0};
   return true;
 }
 
@@ -447,13 +485,32 @@ PairsResult sor_loop(ThreadCtx& c, double* phi, const uint8_t* fx,
                      const float* th, const Theta& t, int stencil, Dims d, double omega,
                      double tol, long max_pairs, PairCtl* ctl_d) {
   const int kind = sweep_kind(th || t.on(), stencil);
-  PairsResult r{0, 0.0, false};
-  if (sor_loop_coop(c, phi, fx, th, t, kind, d, omega, tol, max_pairs, &r)) return r;
   cudaStream_t s = c.s;
-  return run_pairs(c, ctl_d, tol, max_pairs, d.n(), [&](int lp, PairCtl* ctl) {
-    for (int colour = 0; colour < 2; colour++)
-      fine_sweep(s, phi, fx, th, t, kind, d, omega, colour, ctl, lp);
-  });
+  auto launched = [&](long pairs) {
+    return run_pairs(c, ctl_d, tol, pairs, d.n(), [&](int lp, PairCtl* ctl) {
+      for (int colour = 0; colour < 2; colour++)
+        fine_sweep(s, phi, fx, th, t, kind, d, omega, colour, ctl, lp);
+    });
+  };
+  const long slots = d.nx * d.ny * ((d.nz + 1) / 2);
+  Resident R;
+  R.on = !(th && !t.on()) && slots <= kCoopSlots;
+  long base = 0;
+  PairsResult r{0, std::numeric_limits<double>::quiet_NaN(), false};
+  while (R.on && base < max_pairs && !r.converged) {
+    const long left = max_pairs - base;
+    if (may_stay(slots))
+      R.on = resident_pairs(c, R, phi, fx, t, kind, d, omega, tol,
+                            (int)std::min<long>(coop_turn(slots), left), &r);
+    else
+      r = launched(std::min(kLaunchedTurn, left));
+    if (R.on) base += r.pairs;
+  }
+  if ((!R.on && base < max_pairs) || max_pairs < 1) {
+    r = launched(max_pairs - base);
+    base += r.pairs;
+  }
+  return {base, r.delta, r.converged};
 }
 
 // ---------------------------------------------------------------- V-cycle
@@ -858,6 +915,7 @@ int sor_call(const uint8_t* fixed, const Dirichlet& b, const float* theta, long 
              double* phi_out, long* sweeps_out, double* delta_out) {
   if (!fixed || !(b.val || b.mask) || !phi_out) throw Status(IG_BAD_ARG, "null array");
   ThreadCtx& c = ctx();
+  const CallInFlight call(kSorCall);
   FineGrid g;
   load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
   DirichletDev bd;
@@ -883,6 +941,7 @@ int vmg_call(const uint8_t* fixed, const Dirichlet& b, const float* theta, long 
   if (!fixed || !(b.val || b.mask) || !phi_out) throw Status(IG_BAD_ARG, "null array");
   if (nu1 < 0 || nu2 < 0) throw Status(IG_BAD_ARG, "nu1 and nu2 must be >= 0");
   ThreadCtx& c = ctx();
+  const CallInFlight call(kOtherCall);
   FineGrid g;
   load_fine(c, g, fixed, theta, nx, ny, nz, stencil);
   PageTouch touch(phi_out, g.d.n() * 8);
@@ -911,6 +970,12 @@ int vmg_call(const uint8_t* fixed, const Dirichlet& b, const float* theta, long 
 using namespace ig;
 
 void ig::set_last_error(const std::string& m) { t_err = m; }
+
+ig::CallInFlight::CallInFlight(CallKind kind)
+    : n_(kind == kSorCall ? &device_calls().sor : &device_calls().other) {
+  n_->fetch_add(1);
+}
+ig::CallInFlight::~CallInFlight() { n_->fetch_sub(1); }
 
 int ig::call_stream(cudaStream_t* s) {
   return guard([&] {
@@ -986,6 +1051,7 @@ int ig_solve3d_mg(const uint8_t* fixed, const double* val, const float* theta,
     check_dims(nx, ny, nz);
     stencil_check(stencil);
     ThreadCtx& c = ctx();
+    const CallInFlight call(kSorCall);
     const Dims d0{nx, ny, nz};
     std::vector<MgLevel> lv = build_mg_levels(c, fixed, val, d0, min_coarse, std::max(1, max_levels));
     const int nl = (int)lv.size();
@@ -1091,6 +1157,7 @@ int ig_cascadic_relres(const uint8_t* fixed, const double* val, long nx,
     if (check_every < 1) throw Status(IG_BAD_ARG, "check_every must be >= 1");
     check_dims(nx, ny, nz);
     ThreadCtx& c = ctx();
+    const CallInFlight call(kOtherCall);
     const Dims d0{nx, ny, nz};
     std::vector<MgLevel> lv = build_mg_levels(c, fixed, val, d0, min_coarse, std::max(1, max_levels));
     const int nl = (int)lv.size();

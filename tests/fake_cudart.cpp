@@ -1,16 +1,21 @@
 // The library's launchers over a stand-in CUDA runtime of two devices, which
 // keeps kernel attributes by device and refuses a launch beyond them as the
-// real one does; nothing is computed.  Prints one line per check; the first
-// word says what it is, the rest what happened.
+// real one does.  Device memory is host memory, kernels compute nothing: a
+// launched pair's maxima stay 0, which meets any tolerance, and a resident
+// loop runs the pairs it was given without meeting it.  Prints one line per
+// check; the first word says what it is, the rest what happened.
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <map>
 #include <string>
 #include <utility>
+#include <vector>
 
 #include <cuda_runtime.h>
 
 #include "ig_internal.h"
+#include "../include/igsolve.h"
 
 namespace {
 struct Attr {
@@ -22,7 +27,8 @@ struct Config {
   size_t smem = 0;
   cudaStream_t s = nullptr;
 };
-int device = 0, launched = 0, refuse = 0;
+int device = 0, launched = 0, refuse = 0, loops = 0, loops_left = 1 << 30;
+size_t most_memory = size_t(-1);
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, Attr> attrs;
 Config config;
@@ -76,9 +82,17 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void**, size_t smem, 
 cudaError_t cudaLaunchKernel(const void* fn, dim3, dim3, void**, size_t smem, cudaStream_t) {
   return launch(fn, smem, 1);
 }
-cudaError_t cudaLaunchCooperativeKernel(const void* fn, dim3, dim3, void**, size_t smem,
+cudaError_t cudaLaunchCooperativeKernel(const void* fn, dim3, dim3, void** args, size_t smem,
                                         cudaStream_t) {
-  return launch(fn, smem, 1);
+  if (loops == loops_left) return note(cudaErrorInvalidValue);
+  const cudaError_t e = launch(fn, smem, 1);
+  if (e == cudaSuccess) {
+    loops++;
+    ig::CoopCtl* ctl = *static_cast<ig::CoopCtl**>(args[7]);
+    ctl->pairs = *static_cast<int*>(args[6]);
+    ctl->key = 0x7ff0000000000000ULL;
+  }
+  return e;
 }
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void* fn, void**) {
   return launch(fn, c->dynamicSmemBytes, cluster_of(c));
@@ -112,17 +126,60 @@ cudaError_t cudaGetLastError() {
   last = cudaSuccess;
   return e;
 }
-cudaError_t cudaMemsetAsync(void*, int, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaMemsetAsync(void* p, int v, size_t n, cudaStream_t) {
+  std::memset(p, v, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  std::memcpy(d, s, n);
+  return cudaSuccess;
+}
+cudaError_t cudaMalloc(void** p, size_t n) {
+  *p = n > most_memory ? nullptr : std::calloc(1, n);
+  return *p ? cudaSuccess : note(cudaErrorMemoryAllocation);
+}
+cudaError_t cudaMallocAsync(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
+cudaError_t cudaFree(void* p) {
+  std::free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaFreeAsync(void* p, cudaStream_t) { return cudaFree(p); }
+cudaError_t cudaGetDeviceCount(int* n) {
+  *n = 2;
+  return cudaSuccess;
+}
+const char* cudaGetErrorString(cudaError_t) { return "refused"; }
+cudaError_t cudaMemGetInfo(size_t*, size_t*) { return cudaSuccess; }
+cudaError_t cudaDeviceGetDefaultMemPool(cudaMemPool_t*, int) { return cudaSuccess; }
+cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void*) { return cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t*) { return cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float*, cudaEvent_t, cudaEvent_t) { return cudaSuccess; }
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t*, unsigned) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return note(cudaErrorNotSupported); }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t*) { return cudaSuccess; }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long long) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
+cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+  *a = cudaPointerAttributes();
+  return cudaSuccess;
+}
 }
 
 using namespace ig;
 
 static bool sor(long side) {
   char scratch[64];
+  static CoopCtl ctl;
   return launch_sor_coop(nullptr, reinterpret_cast<double*>(scratch),
                          reinterpret_cast<uint8_t*>(scratch), nullptr, kPlain,
-                         Dims{side, side, side}, 1.5, 1e-3, 8, reinterpret_cast<CoopCtl*>(scratch),
-                         scratch, reinterpret_cast<double*>(scratch));
+                         Dims{side, side, side}, 1.5, 1e-3, 8, &ctl, scratch,
+                         reinterpret_cast<double*>(scratch));
 }
 
 static bool tail() {
@@ -140,6 +197,52 @@ static bool bottom(long n) {
 static void say(const char* what, bool took) {
   std::printf("%s took=%d launched=%d error=%d\n", what, took, launched, (int)cudaGetLastError());
   launched = 0;
+}
+
+// A solve of `pairs` pairs at most: which loop it took, and how often.
+static void solve(const char* what, long side, long pairs) {
+  const size_t n = (size_t)side * side * side;
+  std::vector<uint8_t> fixed(n, 0);
+  std::vector<double> val(n, 0.0), phi(n);
+  loops = launched = 0;
+  long sweeps = -1;
+  double delta = 0.0;
+  const int st = ig_solve3d(fixed.data(), val.data(), nullptr, side, side, side, 1e-3, pairs, 1.5,
+                            nullptr, 0, phi.data(), &sweeps, &delta);
+  // one launch sets the Dirichlet values
+  std::printf("%s status=%d loops=%d launched=%d sweeps=%ld\n", what, st, loops,
+              launched - loops - 1 > 0 ? 1 : 0, sweeps);
+  loops = launched = 0;
+  loops_left = 1 << 30;
+  most_memory = size_t(-1);
+}
+
+static void routes() {
+  solve("alone", 65, 100);
+  solve("alone-turns", 65, 600);
+  solve("no-pairs", 65, 0);
+  {
+    const CallInFlight session(kOtherCall);
+    solve("beside-a-session", 65, 100);
+    solve("small-beside-a-session", 33, 100);
+    device = 1;
+    solve("session-on-the-other-device", 65, 100);
+    device = 0;
+  }
+  {
+    const CallInFlight a(kSorCall), b(kSorCall), c(kSorCall);
+    solve("beside-three-solves", 65, 100);
+    const CallInFlight d(kSorCall);
+    solve("beside-four-solves", 65, 100);
+    solve("small-beside-four-solves", 33, 100);
+  }
+  solve("alone-again", 65, 100);
+  loops_left = 0;
+  solve("refused", 65, 100);
+  loops_left = 1;
+  solve("refused-later", 65, 600);
+  most_memory = 3u << 20;  // the potential and the mask, not the loop's words
+  solve("no-memory", 65, 100);
 }
 
 int main() {
@@ -161,5 +264,7 @@ int main() {
   refuse = 1;
   say("tail-refused", tail());
   say("bottom-refused", bottom(21));
+  refuse = device = 0;
+  routes();
   return 0;
 }

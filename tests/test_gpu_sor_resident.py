@@ -73,3 +73,32 @@ def test_threads_with_small_and_large_grids():
 
     with ThreadPoolExecutor(len(decks)) as ex:
         list(ex.map(calls, range(len(decks))))
+
+
+def test_solves_beside_a_session():
+    """The loop makes room for a session's kernels between its turns and takes
+    up again where the launched sweeps left: the same bits as alone."""
+    from ion_gym_gb300.physics import solver3d as S
+    from ion_gym_gb300.physics.mixed import MixedSession
+    decks = [_deck(shape, 50 + q) for q, shape in enumerate([(65, 64, 63), (97, 96, 95)])]
+    want = [S.solve3d(*d, tol=1e-6, omega=1.8) for d in decks]
+    fixed, val = _deck((64, 64, 64), 60)
+    with MixedSession(fixed, 1) as s:
+        field = s.solve_values(val[None], 1e-9)
+
+        def sessions(_):
+            for _ in range(20):
+                assert same_bits(s.solve_values(val[None], 1e-9), field)
+
+        def solves(q):
+            for _ in range(6):
+                a = S.solve3d(*decks[q], tol=1e-6, omega=1.8)
+                assert a[1:] == want[q][1:] and same_bits(a[0], want[q][0])
+
+        with ThreadPoolExecutor(3) as ex:
+            jobs = [ex.submit(sessions, 0)] + [ex.submit(solves, q) for q in (0, 1)]
+            for j in jobs:
+                j.result()
+    for (f, v), a in zip(decks, want):
+        b = port.solve3d(f, v, tol=1e-6, omega=1.8)
+        assert a[1:] == b[1:] and same_bits(a[0], b[0])

@@ -19,7 +19,8 @@ def said(tmp_path_factory):
     include = os.path.join(os.path.dirname(os.path.dirname(B.nvcc())), "include")
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", B.CSRC, "-I", include,
                     os.path.join(HERE, "fake_cudart.cpp"),
-                    os.path.join(B.OUT_DIR, "ig_f64.o"), "-o", exe, "-lpthread"], check=True)
+                    os.path.join(B.OUT_DIR, "ig_f64.o"), os.path.join(B.OUT_DIR, "ig_solvers.o"),
+                    "-o", exe, "-lpthread"], check=True)
     out = subprocess.run([exe], check=True, capture_output=True, text=True).stdout
     return dict(line.split(" ", 1) for line in out.splitlines())
 
@@ -46,3 +47,26 @@ def test_cluster_and_bottom_on_every_device(said, device):
 def test_cluster_and_bottom_refused(said):
     assert said["tail-refused"] == REFUSED
     assert said["bottom-refused"] == REFUSED
+
+
+CAP = 1  # IG_NOT_CONVERGED: the stand-in's loop never meets its tolerance
+
+
+@pytest.mark.parametrize("what,want", [
+    ("alone", (CAP, 1, 0, 100)),
+    ("alone-turns", (CAP, 3, 0, 600)),      # a turn of 65^3 is 258 pairs
+    ("no-pairs", (CAP, 0, 0, 0)),
+    ("beside-a-session", (0, 0, 1, 1)),
+    ("small-beside-a-session", (0, 0, 1, 1)),
+    ("session-on-the-other-device", (CAP, 1, 0, 100)),
+    ("beside-three-solves", (CAP, 1, 0, 100)),
+    ("beside-four-solves", (0, 0, 1, 1)),
+    ("small-beside-four-solves", (CAP, 1, 0, 100)),
+    ("alone-again", (CAP, 1, 0, 100)),
+    ("refused", (0, 0, 1, 1)),
+    ("refused-later", (0, 1, 1, 259)),
+    ("no-memory", (0, 0, 1, 1))])
+def test_who_gets_the_resident_loop(said, what, want):
+    """solve3d's loop holds every SM: alone, or among few or small solves, and
+    nowhere else; what it cannot do the launched sweeps take up."""
+    assert said[what] == "status=%d loops=%d launched=%d sweeps=%d" % want
