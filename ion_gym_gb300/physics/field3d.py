@@ -357,8 +357,7 @@ def compose_drive_channels(spec, bases, ele, verbose=False):
     P = superpose_device(src, plan["rows"], plan["weights"], plan["mult"],
                          shape=shape)
     del src
-    n = int(np.prod(shape))
-    wide = not f32_out and n + 2 * shape[1] * shape[2] < _WIDE_LIMIT
+    wide = not f32_out and (shape[0] + 2) * shape[1] * shape[2] < _WIDE_LIMIT
     E = torch.empty((3, nch) + shape, dtype=torch.float64 if wide else torch.float32,
                     device=dev)
     _field_device(P, ele if eaware else None, h, eaware, out=E)
