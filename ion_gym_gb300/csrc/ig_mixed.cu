@@ -2327,6 +2327,25 @@ __device__ __forceinline__ double block_sum_d(double v, double* sh) {
   return t;  // valid in thread 0
 }
 
+// N sums over the block's threads (kT of them) at once, sum w in lane 0 of
+// warp w: eight values a lane and then the lanes, by one warp a sum, where
+// every warp summing its own lanes first takes the FP64 pipe (16 clocks a warp
+// instruction and SM) for 45 additions a sum instead of 12.
+template <int N>
+__device__ __forceinline__ double block_sums(const double (&v)[N], double (&sh)[N][kT]) {
+#pragma unroll
+  for (int q = 0; q < N; q++) sh[q][threadIdx.x] = v[q];
+  __syncthreads();
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w >= N) return 0.0;
+  double t = sh[w][lane];
+#pragma unroll
+  for (int u = 32; u < kT; u += 32) t += sh[w][lane + u];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return t;
+}
+
 // p = z + beta p on valid free slots (p stays 0 on metal).
 __global__ void __launch_bounds__(kT)
 k_cg_dir(float* __restrict__ p, const float* __restrict__ z,
@@ -2349,7 +2368,7 @@ struct KSum {
     c = __fsub_rn(__fsub_rn(t, s), y);
     s = t;
   }
-  __device__ __forceinline__ double value() const { return (double)s - (double)c; }
+  __device__ __forceinline__ double value() const { return widen(s) - widen(c); }
 };
 
 // The last half-sweep of the finest level's cycle (the same update as k_gs4)
@@ -2358,16 +2377,14 @@ struct KSum {
 // of its slots (the other colour from the half-sweep before) against q, and
 // each block writes one partial (part[b * gridDim.x + blockIdx.x]) --
 // k_cg_dot's read of z folded into the sweep that writes it.  Grid-stride
-// with cg_blocks() blocks a problem: a block's float64 sum takes the FP64
-// pipe (2 lanes per clock and SM) about a microsecond, which 192 blocks for
-// each of 24 problems' 98,000 groups made a third of the launch; and the
-// partial sums follow the grid and the problem count alone, not the tuned
-// launch shape, so equal solves have equal bits.
+// with cg_blocks() blocks a problem, whose partial sums follow the grid alone,
+// not the tuned launch shape or the batch: a problem has the same bits in
+// every session and batch.
 __global__ void __launch_bounds__(kT)
 k_gs4_dot(float* __restrict__ e, const float* __restrict__ g,
           const uint8_t* __restrict__ mask, SGeo G, int c, float omega,
           size_t pstride, const float* __restrict__ q, double* __restrict__ part) {
-  __shared__ double sh[kT / 32];
+  __shared__ double sh[1][kT];
   mask += (size_t)blockIdx.y * G.msplit;
   const uint32_t nq = G.csz >> 2;
   float* eb = e + blockIdx.y * pstride;
@@ -2387,16 +2404,25 @@ k_gs4_dot(float* __restrict__ e, const float* __restrict__ g,
     acc.add(za.x * qa.x); acc.add(za.y * qa.y); acc.add(za.z * qa.z); acc.add(za.w * qa.w);
     acc.add(zb.x * qb.x); acc.add(zb.y * qb.y); acc.add(zb.z * qb.z); acc.add(zb.w * qb.w);
   }
-  const double tot = block_sum_d(acc.value(), sh);
+  const double tot = block_sums<1>({acc.value()}, sh);
   if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = tot;
 }
 
-// Blocks of a grid-stride pass with block sums over `groups` float4 groups
-// for each of n problems (or problem colours): together four a SM, the
-// resident ones, so that each sums once over as much as it can.
-inline unsigned cg_blocks(uint32_t groups, unsigned n) {
+// Blocks a problem of a grid-stride pass with block sums over its float4
+// groups; `colours` 2 where the grid has a dimension for the colour.  By the
+// grid alone: the sums' order, and with it the last bits of alpha and beta,
+// must not change with the other problems of a batch.  A block's sums cost
+// its SM some 0.2 us of the FP64 pipe, so a block takes eight groups a thread
+// (256 x 64 x 48: 48 blocks) between what a small batch of small grids needs
+// and four blocks on each SM.  Against four resident blocks an SM shared by
+// the batch's problems, where the order did change with it: 8 bases of a
+// 193 x 193 x 385 ring stack 1.0 % slower, 24 of a 256 x 64 x 48 board 0.6 to
+// 1.4 %, 16 decks of 33^3 7 % faster, 8 of 65^3 and 257^3 alone alike.  With at
+// least 64 or 32 blocks, or at most 456: none better throughout.
+inline unsigned cg_blocks(uint32_t groups, unsigned colours) {
   const unsigned most = (groups + kT - 1) / kT;
-  return std::max(1u, std::min(most, 4u * 152u / std::max(1u, n)));
+  const unsigned want = std::min(4u * 152u, std::max(48u, groups / (8u * kT)));
+  return std::max(1u, std::min(most, want / colours));
 }
 
 // q = L p (both colours; q = 0 on metal) and block partials of <p, q> and
@@ -2411,7 +2437,7 @@ k_cg_matvec(const float* __restrict__ p, const float* __restrict__ g,
             const uint8_t* __restrict__ mask, SGeo G, float* __restrict__ q,
             double* __restrict__ part, size_t pstride) {
   mask += (size_t)blockIdx.z * G.msplit;
-  __shared__ double sh[kT / 32];
+  __shared__ double sh[2][kT];
   const int c = blockIdx.y;
   const uint32_t nq = G.csz >> 2;
   KSum spq, spg;
@@ -2444,13 +2470,10 @@ k_cg_matvec(const float* __restrict__ p, const float* __restrict__ g,
     *reinterpret_cast<float4*>(q + blockIdx.z * pstride + (size_t)c * G.csz + base) =
         make_float4(out[0], out[1], out[2], out[3]);
   }
-  const double a = block_sum_d(spq.value(), sh);
-  __syncthreads();
-  const double b = block_sum_d(spg.value(), sh);
-  if (threadIdx.x == 0) {
+  const double sum = block_sums<2>({spq.value(), spg.value()}, sh);
+  if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {
     const size_t slot = ((size_t)blockIdx.z * 2 + c) * gridDim.x + blockIdx.x;
-    part[2 * slot] = a;
-    part[2 * slot + 1] = b;
+    part[2 * slot + (threadIdx.x >> 5)] = sum;
   }
 }
 
@@ -2473,7 +2496,7 @@ k_cg_matvec_dir(const float* __restrict__ z, const float* __restrict__ po,
                 float* __restrict__ q, double* __restrict__ part, size_t pstride,
                 float* __restrict__ x) {
   mask += (size_t)blockIdx.z * G.msplit;
-  __shared__ double sh[kT / 32];
+  __shared__ double sh[2][kT];
   const int c = blockIdx.y;
   const uint32_t nq = G.csz >> 2;
   const float b = (float)scal[4 * blockIdx.z + 2];
@@ -2516,13 +2539,10 @@ k_cg_matvec_dir(const float* __restrict__ z, const float* __restrict__ po,
     }
     *reinterpret_cast<float4*>(q + own + base) = make_float4(out[0], out[1], out[2], out[3]);
   }
-  const double a = block_sum_d(spq.value(), sh);
-  __syncthreads();
-  const double bb = block_sum_d(spg.value(), sh);
-  if (threadIdx.x == 0) {
+  const double sum = block_sums<2>({spq.value(), spg.value()}, sh);
+  if ((threadIdx.x & 31) == 0 && threadIdx.x < 64) {
     const size_t slot = ((size_t)blockIdx.z * 2 + c) * gridDim.x + blockIdx.x;
-    part[2 * slot] = a;
-    part[2 * slot + 1] = bb;
+    part[2 * slot + (threadIdx.x >> 5)] = sum;
   }
 }
 
@@ -2531,7 +2551,7 @@ k_cg_matvec_dir(const float* __restrict__ z, const float* __restrict__ po,
 __global__ void __launch_bounds__(kT)
 k_cg_dot(const float* __restrict__ z, const float* __restrict__ q,
          double* __restrict__ part, size_t pstride, uint32_t n) {
-  __shared__ double sh[kT / 32];
+  __shared__ double sh[1][kT];
   KSum s;
   const float* zb = z + blockIdx.y * pstride;
   const float* qb = q + blockIdx.y * pstride;
@@ -2542,7 +2562,7 @@ k_cg_dot(const float* __restrict__ z, const float* __restrict__ q,
     s.add(a.z * b.z);
     s.add(a.w * b.w);
   }
-  const double a = block_sum_d(s.value(), sh);
+  const double a = block_sums<1>({s.value()}, sh);
   if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = a;
 }
 
@@ -2900,7 +2920,7 @@ struct Session {
   // The finest level's last half-sweep with <z, q> folded in (k_gs4_dot):
   // its partials go to `part`, their count to dot_nparts.
   void launch_gs_dot(MLevel& a, int c, int nb, float omega) {
-    const dim3 grid(cg_blocks(a.G.csz / 4, (unsigned)nb), nb);
+    const dim3 grid(cg_blocks(a.G.csz / 4, 1), nb);
     k_gs4_dot<<<grid, kT, 0, s>>>(a.e.p, a.g.p, a.mask.p, a.G, c, omega, a.pstride, qb.p, part.p);
     dot_nparts = (int)grid.x;
   }
@@ -3304,8 +3324,8 @@ struct Session {
     MLevel& f = lv[0];
     const uint32_t n = (uint32_t)f.pstride;
     const dim3 gv(nblk(n), B);
-    const unsigned nb4 = cg_blocks(f.G.csz / 4, 2 * (unsigned)B);
-    const unsigned nbd = cg_blocks(n / 4, (unsigned)B);
+    const unsigned nb4 = cg_blocks(f.G.csz / 4, 2);
+    const unsigned nbd = cg_blocks(n / 4, 1);
     float* pcur = from_b2 ? pb2.p : pb.p;
     float* pnext = from_b2 ? pb.p : pb2.p;
     const bool fold = fold_ok(), three = three_ok();
@@ -4058,7 +4078,7 @@ int ig_mixed_check_fused(void* handle, int n_problems, long long mismatches[8]) 
     if (S->fuse_dir()) {
       MLevel& f = S->lv[0];
       const size_t words = f.pstride * B;
-      const unsigned nb4 = cg_blocks(f.G.csz / 4, 2 * (unsigned)B);
+      const unsigned nb4 = cg_blocks(f.G.csz / 4, 2);
       const size_t nparts = 2 * (size_t)B * 2 * nb4;
       Buf<double> part2;
       part2.alloc(nparts, s);
