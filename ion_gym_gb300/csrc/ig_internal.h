@@ -216,6 +216,11 @@ class CallInFlight {
   std::atomic<int>* n_;
 };
 
+// Whether a kernel may write [p, p + bytes) as elements of `align` bytes: memory
+// of the current device, aligned, within one allocation.  Elsewhere a result is
+// copied, which takes any address and reports a range past its allocation.
+bool device_range(const void* p, size_t bytes, size_t align);
+
 // Waits for the stream when a call leaves, early returns included: copies
 // from pageable memory may still be reading the caller's (or the call's own)
 // arrays.  Declared after them and after the call's CallBufs.

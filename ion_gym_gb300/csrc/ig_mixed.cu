@@ -3618,17 +3618,6 @@ void set_units(Session& S, const std::vector<double>& vmax) {
 
 // The float64 potentials (Dirichlet values exact at the metal: vals, or
 // v_basis on the basis masks) into phi_out.
-// Memory of the current device, which a kernel may write.
-bool on_device(const void* p) {
-  cudaPointerAttributes a;
-  int dev = -1;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeDevice && a.device == dev;
-}
-
 int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
            double* dmax_out, const double* vals, const uint8_t* masks, double v,
            float* unit_out = nullptr) {
@@ -3638,7 +3627,7 @@ int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
     // float32 unit bases, staged in the finest level's correction buffer
     // (scratch once the refinement is done; it holds pstride >= n floats
     // per problem)
-    const bool direct = on_device(unit_out);
+    const bool direct = device_range(unit_out, (size_t)n * S.B * 4, 4);
     float* u = direct ? unit_out : S.lv[0].e.p;
     // every basis of the set has v's exponent as its unit's (set_units)
     UnitScale U;
@@ -3653,7 +3642,7 @@ int finish(Session& S, const MixedResult& r, double* phi_out, int* steps_out,
     MK(cudaGetLastError());
     if (!direct) MK(cudaMemcpyAsync(unit_out, u, (size_t)n * S.B * 4, cudaMemcpyDefault, S.s));
   } else {
-    const bool direct = on_device(phi_out);
+    const bool direct = device_range(phi_out, (size_t)n * S.B * 8, 8);
     double* to = direct ? phi_out : reinterpret_cast<double*>(S.phi.p);
     k_fixed_out<<<dim3(io_blocks(n), S.B), kT, 0, S.s>>>(S.phi.p, to, S.fixed.p, vals, masks, v, n,
                                                     n, S.fexp.p, S.lv[0].G.mnat);

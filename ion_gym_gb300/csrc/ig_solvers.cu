@@ -977,6 +977,31 @@ ig::CallInFlight::CallInFlight(CallKind kind)
 }
 ig::CallInFlight::~CallInFlight() { n_->fetch_sub(1); }
 
+bool ig::device_range(const void* p, size_t bytes, size_t align) {
+  cudaPointerAttributes a;
+  int dev = -1;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  if (a.type != cudaMemoryTypeDevice || a.device != dev || at % align) return false;
+  // the allocation's extent is the driver's to tell
+  using RangeFn = int (*)(unsigned long long*, size_t*, unsigned long long);
+  void* fn = nullptr;
+  cudaDriverEntryPointQueryResult found;
+  if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &fn, 3020, cudaEnableDefault,
+                                       &found) != cudaSuccess ||
+      found != cudaDriverEntryPointSuccess || !fn) {
+    cudaGetLastError();
+    return false;
+  }
+  unsigned long long base = 0;
+  size_t size = 0;
+  if (reinterpret_cast<RangeFn>(fn)(&base, &size, at) != 0) return false;
+  return at >= base && at - base <= size && bytes <= size - (at - base);
+}
+
 int ig::call_stream(cudaStream_t* s) {
   return guard([&] {
     *s = ctx().s;

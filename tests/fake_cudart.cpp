@@ -29,6 +29,9 @@ struct Config {
 };
 int device = 0, launched = 0, refuse = 0, loops = 0, loops_left = 1 << 30;
 size_t most_memory = size_t(-1);
+// an allocation of device 0 that is never touched
+constexpr uintptr_t kRange = 0x7000000000ULL;
+constexpr size_t kRangeSize = 4096;
 cudaError_t last = cudaSuccess;
 std::map<std::pair<int, const void*>, Attr> attrs;
 Config config;
@@ -165,8 +168,24 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t*, cudaGraph_t, unsigned long lo
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
-cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) {
+cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
   *a = cudaPointerAttributes();
+  const auto at = reinterpret_cast<uintptr_t>(p);
+  if (at >= kRange && at < kRange + kRangeSize) {
+    a->type = cudaMemoryTypeDevice;
+    a->device = 0;
+  }
+  return cudaSuccess;
+}
+int range_of(unsigned long long* base, size_t* size, unsigned long long) {
+  *base = kRange;
+  *size = kRangeSize;
+  return 0;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char*, void** fn, unsigned, unsigned long long,
+                                             cudaDriverEntryPointQueryResult* found) {
+  *fn = reinterpret_cast<void*>(range_of);
+  *found = cudaDriverEntryPointSuccess;
   return cudaSuccess;
 }
 }
@@ -245,7 +264,25 @@ static void routes() {
   solve("no-memory", 65, 100);
 }
 
+// offset and bytes of a result in the allocation: may a kernel write it?
+static void ranges() {
+  const struct {
+    const char* what;
+    size_t at, bytes, align;
+  } q[] = {{"range-whole", 0, 4096, 8},  {"range-inside", 24, 800, 8}, {"range-past", 8, 4096, 8},
+           {"range-odd", 4, 800, 8},     {"range-float", 4, 800, 4},   {"range-odd-float", 2, 8, 4},
+           {"range-host", 1u << 20, 8, 8}};
+  for (const auto& r : q)
+    std::printf("%s %d\n", r.what,
+                (int)device_range(reinterpret_cast<void*>(kRange + r.at), r.bytes, r.align));
+  device = 1;
+  std::printf("range-other-device %d\n",
+              (int)device_range(reinterpret_cast<void*>(kRange), 8, 8));
+  device = 0;
+}
+
 int main() {
+  ranges();
   say("sor-large", sor(129));
   say("sor-small", sor(40));
   int lowered = 0;

@@ -32,3 +32,24 @@ def test_device_out(shape, n_b, unit):
     got = out.cpu().numpy()
     assert got.dtype == host.dtype and got.tobytes() == host.tobytes()
     assert bool((room[:3] == -7).all()) and bool((room[-3:] == -7).all())
+
+
+@pytest.mark.parametrize("unit,shift", [(False, 4), (False, 1), (True, 2), (True, 1)])
+def test_device_out_at_any_address(unit, shift):
+    """A result at an address that its type is not aligned to is copied."""
+    import torch
+    from ion_gym_gb300.physics.mixed import MixedSession
+    shape = (17, 19, 21)
+    mask = np.zeros(shape, bool)
+    mask[5:8, 6:9, 7:11] = True
+    metal = mask.copy()
+    metal[0] = metal[-1] = True
+    n = int(np.prod(shape)) * (4 if unit else 8)
+    room = torch.full((n + 16,), 99, dtype=torch.uint8, device="cuda")
+    with MixedSession(metal, 1) as s:
+        solve = s.solve_unit_bases if unit else s.solve_bases
+        host = np.asarray(solve([mask], 1e4, 1e-9)).copy()
+        solve([mask], 1e4, 1e-9, out=room[shift:shift + n])
+    got = room.cpu().numpy()
+    assert got[shift:shift + n].tobytes() == host.tobytes()
+    assert (got[:shift] == 99).all() and (got[shift + n:] == 99).all()

@@ -1,7 +1,8 @@
 """The launchers that set kernel attributes, over a stand-in CUDA runtime
 (fake_cudart.cpp): a call's own size is never left behind for other threads'
 calls, every device gets its attributes, and a refused launch is reported as
-not launched, with no error left, so that the caller takes the other route."""
+not launched, with no error left, so that the caller takes the other route;
+and the caller's memory that a kernel may write."""
 import os
 import subprocess
 
@@ -70,3 +71,10 @@ def test_who_gets_the_resident_loop(said, what, want):
     """solve3d's loop holds every SM: alone, or among few or small solves, and
     nowhere else; what it cannot do the launched sweeps take up."""
     assert said[what] == "status=%d loops=%d launched=%d sweeps=%d" % want
+
+
+@pytest.mark.parametrize("what,direct", [
+    ("whole", 1), ("inside", 1), ("past", 0), ("odd", 0), ("float", 1), ("odd-float", 0),
+    ("host", 0), ("other-device", 0)])
+def test_results_a_kernel_may_write(said, what, direct):
+    assert said["range-" + what] == str(direct)
