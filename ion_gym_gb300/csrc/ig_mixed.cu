@@ -3068,11 +3068,15 @@ struct Session {
   // above the bottom (one is k_tail_cycle's), at most kMTailNodes nodes a
   // problem -- up to there the phases wait for their barriers and loads,
   // which a launch's few microseconds exceed; past it the launched kernels'
-  // 152 SMs win.  Eight 65^3 decks (levels 33^3 to 9^3): 4.52 -> 4.06 ms a
-  // solve; eight 193 x 193 x 385 bases 37.9 -> 37.5; 24 bases of a
-  // 256 x 64 x 48 board 12.1 -> 11.7.  Threads: 640 and 768 measure alike, 896 is slower (its
-  // barriers are).
-  static constexpr size_t kMTailNodes = 65536;
+  // 152 SMs win -- and the clusters of all problems resident at once, since a
+  // second wave of them doubles the time.  Launches against clusters, ms a
+  // solve: levels of 30625 nodes (8 ring stacks of 97 x 97 x 193) 6.68 / 6.48,
+  // of 35937 (decks of 65^3, 1, 2, 4 and 12 of them) 1.11 / 1.25, 1.28 / 1.34,
+  // 2.51 / 2.73, 4.20 / 4.37, of 54872 and 64000 (75^3 and 79^3 alone) 1.69 /
+  // 1.84, 1.65 / 1.87; in two waves, 18 bases of a 128 x 48 x 40 board 4.19 /
+  // 5.62, 16 decks of 65^3 4.99 / 6.79, 24 of 57^3 4.02 / 5.04.  Threads: 640
+  // and 768 measure alike, 896 is slower (its barriers are).
+  static constexpr size_t kMTailNodes = 32768;
   void update_tail_cluster() {
     tail_top = 0;
     tail_ctas = 0;
@@ -3081,18 +3085,44 @@ struct Session {
     while (top > 1 && lv[top - 1].d.n() <= kMTailNodes && lv.size() - (top - 1) <= kMTailLevels &&
            !flat(lv[top - 1]))
       top--;
-    if (top < 1 || top + 2 >= lv.size() || (int)top < tb_levels) return;
-    // CTAs: a group of slots a thread at most, as far as a cluster goes
-    const uint32_t groups = lv[top].G.csz / 4;
-    int n = 1;
-    while (n < kMTailCtas && (uint32_t)(n * kMTailThreads) < groups) n *= 2;
+    if (top < 1) return;
     if (cudaFuncSetAttribute(k_tail_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kTailSmemMax) != cudaSuccess) {
       cudaGetLastError();
       return;
     }
-    tail_top = top;
-    tail_ctas = n;
+    for (; top + 2 < lv.size(); top++) {
+      if ((int)top < tb_levels) continue;
+      // CTAs: a group of slots a thread at most, as far as a cluster goes
+      const uint32_t groups = lv[top].G.csz / 4;
+      int n = 1, resident = 0;
+      while (n < kMTailCtas && (uint32_t)(n * kMTailThreads) < groups) n *= 2;
+      cudaLaunchAttribute at[1];
+      const cudaLaunchConfig_t c = tail_cluster_config(n, bmax, at);
+      if (cudaOccupancyMaxActiveClusters(&resident, k_tail_cluster, &c) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+      }
+      if (resident < bmax) continue;
+      tail_top = top;
+      tail_ctas = n;
+      return;
+    }
+  }
+  // k_tail_cluster's launch for nb problems, n CTAs each
+  cudaLaunchConfig_t tail_cluster_config(int n, int nb, cudaLaunchAttribute* at) const {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)(nb * n));
+    c.blockDim = dim3(kMTailThreads);
+    c.dynamicSmemBytes = tail_smem_bytes(lv[lv.size() - 2].G, lv.back().G);
+    c.stream = s;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)n;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    return c;
   }
   bool tail_cluster(size_t l) const { return tail_top > 0 && l == tail_top && !use_tb(l); }
 
@@ -3109,18 +3139,8 @@ struct Session {
     A.pairs = bottom_pairs;
     A.zero = zero ? 1 : 0;
     A.omega_b = bottom_omega;
-    cudaLaunchConfig_t c{};
     cudaLaunchAttribute at[1];
-    c.gridDim = dim3((unsigned)(B * tail_ctas));
-    c.blockDim = dim3(kMTailThreads);
-    c.dynamicSmemBytes = tail_smem_bytes(lv[lv.size() - 2].G, lv.back().G);
-    c.stream = s;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)tail_ctas;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    c.attrs = at;
-    c.numAttrs = 1;
+    const cudaLaunchConfig_t c = tail_cluster_config(tail_ctas, B, at);
     MK(cudaLaunchKernelEx(&c, k_tail_cluster, A));
   }
 

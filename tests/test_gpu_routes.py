@@ -28,15 +28,20 @@ def _deck(shape, n):
     return masks, np.any(masks, 0)
 
 
-def test_the_cluster_takes_the_small_levels():
-    """64 x 80 x 72 has two levels between the finest and the bottom; with
-    cycles of 2 + 2 pairs each takes 9 launches a cycle (3 and 4 half-sweeps,
-    residual with restriction, prolongation), the bottom one."""
+@pytest.mark.parametrize("n_b,levels", [(3, 2), (24, 1)])
+def test_the_cluster_takes_the_small_levels(n_b, levels):
+    """60^3 has two levels between the finest and the bottom; with cycles of
+    2 + 2 pairs each takes 9 launches a cycle (3 and 4 half-sweeps, residual
+    with restriction, prolongation), the bottom one.  The clusters of three
+    problems take both levels; those of 24 are not resident at once (8 CTAs
+    each on 152 SMs), so that only the last level and the bottom are one launch
+    (k_tail_cycle)."""
     from ion_gym_gb300 import _lib
-    masks, metal = _deck((64, 80, 72), 3)
+    masks, metal = _deck((60, 60, 60), 3)
+    masks = (masks * 8)[:n_b]
     n, steps = {}, {}
     for tail in ("0", "1"):
-        with _session({"IG_MIXED_TAIL": tail, "IG_MIXED_TB_LEVELS": "0"}, metal, 3) as s:
+        with _session({"IG_MIXED_TAIL": tail, "IG_MIXED_TB_LEVELS": "0"}, metal, n_b) as s:
             s.set_cycle(2, 2, 3)
             s.solve_bases(masks, 1.0, 1e-9)
             before = _lib.lib().ig_mixed_launch_count()
@@ -44,7 +49,8 @@ def test_the_cluster_takes_the_small_levels():
             n[tail] = _lib.lib().ig_mixed_launch_count() - before
             steps[tail] = s.last_steps
     assert steps["0"] == steps["1"] > 0
-    assert n["0"] - n["1"] == steps["1"] * 3 * (2 * 9)
+    visits = 2 if n_b >= 4 else 1  # of the first coarse level (the batches' default)
+    assert n["0"] - n["1"] == steps["1"] * 3 * visits * levels * 9
 
 
 @pytest.mark.parametrize("shape,n_b", [((12, 20, 210), 1), ((18, 33, 197), 5), ((40, 31, 33), 2)])
