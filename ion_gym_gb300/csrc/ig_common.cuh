@@ -106,9 +106,9 @@ static __device__ __noinline__ double resid_slow(double S, double phi) {
 //
 // The 257^3 quadrupole's cascadic solve (omega 1.85): 278 ms with the
 // difference and the product alone on the integer pipe (6 FP64 instructions
-// a node), 250 ms now (5, the neighbour sum); both pipes are then about
-// equally busy (320 FP64 and some 340 integer issue cycles a node and
-// scheduler), so moving more of the sum over would not help.
+// a node), 250 ms now (5, the neighbour sum).  The FP64 pipe is then 72 %
+// busy and the integer pipe 60 % (counters of a 257^3 half-sweep), so an
+// addition of the sum moved over would cost there what it saves here.
 __device__ __forceinline__ unsigned long long sor_key(unsigned long long ad, int e) {
   // the IEEE bits of ad * 2^(e - 1075), 0 < ad < 2^54, where that is normal;
   // ~0 where it is not

@@ -566,8 +566,8 @@ k_residual_plan(const double* __restrict__ phi, const ThetaPlan P, FlatGeom g,
 // A grid of some 10^5 nodes is 1.4 us of FP64 work a half-sweep, and a
 // launch 7 us of latency around it (control block, mask, values, sum, block
 // maximum, each waiting for the one before; 43 us with theta's divisions on
-// the last block's chain).  Here one CTA per SM stays for the whole loop (a
-// cooperative launch, so that all of them are resident).  The node arithmetic
+// the last block's chain).  Here one CTA per SM stays for as many pairs as the
+// call's turn has (a cooperative launch, so that all of them are resident).  The node arithmetic
 // is the launched sweeps'.
 //
 // A grid barrier after each half-sweep would be four trips to L2 one after

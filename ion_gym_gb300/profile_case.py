@@ -6,6 +6,8 @@ timing: the arrays are built, a few launches run, the process exits.
 Cases:
   sweep_f64   FP64 red-black sweep (k_sweep<kPlain>) on the 257^3
               quadrupole, `pairs` red-black pairs, omega 1.85
+  sor         solve3d of a sphere in an n^3 box (k_sor_flow up to 129^3)
+  vmg         the FP64 V-cycle of the same (k_err_tail)
   mixed_rings the mixed-precision basis batch of the ring stack (8 bases)
   mixed_quad  the mixed-precision solve of the 257^3 quadrupole (one problem)
   mixed_board the mixed-precision bases of a 512x128x96 planar board
@@ -44,6 +46,17 @@ def sweep_f64(n, pairs):
     print(f"sweep_f64 n={n}: {pairs} pairs in {el * 1e3:.2f} ms "
           f"({n ** 3 * pairs / el / 1e9:.1f} GLUP/s incl. host syncs), "
           f"last max|d| {d.value:.3e}")
+
+
+def fp64_solve(case, n, solves):
+    from ion_gym_gb300.physics import multigrid3d, solver3d
+    from ion_gym_gb300.workloads import sphere_box
+    fixed, val = sphere_box(n, 0.15 * n)
+    solve = solver3d.solve3d if case == "sor" else multigrid3d.solve3d_vmg
+    for _ in range(solves):
+        t0 = time.perf_counter()
+        sweeps = solve(fixed, val, tol=1e-7)[1]
+        print(f"{case} n={n}: {time.perf_counter() - t0:.4f} s, {sweeps} sweeps")
 
 
 def mixed_rings(solves, gs_pairs):
@@ -128,14 +141,16 @@ def mixed_board(solves, n_el=24):
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["sweep_f64", "mixed_rings", "mixed_quad",
-                                     "mixed_board"])
+    ap.add_argument("case", choices=["sweep_f64", "sor", "vmg", "mixed_rings",
+                                     "mixed_quad", "mixed_board"])
     ap.add_argument("--n", type=int, default=257)
     ap.add_argument("--pairs", type=int, default=4)
     ap.add_argument("--solves", type=int, default=1)
     a = ap.parse_args()
     if a.case == "sweep_f64":
         sweep_f64(a.n, a.pairs)
+    elif a.case in ("sor", "vmg"):
+        fp64_solve(a.case, a.n, a.solves)
     elif a.case == "mixed_quad":
         mixed_quad(a.n, a.solves)
     elif a.case == "mixed_board":
