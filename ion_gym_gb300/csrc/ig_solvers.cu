@@ -986,7 +986,7 @@ bool ig::device_range(const void* p, size_t bytes, size_t align) {
   }
   const uintptr_t at = reinterpret_cast<uintptr_t>(p);
   if (a.type != cudaMemoryTypeDevice || a.device != dev || at % align) return false;
-  // the allocation's extent is the driver's to tell
+  // CUDA's own record of the allocation's extent
   using RangeFn = int (*)(unsigned long long*, size_t*, unsigned long long);
   void* fn = nullptr;
   cudaDriverEntryPointQueryResult found;
